@@ -106,6 +106,53 @@ int alloc_persist(tsg_handle* h, Persist64& p, bool soil) {
     return rc ? TSG_E_CUDA : 0;
 }
 
+// Neighbour-row pitch: the lattice points within 1.06 R (WCSPH and soil densities stay within a
+// few percent of the lattice's, 1.06^3 = 1.19) plus 8 for jitter and free-surface clumping;
+// boundary rows hold flow neighbours only, at most about half a sphere of them.
+int row_capacity(const Consts& c) {
+    const double rr = 1.06 * c.R / c.diam;
+    if (!(rr < 64.0)) return 0;
+    const int m = (int)std::ceil(rr);
+    int count = 0;
+    for (int a = -m; a <= m; ++a)
+        for (int b = -m; b <= m; ++b)
+            for (int d = (c.dim == 3 ? -m : 0); d <= (c.dim == 3 ? m : 0); ++d)
+                if (a * a + b * b + d * d < rr * rr) ++count;
+    return count + 8;
+}
+
+// Rows take at most half of the free device memory (2.3 M particles in 3D: 6.3 GB); a scene
+// that would need more, or whose allocation fails, walks the cells instead.
+int alloc_rows(tsg_handle* h) {
+    const Consts& c = h->c;
+    Pairs64& r = h->g.pr;
+    r = Pairs64{};
+    r.rec_stride = c.solver != 1 && c.dim == 3 ? 16 : 8;
+    if (int rc = dalloc(h, &r.rec, (size_t)r.rec_stride * h->n)) return rc;
+    const int cf = row_capacity(c);
+    const int cap_f = (cf + 7) / 8 * 8, cap_b = ((cf * 6) / 10 + 7) / 8 * 8;
+    const size_t sf = (size_t)c.n_flow * cap_f, sb = (size_t)c.n_bdy * cap_b;
+    const int planes = c.dim + (c.solver == 1 ? 1 : 0);
+    size_t free_b = 0, total_b = 0;
+    if (cf <= 0 || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
+    const size_t bytes = sf * (4 + 8 * (size_t)planes) + sb * 12 + 4 * (size_t)h->n;
+    if (bytes > free_b / 2) return 0;
+    auto take = [&](auto** p, size_t count) {
+        void* q = nullptr;
+        if (count && cudaMalloc(&q, count * sizeof(**p)) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (q) h->allocs.push_back(q);
+        *reinterpret_cast<void**>(p) = q;
+        return true;
+    };
+    r.slots_f = sf;
+    if (take(&r.cnt, (size_t)c.n_flow + c.n_bdy) && take(&r.nb_f, sf) && take(&r.nb_b, sb) &&
+        take(&r.gk, sf * c.dim) && take(&r.gw, sb) && (c.solver != 1 || take(&r.gden, sf))) {
+        r.cap_f = cap_f;
+        r.cap_b = cap_b;
+    }
+    return 0;
+}
+
 int alloc_all(tsg_handle* h) {
     const size_t n = h->n;
     const Consts& c = h->c;
@@ -136,6 +183,7 @@ int alloc_all(tsg_handle* h) {
     rc |= dalloc(h, &g.list_count, 2); rc |= dalloc(h, &g.err, 1);
     rc |= dalloc(h, &h->d_stage, 9 * n + 16);
     rc |= dalloc(h, &h->d_scratch, 64);
+    if (!rc) rc = alloc_rows(h);
     return rc ? TSG_E_CUDA : 0;
 }
 
@@ -176,6 +224,55 @@ void refresh_pos32_if_dirty(tsg_handle* h, cudaStream_t s) {
         fp64_refresh_pos32(h->c, h->cur, h->t, s);
         h->pos32_dirty = false;
     }
+}
+
+// FP64 form, a loop called on its own: rows (and the pair geometry) of the positions as they are
+// now, which a caller may have written since the last call through the field views.  The step
+// sequence builds them once per step instead.
+void own_rows(tsg_handle* h, bool geometry, cudaStream_t s) {
+    fp64_refresh_pos32(h->c, h->cur, h->t, s);
+    h->pos32_dirty = false;
+    fp64_build_rows(h->c, h->cur, h->t, h->g, s);
+    if (geometry) fp64_geometry(h->c, h->cur, h->t, h->g, s);
+}
+
+// substep of the FP64 form on the current rows and geometry.
+int substep64(tsg_handle* h, cudaStream_t s) {
+    auto rates = [&] { fp64_one_step(h->c, h->cur, h->t, h->g, s); };
+    auto adv = [&](int which) { fp64_advect(h->c, h->cur, h->t, h->g, which, s); };
+    switch (h->c.ti) {
+    case 1: rates(); adv(TSG_ADVECT_FULL); break;
+    case 2: rates(); adv(TSG_ADVECT_LF_HALF); rates(); adv(TSG_ADVECT_FULL); break;
+    case 4: {
+        adv(TSG_RK_INIT);
+        const int m[4] = {1, 2, 2, 1};
+        for (int k = 0; k < 4; ++k) {
+            rates();
+            fp64_rk_update(h->c, h->cur, h->t, m[k], s);
+            if (k < 3) adv(TSG_RK_STAGE);
+        }
+        adv(TSG_RK_FINAL);
+        break;
+    }
+    default: return TSG_E_CONFIG;
+    }
+    return check_cuda();
+}
+
+// One step of the FP64 form after its sort.
+int step64(tsg_handle* h, bool collide, cudaStream_t s) {
+    const Consts& c = h->c;
+    fp64_build_rows(c, h->cur, h->t, h->g, s);
+    fp64_kernel_corr(c, h->cur, h->t, h->g, s);
+    fp64_init_tmp(c, h->cur, h->t, s);
+    if (int rc = substep64(h, s)) return rc;
+    fp64_advect(c, h->cur, h->t, h->g, TSG_ADVECT_POS, s);
+    h->pos32_dirty = true;
+    fp64_advect(c, h->cur, h->t, h->g, TSG_ADVECT_SOMETHING, s);
+    if (c.n_rigid_dyn) fp64_solve_rigid(c, h->cur, h->rigid, s);
+    // enforce_boundary also clamps dynamic rigid particles in every boundary mode
+    if (collide || c.n_rigid_dyn) fp64_advect(c, h->cur, h->t, h->g, TSG_ENFORCE_BOUNDARY, s);
+    return check_cuda();
 }
 
 }  // namespace
@@ -268,6 +365,10 @@ int tsg_create(const tsg_config* cfg, tsg_handle** out) {
     c.pf_on = 1;
     c.pf_r2 = std::nextafter((float)(c.R * c.R * (1.0 + 1.0 / 1024.0)), 1e30f);
     c.pf_lim = (float)(500.0 * c.R);
+    c.pf_in2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 1024.0)), 0.f);
+    c.R2T = c.R * c.R;
+    while (std::sqrt(c.R2T) >= c.R) c.R2T = std::nextafter(c.R2T, 0.0);
+    while (std::sqrt(c.R2T) < c.R) c.R2T = std::nextafter(c.R2T, 1e300);
     *out = h;
     return 0;
 }
@@ -411,7 +512,7 @@ int tsg_kernel_corr(tsg_handle* h, void* stream) {
     if (!h || !h->sorted) return TSG_E_STATE;
     cudaStream_t s = S(stream);
     if (use_fp32(h)) fp32_kernel_corr(*h->f32, s);
-    else { refresh_pos32_if_dirty(h, s); fp64_kernel_corr(h->c, h->cur, h->t, h->g, s); }
+    else { own_rows(h, false, s); fp64_kernel_corr(h->c, h->cur, h->t, h->g, s); }
     return check_cuda();
 }
 
@@ -427,7 +528,7 @@ int tsg_one_step(tsg_handle* h, void* stream) {
     if (!h || !h->sorted) return TSG_E_STATE;
     cudaStream_t s = S(stream);
     if (use_fp32(h)) fp32_one_step(*h->f32, s);
-    else { refresh_pos32_if_dirty(h, s); fp64_one_step(h->c, h->cur, h->t, h->g, s); }
+    else { own_rows(h, true, s); fp64_one_step(h->c, h->cur, h->t, h->g, s); }
     return check_cuda();
 }
 
@@ -439,7 +540,7 @@ int tsg_advect(tsg_handle* h, int which, void* stream) {
     if (use_fp32(h)) {
         fp32_advect(*h->f32, which, s);
     } else {
-        if (which == TSG_ADVECT_POS) refresh_pos32_if_dirty(h, s);
+        if (which == TSG_ADVECT_POS && h->c.xsph) own_rows(h, false, s);
         fp64_advect(h->c, h->cur, h->t, h->g, which, s);
         if (which == TSG_ADVECT_POS || which == TSG_ENFORCE_BOUNDARY) h->pos32_dirty = true;
     }
@@ -460,6 +561,10 @@ int tsg_rk_update(tsg_handle* h, int32_t m, void* stream) {
 
 int tsg_substep(tsg_handle* h, void* stream) {
     if (!h || !h->sorted) return TSG_E_STATE;
+    if (!use_fp32(h)) {
+        own_rows(h, true, S(stream));
+        return substep64(h, S(stream));
+    }
     int rc = 0;
     switch (h->c.ti) {
     case 1:
@@ -506,14 +611,7 @@ int tsg_step(tsg_handle* h, int nsteps, void* stream) {
             if ((rc = check_cuda())) return rc;
             continue;
         }
-        if ((rc = tsg_kernel_corr(h, stream))) return rc;
-        if ((rc = tsg_init_tmp(h, stream))) return rc;
-        if ((rc = tsg_substep(h, stream))) return rc;
-        if ((rc = tsg_advect(h, TSG_ADVECT_POS, stream))) return rc;
-        if ((rc = tsg_advect(h, TSG_ADVECT_SOMETHING, stream))) return rc;
-        if (h->c.n_rigid_dyn && (rc = tsg_solve_rigid_body(h, stream))) return rc;
-        // enforce_boundary also clamps dynamic rigid particles in every boundary mode
-        if ((collide || h->c.n_rigid_dyn) && (rc = tsg_advect(h, TSG_ENFORCE_BOUNDARY, stream))) return rc;
+        if ((rc = step64(h, collide, S(stream)))) return rc;
     }
     return 0;
 }
@@ -603,7 +701,7 @@ int tsg_write(tsg_handle* h, const char* name, const void* src, int from_device,
     } else {
         upload_planes(h, static_cast<const double*>(src), static_cast<double*>(ptr), comps, from_device != 0, s);
     }
-    if (std::string(name) == "x") h->pos32_dirty = true;
+    if (std::string(name) == "x" || std::string(name) == "mat_type") h->pos32_dirty = true;
     return check_cuda();
 }
 

@@ -25,6 +25,7 @@
 #include <cfloat>
 
 #include "tsg_internal.h"
+#include "tsg_pairs64.cuh"
 #include "tsg_polar.cuh"
 #include "tsg_rigid_list.cuh"
 
@@ -164,55 +165,182 @@ __device__ __forceinline__ double det3(const double* a) {
     return a[0] * (a[4] * a[8] - a[7] * a[5]) - a[3] * (a[1] * a[8] - a[7] * a[2]) + a[6] * (a[1] * a[5] - a[4] * a[2]);
 }
 
+// Pair geometry of row slot `slot` (entry j): r, |r| and grad W into registers, grad W and the
+// viscosity denominator into the row's planes.
 template <int DIM>
-__global__ void k_corr(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ double pair_geometry(const Consts& c, const double* __restrict__ X, const double* xi, int j,
+                                                const Pairs64& pr, size_t slot, double* r, double* kd) {
+    const size_t n = c.n;
+    r[0] = xi[0] - X[j];
+    r[1] = xi[1] - X[n + j];
+    r[2] = DIM == 3 ? xi[2] - X[2 * n + j] : 0.0;
+    double r2 = r[0] * r[0] + r[1] * r[1];
+    if (DIM == 3) r2 = r2 + r[2] * r[2];
+    const double rn = sqrt(r2);
+    kernel_dW<DIM>(c, r, rn, kd);
+    for (int d = 0; d < DIM; ++d) pr.gk[d * pr.slots_f + slot] = kd[d];
+    if (pr.gden) pr.gden[slot] = rn * rn + c.eps_h2;
+    return rn;
+}
+
+// Kernel value of a boundary row's entry.
+template <int DIM>
+__device__ __forceinline__ double pair_W(const Consts& c, const double* __restrict__ X, const double* xi, int j) {
+    const size_t n = c.n;
+    const double rx = xi[0] - X[j], ry = xi[1] - X[n + j];
+    double r2 = rx * rx + ry * ry;
+    if (DIM == 3) { const double rz = xi[2] - X[2 * n + j]; r2 = r2 + rz * rz; }
+    return kernel_W(c, sqrt(r2));
+}
+
+// This thread's row in the row-sum phase: particle index and listed count (0 for a row past the
+// end or above the pitch, which the epilogue walks through the cells).
+struct RowRef { int row, i, cnt; size_t base; };
+template <int G>
+__device__ __forceinline__ RowRef row_ref(const int* __restrict__ list, int count, const int* __restrict__ cnt, int cap) {
+    RowRef q;
+    q.row = blockIdx.x * ROWS + threadIdx.x / G;
+    const bool live = q.row < count;
+    q.i = live ? list[q.row] : list[0];
+    q.cnt = live ? cnt[q.row] : 0;
+    if (q.cnt > cap) q.cnt = 0;
+    q.base = (size_t)q.row * cap;
+    return q;
+}
+
+// Flow rows: pair geometry, Shepard sum and CSPM matrix (eng/solver_sph_base.py:386-423).
+template <int DIM, int G, bool CORR>
+__global__ void __launch_bounds__(ROWS * G) k_corr_flow(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                                                        const int* __restrict__ list, int count, Pairs64 pr) {
+    constexpr int C = 1 + (CORR ? DIM * DIM : 0);
+    __shared__ double S[C][ROWS];
     const int n = c.n;
-    double xi[3];
-    load_x<DIM>(p.x, i, n, xi);
-    const int ti = p.mat_type[i];
-    const bool want_L = c.corr == 1 && is_flow(ti);
+    if (pr.cap_f) {
+        const RowRef q = row_ref<G>(list, count, pr.cnt, pr.cap_f);
+        double xi[3];
+        load_x<DIM>(p.x, q.i, n, xi);
+        block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
+            const int ent = pr.nb_f[q.base + s], j = nb_index(ent);
+            double r[3], kd[3];
+            const double rn = pair_geometry<DIM>(c, p.x, xi, j, pr, q.base + s, r, kd);
+            if (nb_flow(ent)) {
+                const double mVj = p.m_V[j];
+                T[0] = mVj * kernel_W(c, rn);
+                if (CORR)
+                    for (int a = 0; a < DIM; ++a) {
+                        const double av = mVj * (-r[a]);
+                        for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = av * kd[b];
+                    }
+            }
+        });
+    }
+    const int row = blockIdx.x * ROWS + threadIdx.x;
+    if (threadIdx.x >= ROWS || row >= count) return;
+    const int i = list[row];
     double s = 0.0;
     double L[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
-        const int tj = p.mat_type[j];
-        const double mVj = p.m_V[j];
-        if (is_flow(tj)) s += mVj * kernel_W(c, rn);
-        if (want_L && tj == ti) {
-            double k[3];
-            kernel_dW<DIM>(c, r, rn, k);
-            for (int a = 0; a < DIM; ++a) {
-                double av = mVj * (-r[a]);
-                for (int b = 0; b < DIM; ++b) L[3 * a + b] = L[3 * a + b] + av * k[b];
+    if (pr.cap_f && pr.cnt[row] <= pr.cap_f) {
+        s = S[0][threadIdx.x];
+        if (CORR)
+            for (int a = 0; a < DIM; ++a)
+                for (int b = 0; b < DIM; ++b) L[3 * a + b] = S[1 + a * DIM + b][threadIdx.x];
+    } else {
+        double xi[3];
+        load_x<DIM>(p.x, i, n, xi);
+        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
+            if (!is_flow(p.mat_type[j])) return;
+            const double mVj = p.m_V[j];
+            s += mVj * kernel_W(c, rn);
+            if (CORR) {
+                double k[3];
+                kernel_dW<DIM>(c, r, rn, k);
+                for (int a = 0; a < DIM; ++a) {
+                    double av = mVj * (-r[a]);
+                    for (int b = 0; b < DIM; ++b) L[3 * a + b] = L[3 * a + b] + av * k[b];
+                }
             }
-        }
-    });
+        });
+    }
     t.CSPM_f[i] = s != 0.0 ? 1.0 / s : 1.0;
-    if (c.corr == 1) {
+    if (CORR) {
         double inv[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-        if (want_L) {
-            if (DIM == 2) {
-                double dt = det2(L);
-                if (fabs(dt) > EPS) {
-                    double id = 1.0 / dt;
-                    inv[0] = id * L[4]; inv[1] = id * (-L[1]); inv[2] = 0.0;
-                    inv[3] = id * (-L[3]); inv[4] = id * L[0]; inv[5] = 0.0;
-                    inv[6] = 0.0; inv[7] = 0.0; inv[8] = 0.0;
-                }
-            } else {
-                double dt = det3(L);
-                if (fabs(dt) > EPS) {
-                    double id = 1.0 / dt;
-                    for (int a = 0; a < 3; ++a)
-                        for (int b = 0; b < 3; ++b)
-                            inv[3 * b + a] = id * (L[3 * ((a + 1) % 3) + (b + 1) % 3] * L[3 * ((a + 2) % 3) + (b + 2) % 3]
-                                                 - L[3 * ((a + 2) % 3) + (b + 1) % 3] * L[3 * ((a + 1) % 3) + (b + 2) % 3]);
-                }
+        if (DIM == 2) {
+            double dt = det2(L);
+            if (fabs(dt) > EPS) {
+                double id = 1.0 / dt;
+                inv[0] = id * L[4]; inv[1] = id * (-L[1]); inv[2] = 0.0;
+                inv[3] = id * (-L[3]); inv[4] = id * L[0]; inv[5] = 0.0;
+                inv[6] = 0.0; inv[7] = 0.0; inv[8] = 0.0;
+            }
+        } else {
+            double dt = det3(L);
+            if (fabs(dt) > EPS) {
+                double id = 1.0 / dt;
+                for (int a = 0; a < 3; ++a)
+                    for (int b = 0; b < 3; ++b)
+                        inv[3 * b + a] = id * (L[3 * ((a + 1) % 3) + (b + 1) % 3] * L[3 * ((a + 2) % 3) + (b + 2) % 3]
+                                             - L[3 * ((a + 2) % 3) + (b + 1) % 3] * L[3 * ((a + 1) % 3) + (b + 2) % 3]);
             }
         }
         for (int q = 0; q < 9; ++q) t.CSPM_L[(size_t)q * n + i] = inv[q];
     }
+}
+
+// Boundary and rigid rows: kernel values and Shepard sum over the flow neighbours.
+template <int DIM, int G>
+__global__ void __launch_bounds__(ROWS * G) k_corr_bdy(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                                                       const int* __restrict__ list, int count, Pairs64 pr) {
+    __shared__ double S[1][ROWS];
+    const int n = c.n;
+    const int* cnt = pr.cnt + c.n_flow;
+    if (pr.cap_f) {
+        const RowRef q = row_ref<G>(list, count, cnt, pr.cap_b);
+        double xi[3];
+        load_x<DIM>(p.x, q.i, n, xi);
+        block_row_sums<1, G>(q.cnt, S, [&](int s, double* T) {
+            const int j = pr.nb_b[q.base + s];
+            const double w = pair_W<DIM>(c, p.x, xi, j);
+            pr.gw[q.base + s] = w;
+            T[0] = p.m_V[j] * w;
+        });
+    }
+    const int row = blockIdx.x * ROWS + threadIdx.x;
+    if (threadIdx.x >= ROWS || row >= count) return;
+    const int i = list[row];
+    double s = 0.0;
+    if (pr.cap_f && cnt[row] <= pr.cap_b) {
+        s = S[0][threadIdx.x];
+    } else {
+        double xi[3];
+        load_x<DIM>(p.x, i, n, xi);
+        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double*, double rn) {
+            if (is_flow(p.mat_type[j])) s += p.m_V[j] * kernel_W(c, rn);
+        });
+    }
+    t.CSPM_f[i] = s != 0.0 ? 1.0 / s : 1.0;
+    if (c.corr == 1)
+        for (int q = 0; q < 9; ++q) t.CSPM_L[(size_t)q * n + i] = q % 4 == 0 ? 1.0 : 0.0;
+}
+
+// The pair geometry alone, for one_step called without the step sequence around it.
+template <int DIM, int G>
+__global__ void __launch_bounds__(ROWS * G) k_geom_flow(Consts c, Persist64 p, const int* __restrict__ list, int count,
+                                                        Pairs64 pr) {
+    const RowRef q = row_ref<G>(list, count, pr.cnt, pr.cap_f);
+    double xi[3], r[3], kd[3];
+    load_x<DIM>(p.x, q.i, c.n, xi);
+    for (int s = threadIdx.x % G; s < q.cnt; s += G)
+        pair_geometry<DIM>(c, p.x, xi, nb_index(pr.nb_f[q.base + s]), pr, q.base + s, r, kd);
+}
+
+template <int DIM, int G>
+__global__ void __launch_bounds__(ROWS * G) k_geom_bdy(Consts c, Persist64 p, const int* __restrict__ list, int count,
+                                                       Pairs64 pr) {
+    const RowRef q = row_ref<G>(list, count, pr.cnt + c.n_flow, pr.cap_b);
+    double xi[3];
+    load_x<DIM>(p.x, q.i, c.n, xi);
+    for (int s = threadIdx.x % G; s < q.cnt; s += G)
+        pr.gw[q.base + s] = pair_W<DIM>(c, p.x, xi, pr.nb_b[q.base + s]);
 }
 
 // Density summation: calc_density_task summed over for_all_neighbors
@@ -296,79 +424,152 @@ __device__ __forceinline__ double powi(double x, long n) {
     return r;
 }
 
+// What the rates loop reads of a neighbour, one aligned record per particle (the expressions
+// of the pair terms that depend on the neighbour alone, rounded as they are there):
+//   WCSPH  v~ (3), p / (rho~ rho~), m_V, viscosity factor, -rho0 m_V, 0
+//   soil   2D: v~ (2), m_V, m_V rho~, stress~ / (rho~ rho~) (xx, xy, yx, yy)
+//          3D: v~ (3), m_V, m_V rho~, the nine stress entries, 0, 0
+// The viscosity factor is visc_fac m_V for a fluid neighbour and (visc_fac m_V) rho0 for the
+// others (eng/solver_sph_wc.py:47-62).
+__device__ __forceinline__ void wc_record(const Consts& c, double* rec, int i, const double* vt, double pr, double rt,
+                                          double mV, bool fluid) {
+    double2* o = reinterpret_cast<double2*>(rec + (size_t)8 * i);
+    const double vf = c.visc_fac * mV;
+    o[0] = make_double2(vt[0], vt[1]);
+    o[1] = make_double2(vt[2], pr / (rt * rt));
+    o[2] = make_double2(mV, fluid ? vf : vf * c.rho0);
+    o[3] = make_double2(-c.rho0 * mV, 0.0);
+}
+__device__ __forceinline__ void soil_record(const Consts& c, double* rec, int i, const double* vt, const double* st,
+                                            double rt, double mV) {
+    const double r2 = rt * rt;
+    if (c.dim == 2) {
+        double2* o = reinterpret_cast<double2*>(rec + (size_t)8 * i);
+        o[0] = make_double2(vt[0], vt[1]);
+        o[1] = make_double2(mV, mV * rt);
+        o[2] = make_double2(st[0] / r2, st[1] / r2);
+        o[3] = make_double2(st[3] / r2, st[4] / r2);
+    } else {
+        double2* o = reinterpret_cast<double2*>(rec + (size_t)16 * i);
+        o[0] = make_double2(vt[0], vt[1]);
+        o[1] = make_double2(vt[2], mV);
+        o[2] = make_double2(mV * rt, st[0] / r2);
+        for (int q = 0; q < 4; ++q) o[3 + q] = make_double2(st[1 + 2 * q] / r2, st[2 + 2 * q] / r2);
+        o[7] = make_double2(0.0, 0.0);
+    }
+}
+
 // First, per-particle phase of one_step.
-__global__ void k_pre(Consts c, Persist64 p, Trans64 t, const int* __restrict__ list, int count) {
+__global__ void k_pre(Consts c, Persist64 p, Trans64 t, const int* __restrict__ list, int count, Pairs64 pr) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const int i = list[k];
     const int n = c.n;
+    const double rt = t.density_tmp[i], mV = p.m_V[i];
+    double vt[3];
+    for (int d = 0; d < 3; ++d) vt[d] = t.v_tmp[(size_t)d * n + i];
     if (c.solver == 1) {
-        double ratio = t.density_tmp[i] / c.rho0;
+        double ratio = rt / c.rho0;
         double pw = c.exponent_is_int ? powi(ratio, (long)c.gamma) : pow(ratio, c.gamma);
-        p.pressure[i] = fmax(c.B * (pw - 1.0), 0.0);
+        const double pres = fmax(c.B * (pw - 1.0), 0.0);
+        p.pressure[i] = pres;
+        wc_record(c, pr.rec, i, vt, pres, rt, mV, p.mat_type[i] == MAT_FLUID);
     } else if (c.solver == 3) {
         double st[9];
         for (int q = 0; q < 9; ++q) st[q] = t.stress_tmp[(size_t)q * n + i];
         dp_adapt(c, st);
         for (int q = 0; q < 9; ++q) t.stress_tmp[(size_t)q * n + i] = st[q];
+        soil_record(c, pr.rec, i, vt, st, rt, mV);
     }
 }
 
-// Dummy-boundary extrapolation (Adami 2012 style), one traversal for every sum.
-template <int DIM>
-__global__ void k_bdy(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
-                      const int* __restrict__ list, int count) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int i = list[k];
+// One flow neighbour's terms of the dummy extrapolation: v (DIM), then p (WCSPH) or density (1)
+// and stress (9).  w = W(r), r = x_i - x_j.
+template <int DIM, bool SOIL>
+__device__ __forceinline__ void bdy_terms(const Consts& c, const Persist64& p, const Trans64& t, int j,
+                                          const double* r, double w, double* T) {
+    const size_t n = c.n;
+    const double mVj = p.m_V[j], rtj = t.density_tmp[j];
+    for (int d = 0; d < DIM; ++d) T[d] = mVj * t.v_tmp[d * n + j] * w;
+    if (!SOIL) {
+        T[DIM] = mVj * (p.pressure[j] + rtj * c.g[1] * r[1]) * w;
+    } else {
+        T[DIM] = c.solver == 2 ? mVj * rtj * w : 0.0;
+        for (int a = 0; a < 3; ++a)
+            for (int b = 0; b < 3; ++b) {
+                double m = t.stress_tmp[(size_t)(3 * a + b) * n + j];
+                if (a == b) m = m + (rtj * c.g[a]) * r[a];
+                else m = m + (rtj * 0.0) * 0.0;
+                T[DIM + 1 + 3 * a + b] = mVj * m * w;
+            }
+    }
+}
+
+// Dummy-boundary extrapolation (Adami 2012 style), one walk of the row for every sum.
+template <int DIM, int G, bool SOIL>
+__global__ void __launch_bounds__(ROWS * G) k_bdy(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                                                  const int* __restrict__ list, int count, Pairs64 pr) {
+    constexpr int C = DIM + 1 + (SOIL ? 9 : 0);
+    __shared__ double S[C][ROWS];
     const int n = c.n;
+    const int* cnt = pr.cnt + c.n_flow;
+    if (pr.cap_f) {
+        const RowRef q = row_ref<G>(list, count, cnt, pr.cap_b);
+        double xi[3];
+        load_x<DIM>(p.x, q.i, n, xi);
+        block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
+            const int j = pr.nb_b[q.base + s];
+            double r[3] = {0.0, 0.0, 0.0};
+            for (int d = 0; d < DIM; ++d) r[d] = xi[d] - p.x[(size_t)d * n + j];
+            bdy_terms<DIM, SOIL>(c, p, t, j, r, pr.gw[q.base + s], T);
+        });
+    }
+    const int row = blockIdx.x * ROWS + threadIdx.x;
+    if (threadIdx.x >= ROWS || row >= count) return;
+    const int i = list[row];
+    double B[C];
+    if (pr.cap_f && cnt[row] <= pr.cap_b) {
+        for (int q = 0; q < C; ++q) B[q] = S[q][threadIdx.x];
+    } else {
+        double xi[3];
+        load_x<DIM>(p.x, i, n, xi);
+        for (int q = 0; q < C; ++q) B[q] = 0.0;
+        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
+            if (!is_flow(p.mat_type[j])) return;
+            double T[C];
+            bdy_terms<DIM, SOIL>(c, p, t, j, r, kernel_W(c, rn), T);
+            for (int q = 0; q < C; ++q) B[q] += T[q];
+        });
+    }
     const int ti = p.mat_type[i];
-    double xi[3];
-    load_x<DIM>(p.x, i, n, xi);
-    double bv[3] = {0, 0, 0};
-    double bp = 0.0, bd = 0.0;
-    double bs[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const bool soil = c.solver != 1;
-    for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
-        if (!is_flow(p.mat_type[j])) return;
-        const double w = kernel_W(c, rn);
-        const double mVj = p.m_V[j];
-        for (int d = 0; d < DIM; ++d) bv[d] += mVj * t.v_tmp[(size_t)d * n + j] * w;
-        const double rtj = t.density_tmp[j];
-        if (!soil) {
-            bp += mVj * (p.pressure[j] + rtj * c.g[1] * (xi[1] - p.x[(size_t)n + j])) * w;
-        } else {
-            if (c.solver == 2) bd += mVj * rtj * w;
-            for (int a = 0; a < 3; ++a)
-                for (int b = 0; b < 3; ++b) {
-                    double m = t.stress_tmp[(size_t)(3 * a + b) * n + j];
-                    if (a == b) m = m + (rtj * c.g[a]) * r[a];
-                    else m = m + (rtj * 0.0) * 0.0;
-                    bs[3 * a + b] += mVj * m * w;
-                }
-        }
-    });
     const double f = t.CSPM_f[i];
-    for (int d = 0; d < DIM; ++d) t.v_tmp[(size_t)d * n + i] = 2 * p.v[(size_t)d * n + i] - bv[d] * f;
-    if (DIM == 2) t.v_tmp[2 * (size_t)n + i] = 2 * p.v[2 * (size_t)n + i] - 0.0 * f;
-    if (!soil) {
-        t.density_tmp[i] = c.rho0;
-        p.pressure[i] = fmax(bp * f, 0.0);
-    } else {
-        t.density_tmp[i] = c.solver == 2 ? fmax(bd * f, c.rho0) : c.rho0;
-        for (int q = 0; q < 9; ++q) t.stress_tmp[(size_t)q * n + i] = bs[q] * f;
+    double vt[3], rt;
+    for (int d = 0; d < 3; ++d) {
+        vt[d] = 2 * p.v[(size_t)d * n + i] - (d < DIM ? B[d < DIM ? d : 0] : 0.0) * f;
+        t.v_tmp[(size_t)d * n + i] = vt[d];
     }
-    if (ti == MAT_RIGID) {  // static rigid: rates stay zero; dynamic rigid: gravity, then the reaction
-        t.d_density[i] = 0.0;
-        const bool dyn = p.is_dynamic[i] != 0;
-        for (int d = 0; d < 3; ++d) t.d_vel[(size_t)d * n + i] = dyn ? c.g[d] : 0.0;
+    if (!SOIL) {
+        rt = c.rho0;
+        const double pres = fmax(B[DIM] * f, 0.0);
+        p.pressure[i] = pres;
+        wc_record(c, pr.rec, i, vt, pres, rt, p.m_V[i], false);
     } else {
-        // dummy / repulsive particles have no rates: zero, as in the reference, where each
-        // particle's never-written rates travel with it through the sort (the rate arrays
-        // here are not reordered, so a slot may hold another particle's)
-        t.d_density[i] = 0.0;
-        for (int d = 0; d < 3; ++d) t.d_vel[(size_t)d * n + i] = 0.0;
+        rt = c.solver == 2 ? fmax(B[DIM] * f, c.rho0) : c.rho0;
+        double st[9];
+        for (int q = 0; q < 9; ++q) {
+            st[q] = B[(SOIL ? DIM + 1 : 0) + (SOIL ? q : 0)] * f;
+            t.stress_tmp[(size_t)q * n + i] = st[q];
+        }
+        soil_record(c, pr.rec, i, vt, st, rt, p.m_V[i]);
     }
+    t.density_tmp[i] = rt;
+    // static rigid: rates stay zero; dynamic rigid: gravity, then the reaction.  Dummy and
+    // repulsive particles have no rates: zero, as in the reference, where each particle's
+    // never-written rates travel with it through the sort (the rate arrays here are not
+    // reordered, so a slot may hold another particle's)
+    t.d_density[i] = 0.0;
+    const bool dyn = ti == MAT_RIGID && p.is_dynamic[i] != 0;
+    for (int d = 0; d < 3; ++d) t.d_vel[(size_t)d * n + i] = dyn ? c.g[d] : 0.0;
 }
 
 // ---- repulsive particles (eng/solver_sph_base.py:675-689) ----
@@ -406,54 +607,92 @@ __device__ __forceinline__ void wc_force_pair(const Consts& c, int tj, double mV
     }
 }
 
-// ---- WCSPH rates (eng/solver_sph_wc.py:108-126) ----
+// One neighbour's WCSPH terms: continuity, then the acceleration (DIM), from the neighbour's
+// record (v~, P = p / rho~^2, m_V, viscosity factor, -rho0 m_V) and the pair geometry.
 template <int DIM>
-__global__ void k_wc_rates(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
-                           const int* __restrict__ list, int count) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int i = list[k];
+__device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const double* v, double P, double mV, double cvj,
+                                         double cC, const double* vti, double rti, double pri, const double* L,
+                                         const double* r, double den, const double* kd, double* T) {
+    double dvv[3], a[3];
+    for (int d = 0; d < DIM; ++d) { dvv[d] = vti[d] - v[d]; a[d] = mV * dvv[d]; }
+    if (c.corr == 1) {
+        double kc[3];
+        matvec_corr<DIM>(L, kd, kc);
+        T[0] = dotv<DIM>(a, kc);
+    } else {
+        T[0] = dotv<DIM>(a, kd);
+    }
+    const double mn = fmin(dotv<DIM>(dvv, r), 0.0);
+    double cv = cvj;
+    if (!fluid) cv = cv / rti;
+    cv = cv * mn / den;
+    const double cp = cC * (pri + P);
+    for (int d = 0; d < DIM; ++d) T[1 + d] = cv * kd[d] + cp * kd[d];
+}
+
+// ---- WCSPH rates (eng/solver_sph_wc.py:108-126) ----
+template <int DIM, int G>
+__global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                                                       const int* __restrict__ list, int count, Pairs64 pr) {
+    constexpr int C = 1 + DIM;
+    __shared__ double S[C][ROWS];
     const int n = c.n;
-    double xi[3], vti[3];
-    load_x<DIM>(p.x, i, n, xi);
-    for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + i];
-    const double rti = t.density_tmp[i];
-    const double pti = p.pressure[i];
-    const double pri = pti / (rti * rti);
-    double L[9];
-    if (c.corr == 1)
-        for (int q = 0; q < 9; ++q) L[q] = t.CSPM_L[(size_t)q * n + i];
-    double dd = 0.0;
-    double dv[3] = {0, 0, 0};
-    const bool rep = c.boundary == 3 || c.boundary == 4;
-    for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
-        const int tj = p.mat_type[j];
-        const double mVj = p.m_V[j];
-        double vtj[3], dvv[3];
-        for (int d = 0; d < DIM; ++d) { vtj[d] = t.v_tmp[(size_t)d * n + j]; dvv[d] = vti[d] - vtj[d]; }
-        double kd[3];
-        kernel_dW<DIM>(c, r, rn, kd);
-        // continuity: m_Vj (v_i - v_j) . grad~W
-        double a[3];
-        for (int d = 0; d < DIM; ++d) a[d] = mVj * dvv[d];
-        if (c.corr == 1) {
-            double kc[3];
-            matvec_corr<DIM>(L, kd, kc);
-            dd += dotv<DIM>(a, kc);
-        } else {
-            dd += dotv<DIM>(a, kd);
-        }
-        double f[3];
-        wc_force_pair<DIM>(c, tj, mVj, dvv, rti, pri, p.pressure[j], t.density_tmp[j], r, rn, kd, f);
-        for (int d = 0; d < DIM; ++d) dv[d] += f[d];
-    });
-    if (rep) {  // separate traversal: the reference adds these after the whole dv sum
-        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
-            if (p.mat_type[j] == MAT_REP) rep_force<DIM>(c, r, rn, dv);
+    if (pr.cap_f) {
+        const RowRef q = row_ref<G>(list, count, pr.cnt, pr.cap_f);
+        double xi[3], vti[3], L[9];
+        load_x<DIM>(p.x, q.i, n, xi);
+        for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + q.i];
+        const double rti = t.density_tmp[q.i], pri = pr.rec[(size_t)8 * q.i + 3];
+        if (c.corr == 1)
+            for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
+        block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
+            const size_t slot = q.base + s;
+            const int ent = pr.nb_f[slot], j = nb_index(ent);
+            const double2* rj = reinterpret_cast<const double2*>(pr.rec + (size_t)8 * j);
+            const double2 r0 = rj[0], r1 = rj[1], r2 = rj[2], r3 = rj[3];
+            double r[3] = {0.0, 0.0, 0.0}, kd[3] = {0.0, 0.0, 0.0};
+            for (int d = 0; d < DIM; ++d) {
+                r[d] = xi[d] - p.x[(size_t)d * n + j];
+                kd[d] = pr.gk[d * pr.slots_f + slot];
+            }
+            const double v[3] = {r0.x, r0.y, r1.x};
+            wc_terms<DIM>(c, nb_flow(ent), v, r1.y, r2.x, r2.y, r3.x, vti, rti, pri, L, r, pr.gden[slot], kd, T);
         });
     }
-    t.d_density[i] = dd * rti;
-    for (int d = 0; d < DIM; ++d) t.d_vel[(size_t)d * n + i] = dv[d] + c.g[d];
+    const int row = blockIdx.x * ROWS + threadIdx.x;
+    if (threadIdx.x >= ROWS || row >= count) return;
+    const int i = list[row];
+    const double rti = t.density_tmp[i];
+    double A[C];
+    const bool listed = pr.cap_f && pr.cnt[row] <= pr.cap_f;
+    const bool rep = c.boundary == 3 || c.boundary == 4;
+    double xi[3];
+    load_x<DIM>(p.x, i, n, xi);
+    if (listed) {
+        for (int q = 0; q < C; ++q) A[q] = S[q][threadIdx.x];
+    } else {
+        double vti[3], L[9];
+        for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + i];
+        const double pri = pr.rec[(size_t)8 * i + 3];
+        if (c.corr == 1)
+            for (int q = 0; q < 9; ++q) L[q] = t.CSPM_L[(size_t)q * n + i];
+        for (int q = 0; q < C; ++q) A[q] = 0.0;
+        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
+            const double* rj = pr.rec + (size_t)8 * j;
+            double kd[3], T[C];
+            kernel_dW<DIM>(c, r, rn, kd);
+            wc_terms<DIM>(c, p.mat_type[j] == MAT_FLUID, rj, rj[3], rj[4], rj[5], rj[6], vti, rti, pri, L, r,
+                          rn * rn + c.eps_h2, kd, T);
+            for (int q = 0; q < C; ++q) A[q] += T[q];
+        });
+    }
+    if (rep) {  // a separate walk: the reference adds these after the whole acceleration sum
+        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
+            if (p.mat_type[j] == MAT_REP) rep_force<DIM>(c, r, rn, A + 1);
+        });
+    }
+    t.d_density[i] = A[0] * rti;
+    for (int d = 0; d < DIM; ++d) t.d_vel[(size_t)d * n + i] = A[1 + d] + c.g[d];
     if (DIM == 2) t.d_vel[2 * (size_t)n + i] = 0.0 + c.g[2];
 }
 
@@ -463,54 +702,96 @@ __device__ __forceinline__ void damping_acc(const Consts& c, double rti, const d
     for (int d = 0; d < dim; ++d) out[d] = s * vti[d];
 }
 
+// One neighbour's velocity-gradient terms (DIM x DIM) and continuity term (last): the
+// continuity product m_V (v_i - v_j) is the exact negation of the gradient's, so its dot
+// product is the negated trace.
+template <int DIM>
+__device__ __forceinline__ void vgrad_terms(const double* v, double mV, const double* vti, const double* kc, double* T) {
+    for (int a = 0; a < DIM; ++a) {
+        const double av = mV * (v[a] - vti[a]);
+        for (int b = 0; b < DIM; ++b) T[a * DIM + b] = av * kc[b];
+    }
+    double s = T[0] + T[DIM + 1];
+    if (DIM == 3) s = s + T[8];
+    T[DIM * DIM] = -s;
+}
+
+template <int DIM>
+__device__ __forceinline__ void corrected(const Consts& c, const double* L, const double* kd, double* kc) {
+    if (c.corr == 1) matvec_corr<DIM>(L, kd, kc);
+    else { kc[0] = kd[0]; kc[1] = kd[1]; kc[2] = kd[2]; }
+}
+
 // mu(I) loop 1 (eng/solver_sph_muI.py:67-92): velocity gradient, continuity, pressure from
 // density (not density_tmp), mu(I) stress, equivalent strain rate.
-template <int DIM>
-__global__ void k_mui_stress(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
-                             const int* __restrict__ list, int count) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int i = list[k];
+template <int DIM, int G>
+__global__ void __launch_bounds__(ROWS * G) k_mui_stress(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                                                         const int* __restrict__ list, int count, Pairs64 pr) {
+    constexpr int C = DIM * DIM + 1;
+    __shared__ double S[C][ROWS];
     const int n = c.n;
-    double xi[3], vti[3];
-    load_x<DIM>(p.x, i, n, xi);
+    if (pr.cap_f) {
+        const RowRef q = row_ref<G>(list, count, pr.cnt, pr.cap_f);
+        double vti[3], L[9];
+        for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + q.i];
+        if (c.corr == 1)
+            for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
+        block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
+            const size_t slot = q.base + s;
+            const int j = nb_index(pr.nb_f[slot]);
+            double kd[3] = {0.0, 0.0, 0.0}, kc[3], v[3];
+            for (int d = 0; d < DIM; ++d) {
+                kd[d] = pr.gk[d * pr.slots_f + slot];
+                v[d] = t.v_tmp[(size_t)d * n + j];
+            }
+            corrected<DIM>(c, L, kd, kc);
+            vgrad_terms<DIM>(v, p.m_V[j], vti, kc, T);
+        });
+    }
+    const int row = blockIdx.x * ROWS + threadIdx.x;
+    if (threadIdx.x >= ROWS || row >= count) return;
+    const int i = list[row];
+    double A[C], vti[3];
     for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + i];
-    double L[9];
-    if (c.corr == 1)
-        for (int q = 0; q < 9; ++q) L[q] = t.CSPM_L[(size_t)q * n + i];
+    if (pr.cap_f && pr.cnt[row] <= pr.cap_f) {
+        for (int q = 0; q < C; ++q) A[q] = S[q][threadIdx.x];
+    } else {
+        double xi[3], L[9];
+        load_x<DIM>(p.x, i, n, xi);
+        if (c.corr == 1)
+            for (int q = 0; q < 9; ++q) L[q] = t.CSPM_L[(size_t)q * n + i];
+        for (int q = 0; q < C; ++q) A[q] = 0.0;
+        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
+            double kd[3], kc[3], v[3], T[C];
+            kernel_dW<DIM>(c, r, rn, kd);
+            corrected<DIM>(c, L, kd, kc);
+            for (int d = 0; d < DIM; ++d) v[d] = t.v_tmp[(size_t)d * n + j];
+            vgrad_terms<DIM>(v, p.m_V[j], vti, kc, T);
+            for (int q = 0; q < C; ++q) A[q] += T[q];
+        });
+    }
     double vg[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    double dd = 0.0;
-    for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
-        const double mVj = p.m_V[j];
-        double kd[3], kc[3];
-        kernel_dW<DIM>(c, r, rn, kd);
-        if (c.corr == 1) matvec_corr<DIM>(L, kd, kc);
-        else { kc[0] = kd[0]; kc[1] = kd[1]; kc[2] = kd[2]; }
-        double vtj[3];
-        for (int d = 0; d < DIM; ++d) vtj[d] = t.v_tmp[(size_t)d * n + j];
-        for (int a = 0; a < DIM; ++a) {
-            double av = mVj * (vtj[a] - vti[a]);
-            for (int b = 0; b < DIM; ++b) vg[3 * a + b] += av * kc[b];
-        }
-        double aa[3];
-        for (int d = 0; d < DIM; ++d) aa[d] = mVj * (vti[d] - vtj[d]);
-        dd += dotv<DIM>(aa, kc);
-    });
+    for (int a = 0; a < DIM; ++a)
+        for (int b = 0; b < DIM; ++b) vg[3 * a + b] = A[a * DIM + b];
     const double rti = t.density_tmp[i];
     for (int q = 0; q < 9; ++q) t.v_grad[(size_t)q * n + i] = vg[q];
-    t.d_density[i] = dd * rti;
-    const double pr = fmax(c.vsound2 * (p.density[i] - c.rho0), 0.0);
-    p.pressure[i] = pr;
-    double er[9];
+    t.d_density[i] = A[DIM * DIM] * rti;
+    const double pr_i = fmax(c.vsound2 * (p.density[i] - c.rho0), 0.0);
+    p.pressure[i] = pr_i;
+    double er[9], st[9];
     for (int a = 0; a < 3; ++a)
         for (int b = 0; b < 3; ++b) er[3 * a + b] = 0.5 * (vg[3 * a + b] + vg[3 * b + a]);
     const double dbdot = sqrt(0.5 * msum_sq(er)) + EPS;
-    const double sc = 0.0 + (c.coh + pr * c.mu) / dbdot;
-    for (int q = 0; q < 9; ++q) t.stress_tmp[(size_t)q * n + i] = sc * er[q] - pr * ((q % 4 == 0) ? 1.0 : 0.0);
+    const double sc = 0.0 + (c.coh + pr_i * c.mu) / dbdot;
+    for (int q = 0; q < 9; ++q) {
+        st[q] = sc * er[q] - pr_i * ((q % 4 == 0) ? 1.0 : 0.0);
+        t.stress_tmp[(size_t)q * n + i] = st[q];
+    }
     const double t3 = mtrace(er) / 3.0;
     double ed[9];
     for (int q = 0; q < 9; ++q) ed[q] = er[q] - t3 * ((q % 4 == 0) ? 1.0 : 0.0);
     t.d_strain_equ[i] = sqrt(msum_sq(ed) * 2 / 3);
+    soil_record(c, pr.rec, i, vti, st, rti, p.m_V[i]);
 }
 
 // Stress-divergence sum (eng/solver_sph_muI.py:39-46), shared by mu(I) and DP.
@@ -529,90 +810,136 @@ __device__ __forceinline__ void stress_div_val(const double* sti, double ri2, co
         out[a] = s;
     }
 }
+// The same sum from the neighbour's record: S_j = stress_j / rho~_j^2 (DIM x DIM), sc = m_V rho~_j,
+// and S_i likewise.
 template <int DIM>
-__device__ __forceinline__ void stress_div_term(const double* sti, double ri2, const double* stj, double rtj,
-                                                double mVj, const double* kc, double* acc) {
-    double v[3];
-    stress_div_val<DIM>(sti, ri2, stj, rtj, mVj, kc, v);
-    for (int a = 0; a < DIM; ++a) acc[a] += v[a];
+__device__ __forceinline__ void stress_div_rec(const double* Si, const double* Sj, double sc, const double* kc,
+                                               double* out) {
+    for (int a = 0; a < DIM; ++a) {
+        double s = 0.0;
+        for (int b = 0; b < DIM; ++b) {
+            const double v = (sc * (Sj[a * DIM + b] + Si[a * DIM + b])) * kc[b];
+            s = b == 0 ? v : s + v;
+        }
+        out[a] = s;
+    }
 }
 
+// A soil record: v~ (DIM), m_V, m_V rho~, stress~ / rho~^2 (DIM x DIM).
 template <int DIM>
-__global__ void k_mui_mom(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
-                          const int* __restrict__ list, int count) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int i = list[k];
+struct SoilRec {
+    double a[DIM == 2 ? 8 : 16];
+    __device__ __forceinline__ SoilRec(const double* rec, int j) {
+        constexpr int N = DIM == 2 ? 8 : 16;
+        const double2* q = reinterpret_cast<const double2*>(rec + (size_t)N * j);
+#pragma unroll
+        for (int e = 0; e < N / 2 - (DIM == 3 ? 1 : 0); ++e) {
+            const double2 w = q[e];
+            a[2 * e] = w.x;
+            a[2 * e + 1] = w.y;
+        }
+    }
+    __device__ __forceinline__ const double* v() const { return a; }
+    __device__ __forceinline__ double mV() const { return a[DIM]; }
+    __device__ __forceinline__ double sc() const { return a[DIM + 1]; }
+    __device__ __forceinline__ const double* S() const { return a + DIM + 2; }
+};
+
+// mu(I) loop 2 (eng/solver_sph_muI.py:113-128) and the whole Drucker-Prager loop
+// (eng/solver_sph_dp.py:236-270): stress divergence, and for Drucker-Prager the velocity
+// gradient and continuity in the same walk.  Component order: acceleration, gradient, continuity.
+template <int DIM, int G, bool DP>
+__device__ __forceinline__ void soil_sums(const Consts& c, const Persist64& p, const Trans64& t,
+                                          const int* __restrict__ cs, const int* __restrict__ list, int count,
+                                          const Pairs64& pr, double (*S)[ROWS], double* A) {
+    constexpr int C = DIM + (DP ? DIM * DIM + 1 : 0);
     const int n = c.n;
-    double xi[3];
-    load_x<DIM>(p.x, i, n, xi);
-    double L[9], sti[9];
-    if (c.corr == 1)
-        for (int q = 0; q < 9; ++q) L[q] = t.CSPM_L[(size_t)q * n + i];
-    for (int q = 0; q < 9; ++q) sti[q] = t.stress_tmp[(size_t)q * n + i];
-    const double rti = t.density_tmp[i];
-    const double ri2 = rti * rti;
-    double dv[3] = {0, 0, 0};
-    const bool rep = c.boundary == 3 || c.boundary == 4;
-    for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
-        double kd[3], kc[3];
-        kernel_dW<DIM>(c, r, rn, kd);
-        if (c.corr == 1) matvec_corr<DIM>(L, kd, kc);
-        else { kc[0] = kd[0]; kc[1] = kd[1]; kc[2] = kd[2]; }
-        double stj[9];
-        for (int q = 0; q < 9; ++q) stj[q] = t.stress_tmp[(size_t)q * n + j];
-        stress_div_term<DIM>(sti, ri2, stj, t.density_tmp[j], p.m_V[j], kc, dv);
-    });
-    if (rep) {
-        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
-            if (p.mat_type[j] == MAT_REP) rep_force<DIM>(c, r, rn, dv);
+    if (pr.cap_f) {
+        const RowRef q = row_ref<G>(list, count, pr.cnt, pr.cap_f);
+        double L[9];
+        if (c.corr == 1)
+            for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
+        const SoilRec<DIM> ri(pr.rec, q.i);
+        block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
+            const size_t slot = q.base + s;
+            const int j = nb_index(pr.nb_f[slot]);
+            double kd[3] = {0.0, 0.0, 0.0}, kc[3];
+            for (int d = 0; d < DIM; ++d) kd[d] = pr.gk[d * pr.slots_f + slot];
+            corrected<DIM>(c, L, kd, kc);
+            const SoilRec<DIM> rj(pr.rec, j);
+            stress_div_rec<DIM>(ri.S(), rj.S(), rj.sc(), kc, T);
+            if (DP) vgrad_terms<DIM>(rj.v(), rj.mV(), ri.v(), kc, T + DIM);
         });
     }
+    const int row = blockIdx.x * ROWS + threadIdx.x;
+    if (threadIdx.x >= ROWS || row >= count) return;
+    const int i = list[row];
+    const bool rep = c.boundary == 3 || c.boundary == 4;
+    double xi[3];
+    load_x<DIM>(p.x, i, n, xi);
+    if (pr.cap_f && pr.cnt[row] <= pr.cap_f) {
+        for (int q = 0; q < C; ++q) A[q] = S[q][threadIdx.x];
+    } else {
+        double L[9];
+        if (c.corr == 1)
+            for (int q = 0; q < 9; ++q) L[q] = t.CSPM_L[(size_t)q * n + i];
+        const SoilRec<DIM> ri(pr.rec, i);
+        for (int q = 0; q < C; ++q) A[q] = 0.0;
+        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
+            double kd[3], kc[3], T[C];
+            kernel_dW<DIM>(c, r, rn, kd);
+            corrected<DIM>(c, L, kd, kc);
+            const SoilRec<DIM> rj(pr.rec, j);
+            stress_div_rec<DIM>(ri.S(), rj.S(), rj.sc(), kc, T);
+            if (DP) vgrad_terms<DIM>(rj.v(), rj.mV(), ri.v(), kc, T + DIM);
+            for (int q = 0; q < C; ++q) A[q] += T[q];
+        });
+    }
+    // repulsive forces (mu(I) only: the Drucker-Prager loop of the reference adds none)
+    if (rep && !DP)
+        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
+            if (p.mat_type[j] == MAT_REP) rep_force<DIM>(c, r, rn, A);
+        });
+}
+
+template <int DIM, int G>
+__global__ void __launch_bounds__(ROWS * G) k_mui_mom(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                                                      const int* __restrict__ list, int count, Pairs64 pr) {
+    __shared__ double S[DIM][ROWS];
+    double dv[3] = {0, 0, 0};
+    soil_sums<DIM, G, false>(c, p, t, cs, list, count, pr, S, dv);
+    const int row = blockIdx.x * ROWS + threadIdx.x;
+    if (threadIdx.x >= ROWS || row >= count) return;
+    const int i = list[row];
+    const int n = c.n;
     double vti[3], fd[3] = {0, 0, 0};
     for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + i];
-    damping_acc(c, rti, vti, fd, 3);
+    damping_acc(c, t.density_tmp[i], vti, fd, 3);
     for (int d = 0; d < 3; ++d) t.d_vel[(size_t)d * n + i] = (dv[d] + c.g[d]) + fd[d];
 }
 
 // ---- DP rates (eng/solver_sph_dp.py:236-270, Bui 2008 :172-208) ----
-template <int DIM>
-__global__ void k_dp_rates(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
-                           const int* __restrict__ list, int count) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int i = list[k];
+template <int DIM, int G>
+__global__ void __launch_bounds__(ROWS * G) k_dp_rates(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                                                       const int* __restrict__ list, int count, Pairs64 pr) {
+    constexpr int C = DIM + DIM * DIM + 1;
+    __shared__ double S[C][ROWS];
+    double A[C];
+    soil_sums<DIM, G, true>(c, p, t, cs, list, count, pr, S, A);
+    const int row = blockIdx.x * ROWS + threadIdx.x;
+    if (threadIdx.x >= ROWS || row >= count) return;
+    const int i = list[row];
     const int n = c.n;
-    double xi[3], vti[3];
-    load_x<DIM>(p.x, i, n, xi);
+    double vti[3], sti[9], dv[3] = {0, 0, 0};
     for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + i];
-    double L[9], sti[9];
-    if (c.corr == 1)
-        for (int q = 0; q < 9; ++q) L[q] = t.CSPM_L[(size_t)q * n + i];
     for (int q = 0; q < 9; ++q) sti[q] = t.stress_tmp[(size_t)q * n + i];
     const double rti = t.density_tmp[i];
-    const double ri2 = rti * rti;
     double vg[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    double dd = 0.0;
-    double dv[3] = {0, 0, 0};
-    for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
-        const double mVj = p.m_V[j];
-        double kd[3], kc[3];
-        kernel_dW<DIM>(c, r, rn, kd);
-        if (c.corr == 1) matvec_corr<DIM>(L, kd, kc);
-        else { kc[0] = kd[0]; kc[1] = kd[1]; kc[2] = kd[2]; }
-        double vtj[3];
-        for (int d = 0; d < DIM; ++d) vtj[d] = t.v_tmp[(size_t)d * n + j];
-        for (int a = 0; a < DIM; ++a) {
-            double av = mVj * (vtj[a] - vti[a]);
-            for (int b = 0; b < DIM; ++b) vg[3 * a + b] += av * kc[b];
-        }
-        double aa[3];
-        for (int d = 0; d < DIM; ++d) aa[d] = mVj * (vti[d] - vtj[d]);
-        dd += dotv<DIM>(aa, kc);
-        double stj[9];
-        for (int q = 0; q < 9; ++q) stj[q] = t.stress_tmp[(size_t)q * n + j];
-        stress_div_term<DIM>(sti, ri2, stj, t.density_tmp[j], mVj, kc, dv);
-    });
+    for (int a = 0; a < DIM; ++a) {
+        dv[a] = A[a];
+        for (int b = 0; b < DIM; ++b) vg[3 * a + b] = A[DIM + a * DIM + b];
+    }
+    const double dd = A[C - 1];
     for (int q = 0; q < 9; ++q) t.v_grad[(size_t)q * n + i] = vg[q];
     t.d_density[i] = dd * rti;
     // Bui 2008 stress rate
@@ -758,10 +1085,54 @@ __global__ void k_rk_final(Consts c, Persist64 p, Trans64 t, int* err) {
 }
 
 // ---- advect_pos with XSPH (eng/solver_sph_base.py:224-238), two phases ----
+template <int DIM, int G>
+__global__ void __launch_bounds__(ROWS * G) k_xsph(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                                                   const int* __restrict__ list, int count, Pairs64 pr) {
+    __shared__ double S[DIM][ROWS];
+    const int n = c.n;
+    const int tf = c.flow_type;
+    if (pr.cap_f) {
+        const RowRef q = row_ref<G>(list, count, pr.cnt, pr.cap_f);
+        double xi[3], vi[3];
+        load_x<DIM>(p.x, q.i, n, xi);
+        for (int d = 0; d < 3; ++d) vi[d] = p.v[(size_t)d * n + q.i];
+        block_row_sums<DIM, G>(q.cnt, S, [&](int s, double* T) {
+            const int ent = pr.nb_f[q.base + s];
+            if (!nb_flow(ent)) return;
+            const double w = pair_W<DIM>(c, p.x, xi, ent);
+            const double mVj = p.m_V[ent];
+            for (int d = 0; d < DIM; ++d) T[d] = mVj * (p.v[(size_t)d * n + ent] - vi[d]) * w;
+        });
+    }
+    const int row = blockIdx.x * ROWS + threadIdx.x;
+    if (threadIdx.x >= ROWS || row >= count) return;
+    const int i = list[row];
+    if (!p.is_dynamic[i]) return;
+    double s[3] = {0, 0, 0};
+    if (pr.cap_f && pr.cnt[row] <= pr.cap_f) {
+        for (int d = 0; d < DIM; ++d) s[d] = S[d][threadIdx.x];
+    } else {
+        double xi[3], vi[3];
+        load_x<DIM>(p.x, i, n, xi);
+        for (int d = 0; d < 3; ++d) vi[d] = p.v[(size_t)d * n + i];
+        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
+            if (p.mat_type[j] != tf) return;
+            const double w = kernel_W(c, rn);
+            const double mVj = p.m_V[j];
+            for (int d = 0; d < DIM; ++d) s[d] += mVj * (p.v[(size_t)d * n + j] - vi[d]) * w;
+        });
+    }
+    for (int d = 0; d < 3; ++d) t.aux3[(size_t)d * n + i] = s[d];
+}
+
+// Dynamic rigid particles move by the XSPH sum over their own kind (rigid rows list flow
+// neighbours only, so these walk the cells).
 template <int DIM>
-__global__ void k_xsph(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__global__ void k_xsph_rigid(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                             const int* __restrict__ list, int count) {
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= count) return;
+    const int i = list[k];
     const int n = c.n;
     const int ti = p.mat_type[i];
     if (!(ti > 0 && p.is_dynamic[i])) return;
@@ -819,22 +1190,41 @@ __global__ void k_post_mui_a(Consts c, Persist64 p, Trans64 t) {
 }
 
 // Stress regularisation after advect_pos: centres use their moved positions, candidate
-// cells come from this step's sort (eng/solver_sph_muI.py:151-156); exact f64 tests only.
-template <int DIM>
-__global__ void k_post_mui_b(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    if (p.mat_type[i] != MAT_SOIL) return;
+// cells come from this step's sort (eng/solver_sph_muI.py:151-156).  The rows are rebuilt from
+// the moved positions first (flow neighbours only).
+template <int DIM, int G>
+__global__ void __launch_bounds__(ROWS * G) k_post_mui_b(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                                                         const int* __restrict__ list, int count, Pairs64 pr) {
+    constexpr int C = 9;
+    __shared__ double S[C][ROWS];
     const int n = c.n;
-    double xi[3];
-    load_x<DIM>(p.x, i, n, xi);
+    if (pr.cap_f) {
+        const RowRef q = row_ref<G>(list, count, pr.cnt, pr.cap_f);
+        double xi[3];
+        load_x<DIM>(p.x, q.i, n, xi);
+        block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
+            const int j = pr.nb_f[q.base + s];
+            const double w = pair_W<DIM>(c, p.x, xi, j);
+            const double mVj = p.m_V[j];
+            for (int e = 0; e < 9; ++e) T[e] = mVj * p.stress[(size_t)e * n + j] * w;
+        });
+    }
+    const int row = blockIdx.x * ROWS + threadIdx.x;
+    if (threadIdx.x >= ROWS || row >= count) return;
+    const int i = list[row];
     double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, false, [&](int j, const double* r, double rn) {
-        if (p.mat_type[j] != MAT_SOIL) return;
-        const double w = kernel_W(c, rn);
-        const double mVj = p.m_V[j];
-        for (int q = 0; q < 9; ++q) s[q] += mVj * p.stress[(size_t)q * n + j] * w;
-    });
+    if (pr.cap_f && pr.cnt[row] <= pr.cap_f) {
+        for (int q = 0; q < 9; ++q) s[q] = S[q][threadIdx.x];
+    } else {
+        double xi[3];
+        load_x<DIM>(p.x, i, n, xi);
+        for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, false, [&](int j, const double* r, double rn) {
+            if (p.mat_type[j] != MAT_SOIL) return;
+            const double w = kernel_W(c, rn);
+            const double mVj = p.m_V[j];
+            for (int q = 0; q < 9; ++q) s[q] += mVj * p.stress[(size_t)q * n + j] * w;
+        });
+    }
     const double f = t.CSPM_f[i];
     for (int q = 0; q < 9; ++q) t.aux9[(size_t)q * n + i] = s[q] * f;
 }
@@ -1188,9 +1578,59 @@ static void rigid_lists64(const Consts& c, const Persist64& p, const Rigid64& r,
         else TSG_LAUNCH(KERNEL<3>, GRID, TPB, s, __VA_ARGS__);                    \
     } while (0)
 
+// Lanes per row of the pair loops.
+constexpr int LANES = 8;
+inline int nrows(int count) { return (count + ROWS - 1) / ROWS; }
+// Threads of a row kernel: without rows only the epilogue's threads have work.
+inline int row_threads(const Grid& g) { return g.pr.cap_f ? ROWS * LANES : ROWS; }
+
+#define DISPATCH_ROWS(c, g, KERNEL, COUNT, ...)                                                            \
+    do {                                                                                                   \
+        if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LANES>), nrows(COUNT), row_threads(g), s, __VA_ARGS__);    \
+        else TSG_LAUNCH((KERNEL<3, LANES>), nrows(COUNT), row_threads(g), s, __VA_ARGS__);                 \
+    } while (0)
+#define DISPATCH_ROWS_B(c, g, KERNEL, FLAG, COUNT, ...)                                                          \
+    do {                                                                                                         \
+        if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LANES, FLAG>), nrows(COUNT), row_threads(g), s, __VA_ARGS__);    \
+        else TSG_LAUNCH((KERNEL<3, LANES, FLAG>), nrows(COUNT), row_threads(g), s, __VA_ARGS__);                 \
+    } while (0)
+
+static void build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, bool flow_only,
+                       cudaStream_t s) {
+    if (!g.pr.cap_f) return;
+    const int nb = flow_only ? 0 : c.n_bdy;
+    const long long threads = 32ll * (c.n_flow + nb);
+    if (threads <= 0) return;
+    const int blocks = (int)((threads + 255) / 256);
+    if (c.dim == 2)
+        TSG_LAUNCH(k_list64<2>, blocks, 256, s, c, p.x, t.pos32, g.cell_start, g.list_flow, c.n_flow, g.list_bdy, nb,
+                   flow_only, g.pr);
+    else
+        TSG_LAUNCH(k_list64<3>, blocks, 256, s, c, p.x, t.pos32, g.cell_start, g.list_flow, c.n_flow, g.list_bdy, nb,
+                   flow_only, g.pr);
+}
+
+void fp64_build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, cudaStream_t s) {
+    PhaseScope ph(s, PH_LISTS);
+    build_rows(c, p, t, g, false, s);
+}
+
+void fp64_geometry(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+    if (!g.pr.cap_f) return;
+    PhaseScope ph(s, PH_LISTS);
+    if (c.n_flow > 0) DISPATCH_ROWS(c, g, k_geom_flow, c.n_flow, c, p, g.list_flow, c.n_flow, g.pr);
+    if (c.n_bdy > 0) DISPATCH_ROWS(c, g, k_geom_bdy, c.n_bdy, c, p, g.list_bdy, c.n_bdy, g.pr);
+}
+
 void fp64_kernel_corr(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
     PhaseScope ph(s, PH_CORR);
-    DISPATCH_DIM(c, k_corr, nblk(c.n), c, p, t, g.cell_start);
+    if (c.n_flow > 0) {
+        if (c.corr == 1)
+            DISPATCH_ROWS_B(c, g, k_corr_flow, true, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+        else
+            DISPATCH_ROWS_B(c, g, k_corr_flow, false, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+    }
+    if (c.n_bdy > 0) DISPATCH_ROWS(c, g, k_corr_bdy, c.n_bdy, c, p, t, g.cell_start, g.list_bdy, c.n_bdy, g.pr);
 }
 
 void fp64_rest_cm(const Consts& c, const Persist64& p, const Rigid64& r, cudaStream_t s) {
@@ -1220,21 +1660,24 @@ void fp64_init_tmp(const Consts& c, const Persist64& p, Trans64& t, cudaStream_t
 void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
     if (c.n_flow > 0 && (c.solver == 1 || c.solver == 3)) {
         PhaseScope ph(s, PH_PRE);
-        TSG_LAUNCH(k_pre, nblk(c.n_flow), TPB, s, c, p, t, g.list_flow, c.n_flow);
+        TSG_LAUNCH(k_pre, nblk(c.n_flow), TPB, s, c, p, t, g.list_flow, c.n_flow, g.pr);
     }
     if (c.solver == 2 && c.n_flow > 0) {
         PhaseScope ph(s, PH_PRE);
-        DISPATCH_DIM(c, k_mui_stress, nblk(c.n_flow), c, p, t, g.cell_start, g.list_flow, c.n_flow);
+        DISPATCH_ROWS(c, g, k_mui_stress, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
     }
     if (c.n_bdy > 0) {
         PhaseScope ph(s, PH_BDY);
-        DISPATCH_DIM(c, k_bdy, nblk(c.n_bdy), c, p, t, g.cell_start, g.list_bdy, c.n_bdy);
+        if (c.solver == 1)
+            DISPATCH_ROWS_B(c, g, k_bdy, false, c.n_bdy, c, p, t, g.cell_start, g.list_bdy, c.n_bdy, g.pr);
+        else
+            DISPATCH_ROWS_B(c, g, k_bdy, true, c.n_bdy, c, p, t, g.cell_start, g.list_bdy, c.n_bdy, g.pr);
     }
     if (c.n_flow > 0) {
         PhaseScope ph(s, PH_RATES);
-        if (c.solver == 1) DISPATCH_DIM(c, k_wc_rates, nblk(c.n_flow), c, p, t, g.cell_start, g.list_flow, c.n_flow);
-        else if (c.solver == 2) DISPATCH_DIM(c, k_mui_mom, nblk(c.n_flow), c, p, t, g.cell_start, g.list_flow, c.n_flow);
-        else DISPATCH_DIM(c, k_dp_rates, nblk(c.n_flow), c, p, t, g.cell_start, g.list_flow, c.n_flow);
+        if (c.solver == 1) DISPATCH_ROWS(c, g, k_wc_rates, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+        else if (c.solver == 2) DISPATCH_ROWS(c, g, k_mui_mom, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+        else DISPATCH_ROWS(c, g, k_dp_rates, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
     }
     if (c.n_rigid_dyn > 0 && c.n_bdy > 0) {  // the flow's reaction on dynamic rigid particles
         PhaseScope ph(s, PH_RATES);
@@ -1250,14 +1693,23 @@ void fp64_advect(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int w
     case TSG_ADVECT_FULL: TSG_LAUNCH(k_advect_full, nb, TPB, s, c, p, t, g.err); break;
     case TSG_ADVECT_LF_HALF: TSG_LAUNCH(k_advect_half, nb, TPB, s, c, p, t); break;
     case TSG_ADVECT_POS:
-        if (c.xsph) DISPATCH_DIM(c, k_xsph, nb, c, p, t, g.cell_start);
+        if (c.xsph) {
+            if (c.n_flow > 0)
+                DISPATCH_ROWS(c, g, k_xsph, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+            if (c.n_rigid_dyn > 0)
+                DISPATCH_DIM(c, k_xsph_rigid, nblk(c.n_bdy), c, p, t, g.cell_start, g.list_bdy, c.n_bdy);
+        }
         TSG_LAUNCH(k_advect_pos, nb, TPB, s, c, p, t, g.err);
         break;
     case TSG_ADVECT_SOMETHING:
         if (c.solver == 1) TSG_LAUNCH(k_post_wc, nb, TPB, s, c, p);
         else if (c.solver == 2) {
             TSG_LAUNCH(k_post_mui_a, nb, TPB, s, c, p, t);
-            DISPATCH_DIM(c, k_post_mui_b, nb, c, p, t, g.cell_start);
+            if (c.n_flow > 0) {
+                if (g.pr.cap_f) fp64_refresh_pos32(c, p, t, s);
+                build_rows(c, p, t, g, true, s);
+                DISPATCH_ROWS(c, g, k_post_mui_b, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+            }
             TSG_LAUNCH(k_post_mui_c, nb, TPB, s, c, p, t);
         } else TSG_LAUNCH(k_post_dp, nb, TPB, s, c, p, t);
         break;
@@ -1298,15 +1750,17 @@ void fp64_init_geostatic(const Consts& c, Persist64& p, double* scratch, cudaStr
     TSG_LAUNCH(k_geostatic, nblk(c.n), TPB, s, c, p, scratch, c.K0);
 }
 
-__global__ void k_refresh_pos32_impl(Consts c, const double* __restrict__ x, float4* __restrict__ pos32) {
+__global__ void k_refresh_pos32_impl(Consts c, const double* __restrict__ x, const int* __restrict__ mt,
+                                     float4* __restrict__ pos32) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
     const size_t n = c.n;
-    pos32[i] = make_float4((float)(x[i] - c.vs[0]), (float)(x[n + i] - c.vs[1]), (float)(x[2 * n + i] - c.vs[2]), 0.f);
+    pos32[i] = make_float4((float)(x[i] - c.vs[0]), (float)(x[n + i] - c.vs[1]), (float)(x[2 * n + i] - c.vs[2]),
+                           is_flow(mt[i]) ? 1.f : 0.f);
 }
 
 void fp64_refresh_pos32(const Consts& c, const Persist64& p, Trans64& t, cudaStream_t s) {
-    TSG_LAUNCH(k_refresh_pos32_impl, nblk(c.n), TPB, s, c, p.x, t.pos32);
+    TSG_LAUNCH(k_refresh_pos32_impl, nblk(c.n), TPB, s, c, p.x, p.mat_type, t.pos32);
 }
 
 }  // namespace tsg

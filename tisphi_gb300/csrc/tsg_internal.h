@@ -53,6 +53,8 @@ struct Consts {
     // every |x - vdomain_start| below pf_lim
     int pf_on;
     float pf_r2, pf_lim;
+    float pf_in2;       // below this f32 distance^2 a pair is certainly a neighbour
+    double R2T;         // r2 < R2T exactly when sqrt(r2) < R
     int n_rigid_dyn;    // dynamic rigid particles (shape-matched bodies)
 };
 
@@ -117,7 +119,24 @@ struct Trans64 {
     double* d_stress_RK;// 9 planes or nullptr
     double* aux3;       // 3 planes: XSPH sums
     double* aux9;       // 9 planes: regularised stress (mu(I))
-    float4* pos32;      // (x - vdomain_start) as f32, candidate prefilter
+    float4* pos32;      // (x - vdomain_start) as f32, candidate prefilter; w = 1 for flow particles
+};
+
+// Neighbour rows of the current positions (tsg_pairs64.cuh): row k of the flow block belongs to
+// particle list_flow[k], row k of the boundary block to list_bdy[k].  Row-major with a fixed
+// pitch (a multiple of 8 slots); a row whose count exceeds it is walked through the cells.
+// cap_f == 0: no rows (not enough device memory), every particle walks the cells.
+struct Pairs64 {
+    int cap_f, cap_b;
+    size_t slots_f;     // n_flow * cap_f: plane stride of gk
+    int* cnt;           // n_flow + n_bdy
+    int* nb_f;          // entries: particle index, sign bit set for a non-flow neighbour
+    int* nb_b;
+    double* gk;         // dim planes: kernel gradient of each flow entry
+    double* gden;       // |r|^2 + 0.01 h^2 of each flow entry (WCSPH)
+    double* gw;         // kernel value of each boundary entry
+    double* rec;        // rec_stride doubles per particle: what the rates loop reads of a neighbour
+    int rec_stride;
 };
 
 // Sort scratch and cell table.
@@ -134,6 +153,7 @@ struct Grid {
     int* err;           // device error word
     int* big;           // cells above kSortSmall particles (cellsort_big_ints)
     int* nbig;          // their count
+    Pairs64 pr;         // neighbour rows
 };
 
 // ---- headless visual buffer (tsg_visual.cu) ----
@@ -153,6 +173,10 @@ void scan_exclusive(const int* in, int* out, int n, int* tile_sum, cudaStream_t 
 
 // ---- launchers (tsg_fp64.cu) ----
 void fp64_kernel_corr(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
+// Neighbour rows of the current positions, and the pair geometry without the correction
+// factors (for a loop called on its own; fp64_kernel_corr writes the geometry too).
+void fp64_build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, cudaStream_t s);
+void fp64_geometry(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
 void fp64_init_tmp(const Consts& c, const Persist64& p, Trans64& t, cudaStream_t s);
 void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
 void fp64_advect(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int which, cudaStream_t s);

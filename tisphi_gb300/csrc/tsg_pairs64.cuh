@@ -1,0 +1,155 @@
+// Neighbour rows of the FP64 form: built once per step, walked by every pair loop of it.
+//
+// Positions are fixed from the sort to advect_pos, so the neighbours of a step, their kernel
+// gradients and the dummies' kernel values are the same in every loop.  k_list64 writes each
+// particle's neighbours in the reference's traversal order (for_all_neighbors,
+// eng/particle_system.py:259-269): flow particles list all neighbours, boundary and rigid
+// particles only flow neighbours (all that any loop reads).  The correction pass computes the
+// pair geometry and stores it beside the entries.
+//
+// What bounds these loops is the FP64 pipe: sm_103a issues one FP64 warp instruction per SM
+// in 16 cycles, against four of any other kind per cycle, so everything that is not FP64
+// arithmetic (list and record traffic, shared-memory exchange) hides behind it and every FP64
+// operation saved counts.  A traversal of the cells ran the FP64 body for a third of a warp's
+// lanes (the candidates of different particles pass the distance test at different trips);
+// rows keep the lanes full.
+//
+// G lanes share a row: lane g evaluates the pair terms of slots g, g + G, ..., the terms of a
+// trip go through shared memory, and lane c adds component c of them in slot order.  The sums
+// therefore round exactly as one thread adding them in traversal order (a missing slot adds
+// +0.0, which changes no sum that starts at +0.0), C chains of additions cost one lane group
+// G additions instead of C x G, and small scenes get G times the threads.
+#pragma once
+
+#include "tsg_internal.h"
+
+namespace tsg {
+namespace {
+
+constexpr int ROWS = 32;           // rows per block; one thread each in the epilogue
+constexpr int NB_BDY = 1 << 31;    // entry flag: not a flow particle (sign bit)
+
+__device__ __forceinline__ int nb_index(int ent) { return ent & 0x7fffffff; }
+__device__ __forceinline__ bool nb_flow(int ent) { return ent >= 0; }
+
+// One warp per row.  The candidates of one stencil row of cells are contiguous; 32 of them are
+// tested at a time and the accepted ones compacted in order by ballot.  The f32 distance
+// decides all but the pairs within 2^-10 of R^2 (the rounding of f32 coordinates below 500 R
+// stays under a fifth of that), which take the reference's f64 test: r2 < R2T is
+// sqrt(r2) < support_radius, exactly, sqrt being monotone.
+template <int DIM>
+__global__ void __launch_bounds__(256) k_list64(Consts c, const double* __restrict__ X,
+                                                const float4* __restrict__ P32, const int* __restrict__ cs,
+                                                const int* __restrict__ list_flow, int n_flow,
+                                                const int* __restrict__ list_bdy, int n_bdy, bool flow_only,
+                                                Pairs64 pr) {
+    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (row >= n_flow + n_bdy) return;
+    const bool bdy = row >= n_flow;
+    const int i = bdy ? list_bdy[row - n_flow] : list_flow[row];
+    const bool want_flow = bdy || flow_only;
+    const int cap = bdy ? pr.cap_b : pr.cap_f;
+    int* out = bdy ? pr.nb_b + (size_t)(row - n_flow) * cap : pr.nb_f + (size_t)row * cap;
+    const size_t n = c.n;
+    double xi[3];
+    long long cc[3];
+    bool ok = true;
+    for (int d = 0; d < 3; ++d) {
+        xi[d] = X[d * n + i];
+        const double t = (xi[d] - c.vs[d]) / c.grid;
+        ok = ok && fabs(t) < 2147483647.0;
+        cc[d] = ok ? (int)t : 0;
+    }
+    const float4 pi = P32[i];
+    const bool pf = c.pf_on && fabsf(pi.x) < c.pf_lim && fabsf(pi.y) < c.pf_lim && fabsf(pi.z) < c.pf_lim;
+    constexpr int NR = DIM == 3 ? 9 : 3;
+    int jb_l = 0, je_l = 0;
+    if (ok && lane < NR) {
+        const long long ny = c.gnum[1], nz = c.gnum[2], G = c.G;
+        const int ox = DIM == 3 ? lane / 3 - 1 : lane - 1, oy = DIM == 3 ? lane % 3 - 1 : 0;
+        const long long f0 = (cc[0] + ox) * ny * nz + (cc[1] + oy) * nz + cc[2];
+        const long long lo = f0 - 1 > 0 ? f0 - 1 : 0;
+        const long long hi = f0 + 1 < G - 1 ? f0 + 1 : G - 1;
+        if (lo <= hi) { jb_l = cs[lo]; je_l = cs[hi + 1]; }
+    }
+    int m = 0;
+    for (int q = 0; q < NR; ++q) {
+        const int jb = __shfl_sync(0xffffffffu, jb_l, q), je = __shfl_sync(0xffffffffu, je_l, q);
+        for (int b = jb; b < je; b += 32) {
+            const int j = b + lane;
+            bool in = false, flow = false;
+            if (j < je && j != i) {
+                const float4 pj = P32[j];
+                flow = pj.w != 0.f;
+                if (flow || !want_flow) {
+                    bool exact = !pf;
+                    if (pf) {
+                        const float fx = pi.x - pj.x, fy = pi.y - pj.y, fz = pi.z - pj.z;
+                        float r2f = fx * fx + fy * fy;
+                        if (DIM == 3) r2f += fz * fz;
+                        in = r2f < c.pf_in2;
+                        exact = !in && !(r2f > c.pf_r2);
+                    }
+                    if (exact) {
+                        const double rx = xi[0] - X[j], ry = xi[1] - X[n + j];
+                        double r2 = rx * rx + ry * ry;
+                        if (DIM == 3) { const double rz = xi[2] - X[2 * n + j]; r2 = r2 + rz * rz; }
+                        in = r2 < c.R2T;
+                    }
+                }
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, in);
+            const int pos = m + __popc(bal & ((1u << lane) - 1u));
+            if (in && pos < cap) out[pos] = flow ? j : j | NB_BDY;
+            m += __popc(bal);
+        }
+    }
+    if (lane == 0) pr.cnt[row] = m;
+}
+
+// The ordered sums of one row's C pair terms by its G lanes; acc[m] of lane g is component
+// g + m G.  `term(s, T)` evaluates slot s.  sh: this warp's C x 33 doubles (the pitch keeps
+// the column reads off each other's banks).
+template <int C, int G, class F>
+__device__ __forceinline__ void row_sums(int cnt, double* sh, double (&acc)[(C + G - 1) / G], F&& term) {
+    const int lane = threadIdx.x & 31, g = lane % G, gb = lane - g;
+    const int mx = __reduce_max_sync(0xffffffffu, cnt);
+    for (int k0 = 0; k0 < mx; k0 += G) {
+        double T[C];
+#pragma unroll
+        for (int q = 0; q < C; ++q) T[q] = 0.0;
+        if (k0 + g < cnt) term(k0 + g, T);
+#pragma unroll
+        for (int q = 0; q < C; ++q) sh[q * 33 + lane] = T[q];
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < (C + G - 1) / G; ++m) {
+            const int q = g + m * G;
+            if (q < C) {
+#pragma unroll
+                for (int e = 0; e < G; ++e) acc[m] = acc[m] + sh[q * 33 + gb + e];
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// Row sums of a block of ROWS rows: fills S[q][row in block] (shared) for every listed row.
+// cnt is this thread's row's count, 0 for rows to skip.  Ends with a block barrier.
+template <int C, int G, class F>
+__device__ __forceinline__ void block_row_sums(int cnt, double (*S)[ROWS], F&& term) {
+    __shared__ double sh[G][C * 33];
+    double acc[(C + G - 1) / G];
+#pragma unroll
+    for (int m = 0; m < (C + G - 1) / G; ++m) acc[m] = 0.0;
+    row_sums<C, G>(cnt, sh[threadIdx.x >> 5], acc, term);
+    const int g = threadIdx.x % G, r = threadIdx.x / G;
+#pragma unroll
+    for (int m = 0; m < (C + G - 1) / G; ++m)
+        if (g + m * G < C) S[g + m * G][r] = acc[m];
+    __syncthreads();
+}
+
+}  // namespace
+}  // namespace tsg

@@ -180,7 +180,8 @@ __global__ void k_reorder64(Consts c, const int* __restrict__ perm, Persist64 a,
         b.id0[k] = a.id0[s];
         if (vt_src)
             for (int d = 0; d < 3; ++d) vt_dst[d * n + k] = vt_src[d * n + s];
-        pos32[k] = make_float4((float)(xv[0] - c.vs[0]), (float)(xv[1] - c.vs[1]), (float)(xv[2] - c.vs[2]), 0.f);
+        pos32[k] = make_float4((float)(xv[0] - c.vs[0]), (float)(xv[1] - c.vs[1]), (float)(xv[2] - c.vs[2]),
+                               mt == MAT_FLUID || mt == MAT_SOIL ? 1.f : 0.f);
     }
     append(list_flow, list_count + 0, live && mt == c.flow_type, k);
     append(list_bdy, list_count + 1, live && (mt == MAT_DUMMY || mt == MAT_REP || mt == MAT_RIGID), k);
