@@ -172,9 +172,10 @@ int alloc_all(tsg_handle* h) {
     rc |= dalloc(h, &t.d_density_RK, n); rc |= dalloc(h, &t.d_vel_RK, 3 * n);
     if (c.solver == 3) rc |= dalloc(h, &t.d_stress_RK, 9 * n);
     rc |= dalloc(h, &t.aux3, 3 * n);
-    rc |= dalloc(h, &t.pos32, n);
+    rc |= dalloc(h, &t.pos32, n); rc |= dalloc(h, &t.pos32l, n); rc |= dalloc(h, &t.cell0, n);
     Grid& g = h->g;
     const size_t nb = (size_t)c.G + 1;
+    rc |= dalloc(h, &g.cell0_old, n); rc |= dalloc(h, &g.cell_flow, (size_t)c.G);
     rc |= dalloc(h, &g.cell_of, n); rc |= dalloc(h, &g.rank, n); rc |= dalloc(h, &g.count, nb);
     rc |= dalloc(h, &g.cell_start, nb + 1); rc |= dalloc(h, &g.perm, n);
     rc |= dalloc(h, &g.tile_sum, nb / 2048 + 2);
@@ -232,7 +233,7 @@ void refresh_pos32_if_dirty(tsg_handle* h, cudaStream_t s) {
 void own_rows(tsg_handle* h, bool geometry, cudaStream_t s) {
     fp64_refresh_pos32(h->c, h->cur, h->t, s);
     h->pos32_dirty = false;
-    fp64_build_rows(h->c, h->cur, h->t, h->g, s);
+    fp64_build_rows(h->c, h->cur, h->t, h->g, false, s);
     if (geometry) fp64_geometry(h->c, h->cur, h->t, h->g, s);
 }
 
@@ -262,7 +263,7 @@ int substep64(tsg_handle* h, cudaStream_t s) {
 // One step of the FP64 form after its sort.
 int step64(tsg_handle* h, bool collide, cudaStream_t s) {
     const Consts& c = h->c;
-    fp64_build_rows(c, h->cur, h->t, h->g, s);
+    fp64_build_rows(c, h->cur, h->t, h->g, true, s);
     fp64_kernel_corr(c, h->cur, h->t, h->g, s);
     fp64_init_tmp(c, h->cur, h->t, s);
     if (int rc = substep64(h, s)) return rc;
@@ -366,6 +367,8 @@ int tsg_create(const tsg_config* cfg, tsg_handle** out) {
     c.pf_r2 = std::nextafter((float)(c.R * c.R * (1.0 + 1.0 / 1024.0)), 1e30f);
     c.pf_lim = (float)(500.0 * c.R);
     c.pf_in2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 1024.0)), 0.f);
+    c.pf_lo2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 262144.0)), 0.f);
+    c.pf_hi2 = std::nextafter((float)(c.R * c.R * (1.0 + 1.0 / 262144.0)), 1e30f);
     c.R2T = c.R * c.R;
     while (std::sqrt(c.R2T) >= c.R) c.R2T = std::nextafter(c.R2T, 0.0);
     while (std::sqrt(c.R2T) < c.R) c.R2T = std::nextafter(c.R2T, 1e300);

@@ -1596,23 +1596,24 @@ inline int row_threads(const Grid& g) { return g.pr.cap_f ? ROWS * LANES : ROWS;
     } while (0)
 
 static void build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, bool flow_only,
-                       cudaStream_t s) {
+                       bool sorted, cudaStream_t s) {
     if (!g.pr.cap_f) return;
     const int nb = flow_only ? 0 : c.n_bdy;
-    const long long threads = 32ll * (c.n_flow + nb);
-    if (threads <= 0) return;
-    const int blocks = (int)((threads + 255) / 256);
+    const int blocks = (c.n_flow + nb + 7) / 8;
+    if (blocks <= 0) return;
+    const unsigned char* cf = sorted ? g.cell_flow : nullptr;
     if (c.dim == 2)
-        TSG_LAUNCH(k_list64<2>, blocks, 256, s, c, p.x, t.pos32, g.cell_start, g.list_flow, c.n_flow, g.list_bdy, nb,
-                   flow_only, g.pr);
+        TSG_LAUNCH(k_list64<2>, blocks, 256, s, c, p.x, t.pos32, t.pos32l, t.cell0, g.cell_start, cf, g.list_flow,
+                   c.n_flow, g.list_bdy, nb, flow_only, g.pr);
     else
-        TSG_LAUNCH(k_list64<3>, blocks, 256, s, c, p.x, t.pos32, g.cell_start, g.list_flow, c.n_flow, g.list_bdy, nb,
-                   flow_only, g.pr);
+        TSG_LAUNCH(k_list64<3>, blocks, 256, s, c, p.x, t.pos32, t.pos32l, t.cell0, g.cell_start, cf, g.list_flow,
+                   c.n_flow, g.list_bdy, nb, flow_only, g.pr);
 }
 
-void fp64_build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, cudaStream_t s) {
+void fp64_build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, bool sorted,
+                     cudaStream_t s) {
     PhaseScope ph(s, PH_LISTS);
-    build_rows(c, p, t, g, false, s);
+    build_rows(c, p, t, g, false, sorted, s);
 }
 
 void fp64_geometry(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
@@ -1707,7 +1708,7 @@ void fp64_advect(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int w
             TSG_LAUNCH(k_post_mui_a, nb, TPB, s, c, p, t);
             if (c.n_flow > 0) {
                 if (g.pr.cap_f) fp64_refresh_pos32(c, p, t, s);
-                build_rows(c, p, t, g, true, s);
+                build_rows(c, p, t, g, true, false, s);
                 DISPATCH_ROWS(c, g, k_post_mui_b, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
             }
             TSG_LAUNCH(k_post_mui_c, nb, TPB, s, c, p, t);
@@ -1751,16 +1752,18 @@ void fp64_init_geostatic(const Consts& c, Persist64& p, double* scratch, cudaStr
 }
 
 __global__ void k_refresh_pos32_impl(Consts c, const double* __restrict__ x, const int* __restrict__ mt,
-                                     float4* __restrict__ pos32) {
+                                     float4* __restrict__ pos32, float4* __restrict__ pos32l,
+                                     long long* __restrict__ cell0) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
     const size_t n = c.n;
-    pos32[i] = make_float4((float)(x[i] - c.vs[0]), (float)(x[n + i] - c.vs[1]), (float)(x[2 * n + i] - c.vs[2]),
-                           is_flow(mt[i]) ? 1.f : 0.f);
+    const double xi[3] = {x[i], x[n + i], x[2 * n + i]};
+    write_pos32(c, xi, is_flow(mt[i]), pos32 + i, pos32l + i);
+    cell0[i] = flat_cell(c, xi);
 }
 
 void fp64_refresh_pos32(const Consts& c, const Persist64& p, Trans64& t, cudaStream_t s) {
-    TSG_LAUNCH(k_refresh_pos32_impl, nblk(c.n), TPB, s, c, p.x, p.mat_type, t.pos32);
+    TSG_LAUNCH(k_refresh_pos32_impl, nblk(c.n), TPB, s, c, p.x, p.mat_type, t.pos32, t.pos32l, t.cell0);
 }
 
 }  // namespace tsg

@@ -54,6 +54,7 @@ struct Consts {
     int pf_on;
     float pf_r2, pf_lim;
     float pf_in2;       // below this f32 distance^2 a pair is certainly a neighbour
+    float pf_lo2, pf_hi2;  // the same two bounds for the distance^2 with the low parts added
     double R2T;         // r2 < R2T exactly when sqrt(r2) < R
     int n_rigid_dyn;    // dynamic rigid particles (shape-matched bodies)
 };
@@ -120,7 +121,10 @@ struct Trans64 {
     double* aux3;       // 3 planes: XSPH sums
     double* aux9;       // 9 planes: regularised stress (mu(I))
     float4* pos32;      // (x - vdomain_start) as f32, candidate prefilter; w = 1 for flow particles
+    float4* pos32l;     // what pos32 rounds off, as f32
+    long long* cell0;   // flattened cell index of the position, kNoCell if it has none
 };
+constexpr long long kNoCell = (long long)1 << 62;
 
 // Neighbour rows of the current positions (tsg_pairs64.cuh): row k of the flow block belongs to
 // particle list_flow[k], row k of the boundary block to list_bdy[k].  Row-major with a fixed
@@ -143,6 +147,7 @@ struct Pairs64 {
 struct Grid {
     int* cell_of;       // per particle (old order)
     int* rank;          // per particle within-cell arrival rank
+    long long* cell0_old;  // per particle (old order): unclipped flattened cell index
     int* count;         // G + 1
     int* cell_start;    // G + 2 exclusive starts; [G] = out-of-grid bin, [G+1] = n
     int* perm;          // new -> old
@@ -153,6 +158,7 @@ struct Grid {
     int* err;           // device error word
     int* big;           // cells above kSortSmall particles (cellsort_big_ints)
     int* nbig;          // their count
+    unsigned char* cell_flow;  // per cell: 1 if it holds flow particles (as of the last sort)
     Pairs64 pr;         // neighbour rows
 };
 
@@ -175,7 +181,9 @@ void scan_exclusive(const int* in, int* out, int n, int* tile_sum, cudaStream_t 
 void fp64_kernel_corr(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
 // Neighbour rows of the current positions, and the pair geometry without the correction
 // factors (for a loop called on its own; fp64_kernel_corr writes the geometry too).
-void fp64_build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, cudaStream_t s);
+// sorted: positions and types are those of the last sort (cell_flow holds).
+void fp64_build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, bool sorted,
+                     cudaStream_t s);
 void fp64_geometry(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
 void fp64_init_tmp(const Consts& c, const Persist64& p, Trans64& t, cudaStream_t s);
 void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);

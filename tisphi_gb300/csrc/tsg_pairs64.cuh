@@ -33,13 +33,22 @@ __device__ __forceinline__ int nb_index(int ent) { return ent & 0x7fffffff; }
 __device__ __forceinline__ bool nb_flow(int ent) { return ent >= 0; }
 
 // One warp per row.  The candidates of one stencil row of cells are contiguous; 32 of them are
-// tested at a time and the accepted ones compacted in order by ballot.  The f32 distance
-// decides all but the pairs within 2^-10 of R^2 (the rounding of f32 coordinates below 500 R
-// stays under a fifth of that), which take the reference's f64 test: r2 < R2T is
-// sqrt(r2) < support_radius, exactly, sqrt being monotone.
+// tested at a time and the accepted ones compacted in order by ballot.  An FP64 instruction
+// costs a warp the same 16 cycles for one lane as for 32, so no FP64 runs here but for pairs
+// within 2^-18 of R^2: the f32 distance decides all but those within 2^-10 (the rounding of f32
+// coordinates below 500 R stays under a fifth of that), the same distance with the low parts of
+// the coordinates added all but those within 2^-18 (its error is below 2^-20), and the rest
+// take the reference's test: r2 < R2T is sqrt(r2) < support_radius, exactly, sqrt being
+// monotone.  The cell index comes from the sort (or the position refresh), one division per
+// particle there instead of one per warp here.  Boundary rows skip stencil rows without flow
+// particles (three quarters of a tank's dummies see none).
+// 118 k fluid + 357 k dummy particles in 3D: 301 us (911,754 + 1,413,114: 6.34 ms with FP64 cell
+// indices and shell tests in the warp, about 2 ms without).
 template <int DIM>
 __global__ void __launch_bounds__(256) k_list64(Consts c, const double* __restrict__ X,
-                                                const float4* __restrict__ P32, const int* __restrict__ cs,
+                                                const float4* __restrict__ P32, const float4* __restrict__ P32L,
+                                                const long long* __restrict__ cell0, const int* __restrict__ cs,
+                                                const unsigned char* __restrict__ cell_flow,
                                                 const int* __restrict__ list_flow, int n_flow,
                                                 const int* __restrict__ list_bdy, int n_bdy, bool flow_only,
                                                 Pairs64 pr) {
@@ -52,60 +61,88 @@ __global__ void __launch_bounds__(256) k_list64(Consts c, const double* __restri
     const int cap = bdy ? pr.cap_b : pr.cap_f;
     int* out = bdy ? pr.nb_b + (size_t)(row - n_flow) * cap : pr.nb_f + (size_t)row * cap;
     const size_t n = c.n;
-    double xi[3];
-    long long cc[3];
-    bool ok = true;
-    for (int d = 0; d < 3; ++d) {
-        xi[d] = X[d * n + i];
-        const double t = (xi[d] - c.vs[d]) / c.grid;
-        ok = ok && fabs(t) < 2147483647.0;
-        cc[d] = ok ? (int)t : 0;
-    }
-    const float4 pi = P32[i];
-    const bool pf = c.pf_on && fabsf(pi.x) < c.pf_lim && fabsf(pi.y) < c.pf_lim && fabsf(pi.z) < c.pf_lim;
     constexpr int NR = DIM == 3 ? 9 : 3;
+    const long long fc = cell0[i];
     int jb_l = 0, je_l = 0;
-    if (ok && lane < NR) {
-        const long long ny = c.gnum[1], nz = c.gnum[2], G = c.G;
+    if (fc != kNoCell && lane < NR) {
+        const long long nz = c.gnum[2], sx = c.gnum[1] * nz, G = c.G;
         const int ox = DIM == 3 ? lane / 3 - 1 : lane - 1, oy = DIM == 3 ? lane % 3 - 1 : 0;
-        const long long f0 = (cc[0] + ox) * ny * nz + (cc[1] + oy) * nz + cc[2];
+        const long long f0 = fc + ox * sx + oy * nz;
         const long long lo = f0 - 1 > 0 ? f0 - 1 : 0;
         const long long hi = f0 + 1 < G - 1 ? f0 + 1 : G - 1;
-        if (lo <= hi) { jb_l = cs[lo]; je_l = cs[hi + 1]; }
+        bool any = lo <= hi;
+        if (any && want_flow && cell_flow) {
+            any = false;
+            for (long long f = lo; f <= hi; ++f) any = any || cell_flow[f];
+        }
+        if (any) { jb_l = cs[lo]; je_l = cs[hi + 1]; }
     }
     int m = 0;
-    for (int q = 0; q < NR; ++q) {
-        const int jb = __shfl_sync(0xffffffffu, jb_l, q), je = __shfl_sync(0xffffffffu, je_l, q);
-        for (int b = jb; b < je; b += 32) {
-            const int j = b + lane;
-            bool in = false, flow = false;
-            if (j < je && j != i) {
-                const float4 pj = P32[j];
-                flow = pj.w != 0.f;
-                if (flow || !want_flow) {
-                    bool exact = !pf;
-                    if (pf) {
-                        const float fx = pi.x - pj.x, fy = pi.y - pj.y, fz = pi.z - pj.z;
-                        float r2f = fx * fx + fy * fy;
-                        if (DIM == 3) r2f += fz * fz;
-                        in = r2f < c.pf_in2;
-                        exact = !in && !(r2f > c.pf_r2);
-                    }
-                    if (exact) {
-                        const double rx = xi[0] - X[j], ry = xi[1] - X[n + j];
-                        double r2 = rx * rx + ry * ry;
-                        if (DIM == 3) { const double rz = xi[2] - X[2 * n + j]; r2 = r2 + rz * rz; }
-                        in = r2 < c.R2T;
+    if (__any_sync(0xffffffffu, jb_l < je_l)) {
+        const float4 pi = P32[i];
+        const bool pf = c.pf_on && fabsf(pi.x) < c.pf_lim && fabsf(pi.y) < c.pf_lim && fabsf(pi.z) < c.pf_lim;
+        for (int q = 0; q < NR; ++q) {
+            const int jb = __shfl_sync(0xffffffffu, jb_l, q), je = __shfl_sync(0xffffffffu, je_l, q);
+            for (int b = jb; b < je; b += 32) {
+                const int j = b + lane;
+                bool in = false, flow = false;
+                if (j < je && j != i) {
+                    const float4 pj = P32[j];
+                    flow = pj.w != 0.f;
+                    if (flow || !want_flow) {
+                        bool exact = !pf;
+                        if (pf) {
+                            float fx = pi.x - pj.x, fy = pi.y - pj.y, fz = pi.z - pj.z;
+                            float r2f = fx * fx + fy * fy;
+                            if (DIM == 3) r2f += fz * fz;
+                            in = r2f < c.pf_in2;
+                            if (!in && !(r2f > c.pf_r2)) {
+                                const float4 li = P32L[i], lj = P32L[j];
+                                fx += li.x - lj.x;
+                                fy += li.y - lj.y;
+                                r2f = fx * fx + fy * fy;
+                                if (DIM == 3) { fz += li.z - lj.z; r2f += fz * fz; }
+                                in = r2f < c.pf_lo2;
+                                exact = !in && !(r2f > c.pf_hi2);
+                            }
+                        }
+                        if (exact) {
+                            const double rx = X[i] - X[j], ry = X[n + i] - X[n + j];
+                            double r2 = rx * rx + ry * ry;
+                            if (DIM == 3) { const double rz = X[2 * n + i] - X[2 * n + j]; r2 = r2 + rz * rz; }
+                            in = r2 < c.R2T;
+                        }
                     }
                 }
+                const unsigned bal = __ballot_sync(0xffffffffu, in);
+                const int pos = m + __popc(bal & ((1u << lane) - 1u));
+                if (in && pos < cap) out[pos] = flow ? j : j | NB_BDY;
+                m += __popc(bal);
             }
-            const unsigned bal = __ballot_sync(0xffffffffu, in);
-            const int pos = m + __popc(bal & ((1u << lane) - 1u));
-            if (in && pos < cap) out[pos] = flow ? j : j | NB_BDY;
-            m += __popc(bal);
         }
     }
     if (lane == 0) pr.cnt[row] = m;
+}
+
+// f32 coordinates of a position: high part (w: flow flag) and what it rounds off.
+__device__ __forceinline__ void write_pos32(const Consts& c, const double* x, bool flow, float4* hi, float4* lo) {
+    double d[3];
+    float h[3];
+    for (int q = 0; q < 3; ++q) { d[q] = x[q] - c.vs[q]; h[q] = (float)d[q]; }
+    *hi = make_float4(h[0], h[1], h[2], flow ? 1.f : 0.f);
+    *lo = make_float4((float)(d[0] - h[0]), (float)(d[1] - h[1]), (float)(d[2] - h[2]), 0.f);
+}
+
+// Flattened cell index (truncating cast, eng/particle_system.py:216-226), unclipped; kNoCell
+// where a coordinate leaves the int range or is not finite.
+__device__ __forceinline__ long long flat_cell(const Consts& c, const double* x) {
+    long long idx[3];
+    for (int d = 0; d < 3; ++d) {
+        const double t = (x[d] - c.vs[d]) / c.grid;
+        if (!(fabs(t) < 2147483647.0)) return kNoCell;
+        idx[d] = (long long)(int)t;
+    }
+    return idx[0] * c.gnum[1] * c.gnum[2] + idx[1] * c.gnum[2] + idx[2];
 }
 
 // The ordered sums of one row's C pair terms by its G lanes; acc[m] of lane g is component

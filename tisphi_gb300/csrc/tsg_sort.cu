@@ -18,6 +18,7 @@
 
 #include "tsg_cellsort.cuh"
 #include "tsg_internal.h"
+#include "tsg_pairs64.cuh"
 
 namespace tsg {
 
@@ -26,20 +27,17 @@ namespace {
 constexpr int TPB = 256;
 
 __global__ void k_hash(Consts c, const double* __restrict__ x, int* __restrict__ cell_of,
-                       int* __restrict__ rank, int* __restrict__ count, int* __restrict__ err) {
+                       int* __restrict__ rank, int* __restrict__ count, long long* __restrict__ cell0,
+                       int* __restrict__ err) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
-    long long idx[3];
-    bool ok = true;
-    for (int d = 0; d < 3; ++d) {
-        double t = (x[(size_t)d * c.n + i] - c.vs[d]) / c.grid;
-        if (!(fabs(t) < 2147483647.0)) { ok = false; idx[d] = 0; }
-        else idx[d] = (long long)(int)t;
-    }
-    long long f = idx[0] * c.gnum[1] * c.gnum[2] + idx[1] * c.gnum[2] + idx[2];
-    if (!ok || f < 0 || f >= c.G) {
+    double xi[3];
+    for (int d = 0; d < 3; ++d) xi[d] = x[(size_t)d * c.n + i];
+    long long f = flat_cell(c, xi);
+    cell0[i] = f;
+    if (f < 0 || f >= c.G) {
+        atomicOr(err, f != kNoCell ? TSG_ERR_CELL_OOB : (TSG_ERR_CELL_OOB | TSG_ERR_NONFINITE));
         f = c.G;
-        atomicOr(err, ok ? TSG_ERR_CELL_OOB : (TSG_ERR_CELL_OOB | TSG_ERR_NONFINITE));
     }
     cell_of[i] = (int)f;
     rank[i] = atomicAdd(&count[f], 1);
@@ -146,7 +144,9 @@ __device__ __forceinline__ void append(int* list, int* counter, bool pred, int v
 // array-of-structs sort moves it with the particle.
 template <bool SOIL>
 __global__ void k_reorder64(Consts c, const int* __restrict__ perm, Persist64 a, Persist64 b,
-                            float4* __restrict__ pos32, int* __restrict__ list_flow,
+                            float4* __restrict__ pos32, float4* __restrict__ pos32l,
+                            const long long* __restrict__ cell_src, long long* __restrict__ cell0,
+                            unsigned char* __restrict__ cell_flow, int* __restrict__ list_flow,
                             int* __restrict__ list_bdy, int* __restrict__ list_count,
                             const double* __restrict__ vt_src, double* __restrict__ vt_dst) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -180,8 +180,11 @@ __global__ void k_reorder64(Consts c, const int* __restrict__ perm, Persist64 a,
         b.id0[k] = a.id0[s];
         if (vt_src)
             for (int d = 0; d < 3; ++d) vt_dst[d * n + k] = vt_src[d * n + s];
-        pos32[k] = make_float4((float)(xv[0] - c.vs[0]), (float)(xv[1] - c.vs[1]), (float)(xv[2] - c.vs[2]),
-                               mt == MAT_FLUID || mt == MAT_SOIL ? 1.f : 0.f);
+        const bool flow = mt == MAT_FLUID || mt == MAT_SOIL;
+        write_pos32(c, xv, flow, pos32 + k, pos32l + k);
+        const long long f = cell_src[s];
+        cell0[k] = f;
+        if (flow && f >= 0 && f < c.G) cell_flow[f] = 1;
     }
     append(list_flow, list_count + 0, live && mt == c.flow_type, k);
     append(list_bdy, list_count + 1, live && (mt == MAT_DUMMY || mt == MAT_REP || mt == MAT_RIGID), k);
@@ -203,13 +206,14 @@ void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid
     const long long nbins = c.G + 1;
     cudaMemsetAsync(g.count, 0, sizeof(int) * nbins, s);
     cudaMemsetAsync(g.list_count, 0, sizeof(int) * 2, s);
-    TSG_LAUNCH(k_hash, nblk(c.n), TPB, s, c, cur.x, g.cell_of, g.rank, g.count, g.err);
+    cudaMemsetAsync(g.cell_flow, 0, (size_t)c.G, s);
+    TSG_LAUNCH(k_hash, nblk(c.n), TPB, s, c, cur.x, g.cell_of, g.rank, g.count, g.cell0_old, g.err);
     scan_exclusive(g.count, g.cell_start, (int)nbins, g.tile_sum, s);
     TSG_LAUNCH(k_scatter, nblk(c.n), TPB, s, c.n, g.cell_of, g.rank, g.cell_start, g.perm);
     sort_within_cells(nbins, g.cell_start, g.cell_of, c.n, g.perm, g.big, g.nbig, s);
     if (c.solver == 1) {
-        TSG_LAUNCH(k_reorder64<false>, nblk(c.n), TPB, s, c, g.perm, cur, nxt, t.pos32, g.list_flow, g.list_bdy,
-                   g.list_count, nullptr, nullptr);
+        TSG_LAUNCH(k_reorder64<false>, nblk(c.n), TPB, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell0_old,
+                   t.cell0, g.cell_flow, g.list_flow, g.list_bdy, g.list_count, nullptr, nullptr);
     } else {
         // mu(I) keeps v_tmp across steps: stage it in aux3 (free until advect_pos) and gather
         const double* src = nullptr;
@@ -217,8 +221,8 @@ void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid
             cudaMemcpyAsync(t.aux3, t.v_tmp, sizeof(double) * 3 * (size_t)c.n, cudaMemcpyDeviceToDevice, s);
             src = t.aux3;
         }
-        TSG_LAUNCH(k_reorder64<true>, nblk(c.n), TPB, s, c, g.perm, cur, nxt, t.pos32, g.list_flow, g.list_bdy,
-                   g.list_count, src, src ? t.v_tmp : nullptr);
+        TSG_LAUNCH(k_reorder64<true>, nblk(c.n), TPB, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell0_old,
+                   t.cell0, g.cell_flow, g.list_flow, g.list_bdy, g.list_count, src, src ? t.v_tmp : nullptr);
     }
     Persist64 tmp = cur;
     cur = nxt;
