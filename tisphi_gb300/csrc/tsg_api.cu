@@ -132,7 +132,7 @@ int alloc_rows(tsg_handle* h) {
     const int cf = row_capacity(c);
     const int cap_f = (cf + 7) / 8 * 8, cap_b = ((cf * 6) / 10 + 7) / 8 * 8;
     const size_t sf = (size_t)c.n_flow * cap_f, sb = (size_t)c.n_bdy * cap_b;
-    const int planes = c.dim + (c.solver == 1 ? 1 : 0);
+    const int planes = c.dim + (c.solver == 1 ? 2 : 0);
     size_t free_b = 0, total_b = 0;
     if (cf <= 0 || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     const size_t bytes = sf * (4 + 8 * (size_t)planes) + sb * 12 + 4 * (size_t)h->n;
@@ -367,6 +367,8 @@ int tsg_create(const tsg_config* cfg, tsg_handle** out) {
     c.pf_r2 = std::nextafter((float)(c.R * c.R * (1.0 + 1.0 / 1024.0)), 1e30f);
     c.pf_lim = (float)(500.0 * c.R);
     c.pf_in2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 1024.0)), 0.f);
+    // div_by: divisors |r| in (EPS, R) and |r|^2 + eps_h2 stay within 2^+-200 of 1
+    c.div_span = c.R < 0x1p100 && c.eps_h2 > 0x1p-200 ? 1000u << 20 : 0u;
     c.pf_lo2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 262144.0)), 0.f);
     c.pf_hi2 = std::nextafter((float)(c.R * c.R * (1.0 + 1.0 / 262144.0)), 1e30f);
     c.R2T = c.R * c.R;

@@ -45,8 +45,8 @@ __device__ __forceinline__ double kernel_W(const Consts& c, double rn) {
     double q = rn * c.h1;
     if (rn > EPS && q <= 2.0) {
         if (c.kernel == 1) {
-            double q1 = 1.0 - 0.5 * q;
-            res = c.kk * ((q1 * q1) * (q1 * q1)) * (1.0 + 2.0 * q);
+            double q1 = __fma_rn(-0.5, q, 1.0);  // 0.5 q and 2 q are exact: one rounding either way
+            res = c.kk * ((q1 * q1) * (q1 * q1)) * __fma_rn(2.0, q, 1.0);
         } else if (q <= 1.0) {
             double q2 = q * q, q3 = q2 * q;
             res = c.kk * (0.5 * q3 - q2 + 2.0 / 3.0);
@@ -63,15 +63,16 @@ __device__ __forceinline__ void kernel_dW(const Consts& c, const double* r, doub
     out[0] = out[1] = out[2] = 0.0;
     double q = rn * c.h1;
     if (rn > EPS && q <= 2.0) {
+        const double y = __drcp_rn(rn);
         if (c.kernel == 1) {
-            double q1 = 1.0 - 0.5 * q;
+            double q1 = __fma_rn(-0.5, q, 1.0);
             double s = c.kk * ((q1 * q1) * q1) * (-5.0 * q) * c.h1;
-            for (int d = 0; d < DIM; ++d) out[d] = s * r[d] / rn;
+            for (int d = 0; d < DIM; ++d) out[d] = div_by(s * r[d], rn, y, c.div_span);
         } else {
             double s;
             if (q <= 1.0) s = c.kk * q * (1.5 * q - 2.0);
             else { double f = 2.0 - q; s = c.kk * (-0.5 * f * f); }
-            for (int d = 0; d < DIM; ++d) out[d] = s * (r[d] / rn * c.h1);
+            for (int d = 0; d < DIM; ++d) out[d] = s * (div_by(r[d], rn, y, c.div_span) * c.h1);
         }
     }
 }
@@ -179,7 +180,10 @@ __device__ __forceinline__ double pair_geometry(const Consts& c, const double* _
     const double rn = sqrt(r2);
     kernel_dW<DIM>(c, r, rn, kd);
     for (int d = 0; d < DIM; ++d) pr.gk[d * pr.slots_f + slot] = kd[d];
-    if (pr.gden) pr.gden[slot] = rn * rn + c.eps_h2;
+    if (pr.gden) {
+        const double den = rn * rn + c.eps_h2;
+        pr.gden[slot] = make_double2(den, __drcp_rn(den));
+    }
     return rn;
 }
 
@@ -608,11 +612,19 @@ __device__ __forceinline__ void wc_force_pair(const Consts& c, int tj, double mV
 }
 
 // One neighbour's WCSPH terms: continuity, then the acceleration (DIM), from the neighbour's
-// record (v~, P = p / rho~^2, m_V, viscosity factor, -rho0 m_V) and the pair geometry.
+// record (v~, P = p / rho~^2, m_V, viscosity factor, -rho0 m_V) and the pair geometry
+// (den.y = 1 / den.x).
+struct Divisor {  // a divisor with its reciprocal; span 0 where div_by's window does not hold
+    double b, y;
+    unsigned span;
+    __device__ __forceinline__ Divisor(const Consts& c, double v) : b(v), y(1.0 / v) {
+        span = (unsigned)__double2hiint(v) - (923u << 20) < 200u << 20 ? c.div_span : 0u;
+    }
+};
 template <int DIM>
 __device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const double* v, double P, double mV, double cvj,
-                                         double cC, const double* vti, double rti, double pri, const double* L,
-                                         const double* r, double den, const double* kd, double* T) {
+                                         double cC, const double* vti, const Divisor& rti, double pri, const double* L,
+                                         const double* r, double2 den, const double* kd, double* T) {
     double dvv[3], a[3];
     for (int d = 0; d < DIM; ++d) { dvv[d] = vti[d] - v[d]; a[d] = mV * dvv[d]; }
     if (c.corr == 1) {
@@ -622,10 +634,10 @@ __device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const doub
     } else {
         T[0] = dotv<DIM>(a, kd);
     }
-    const double mn = fmin(dotv<DIM>(dvv, r), 0.0);
+    const double mn = min0(dotv<DIM>(dvv, r));
     double cv = cvj;
-    if (!fluid) cv = cv / rti;
-    cv = cv * mn / den;
+    if (!fluid) cv = div_by(cv, rti.b, rti.y, rti.span);
+    cv = div_by(cv * mn, den.x, den.y, c.div_span);
     const double cp = cC * (pri + P);
     for (int d = 0; d < DIM; ++d) T[1 + d] = cv * kd[d] + cp * kd[d];
 }
@@ -642,7 +654,8 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
         double xi[3], vti[3], L[9];
         load_x<DIM>(p.x, q.i, n, xi);
         for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + q.i];
-        const double rti = t.density_tmp[q.i], pri = pr.rec[(size_t)8 * q.i + 3];
+        const Divisor rti(c, t.density_tmp[q.i]);
+        const double pri = pr.rec[(size_t)8 * q.i + 3];
         if (c.corr == 1)
             for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
@@ -662,7 +675,7 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
     const int row = blockIdx.x * ROWS + threadIdx.x;
     if (threadIdx.x >= ROWS || row >= count) return;
     const int i = list[row];
-    const double rti = t.density_tmp[i];
+    const Divisor rti(c, t.density_tmp[i]);
     double A[C];
     const bool listed = pr.cap_f && pr.cnt[row] <= pr.cap_f;
     const bool rep = c.boundary == 3 || c.boundary == 4;
@@ -681,8 +694,9 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
             const double* rj = pr.rec + (size_t)8 * j;
             double kd[3], T[C];
             kernel_dW<DIM>(c, r, rn, kd);
+            const double den = rn * rn + c.eps_h2;
             wc_terms<DIM>(c, p.mat_type[j] == MAT_FLUID, rj, rj[3], rj[4], rj[5], rj[6], vti, rti, pri, L, r,
-                          rn * rn + c.eps_h2, kd, T);
+                          make_double2(den, __drcp_rn(den)), kd, T);
             for (int q = 0; q < C; ++q) A[q] += T[q];
         });
     }
@@ -691,7 +705,7 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
             if (p.mat_type[j] == MAT_REP) rep_force<DIM>(c, r, rn, A + 1);
         });
     }
-    t.d_density[i] = A[0] * rti;
+    t.d_density[i] = A[0] * rti.b;
     for (int d = 0; d < DIM; ++d) t.d_vel[(size_t)d * n + i] = A[1 + d] + c.g[d];
     if (DIM == 2) t.d_vel[2 * (size_t)n + i] = 0.0 + c.g[2];
 }
@@ -1578,21 +1592,26 @@ static void rigid_lists64(const Consts& c, const Persist64& p, const Rigid64& r,
         else TSG_LAUNCH(KERNEL<3>, GRID, TPB, s, __VA_ARGS__);                    \
     } while (0)
 
-// Lanes per row of the pair loops.
-constexpr int LANES = 8;
+// Lanes per row: about as many as a loop has sums (2 to 5 in most), so that the additions in
+// slot order cost what one thread's would; the Drucker-Prager loop has 7 (2D) or 13 sums and a
+// long epilogue, and wants the threads.  us per launch with 8 -> 4 lanes: 3D rates (118 k rows)
+// 1,915 -> 1,834, correction 2,141 -> 2,055; 2D mu(I) (20 k rows) correction 81 -> 66, stress
+// 56 -> 47, momentum 49 -> 40; 2D rates (7 k rows) 42 -> 36; Drucker-Prager 90 -> 101.
+constexpr int LANES = 4, LANES_DP = 8;
 inline int nrows(int count) { return (count + ROWS - 1) / ROWS; }
 // Threads of a row kernel: without rows only the epilogue's threads have work.
-inline int row_threads(const Grid& g) { return g.pr.cap_f ? ROWS * LANES : ROWS; }
+inline int row_threads(const Grid& g, int lanes) { return g.pr.cap_f ? ROWS * lanes : ROWS; }
 
-#define DISPATCH_ROWS(c, g, KERNEL, COUNT, ...)                                                            \
-    do {                                                                                                   \
-        if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LANES>), nrows(COUNT), row_threads(g), s, __VA_ARGS__);    \
-        else TSG_LAUNCH((KERNEL<3, LANES>), nrows(COUNT), row_threads(g), s, __VA_ARGS__);                 \
+#define DISPATCH_LANES(c, g, KERNEL, LN, COUNT, ...)                                                          \
+    do {                                                                                                      \
+        if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LN>), nrows(COUNT), row_threads(g, LN), s, __VA_ARGS__);      \
+        else TSG_LAUNCH((KERNEL<3, LN>), nrows(COUNT), row_threads(g, LN), s, __VA_ARGS__);                   \
     } while (0)
-#define DISPATCH_ROWS_B(c, g, KERNEL, FLAG, COUNT, ...)                                                          \
-    do {                                                                                                         \
-        if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LANES, FLAG>), nrows(COUNT), row_threads(g), s, __VA_ARGS__);    \
-        else TSG_LAUNCH((KERNEL<3, LANES, FLAG>), nrows(COUNT), row_threads(g), s, __VA_ARGS__);                 \
+#define DISPATCH_ROWS(c, g, KERNEL, COUNT, ...) DISPATCH_LANES(c, g, KERNEL, LANES, COUNT, __VA_ARGS__)
+#define DISPATCH_ROWS_B(c, g, KERNEL, FLAG, COUNT, ...)                                                                 \
+    do {                                                                                                                \
+        if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LANES, FLAG>), nrows(COUNT), row_threads(g, LANES), s, __VA_ARGS__);    \
+        else TSG_LAUNCH((KERNEL<3, LANES, FLAG>), nrows(COUNT), row_threads(g, LANES), s, __VA_ARGS__);                 \
     } while (0)
 
 static void build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, bool flow_only,
@@ -1678,7 +1697,7 @@ void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cud
         PhaseScope ph(s, PH_RATES);
         if (c.solver == 1) DISPATCH_ROWS(c, g, k_wc_rates, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
         else if (c.solver == 2) DISPATCH_ROWS(c, g, k_mui_mom, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
-        else DISPATCH_ROWS(c, g, k_dp_rates, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+        else DISPATCH_LANES(c, g, k_dp_rates, LANES_DP, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
     }
     if (c.n_rigid_dyn > 0 && c.n_bdy > 0) {  // the flow's reaction on dynamic rigid particles
         PhaseScope ph(s, PH_RATES);

@@ -55,6 +55,7 @@ struct Consts {
     float pf_r2, pf_lim;
     float pf_in2;       // below this f32 distance^2 a pair is certainly a neighbour
     float pf_lo2, pf_hi2;  // the same two bounds for the distance^2 with the low parts added
+    unsigned div_span;  // exponent window of div_by (0 closes it)
     double R2T;         // r2 < R2T exactly when sqrt(r2) < R
     int n_rigid_dyn;    // dynamic rigid particles (shape-matched bodies)
 };
@@ -137,7 +138,7 @@ struct Pairs64 {
     int* nb_f;          // entries: particle index, sign bit set for a non-flow neighbour
     int* nb_b;
     double* gk;         // dim planes: kernel gradient of each flow entry
-    double* gden;       // |r|^2 + 0.01 h^2 of each flow entry (WCSPH)
+    double2* gden;      // |r|^2 + 0.01 h^2 of each flow entry and its reciprocal (WCSPH)
     double* gw;         // kernel value of each boundary entry
     double* rec;        // rec_stride doubles per particle: what the rates loop reads of a neighbour
     int rec_stride;

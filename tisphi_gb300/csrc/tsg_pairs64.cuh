@@ -17,8 +17,8 @@
 // G lanes share a row: lane g evaluates the pair terms of slots g, g + G, ..., the terms of a
 // trip go through shared memory, and lane c adds component c of them in slot order.  The sums
 // therefore round exactly as one thread adding them in traversal order (a missing slot adds
-// +0.0, which changes no sum that starts at +0.0), C chains of additions cost one lane group
-// G additions instead of C x G, and small scenes get G times the threads.
+// +0.0, which changes no sum that starts at +0.0), C chains of additions cost the lanes
+// of a row about G additions instead of C x G, and small scenes get G times the threads.
 #pragma once
 
 #include "tsg_internal.h"
@@ -122,6 +122,29 @@ __global__ void __launch_bounds__(256) k_list64(Consts c, const double* __restri
         }
     }
     if (lane == 0) pr.cnt[row] = m;
+}
+
+// a / b, correctly rounded, from y = RN(1 / b): one product and two fused multiply-adds instead
+// of the division's ten-odd FP64 instructions (Markstein 1990; Brisebarre, Muller and Raina,
+// "Accelerating correctly rounded floating-point division when the divisor is known in
+// advance", 2004).  The residual must not underflow nor the quotient leave the normal range:
+// b is a caller's positive divisor within 2^+-200 of 1, and |a| outside [2^-500, 2^500) takes
+// the division, except +-0, whose quotient is itself.
+__device__ __forceinline__ double div_by(double a, double b, double y, unsigned span) {
+    const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    if (hi - (523u << 20) < span) {
+        const double q = a * y;
+        return __fma_rn(__fma_rn(-b, q, a), y, q);
+    }
+    if ((hi | (unsigned)__double2loint(a)) == 0u) return a;
+    return a / b;
+}
+
+// fmin(x, 0.0) without an FP64 comparison: x where its sign is set (and it is no NaN), else 0.
+__device__ __forceinline__ double min0(double x) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const bool keep = hi < 0 && ((unsigned)hi < 0xfff00000u || ((unsigned)hi == 0xfff00000u && lo == 0));
+    return keep ? x : 0.0;
 }
 
 // f32 coordinates of a position: high part (w: flow flag) and what it rounds off.
