@@ -45,9 +45,10 @@ def _check(d, oracle_lib, names, steps):
 
 SCENES = {
     "wc2d_cspm_xsph": lambda: (small_dambreak_2d(corr=1, xsph=True), WC),
-    "wc2d_rk4_cubic": lambda: (small_dambreak_2d(integration=4, kernel=0), WC),
+    "wc2d_rk4_cubic_cspm": lambda: (small_dambreak_2d(integration=4, kernel=0, corr=1), WC),
     "wc3d_cspm": lambda: (small_dambreak_3d(corr=1, spacing=0.025), WC),
-    "mui": lambda: (small_column(2, corr=1), SOIL),
+    "mui_cspm": lambda: (small_column(2, corr=1), SOIL),
+    "mui_lf_cspm": lambda: (small_column(2, integration=2, corr=1), SOIL),
     "dp_lf_xsph": lambda: (small_column(3, integration=2, xsph=True), SOIL),
 }
 

@@ -132,7 +132,8 @@ int alloc_rows(tsg_handle* h) {
     const int cf = row_capacity(c);
     const int cap_f = (cf + 7) / 8 * 8, cap_b = ((cf * 6) / 10 + 7) / 8 * 8;
     const size_t sf = (size_t)c.n_flow * cap_f, sb = (size_t)c.n_bdy * cap_b;
-    const int planes = c.dim + (c.solver == 1 ? 2 : 0);
+    const bool own_gc = c.solver == 1 && c.corr == 1;
+    const int planes = c.dim + (c.solver == 1 ? 2 : 0) + (own_gc ? c.dim : 0);
     size_t free_b = 0, total_b = 0;
     if (cf <= 0 || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     const size_t bytes = sf * (4 + 8 * (size_t)planes) + sb * 12 + 4 * (size_t)h->n;
@@ -146,7 +147,9 @@ int alloc_rows(tsg_handle* h) {
     };
     r.slots_f = sf;
     if (take(&r.cnt, (size_t)c.n_flow + c.n_bdy) && take(&r.nb_f, sf) && take(&r.nb_b, sb) &&
-        take(&r.gk, sf * c.dim) && take(&r.gw, sb) && (c.solver != 1 || take(&r.gden, sf))) {
+        take(&r.gk, sf * c.dim) && take(&r.gw, sb) && (c.solver != 1 || take(&r.gden, sf)) &&
+        (!own_gc || take(&r.gc, sf * c.dim))) {
+        if (!own_gc) r.gc = r.gk;
         r.cap_f = cap_f;
         r.cap_b = cap_b;
     }
@@ -239,7 +242,11 @@ void own_rows(tsg_handle* h, bool geometry, cudaStream_t s) {
 
 // substep of the FP64 form on the current rows and geometry.
 int substep64(tsg_handle* h, cudaStream_t s) {
-    auto rates = [&] { fp64_one_step(h->c, h->cur, h->t, h->g, s); };
+    int stage = h->c.ti == 1 ? -1 : 0;
+    auto rates = [&] {
+        fp64_one_step(h->c, h->cur, h->t, h->g, stage, s);
+        if (stage >= 0) ++stage;
+    };
     auto adv = [&](int which) { fp64_advect(h->c, h->cur, h->t, h->g, which, s); };
     switch (h->c.ti) {
     case 1: rates(); adv(TSG_ADVECT_FULL); break;
@@ -533,7 +540,7 @@ int tsg_one_step(tsg_handle* h, void* stream) {
     if (!h || !h->sorted) return TSG_E_STATE;
     cudaStream_t s = S(stream);
     if (use_fp32(h)) fp32_one_step(*h->f32, s);
-    else { own_rows(h, true, s); fp64_one_step(h->c, h->cur, h->t, h->g, s); }
+    else { own_rows(h, true, s); fp64_one_step(h->c, h->cur, h->t, h->g, -1, s); }
     return check_cuda();
 }
 

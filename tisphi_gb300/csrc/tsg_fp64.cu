@@ -611,6 +611,29 @@ __device__ __forceinline__ void wc_force_pair(const Consts& c, int tj, double mV
     }
 }
 
+// The corrected gradient L_i grad W of a pair is the same in every loop of a step.  KC_MAKE
+// forms it, KC_KEEP also stores it in the row, KC_READ reads it back (3D WCSPH: 15 of a pair's
+// 57 FP64 operations for 24 bytes of stream).
+enum { KC_MAKE = 0, KC_KEEP = 1, KC_READ = 2 };
+template <int DIM>
+__device__ __forceinline__ void corrected(const Consts& c, const double* L, const double* kd, double* kc) {
+    if (c.corr == 1) matvec_corr<DIM>(L, kd, kc);
+    else { kc[0] = kd[0]; kc[1] = kd[1]; kc[2] = kd[2]; }
+}
+template <int DIM, int KC>
+__device__ __forceinline__ void row_gradient(const Consts& c, const Pairs64& pr, size_t slot, const double* L,
+                                             double* kc) {
+    if (KC == KC_READ) {
+        for (int d = 0; d < DIM; ++d) kc[d] = pr.gc[d * pr.slots_f + slot];
+        return;
+    }
+    double kd[3] = {0.0, 0.0, 0.0};
+    for (int d = 0; d < DIM; ++d) kd[d] = pr.gk[d * pr.slots_f + slot];
+    corrected<DIM>(c, L, kd, kc);
+    if (KC == KC_KEEP)
+        for (int d = 0; d < DIM; ++d) pr.gc[d * pr.slots_f + slot] = kc[d];
+}
+
 // One neighbour's WCSPH terms: continuity, then the acceleration (DIM), from the neighbour's
 // record (v~, P = p / rho~^2, m_V, viscosity factor, -rho0 m_V) and the pair geometry
 // (den.y = 1 / den.x).
@@ -623,17 +646,11 @@ struct Divisor {  // a divisor with its reciprocal; span 0 where div_by's window
 };
 template <int DIM>
 __device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const double* v, double P, double mV, double cvj,
-                                         double cC, const double* vti, const Divisor& rti, double pri, const double* L,
-                                         const double* r, double2 den, const double* kd, double* T) {
+                                         double cC, const double* vti, const Divisor& rti, double pri, const double* r,
+                                         double2 den, const double* kd, const double* kc, double* T) {
     double dvv[3], a[3];
     for (int d = 0; d < DIM; ++d) { dvv[d] = vti[d] - v[d]; a[d] = mV * dvv[d]; }
-    if (c.corr == 1) {
-        double kc[3];
-        matvec_corr<DIM>(L, kd, kc);
-        T[0] = dotv<DIM>(a, kc);
-    } else {
-        T[0] = dotv<DIM>(a, kd);
-    }
+    T[0] = dotv<DIM>(a, kc);
     const double mn = min0(dotv<DIM>(dvv, r));
     double cv = cvj;
     if (!fluid) cv = div_by(cv, rti.b, rti.y, rti.span);
@@ -643,7 +660,7 @@ __device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const doub
 }
 
 // ---- WCSPH rates (eng/solver_sph_wc.py:108-126) ----
-template <int DIM, int G>
+template <int DIM, int G, int KC>
 __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
                                                        const int* __restrict__ list, int count, Pairs64 pr) {
     constexpr int C = 1 + DIM;
@@ -656,20 +673,21 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
         for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + q.i];
         const Divisor rti(c, t.density_tmp[q.i]);
         const double pri = pr.rec[(size_t)8 * q.i + 3];
-        if (c.corr == 1)
+        if (c.corr == 1 && KC != KC_READ)
             for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
             const int ent = pr.nb_f[slot], j = nb_index(ent);
             const double2* rj = reinterpret_cast<const double2*>(pr.rec + (size_t)8 * j);
             const double2 r0 = rj[0], r1 = rj[1], r2 = rj[2], r3 = rj[3];
-            double r[3] = {0.0, 0.0, 0.0}, kd[3] = {0.0, 0.0, 0.0};
+            double r[3] = {0.0, 0.0, 0.0}, kd[3] = {0.0, 0.0, 0.0}, kc[3];
             for (int d = 0; d < DIM; ++d) {
                 r[d] = xi[d] - p.x[(size_t)d * n + j];
                 kd[d] = pr.gk[d * pr.slots_f + slot];
             }
+            row_gradient<DIM, KC>(c, pr, slot, L, kc);
             const double v[3] = {r0.x, r0.y, r1.x};
-            wc_terms<DIM>(c, nb_flow(ent), v, r1.y, r2.x, r2.y, r3.x, vti, rti, pri, L, r, pr.gden[slot], kd, T);
+            wc_terms<DIM>(c, nb_flow(ent), v, r1.y, r2.x, r2.y, r3.x, vti, rti, pri, r, pr.gden[slot], kd, kc, T);
         });
     }
     const int row = blockIdx.x * ROWS + threadIdx.x;
@@ -692,11 +710,12 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
         for (int q = 0; q < C; ++q) A[q] = 0.0;
         for_neighbors<DIM>(c, p.x, t.pos32, cs, i, xi, true, [&](int j, const double* r, double rn) {
             const double* rj = pr.rec + (size_t)8 * j;
-            double kd[3], T[C];
+            double kd[3], kc[3], T[C];
             kernel_dW<DIM>(c, r, rn, kd);
+            corrected<DIM>(c, L, kd, kc);
             const double den = rn * rn + c.eps_h2;
-            wc_terms<DIM>(c, p.mat_type[j] == MAT_FLUID, rj, rj[3], rj[4], rj[5], rj[6], vti, rti, pri, L, r,
-                          make_double2(den, __drcp_rn(den)), kd, T);
+            wc_terms<DIM>(c, p.mat_type[j] == MAT_FLUID, rj, rj[3], rj[4], rj[5], rj[6], vti, rti, pri, r,
+                          make_double2(den, __drcp_rn(den)), kd, kc, T);
             for (int q = 0; q < C; ++q) A[q] += T[q];
         });
     }
@@ -730,15 +749,9 @@ __device__ __forceinline__ void vgrad_terms(const double* v, double mV, const do
     T[DIM * DIM] = -s;
 }
 
-template <int DIM>
-__device__ __forceinline__ void corrected(const Consts& c, const double* L, const double* kd, double* kc) {
-    if (c.corr == 1) matvec_corr<DIM>(L, kd, kc);
-    else { kc[0] = kd[0]; kc[1] = kd[1]; kc[2] = kd[2]; }
-}
-
 // mu(I) loop 1 (eng/solver_sph_muI.py:67-92): velocity gradient, continuity, pressure from
 // density (not density_tmp), mu(I) stress, equivalent strain rate.
-template <int DIM, int G>
+template <int DIM, int G, int KC>
 __global__ void __launch_bounds__(ROWS * G) k_mui_stress(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
                                                          const int* __restrict__ list, int count, Pairs64 pr) {
     constexpr int C = DIM * DIM + 1;
@@ -753,12 +766,9 @@ __global__ void __launch_bounds__(ROWS * G) k_mui_stress(Consts c, Persist64 p, 
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
             const int j = nb_index(pr.nb_f[slot]);
-            double kd[3] = {0.0, 0.0, 0.0}, kc[3], v[3];
-            for (int d = 0; d < DIM; ++d) {
-                kd[d] = pr.gk[d * pr.slots_f + slot];
-                v[d] = t.v_tmp[(size_t)d * n + j];
-            }
-            corrected<DIM>(c, L, kd, kc);
+            double kc[3], v[3];
+            for (int d = 0; d < DIM; ++d) v[d] = t.v_tmp[(size_t)d * n + j];
+            row_gradient<DIM, KC>(c, pr, slot, L, kc);
             vgrad_terms<DIM>(v, p.m_V[j], vti, kc, T);
         });
     }
@@ -862,7 +872,7 @@ struct SoilRec {
 // mu(I) loop 2 (eng/solver_sph_muI.py:113-128) and the whole Drucker-Prager loop
 // (eng/solver_sph_dp.py:236-270): stress divergence, and for Drucker-Prager the velocity
 // gradient and continuity in the same walk.  Component order: acceleration, gradient, continuity.
-template <int DIM, int G, bool DP>
+template <int DIM, int G, bool DP, int KC>
 __device__ __forceinline__ void soil_sums(const Consts& c, const Persist64& p, const Trans64& t,
                                           const int* __restrict__ cs, const int* __restrict__ list, int count,
                                           const Pairs64& pr, double (*S)[ROWS], double* A) {
@@ -877,9 +887,8 @@ __device__ __forceinline__ void soil_sums(const Consts& c, const Persist64& p, c
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
             const int j = nb_index(pr.nb_f[slot]);
-            double kd[3] = {0.0, 0.0, 0.0}, kc[3];
-            for (int d = 0; d < DIM; ++d) kd[d] = pr.gk[d * pr.slots_f + slot];
-            corrected<DIM>(c, L, kd, kc);
+            double kc[3];
+            row_gradient<DIM, KC>(c, pr, slot, L, kc);
             const SoilRec<DIM> rj(pr.rec, j);
             stress_div_rec<DIM>(ri.S(), rj.S(), rj.sc(), kc, T);
             if (DP) vgrad_terms<DIM>(rj.v(), rj.mV(), ri.v(), kc, T + DIM);
@@ -916,12 +925,12 @@ __device__ __forceinline__ void soil_sums(const Consts& c, const Persist64& p, c
         });
 }
 
-template <int DIM, int G>
+template <int DIM, int G, int KC>
 __global__ void __launch_bounds__(ROWS * G) k_mui_mom(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
                                                       const int* __restrict__ list, int count, Pairs64 pr) {
     __shared__ double S[DIM][ROWS];
     double dv[3] = {0, 0, 0};
-    soil_sums<DIM, G, false>(c, p, t, cs, list, count, pr, S, dv);
+    soil_sums<DIM, G, false, KC>(c, p, t, cs, list, count, pr, S, dv);
     const int row = blockIdx.x * ROWS + threadIdx.x;
     if (threadIdx.x >= ROWS || row >= count) return;
     const int i = list[row];
@@ -933,13 +942,13 @@ __global__ void __launch_bounds__(ROWS * G) k_mui_mom(Consts c, Persist64 p, Tra
 }
 
 // ---- DP rates (eng/solver_sph_dp.py:236-270, Bui 2008 :172-208) ----
-template <int DIM, int G>
+template <int DIM, int G, int KC>
 __global__ void __launch_bounds__(ROWS * G) k_dp_rates(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
                                                        const int* __restrict__ list, int count, Pairs64 pr) {
     constexpr int C = DIM + DIM * DIM + 1;
     __shared__ double S[C][ROWS];
     double A[C];
-    soil_sums<DIM, G, true>(c, p, t, cs, list, count, pr, S, A);
+    soil_sums<DIM, G, true, KC>(c, p, t, cs, list, count, pr, S, A);
     const int row = blockIdx.x * ROWS + threadIdx.x;
     if (threadIdx.x >= ROWS || row >= count) return;
     const int i = list[row];
@@ -1608,6 +1617,17 @@ inline int row_threads(const Grid& g, int lanes) { return g.pr.cap_f ? ROWS * la
         else TSG_LAUNCH((KERNEL<3, LN>), nrows(COUNT), row_threads(g, LN), s, __VA_ARGS__);                   \
     } while (0)
 #define DISPATCH_ROWS(c, g, KERNEL, COUNT, ...) DISPATCH_LANES(c, g, KERNEL, LANES, COUNT, __VA_ARGS__)
+#define DISPATCH_KC(c, g, KERNEL, LN, KC, COUNT, ...)                                                            \
+    do {                                                                                                         \
+        if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LN, KC>), nrows(COUNT), row_threads(g, LN), s, __VA_ARGS__);     \
+        else TSG_LAUNCH((KERNEL<3, LN, KC>), nrows(COUNT), row_threads(g, LN), s, __VA_ARGS__);                  \
+    } while (0)
+#define DISPATCH_KC3(c, g, KERNEL, LN, MODE, COUNT, ...)                                                         \
+    do {                                                                                                         \
+        if ((MODE) == KC_READ) DISPATCH_KC(c, g, KERNEL, LN, KC_READ, COUNT, __VA_ARGS__);                       \
+        else if ((MODE) == KC_KEEP) DISPATCH_KC(c, g, KERNEL, LN, KC_KEEP, COUNT, __VA_ARGS__);                  \
+        else DISPATCH_KC(c, g, KERNEL, LN, KC_MAKE, COUNT, __VA_ARGS__);                                         \
+    } while (0)
 #define DISPATCH_ROWS_B(c, g, KERNEL, FLAG, COUNT, ...)                                                                 \
     do {                                                                                                                \
         if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LANES, FLAG>), nrows(COUNT), row_threads(g, LANES), s, __VA_ARGS__);    \
@@ -1677,14 +1697,17 @@ void fp64_init_tmp(const Consts& c, const Persist64& p, Trans64& t, cudaStream_t
     TSG_LAUNCH(k_init_tmp, nblk(c.n), TPB, s, c, p, t);
 }
 
-void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int stage, cudaStream_t s) {
+    // without the correction the gradient is grad W itself: nothing to keep
+    const int kc = c.corr != 1 || stage < 0 ? KC_MAKE : stage == 0 ? KC_KEEP : KC_READ;
     if (c.n_flow > 0 && (c.solver == 1 || c.solver == 3)) {
         PhaseScope ph(s, PH_PRE);
         TSG_LAUNCH(k_pre, nblk(c.n_flow), TPB, s, c, p, t, g.list_flow, c.n_flow, g.pr);
     }
     if (c.solver == 2 && c.n_flow > 0) {
         PhaseScope ph(s, PH_PRE);
-        DISPATCH_ROWS(c, g, k_mui_stress, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+        const int kc1 = c.corr == 1 && kc == KC_MAKE ? KC_KEEP : kc;  // the momentum loop reads it
+        DISPATCH_KC3(c, g, k_mui_stress, LANES, kc1, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
     }
     if (c.n_bdy > 0) {
         PhaseScope ph(s, PH_BDY);
@@ -1695,9 +1718,14 @@ void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cud
     }
     if (c.n_flow > 0) {
         PhaseScope ph(s, PH_RATES);
-        if (c.solver == 1) DISPATCH_ROWS(c, g, k_wc_rates, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
-        else if (c.solver == 2) DISPATCH_ROWS(c, g, k_mui_mom, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
-        else DISPATCH_LANES(c, g, k_dp_rates, LANES_DP, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+        if (c.solver == 1)
+            DISPATCH_KC3(c, g, k_wc_rates, LANES, kc, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+        else if (c.solver == 2 && c.corr == 1)
+            DISPATCH_KC(c, g, k_mui_mom, LANES, KC_READ, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+        else if (c.solver == 2)
+            DISPATCH_KC(c, g, k_mui_mom, LANES, KC_MAKE, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+        else
+            DISPATCH_KC3(c, g, k_dp_rates, LANES_DP, kc, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
     }
     if (c.n_rigid_dyn > 0 && c.n_bdy > 0) {  // the flow's reaction on dynamic rigid particles
         PhaseScope ph(s, PH_RATES);

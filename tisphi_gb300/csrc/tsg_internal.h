@@ -139,6 +139,8 @@ struct Pairs64 {
     int* nb_b;
     double* gk;         // dim planes: kernel gradient of each flow entry
     double2* gden;      // |r|^2 + 0.01 h^2 of each flow entry and its reciprocal (WCSPH)
+    double* gc;         // dim planes: corrected gradient L_i grad W of each flow entry (CSPM);
+                        // the soil solvers, which use no other gradient, keep it in gk
     double* gw;         // kernel value of each boundary entry
     double* rec;        // rec_stride doubles per particle: what the rates loop reads of a neighbour
     int rec_stride;
@@ -187,7 +189,9 @@ void fp64_build_rows(const Consts& c, const Persist64& p, const Trans64& t, cons
                      cudaStream_t s);
 void fp64_geometry(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
 void fp64_init_tmp(const Consts& c, const Persist64& p, Trans64& t, cudaStream_t s);
-void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
+// stage: how often this step's loops have run before (the first stores the corrected gradients
+// for the others); -1: a loop on its own.
+void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int stage, cudaStream_t s);
 void fp64_advect(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int which, cudaStream_t s);
 void fp64_rk_update(const Consts& c, Persist64& p, Trans64& t, int m, cudaStream_t s);
 void fp64_neighbors(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g,
