@@ -376,6 +376,7 @@ int tsg_create(const tsg_config* cfg, tsg_handle** out) {
     c.pf_in2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 1024.0)), 0.f);
     // div_by: divisors |r| in (EPS, R) and |r|^2 + eps_h2 stay within 2^+-200 of 1
     c.div_span = c.R < 0x1p100 && c.eps_h2 > 0x1p-200 ? 1000u << 20 : 0u;
+    c.wend_int = f.kernel == 1 && c.kk > 0x1p-100 && c.kk < 0x1p100 && c.h1 > 0x1p-100 && c.h1 < 0x1p100;
     c.pf_lo2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 262144.0)), 0.f);
     c.pf_hi2 = std::nextafter((float)(c.R * c.R * (1.0 + 1.0 / 262144.0)), 1e30f);
     c.R2T = c.R * c.R;

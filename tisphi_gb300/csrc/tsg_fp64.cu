@@ -77,21 +77,33 @@ __device__ __forceinline__ void kernel_dW(const Consts& c, const double* r, doub
     }
 }
 
-template <int DIM>
+template <int DIM, bool INT = false>
 __device__ __forceinline__ void matvec_corr(const double* L, const double* k, double* out) {
     for (int p = 0; p < DIM; ++p) {
-        double s = L[3 * p] * k[0] + L[3 * p + 1] * k[1];
-        if (DIM == 3) s = s + L[3 * p + 2] * k[2];
+        double s = mul<INT>(L[3 * p], k[0]) + mul<INT>(L[3 * p + 1], k[1]);
+        if (DIM == 3) s = s + mul<INT>(L[3 * p + 2], k[2]);
         out[p] = s;
     }
     if (DIM == 2) out[2] = 0.0;
 }
 
-template <int DIM>
+template <int DIM, bool INT = false>
 __device__ __forceinline__ double dotv(const double* a, const double* b) {
-    double s = a[0] * b[0] + a[1] * b[1];
-    if (DIM == 3) s = s + a[2] * b[2];
+    double s = mul<INT>(a[0], b[0]) + mul<INT>(a[1], b[1]);
+    if (DIM == 3) s = s + mul<INT>(a[2], b[2]);
     return s;
+}
+// Every entry usable by int_mul.
+template <int DIM>
+__device__ __forceinline__ bool in_window_v(const double* a) {
+    return in_window(a[0]) && in_window(a[1]) && (DIM == 2 || in_window(a[2]));
+}
+template <int DIM>
+__device__ __forceinline__ bool in_window_m(const double* L) {
+    bool ok = true;
+    for (int a = 0; a < DIM; ++a)
+        for (int b = 0; b < DIM; ++b) ok = ok && in_window(L[3 * a + b]);
+    return ok;
 }
 
 // ---- neighbour traversal (eng/particle_system.py:259-269) ----
@@ -166,25 +178,39 @@ __device__ __forceinline__ double det3(const double* a) {
     return a[0] * (a[4] * a[8] - a[7] * a[5]) - a[3] * (a[1] * a[8] - a[7] * a[2]) + a[6] * (a[1] * a[5] - a[4] * a[2]);
 }
 
-// Pair geometry of row slot `slot` (entry j): r, |r| and grad W into registers, grad W and the
-// viscosity denominator into the row's planes.
+// Pair geometry of row slot `slot` (entry j): r, grad W and, for a flow neighbour, W into
+// registers, grad W and the viscosity denominator into the row's planes.  The Wendland kernel
+// away from its ends runs its products on the integer pipes; the others take the kernel functions.
 template <int DIM>
 __device__ __forceinline__ double pair_geometry(const Consts& c, const double* __restrict__ X, const double* xi, int j,
-                                                const Pairs64& pr, size_t slot, double* r, double* kd) {
+                                                const Pairs64& pr, size_t slot, bool want_W, double* r, double* kd) {
     const size_t n = c.n;
     r[0] = xi[0] - X[j];
     r[1] = xi[1] - X[n + j];
     r[2] = DIM == 3 ? xi[2] - X[2 * n + j] : 0.0;
-    double r2 = r[0] * r[0] + r[1] * r[1];
-    if (DIM == 3) r2 = r2 + r[2] * r[2];
+    const bool r_ok = in_window_v<DIM>(r);
+    const double r2 = r_ok ? dotv<DIM, true>(r, r) : dotv<DIM>(r, r);
     const double rn = sqrt(r2);
-    kernel_dW<DIM>(c, r, rn, kd);
+    double W = 0.0, den;
+    const double q = rn * c.h1, q1 = __fma_rn(-0.5, q, 1.0);
+    if (c.wend_int && r_ok && rn > EPS && q <= 2.0 && in_window(q) && q1 > 0x1p-50) {
+        const double y = __drcp_rn(rn);
+        const double q2 = int_mul(q1, q1);
+        const double s = int_mul(int_mul(int_mul(c.kk, int_mul(q2, q1)), int_mul(-5.0, q)), c.h1);
+        for (int d = 0; d < DIM; ++d) kd[d] = div_by(int_mul(s, r[d]), rn, y, c.div_span);
+        if (want_W) W = int_mul(int_mul(c.kk, int_mul(q2, q2)), __fma_rn(2.0, q, 1.0));
+        den = int_mul(rn, rn);
+    } else {
+        kernel_dW<DIM>(c, r, rn, kd);
+        if (want_W) W = kernel_W(c, rn);
+        den = rn * rn;
+    }
     for (int d = 0; d < DIM; ++d) pr.gk[d * pr.slots_f + slot] = kd[d];
     if (pr.gden) {
-        const double den = rn * rn + c.eps_h2;
+        den = den + c.eps_h2;
         pr.gden[slot] = make_double2(den, __drcp_rn(den));
     }
-    return rn;
+    return W;
 }
 
 // Kernel value of a boundary row's entry.
@@ -226,15 +252,24 @@ __global__ void __launch_bounds__(ROWS * G) k_corr_flow(Consts c, Persist64 p, T
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const int ent = pr.nb_f[q.base + s], j = nb_index(ent);
             double r[3], kd[3];
-            const double rn = pair_geometry<DIM>(c, p.x, xi, j, pr, q.base + s, r, kd);
+            const double W = pair_geometry<DIM>(c, p.x, xi, j, pr, q.base + s, nb_flow(ent), r, kd);
             if (nb_flow(ent)) {
                 const double mVj = p.m_V[j];
-                T[0] = mVj * kernel_W(c, rn);
-                if (CORR)
-                    for (int a = 0; a < DIM; ++a) {
-                        const double av = mVj * (-r[a]);
-                        for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = av * kd[b];
-                    }
+                if (in_window(mVj) && in_window(W) && (!CORR || (in_window_v<DIM>(r) && in_window_v<DIM>(kd)))) {
+                    T[0] = int_mul(mVj, W);
+                    if (CORR)
+                        for (int a = 0; a < DIM; ++a) {
+                            const double av = int_mul(mVj, -r[a]);
+                            for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = int_mul(av, kd[b]);
+                        }
+                } else {
+                    T[0] = mVj * W;
+                    if (CORR)
+                        for (int a = 0; a < DIM; ++a) {
+                            const double av = mVj * (-r[a]);
+                            for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = av * kd[b];
+                        }
+                }
             }
         });
     }
@@ -334,7 +369,7 @@ __global__ void __launch_bounds__(ROWS * G) k_geom_flow(Consts c, Persist64 p, c
     double xi[3], r[3], kd[3];
     load_x<DIM>(p.x, q.i, c.n, xi);
     for (int s = threadIdx.x % G; s < q.cnt; s += G)
-        pair_geometry<DIM>(c, p.x, xi, nb_index(pr.nb_f[q.base + s]), pr, q.base + s, r, kd);
+        pair_geometry<DIM>(c, p.x, xi, nb_index(pr.nb_f[q.base + s]), pr, q.base + s, false, r, kd);
 }
 
 template <int DIM, int G>
@@ -622,14 +657,15 @@ __device__ __forceinline__ void corrected(const Consts& c, const double* L, cons
 }
 template <int DIM, int KC>
 __device__ __forceinline__ void row_gradient(const Consts& c, const Pairs64& pr, size_t slot, const double* L,
-                                             double* kc) {
+                                             bool L_ok, double* kc) {
     if (KC == KC_READ) {
         for (int d = 0; d < DIM; ++d) kc[d] = pr.gc[d * pr.slots_f + slot];
         return;
     }
     double kd[3] = {0.0, 0.0, 0.0};
     for (int d = 0; d < DIM; ++d) kd[d] = pr.gk[d * pr.slots_f + slot];
-    corrected<DIM>(c, L, kd, kc);
+    if (c.corr == 1 && L_ok && in_window_v<DIM>(kd)) matvec_corr<DIM, true>(L, kd, kc);
+    else corrected<DIM>(c, L, kd, kc);
     if (KC == KC_KEEP)
         for (int d = 0; d < DIM; ++d) pr.gc[d * pr.slots_f + slot] = kc[d];
 }
@@ -648,15 +684,26 @@ template <int DIM>
 __device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const double* v, double P, double mV, double cvj,
                                          double cC, const double* vti, const Divisor& rti, double pri, const double* r,
                                          double2 den, const double* kd, const double* kc, double* T) {
-    double dvv[3], a[3];
-    for (int d = 0; d < DIM; ++d) { dvv[d] = vti[d] - v[d]; a[d] = mV * dvv[d]; }
-    T[0] = dotv<DIM>(a, kc);
-    const double mn = min0(dotv<DIM>(dvv, r));
+    double dvv[3], a[3], dr;
+    for (int d = 0; d < DIM; ++d) dvv[d] = vti[d] - v[d];
+    if (in_window(mV) && in_window_v<DIM>(dvv) && in_window_v<DIM>(r) && in_window_v<DIM>(kc)) {
+        for (int d = 0; d < DIM; ++d) a[d] = int_mul(mV, dvv[d]);
+        T[0] = dotv<DIM, true>(a, kc);
+        dr = dotv<DIM, true>(dvv, r);
+    } else {
+        for (int d = 0; d < DIM; ++d) a[d] = mV * dvv[d];
+        T[0] = dotv<DIM>(a, kc);
+        dr = dotv<DIM>(dvv, r);
+    }
+    const double mn = min0(dr);
     double cv = cvj;
     if (!fluid) cv = div_by(cv, rti.b, rti.y, rti.span);
     cv = div_by(cv * mn, den.x, den.y, c.div_span);
     const double cp = cC * (pri + P);
-    for (int d = 0; d < DIM; ++d) T[1 + d] = cv * kd[d] + cp * kd[d];
+    if (in_window(cp) && in_window_v<DIM>(kd))
+        for (int d = 0; d < DIM; ++d) T[1 + d] = cv * kd[d] + int_mul(cp, kd[d]);
+    else
+        for (int d = 0; d < DIM; ++d) T[1 + d] = cv * kd[d] + cp * kd[d];
 }
 
 // ---- WCSPH rates (eng/solver_sph_wc.py:108-126) ----
@@ -675,6 +722,7 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
         const double pri = pr.rec[(size_t)8 * q.i + 3];
         if (c.corr == 1 && KC != KC_READ)
             for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
+        const bool L_ok = c.corr == 1 && KC != KC_READ && in_window_m<DIM>(L);
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
             const int ent = pr.nb_f[slot], j = nb_index(ent);
@@ -685,7 +733,7 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
                 r[d] = xi[d] - p.x[(size_t)d * n + j];
                 kd[d] = pr.gk[d * pr.slots_f + slot];
             }
-            row_gradient<DIM, KC>(c, pr, slot, L, kc);
+            row_gradient<DIM, KC>(c, pr, slot, L, L_ok, kc);
             const double v[3] = {r0.x, r0.y, r1.x};
             wc_terms<DIM>(c, nb_flow(ent), v, r1.y, r2.x, r2.y, r3.x, vti, rti, pri, r, pr.gden[slot], kd, kc, T);
         });
@@ -740,9 +788,18 @@ __device__ __forceinline__ void damping_acc(const Consts& c, double rti, const d
 // product is the negated trace.
 template <int DIM>
 __device__ __forceinline__ void vgrad_terms(const double* v, double mV, const double* vti, const double* kc, double* T) {
-    for (int a = 0; a < DIM; ++a) {
-        const double av = mV * (v[a] - vti[a]);
-        for (int b = 0; b < DIM; ++b) T[a * DIM + b] = av * kc[b];
+    double dv[3];
+    for (int a = 0; a < DIM; ++a) dv[a] = v[a] - vti[a];
+    if (in_window(mV) && in_window_v<DIM>(dv) && in_window_v<DIM>(kc)) {
+        for (int a = 0; a < DIM; ++a) {
+            const double av = int_mul(mV, dv[a]);
+            for (int b = 0; b < DIM; ++b) T[a * DIM + b] = int_mul(av, kc[b]);
+        }
+    } else {
+        for (int a = 0; a < DIM; ++a) {
+            const double av = mV * dv[a];
+            for (int b = 0; b < DIM; ++b) T[a * DIM + b] = av * kc[b];
+        }
     }
     double s = T[0] + T[DIM + 1];
     if (DIM == 3) s = s + T[8];
@@ -761,14 +818,15 @@ __global__ void __launch_bounds__(ROWS * G) k_mui_stress(Consts c, Persist64 p, 
         const RowRef q = row_ref<G>(list, count, pr.cnt, pr.cap_f);
         double vti[3], L[9];
         for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + q.i];
-        if (c.corr == 1)
+        if (c.corr == 1 && KC != KC_READ)
             for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
+        const bool L_ok = c.corr == 1 && KC != KC_READ && in_window_m<DIM>(L);
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
             const int j = nb_index(pr.nb_f[slot]);
             double kc[3], v[3];
             for (int d = 0; d < DIM; ++d) v[d] = t.v_tmp[(size_t)d * n + j];
-            row_gradient<DIM, KC>(c, pr, slot, L, kc);
+            row_gradient<DIM, KC>(c, pr, slot, L, L_ok, kc);
             vgrad_terms<DIM>(v, p.m_V[j], vti, kc, T);
         });
     }
@@ -839,13 +897,20 @@ __device__ __forceinline__ void stress_div_val(const double* sti, double ri2, co
 template <int DIM>
 __device__ __forceinline__ void stress_div_rec(const double* Si, const double* Sj, double sc, const double* kc,
                                                double* out) {
+    double m[DIM * DIM];
+    bool ok = in_window(sc) && in_window_v<DIM>(kc);
+    for (int q = 0; q < DIM * DIM; ++q) {
+        m[q] = Sj[q] + Si[q];
+        ok = ok && in_window(m[q]);
+    }
+    if (ok) {
+        for (int q = 0; q < DIM * DIM; ++q) m[q] = int_mul(int_mul(sc, m[q]), kc[q % DIM]);
+    } else {
+        for (int q = 0; q < DIM * DIM; ++q) m[q] = (sc * m[q]) * kc[q % DIM];
+    }
     for (int a = 0; a < DIM; ++a) {
-        double s = 0.0;
-        for (int b = 0; b < DIM; ++b) {
-            const double v = (sc * (Sj[a * DIM + b] + Si[a * DIM + b])) * kc[b];
-            s = b == 0 ? v : s + v;
-        }
-        out[a] = s;
+        out[a] = m[a * DIM] + m[a * DIM + 1];
+        if (DIM == 3) out[a] = out[a] + m[a * DIM + 2];
     }
 }
 
@@ -881,14 +946,15 @@ __device__ __forceinline__ void soil_sums(const Consts& c, const Persist64& p, c
     if (pr.cap_f) {
         const RowRef q = row_ref<G>(list, count, pr.cnt, pr.cap_f);
         double L[9];
-        if (c.corr == 1)
+        if (c.corr == 1 && KC != KC_READ)
             for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
+        const bool L_ok = c.corr == 1 && KC != KC_READ && in_window_m<DIM>(L);
         const SoilRec<DIM> ri(pr.rec, q.i);
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
             const int j = nb_index(pr.nb_f[slot]);
             double kc[3];
-            row_gradient<DIM, KC>(c, pr, slot, L, kc);
+            row_gradient<DIM, KC>(c, pr, slot, L, L_ok, kc);
             const SoilRec<DIM> rj(pr.rec, j);
             stress_div_rec<DIM>(ri.S(), rj.S(), rj.sc(), kc, T);
             if (DP) vgrad_terms<DIM>(rj.v(), rj.mV(), ri.v(), kc, T + DIM);

@@ -55,6 +55,7 @@ struct Consts {
     float pf_r2, pf_lim;
     float pf_in2;       // below this f32 distance^2 a pair is certainly a neighbour
     float pf_lo2, pf_hi2;  // the same two bounds for the distance^2 with the low parts added
+    int wend_int;       // Wendland kernel with constants inside 2^+-100 (int_mul chains stay normal)
     unsigned div_span;  // exponent window of div_by (0 closes it)
     double R2T;         // r2 < R2T exactly when sqrt(r2) < R
     int n_rigid_dyn;    // dynamic rigid particles (shape-matched bodies)

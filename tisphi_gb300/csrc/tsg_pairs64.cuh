@@ -140,6 +140,42 @@ __device__ __forceinline__ double div_by(double a, double b, double y, unsigned 
     return a / b;
 }
 
+// a * b, correctly rounded, on the integer pipes.  sm_103a issues an FP64 warp instruction per SM
+// in 16 cycles; this takes about as long on the other pipes and runs beside it (measured: 18.5
+// cycles at the nominal clock for the FP64 product, 15.8 for this one, 9.3 for each of two in
+// parallel), so the pair loops give it most of their products.  The 53 x 53 bit product of the
+// significands is formed in 128 bits, normalised, and rounded to nearest even with the bits
+// below jammed into one word; the sign and the exponent are put together beside it.  Operands
+// and result must be normal numbers (in_window(a), in_window(b): then so are products of up to
+// three of them).
+__device__ __forceinline__ bool in_window(double a) {  // 2^-255 <= |a| < 2^257
+    return ((unsigned)__double2hiint(a) & 0x7fffffffu) - (768u << 20) < (512u << 20);
+}
+__device__ __forceinline__ double int_mul(double a, double b) {
+    const unsigned ah = __double2hiint(a), al = __double2loint(a);
+    const unsigned bh = __double2hiint(b), bl = __double2loint(b);
+    // significands: a's in 53 bits, b's shifted up to 64
+    const unsigned ma = (ah & 0xfffffu) | 0x100000u;
+    const unsigned mh = __funnelshift_l(bl, bh, 11) | 0x80000000u, ml = bl << 11;
+    const unsigned long long p0 = (unsigned long long)al * ml;
+    const unsigned long long p1 = (unsigned long long)al * mh + (p0 >> 32);
+    const unsigned long long p2 = (unsigned long long)ma * ml + (unsigned)p1;
+    const unsigned long long p3 = (unsigned long long)ma * mh + (p1 >> 32) + (p2 >> 32);  // [2^51, 2^53)
+    unsigned w = (unsigned)p2 | min((unsigned)p0, 1u);  // the bits below p3, the last ones jammed
+    unsigned h1 = (unsigned)(p3 >> 32), h0 = (unsigned)p3;
+    const unsigned sh = (h1 >> 20) ^ 1u;  // one bit short: shift up
+    h1 = __funnelshift_l(h0, h1, sh);
+    h0 = __funnelshift_l(w, h0, sh);
+    w <<= sh;
+    const unsigned up = w > 0x80000000u - (h0 & 1u);  // above half, or half and odd
+    const unsigned e = (ah & 0x7ff00000u) + (bh & 0x7ff00000u) - (1023u << 20) - (sh << 20) + h1;
+    const unsigned long long r = (((unsigned long long)e << 32) | h0) + up;
+    return __hiloint2double((int)((unsigned)(r >> 32) | ((ah ^ bh) & 0x80000000u)), (int)(unsigned)r);
+}
+// The product on the pipe a loop chose for it.
+template <bool INT>
+__device__ __forceinline__ double mul(double a, double b) { return INT ? int_mul(a, b) : a * b; }
+
 // fmin(x, 0.0) without an FP64 comparison: x where its sign is set (and it is no NaN), else 0.
 __device__ __forceinline__ double min0(double x) {
     const int hi = __double2hiint(x), lo = __double2loint(x);
