@@ -40,7 +40,8 @@ inline int nblk(long long n, int tpb = TPB) { return (int)((n + tpb - 1) / tpb);
 // ---- kernel functions (eng/solver_sph_base.py:299-358) ----
 // W and |grad W| factor from the precomputed norm rn; dW_c = s * r_c / rn (Wendland) or
 // s * (r_c / rn * h1) (cubic), matching the reference's expression trees.
-__device__ __forceinline__ double kernel_W(const Consts& c, double rn) {
+template <class P>
+__device__ __forceinline__ double kernel_W(const P& c, double rn) {
     double res = 0.0;
     double q = rn * c.h1;
     if (rn > EPS && q <= 2.0) {
@@ -58,8 +59,8 @@ __device__ __forceinline__ double kernel_W(const Consts& c, double rn) {
     return res;
 }
 
-template <int DIM>
-__device__ __forceinline__ void kernel_dW(const Consts& c, const double* r, double rn, double* out) {
+template <int DIM, class P>
+__device__ __forceinline__ void kernel_dW(const P& c, const double* r, double rn, double* out) {
     out[0] = out[1] = out[2] = 0.0;
     double q = rn * c.h1;
     if (rn > EPS && q <= 2.0) {
@@ -77,32 +78,41 @@ __device__ __forceinline__ void kernel_dW(const Consts& c, const double* r, doub
     }
 }
 
-template <int DIM, bool INT = false>
-__device__ __forceinline__ void matvec_corr(const double* L, const double* k, double* out) {
+template <int DIM, class M>
+__device__ __forceinline__ void matvec_corr(const double* L, const double* k, double* out, M mul) {
     for (int p = 0; p < DIM; ++p) {
-        double s = mul<INT>(L[3 * p], k[0]) + mul<INT>(L[3 * p + 1], k[1]);
-        if (DIM == 3) s = s + mul<INT>(L[3 * p + 2], k[2]);
+        double s = mul(L[3 * p], k[0]) + mul(L[3 * p + 1], k[1]);
+        if (DIM == 3) s = s + mul(L[3 * p + 2], k[2]);
         out[p] = s;
     }
     if (DIM == 2) out[2] = 0.0;
 }
 
-template <int DIM, bool INT = false>
-__device__ __forceinline__ double dotv(const double* a, const double* b) {
-    double s = mul<INT>(a[0], b[0]) + mul<INT>(a[1], b[1]);
-    if (DIM == 3) s = s + mul<INT>(a[2], b[2]);
+template <int DIM, class M>
+__device__ __forceinline__ double dotv(const double* a, const double* b, M mul) {
+    double s = mul(a[0], b[0]) + mul(a[1], b[1]);
+    if (DIM == 3) s = s + mul(a[2], b[2]);
     return s;
+}
+// The pipe of a run of products: integer where every operand is usable, else calls.
+struct IntMul { __device__ __forceinline__ double operator()(double a, double b) const { return int_mul(a, b); } };
+struct SlowMul { __device__ __forceinline__ double operator()(double a, double b) const { return slow_mul(a, b); } };
+struct PlainMul { __device__ __forceinline__ double operator()(double a, double b) const { return a * b; } };
+template <class F>
+__device__ __forceinline__ void on_pipe(bool usable_operands, F&& f) {
+    if (usable_operands) f(IntMul());
+    else f(SlowMul());
 }
 // Every entry usable by int_mul.
 template <int DIM>
-__device__ __forceinline__ bool in_window_v(const double* a) {
-    return in_window(a[0]) && in_window(a[1]) && (DIM == 2 || in_window(a[2]));
+__device__ __forceinline__ bool usable_v(const double* a) {
+    return usable(a[0]) && usable(a[1]) && (DIM == 2 || usable(a[2]));
 }
 template <int DIM>
-__device__ __forceinline__ bool in_window_m(const double* L) {
+__device__ __forceinline__ bool usable_m(const double* L) {
     bool ok = true;
     for (int a = 0; a < DIM; ++a)
-        for (int b = 0; b < DIM; ++b) ok = ok && in_window(L[3 * a + b]);
+        for (int b = 0; b < DIM; ++b) ok = ok && usable(L[3 * a + b]);
     return ok;
 }
 
@@ -178,6 +188,18 @@ __device__ __forceinline__ double det3(const double* a) {
     return a[0] * (a[4] * a[8] - a[7] * a[5]) - a[3] * (a[1] * a[8] - a[7] * a[2]) + a[6] * (a[1] * a[5] - a[4] * a[2]);
 }
 
+// The kernel functions behind a call (see slow_mul), their constants by value: grad W and W.
+struct KernelConsts { int kernel; unsigned div_span; double h1, kk; };
+struct KernelVals { double kd[3], W; };
+template <int DIM>
+__device__ __noinline__ KernelVals slow_kernel(KernelConsts c, double r0, double r1, double r2, double rn) {
+    const double r[3] = {r0, r1, r2};
+    KernelVals k;
+    kernel_dW<DIM>(c, r, rn, k.kd);
+    k.W = kernel_W(c, rn);
+    return k;
+}
+
 // Pair geometry of row slot `slot` (entry j): r, grad W and, for a flow neighbour, W into
 // registers, grad W and the viscosity denominator into the row's planes.  The Wendland kernel
 // away from its ends runs its products on the integer pipes; the others take the kernel functions.
@@ -188,12 +210,13 @@ __device__ __forceinline__ double pair_geometry(const Consts& c, const double* _
     r[0] = xi[0] - X[j];
     r[1] = xi[1] - X[n + j];
     r[2] = DIM == 3 ? xi[2] - X[2 * n + j] : 0.0;
-    const bool r_ok = in_window_v<DIM>(r);
-    const double r2 = r_ok ? dotv<DIM, true>(r, r) : dotv<DIM>(r, r);
+    const bool r_ok = usable_v<DIM>(r);
+    double r2;
+    on_pipe(r_ok, [&](auto mul) { r2 = dotv<DIM>(r, r, mul); });
     const double rn = sqrt(r2);
     double W = 0.0, den;
     const double q = rn * c.h1, q1 = __fma_rn(-0.5, q, 1.0);
-    if (c.wend_int && r_ok && rn > EPS && q <= 2.0 && in_window(q) && q1 > 0x1p-50) {
+    if (c.wend_int && r_ok && above(rn, EPS) && !above(q, 2.0) && usable(q) && above(q1, 0x1p-50)) {
         const double y = __drcp_rn(rn);
         const double q2 = int_mul(q1, q1);
         const double s = int_mul(int_mul(int_mul(c.kk, int_mul(q2, q1)), int_mul(-5.0, q)), c.h1);
@@ -201,9 +224,10 @@ __device__ __forceinline__ double pair_geometry(const Consts& c, const double* _
         if (want_W) W = int_mul(int_mul(c.kk, int_mul(q2, q2)), __fma_rn(2.0, q, 1.0));
         den = int_mul(rn, rn);
     } else {
-        kernel_dW<DIM>(c, r, rn, kd);
-        if (want_W) W = kernel_W(c, rn);
-        den = rn * rn;
+        const KernelVals k = slow_kernel<DIM>(KernelConsts{c.kernel, c.div_span, c.h1, c.kk}, r[0], r[1], r[2], rn);
+        for (int d = 0; d < DIM; ++d) kd[d] = k.kd[d];
+        W = k.W;
+        den = slow_mul(rn, rn);
     }
     for (int d = 0; d < DIM; ++d) pr.gk[d * pr.slots_f + slot] = kd[d];
     if (pr.gden) {
@@ -255,21 +279,14 @@ __global__ void __launch_bounds__(ROWS * G) k_corr_flow(Consts c, Persist64 p, T
             const double W = pair_geometry<DIM>(c, p.x, xi, j, pr, q.base + s, nb_flow(ent), r, kd);
             if (nb_flow(ent)) {
                 const double mVj = p.m_V[j];
-                if (in_window(mVj) && in_window(W) && (!CORR || (in_window_v<DIM>(r) && in_window_v<DIM>(kd)))) {
-                    T[0] = int_mul(mVj, W);
+                on_pipe(usable(mVj) && usable(W) && (!CORR || (usable_v<DIM>(r) && usable_v<DIM>(kd))), [&](auto mul) {
+                    T[0] = mul(mVj, W);
                     if (CORR)
                         for (int a = 0; a < DIM; ++a) {
-                            const double av = int_mul(mVj, -r[a]);
-                            for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = int_mul(av, kd[b]);
+                            const double av = mul(mVj, -r[a]);
+                            for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = mul(av, kd[b]);
                         }
-                } else {
-                    T[0] = mVj * W;
-                    if (CORR)
-                        for (int a = 0; a < DIM; ++a) {
-                            const double av = mVj * (-r[a]);
-                            for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = av * kd[b];
-                        }
-                }
+                });
             }
         });
     }
@@ -631,7 +648,7 @@ template <int DIM>
 __device__ __forceinline__ void wc_force_pair(const Consts& c, int tj, double mVj, const double* dvv, double rti,
                                               double pri, double ptj, double rtj, const double* r, double rn,
                                               const double* kd, double* out) {
-    const double mn = fmin(dotv<DIM>(dvv, r), 0.0);
+    const double mn = fmin(dotv<DIM>(dvv, r, PlainMul()), 0.0);
     const double den = rn * rn + c.eps_h2;
     double cv = 0.0;
     bool visc = false;
@@ -652,7 +669,7 @@ __device__ __forceinline__ void wc_force_pair(const Consts& c, int tj, double mV
 enum { KC_MAKE = 0, KC_KEEP = 1, KC_READ = 2 };
 template <int DIM>
 __device__ __forceinline__ void corrected(const Consts& c, const double* L, const double* kd, double* kc) {
-    if (c.corr == 1) matvec_corr<DIM>(L, kd, kc);
+    if (c.corr == 1) matvec_corr<DIM>(L, kd, kc, PlainMul());
     else { kc[0] = kd[0]; kc[1] = kd[1]; kc[2] = kd[2]; }
 }
 template <int DIM, int KC>
@@ -664,8 +681,10 @@ __device__ __forceinline__ void row_gradient(const Consts& c, const Pairs64& pr,
     }
     double kd[3] = {0.0, 0.0, 0.0};
     for (int d = 0; d < DIM; ++d) kd[d] = pr.gk[d * pr.slots_f + slot];
-    if (c.corr == 1 && L_ok && in_window_v<DIM>(kd)) matvec_corr<DIM, true>(L, kd, kc);
-    else corrected<DIM>(c, L, kd, kc);
+    if (c.corr == 1)
+        on_pipe(L_ok && usable_v<DIM>(kd), [&](auto mul) { matvec_corr<DIM>(L, kd, kc, mul); });
+    else
+        for (int d = 0; d < 3; ++d) kc[d] = kd[d];
     if (KC == KC_KEEP)
         for (int d = 0; d < DIM; ++d) pr.gc[d * pr.slots_f + slot] = kc[d];
 }
@@ -686,24 +705,19 @@ __device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const doub
                                          double2 den, const double* kd, const double* kc, double* T) {
     double dvv[3], a[3], dr;
     for (int d = 0; d < DIM; ++d) dvv[d] = vti[d] - v[d];
-    if (in_window(mV) && in_window_v<DIM>(dvv) && in_window_v<DIM>(r) && in_window_v<DIM>(kc)) {
-        for (int d = 0; d < DIM; ++d) a[d] = int_mul(mV, dvv[d]);
-        T[0] = dotv<DIM, true>(a, kc);
-        dr = dotv<DIM, true>(dvv, r);
-    } else {
-        for (int d = 0; d < DIM; ++d) a[d] = mV * dvv[d];
-        T[0] = dotv<DIM>(a, kc);
-        dr = dotv<DIM>(dvv, r);
-    }
+    on_pipe(usable(mV) && usable_v<DIM>(dvv) && usable_v<DIM>(r) && usable_v<DIM>(kc), [&](auto mul) {
+        for (int d = 0; d < DIM; ++d) a[d] = mul(mV, dvv[d]);
+        T[0] = dotv<DIM>(a, kc, mul);
+        dr = dotv<DIM>(dvv, r, mul);
+    });
     const double mn = min0(dr);
     double cv = cvj;
     if (!fluid) cv = div_by(cv, rti.b, rti.y, rti.span);
     cv = div_by(cv * mn, den.x, den.y, c.div_span);
     const double cp = cC * (pri + P);
-    if (in_window(cp) && in_window_v<DIM>(kd))
-        for (int d = 0; d < DIM; ++d) T[1 + d] = cv * kd[d] + int_mul(cp, kd[d]);
-    else
-        for (int d = 0; d < DIM; ++d) T[1 + d] = cv * kd[d] + cp * kd[d];
+    on_pipe(usable(cp) && usable(cv) && usable_v<DIM>(kd), [&](auto mul) {
+        for (int d = 0; d < DIM; ++d) T[1 + d] = mul(cv, kd[d]) + mul(cp, kd[d]);
+    });
 }
 
 // ---- WCSPH rates (eng/solver_sph_wc.py:108-126) ----
@@ -722,7 +736,7 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
         const double pri = pr.rec[(size_t)8 * q.i + 3];
         if (c.corr == 1 && KC != KC_READ)
             for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
-        const bool L_ok = c.corr == 1 && KC != KC_READ && in_window_m<DIM>(L);
+        const bool L_ok = c.corr == 1 && KC != KC_READ && usable_m<DIM>(L);
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
             const int ent = pr.nb_f[slot], j = nb_index(ent);
@@ -790,17 +804,12 @@ template <int DIM>
 __device__ __forceinline__ void vgrad_terms(const double* v, double mV, const double* vti, const double* kc, double* T) {
     double dv[3];
     for (int a = 0; a < DIM; ++a) dv[a] = v[a] - vti[a];
-    if (in_window(mV) && in_window_v<DIM>(dv) && in_window_v<DIM>(kc)) {
+    on_pipe(usable(mV) && usable_v<DIM>(dv) && usable_v<DIM>(kc), [&](auto mul) {
         for (int a = 0; a < DIM; ++a) {
-            const double av = int_mul(mV, dv[a]);
-            for (int b = 0; b < DIM; ++b) T[a * DIM + b] = int_mul(av, kc[b]);
+            const double av = mul(mV, dv[a]);
+            for (int b = 0; b < DIM; ++b) T[a * DIM + b] = mul(av, kc[b]);
         }
-    } else {
-        for (int a = 0; a < DIM; ++a) {
-            const double av = mV * dv[a];
-            for (int b = 0; b < DIM; ++b) T[a * DIM + b] = av * kc[b];
-        }
-    }
+    });
     double s = T[0] + T[DIM + 1];
     if (DIM == 3) s = s + T[8];
     T[DIM * DIM] = -s;
@@ -820,7 +829,7 @@ __global__ void __launch_bounds__(ROWS * G) k_mui_stress(Consts c, Persist64 p, 
         for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + q.i];
         if (c.corr == 1 && KC != KC_READ)
             for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
-        const bool L_ok = c.corr == 1 && KC != KC_READ && in_window_m<DIM>(L);
+        const bool L_ok = c.corr == 1 && KC != KC_READ && usable_m<DIM>(L);
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
             const int j = nb_index(pr.nb_f[slot]);
@@ -898,16 +907,14 @@ template <int DIM>
 __device__ __forceinline__ void stress_div_rec(const double* Si, const double* Sj, double sc, const double* kc,
                                                double* out) {
     double m[DIM * DIM];
-    bool ok = in_window(sc) && in_window_v<DIM>(kc);
+    bool ok = usable(sc) && usable_v<DIM>(kc);
     for (int q = 0; q < DIM * DIM; ++q) {
         m[q] = Sj[q] + Si[q];
-        ok = ok && in_window(m[q]);
+        ok = ok && usable(m[q]);
     }
-    if (ok) {
-        for (int q = 0; q < DIM * DIM; ++q) m[q] = int_mul(int_mul(sc, m[q]), kc[q % DIM]);
-    } else {
-        for (int q = 0; q < DIM * DIM; ++q) m[q] = (sc * m[q]) * kc[q % DIM];
-    }
+    on_pipe(ok, [&](auto mul) {
+        for (int q = 0; q < DIM * DIM; ++q) m[q] = mul(mul(sc, m[q]), kc[q % DIM]);
+    });
     for (int a = 0; a < DIM; ++a) {
         out[a] = m[a * DIM] + m[a * DIM + 1];
         if (DIM == 3) out[a] = out[a] + m[a * DIM + 2];
@@ -948,7 +955,7 @@ __device__ __forceinline__ void soil_sums(const Consts& c, const Persist64& p, c
         double L[9];
         if (c.corr == 1 && KC != KC_READ)
             for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
-        const bool L_ok = c.corr == 1 && KC != KC_READ && in_window_m<DIM>(L);
+        const bool L_ok = c.corr == 1 && KC != KC_READ && usable_m<DIM>(L);
         const SoilRec<DIM> ri(pr.rec, q.i);
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
@@ -1507,7 +1514,7 @@ __global__ void k_rigid_reaction(Consts c, Persist64 p, Trans64 t, const int* __
             if (c.corr == 1) {
                 double L[9];
                 for (int q = 0; q < 9; ++q) L[q] = t.CSPM_L[(size_t)q * n + i];
-                matvec_corr<DIM>(L, kd, kc);
+                matvec_corr<DIM>(L, kd, kc, PlainMul());
             } else {
                 kc[0] = kd[0]; kc[1] = kd[1]; kc[2] = kd[2];
             }

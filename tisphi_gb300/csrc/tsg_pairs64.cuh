@@ -124,6 +124,12 @@ __global__ void __launch_bounds__(256) k_list64(Consts c, const double* __restri
     if (lane == 0) pr.cnt[row] = m;
 }
 
+// FP64 products and quotients of the rare operands that the paths below leave out.  Calls, so
+// that they stay behind a branch: inlined, the compiler predicates them, and an FP64 instruction
+// with every lane off holds the pipe like any other.
+__device__ __noinline__ double slow_mul(double a, double b) { return a * b; }
+__device__ __noinline__ double slow_div(double a, double b) { return a / b; }
+
 // a / b, correctly rounded, from y = RN(1 / b): one product and two fused multiply-adds instead
 // of the division's ten-odd FP64 instructions (Markstein 1990; Brisebarre, Muller and Raina,
 // "Accelerating correctly rounded floating-point division when the divisor is known in
@@ -137,19 +143,21 @@ __device__ __forceinline__ double div_by(double a, double b, double y, unsigned 
         return __fma_rn(__fma_rn(-b, q, a), y, q);
     }
     if ((hi | (unsigned)__double2loint(a)) == 0u) return a;
-    return a / b;
+    return slow_div(a, b);
 }
 
 // a * b, correctly rounded, on the integer pipes.  sm_103a issues an FP64 warp instruction per SM
 // in 16 cycles; this takes about as long on the other pipes and runs beside it (measured: 18.5
 // cycles at the nominal clock for the FP64 product, 15.8 for this one, 9.3 for each of two in
-// parallel), so the pair loops give it most of their products.  The 53 x 53 bit product of the
+// parallel), so the pair loops give it most of their products.  3D, 118 k rows, us per launch:
+// rates 1,835 -> 855 (first loop) and 1,476 -> 655 (second), correction 2,057 -> 1,376.  The 53 x 53 bit product of the
 // significands is formed in 128 bits, normalised, and rounded to nearest even with the bits
 // below jammed into one word; the sign and the exponent are put together beside it.  Operands
-// and result must be normal numbers (in_window(a), in_window(b): then so are products of up to
-// three of them).
-__device__ __forceinline__ bool in_window(double a) {  // 2^-255 <= |a| < 2^257
-    return ((unsigned)__double2hiint(a) & 0x7fffffffu) - (768u << 20) < (512u << 20);
+// are +-0 or normal numbers with normal products (usable(a), usable(b): then so are products of
+// up to three of them).
+__device__ __forceinline__ bool usable(double a) {  // +-0 or 2^-255 <= |a| < 2^257
+    const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    return hi - (768u << 20) < (512u << 20) || (hi | (unsigned)__double2loint(a)) == 0u;
 }
 __device__ __forceinline__ double int_mul(double a, double b) {
     const unsigned ah = __double2hiint(a), al = __double2loint(a);
@@ -168,13 +176,19 @@ __device__ __forceinline__ double int_mul(double a, double b) {
     h0 = __funnelshift_l(w, h0, sh);
     w <<= sh;
     const unsigned up = w > 0x80000000u - (h0 & 1u);  // above half, or half and odd
-    const unsigned e = (ah & 0x7ff00000u) + (bh & 0x7ff00000u) - (1023u << 20) - (sh << 20) + h1;
+    const unsigned ea = ah & 0x7ff00000u, eb = bh & 0x7ff00000u;
+    const unsigned e = ea + eb - (1023u << 20) - (sh << 20) + h1;
     const unsigned long long r = (((unsigned long long)e << 32) | h0) + up;
-    return __hiloint2double((int)((unsigned)(r >> 32) | ((ah ^ bh) & 0x80000000u)), (int)(unsigned)r);
+    const bool zero = min(ea, eb) == 0u;
+    return __hiloint2double((int)((zero ? 0u : (unsigned)(r >> 32)) | ((ah ^ bh) & 0x80000000u)),
+                            zero ? 0 : (int)(unsigned)r);
 }
-// The product on the pipe a loop chose for it.
-template <bool INT>
-__device__ __forceinline__ double mul(double a, double b) { return INT ? int_mul(a, b) : a * b; }
+
+
+// a > b for b >= 0 and a that is not a NaN, on the bits (an FP64 comparison holds the pipe too).
+__device__ __forceinline__ bool above(double a, double b) {
+    return __double_as_longlong(a) > __double_as_longlong(b);
+}
 
 // fmin(x, 0.0) without an FP64 comparison: x where its sign is set (and it is no NaN), else 0.
 __device__ __forceinline__ double min0(double x) {
