@@ -63,6 +63,12 @@ struct tsg_handle {
     int nscenes = 0;                // batched ensemble (tsg_batch_create): scenes and x pitch
     double batch_pitch = 0.0;
     Rigid64 rigid{};                // dynamic rigid bodies (FP64 form)
+    // Captured steps of the FP64 form, [buffer parity][1 or 2 steps] (see step_graph64)
+    struct StepGraph { cudaGraphExec_t exec = nullptr; long long kernels = 0; bool collide = false; };
+    StepGraph graphs[2][2];
+    const double* x_first = nullptr;  // cur.x at upload: tells the buffer parity
+    int eager_steps = 0;
+    bool no_graphs = false;         // a capture failed: launch eagerly
 };
 
 namespace {
@@ -280,6 +286,83 @@ int step64(tsg_handle* h, bool collide, cudaStream_t s) {
     if (c.n_rigid_dyn) fp64_solve_rigid(c, h->cur, h->rigid, s);
     // enforce_boundary also clamps dynamic rigid particles in every boundary mode
     if (collide || c.n_rigid_dyn) fp64_advect(c, h->cur, h->t, h->g, TSG_ENFORCE_BOUNDARY, s);
+    return check_cuda();
+}
+
+void drop_graphs64(tsg_handle* h) {
+    for (auto& side : h->graphs)
+        for (auto& g : side) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g = tsg_handle::StepGraph{};
+        }
+}
+
+// The captured graph of one or two FP64 steps from the current buffers.  A small scene's step is
+// some twenty-five launches of a few microseconds, each waiting for the host's next one when
+// launched one by one; the graph issues them back to back.  Nothing in a step depends on the
+// host, the constants are the launches' own copies (dropped when a material is set), and the
+// sort swaps the buffer sets, hence a graph per parity.
+tsg_handle::StepGraph* step_graph64(tsg_handle* h, int steps, bool collide) {
+    tsg_handle::StepGraph& g = h->graphs[h->cur.x == h->x_first ? 0 : 1][steps - 1];
+    if (g.exec && g.collide == collide) return &g;
+    if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
+    cudaStream_t cs = nullptr;
+    if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    const Persist64 cur = h->cur, nxt = h->nxt;
+    const long long c0 = launch_total();
+    cudaGraph_t graph = nullptr;
+    bool ok = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed) == cudaSuccess;
+    if (ok) {
+        for (int q = 0; q < steps && ok; ++q) {
+            sort_fp64(h->c, h->cur, h->nxt, h->t, h->g, cs);
+            ok = step64(h, collide, cs) == 0;
+        }
+        ok = cudaStreamEndCapture(cs, &graph) == cudaSuccess && graph && ok;
+    }
+    g.kernels = launch_total() - c0;
+    add_launches(-g.kernels);  // nodes, not launches
+    h->cur = cur;
+    h->nxt = nxt;
+    ok = ok && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
+    if (!ok) g.exec = nullptr;
+    if (graph) cudaGraphDestroy(graph);
+    cudaStreamDestroy(cs);
+    cudaGetLastError();
+    g.collide = collide;
+    return ok ? &g : nullptr;
+}
+
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) { cudaGetLastError(); return true; }
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// FP64 steps.  The first two of a handle run eagerly (a script that steps once or twice does
+// not pay for a capture), as do profiled steps and steps inside a caller's own capture.
+int steps64(tsg_handle* h, int nsteps, bool collide, cudaStream_t s) {
+    bool graphs = !h->no_graphs && !profiling_on() && !capturing(s);
+    while (nsteps > 0) {
+        if (graphs && h->eager_steps >= 2) {
+            const int take = nsteps >= 2 ? 2 : 1;
+            if (tsg_handle::StepGraph* g = step_graph64(h, take, collide)) {
+                if (cudaGraphLaunch(g->exec, s) != cudaSuccess) { check_cuda(); return TSG_E_CUDA; }
+                add_launches(g->kernels);
+                if (take == 1) std::swap(h->cur, h->nxt);
+                h->sorted = true;
+                h->pos32_dirty = true;
+                nsteps -= take;
+                continue;
+            }
+            h->no_graphs = true;
+            graphs = false;
+        }
+        sort_fp64(h->c, h->cur, h->nxt, h->t, h->g, s);
+        h->sorted = true;
+        if (int rc = step64(h, collide, s)) return rc;
+        ++h->eager_steps;
+        --nsteps;
+    }
     return check_cuda();
 }
 
@@ -503,6 +586,7 @@ int upload_impl(tsg_handle* h, const tsg_particles* p, int from_device, void* st
     if (nrdyn) fp64_rest_cm(c, h->cur, h->rigid, s);
     h->uploaded = true;
     h->pos32_dirty = true;
+    h->x_first = h->cur.x;
     return check_cuda();
 }
 }  // namespace
@@ -614,17 +698,14 @@ int tsg_step(tsg_handle* h, int nsteps, void* stream) {
         h->sorted = true;
         return check_cuda();
     }
-    for (int k = 0; k < nsteps; ++k) {
+    if (!use_fp32(h)) return steps64(h, nsteps, collide, S(stream));
+    for (int k = 0; k < nsteps; ++k) {  // FP32-mixed, profiled: what the captured graphs replay, eagerly
         int rc;
-        // FP32-mixed with a neighbour skin re-sorts only when its lists expire
-        if (!use_fp32(h) || fp32_rebuild_due(*h->f32, S(stream)))
+        // with a neighbour skin the particles are re-sorted only when the lists expire
+        if (fp32_rebuild_due(*h->f32, S(stream)))
             if ((rc = tsg_sort(h, stream))) return rc;
-        if (use_fp32(h)) {  // the kernel sequence the captured graphs replay, launched eagerly
-            fp32_step_body(*h->f32, collide, S(stream));
-            if ((rc = check_cuda())) return rc;
-            continue;
-        }
-        if ((rc = step64(h, collide, S(stream)))) return rc;
+        fp32_step_body(*h->f32, collide, S(stream));
+        if ((rc = check_cuda())) return rc;
     }
     return 0;
 }
@@ -944,6 +1025,7 @@ int tsg_set_soil(tsg_handle* h, double friction, double cohesion) {
         c.lam_den = 27.0 * c.alpha * c.Km * c.sin_dila + c.Gm;
         c.three_aK = 3.0 * c.alpha * c.Km;
     }
+    drop_graphs64(h);
     if (use_fp32(h)) fp32_set_soil(*h->f32, c);
     return 0;
 }
@@ -956,6 +1038,7 @@ int tsg_set_fluid(tsg_handle* h, double stiffness, double viscosity) {
     h->cfg.viscosity = viscosity;
     c.B = stiffness;
     c.visc_fac = 2 * (c.dim + 2) * viscosity;
+    drop_graphs64(h);
     if (use_fp32(h)) fp32_set_fluid(*h->f32, c);
     return 0;
 }
@@ -1106,6 +1189,7 @@ double tsg_batch_pitch(const tsg_handle* h) { return h ? h->batch_pitch : 0.0; }
 void tsg_destroy(tsg_handle* h) {
     if (!h) return;
     cudaDeviceSynchronize();
+    drop_graphs64(h);
     if (h->f32) fp32_destroy(h->f32);
     for (void* p : h->allocs) cudaFree(p);
     delete h;
