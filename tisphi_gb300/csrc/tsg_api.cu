@@ -184,13 +184,19 @@ int alloc_all(tsg_handle* h) {
     rc |= dalloc(h, &t.pos32, n); rc |= dalloc(h, &t.pos32l, n); rc |= dalloc(h, &t.cell0, n);
     Grid& g = h->g;
     const size_t nb = (size_t)c.G + 1;
-    rc |= dalloc(h, &g.cell0_old, n); rc |= dalloc(h, &g.cell_flow, (size_t)c.G);
-    rc |= dalloc(h, &g.cell_of, n); rc |= dalloc(h, &g.rank, n); rc |= dalloc(h, &g.count, nb);
+    rc |= dalloc(h, &g.cell0_old, n);
+    rc |= dalloc(h, &g.cell_of, n); rc |= dalloc(h, &g.rank, n);
+    const size_t zero_ints = nb + 3 + ((size_t)c.G + 3) / 4;
+    rc |= dalloc(h, &g.count, zero_ints);
+    g.zero_bytes = zero_ints * sizeof(int);
+    g.list_count = g.count + nb;
+    g.nbig = g.count + nb + 2;
+    g.cell_flow = reinterpret_cast<unsigned char*>(g.count + nb + 3);
     rc |= dalloc(h, &g.cell_start, nb + 1); rc |= dalloc(h, &g.perm, n);
     rc |= dalloc(h, &g.tile_sum, nb / 2048 + 2);
-    rc |= dalloc(h, &g.big, cellsort_big_ints(n)); rc |= dalloc(h, &g.nbig, 1);
+    rc |= dalloc(h, &g.big, cellsort_big_ints(n));
     rc |= dalloc(h, &g.list_flow, n + 1); rc |= dalloc(h, &g.list_bdy, n + 1);
-    rc |= dalloc(h, &g.list_count, 2); rc |= dalloc(h, &g.err, 1);
+    rc |= dalloc(h, &g.err, 1);
     rc |= dalloc(h, &h->d_stage, 9 * n + 16);
     rc |= dalloc(h, &h->d_scratch, 64);
     if (!rc) rc = alloc_rows(h);
@@ -459,6 +465,8 @@ int tsg_create(const tsg_config* cfg, tsg_handle** out) {
     c.pf_in2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 1024.0)), 0.f);
     // div_by: divisors |r| in (EPS, R) and |r|^2 + eps_h2 stay within 2^+-200 of 1
     c.div_span = c.R < 0x1p100 && c.eps_h2 > 0x1p-200 ? 1000u << 20 : 0u;
+    c.rgrid = 1.0 / c.grid;
+    c.grid_span = c.grid > 0x1p-100 && c.grid < 0x1p100 ? 1000u << 20 : 0u;
     c.wend_int = f.kernel == 1 && c.kk > 0x1p-100 && c.kk < 0x1p100 && c.h1 > 0x1p-100 && c.h1 < 0x1p100;
     c.pf_lo2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 262144.0)), 0.f);
     c.pf_hi2 = std::nextafter((float)(c.R * c.R * (1.0 + 1.0 / 262144.0)), 1e30f);

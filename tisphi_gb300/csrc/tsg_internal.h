@@ -56,6 +56,8 @@ struct Consts {
     float pf_in2;       // below this f32 distance^2 a pair is certainly a neighbour
     float pf_lo2, pf_hi2;  // the same two bounds for the distance^2 with the low parts added
     int wend_int;       // Wendland kernel with constants inside 2^+-100 (int_mul chains stay normal)
+    double rgrid;       // 1 / grid, and div_by's window for it
+    unsigned grid_span;
     unsigned div_span;  // exponent window of div_by (0 closes it)
     double R2T;         // r2 < R2T exactly when sqrt(r2) < R
     int n_rigid_dyn;    // dynamic rigid particles (shape-matched bodies)
@@ -152,7 +154,9 @@ struct Grid {
     int* cell_of;       // per particle (old order)
     int* rank;          // per particle within-cell arrival rank
     long long* cell0_old;  // per particle (old order): unclipped flattened cell index
-    int* count;         // G + 1
+    int* count;         // G + 1; zeroed with what follows it in one memory set per sort:
+                        // list_count, nbig, cell_flow
+    size_t zero_bytes;
     int* cell_start;    // G + 2 exclusive starts; [G] = out-of-grid bin, [G+1] = n
     int* perm;          // new -> old
     int* tile_sum;      // scan partials

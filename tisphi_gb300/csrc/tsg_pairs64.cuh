@@ -197,6 +197,18 @@ __device__ __forceinline__ double min0(double x) {
     return keep ? x : 0.0;
 }
 
+// Flattened cell index (truncating cast, eng/particle_system.py:216-226), unclipped; kNoCell
+// where a coordinate leaves the int range or is not finite.
+__device__ __forceinline__ long long flat_cell(const Consts& c, const double* x) {
+    long long idx[3];
+    for (int d = 0; d < 3; ++d) {
+        const double t = div_by(x[d] - c.vs[d], c.grid, c.rgrid, c.grid_span);
+        if (!(fabs(t) < 2147483647.0)) return kNoCell;
+        idx[d] = (long long)(int)t;
+    }
+    return idx[0] * c.gnum[1] * c.gnum[2] + idx[1] * c.gnum[2] + idx[2];
+}
+
 // f32 coordinates of a position: high part (w: flow flag) and what it rounds off.
 __device__ __forceinline__ void write_pos32(const Consts& c, const double* x, bool flow, float4* hi, float4* lo) {
     double d[3];
@@ -204,18 +216,6 @@ __device__ __forceinline__ void write_pos32(const Consts& c, const double* x, bo
     for (int q = 0; q < 3; ++q) { d[q] = x[q] - c.vs[q]; h[q] = (float)d[q]; }
     *hi = make_float4(h[0], h[1], h[2], flow ? 1.f : 0.f);
     *lo = make_float4((float)(d[0] - h[0]), (float)(d[1] - h[1]), (float)(d[2] - h[2]), 0.f);
-}
-
-// Flattened cell index (truncating cast, eng/particle_system.py:216-226), unclipped; kNoCell
-// where a coordinate leaves the int range or is not finite.
-__device__ __forceinline__ long long flat_cell(const Consts& c, const double* x) {
-    long long idx[3];
-    for (int d = 0; d < 3; ++d) {
-        const double t = (x[d] - c.vs[d]) / c.grid;
-        if (!(fabs(t) < 2147483647.0)) return kNoCell;
-        idx[d] = (long long)(int)t;
-    }
-    return idx[0] * c.gnum[1] * c.gnum[2] + idx[1] * c.gnum[2] + idx[2];
 }
 
 // The ordered sums of one row's C pair terms by its G lanes; acc[m] of lane g is component

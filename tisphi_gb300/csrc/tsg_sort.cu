@@ -10,8 +10,8 @@
 //   scan        exclusive prefix sum of the G + 1 counts (the extra bin collects
 //               particles whose flattened index falls outside [0, G));
 //   k_scatter   perm[cell_start + rank] = old index (unstable inside a cell);
-//   sort_within_cells (tsg_cellsort.cuh) orders each cell by old index (stable result);
-//   k_reorder   gathers every persistent field into the other buffer set, writes the f32
+//   k_cell_sort_big (tsg_cellsort.cuh) orders cells above kSortSmall by old index;
+//   k_reorder64 ranks the others' particles by old index (stable result), gathers every persistent field into the other buffer set, writes the f32
 //               prefilter positions and the flow / boundary index lists.
 // Compiled with -fmad=false: the f64 cell arithmetic must round exactly like the oracle's.
 #include <cstdio>
@@ -120,11 +120,46 @@ __global__ void k_tile_rescan(const int* __restrict__ in, int n, const int* __re
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) out[n] = e;  // grand total
 }
 
+// One block scans up to SCAN_ONE counts (a 2D scene's grid): one launch instead of three whose
+// few blocks each take a launch's latency.
+constexpr int SCAN_ONE_TPB = 1024, SCAN_ONE_ITEMS = 16, SCAN_ONE = SCAN_ONE_TPB * SCAN_ONE_ITEMS;
+__global__ void __launch_bounds__(SCAN_ONE_TPB) k_scan_one(const int* __restrict__ in, int n, int* __restrict__ out) {
+    __shared__ int warp_sums[SCAN_ONE_TPB / 32];
+    const int per = (n + SCAN_ONE_TPB - 1) / SCAN_ONE_TPB, base = threadIdx.x * per;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int v[SCAN_ONE_ITEMS], s = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_ONE_ITEMS; ++k) {
+        v[k] = k < per && base + k < n ? in[base + k] : 0;
+        s += v[k];
+    }
+    const int incl = warp_incl_scan(s);
+    if (lane == 31) warp_sums[wid] = incl;
+    __syncthreads();
+    if (wid == 0) {
+        const int w = warp_sums[lane];
+        warp_sums[lane] = warp_incl_scan(w) - w;
+    }
+    __syncthreads();
+    int e = warp_sums[wid] + incl - s;
+#pragma unroll
+    for (int k = 0; k < SCAN_ONE_ITEMS; ++k) {
+        if (k < per && base + k < n) out[base + k] = e;
+        e += v[k];
+    }
+    if (threadIdx.x == SCAN_ONE_TPB - 1) out[n] = e;  // grand total
+}
+
+// Places the particles in arrival order inside their cells and lists the cells above
+// kSortSmall, which k_cell_sort_big orders; k_reorder64 ranks the particles of the others.
 __global__ void k_scatter(int n, const int* __restrict__ cell_of, const int* __restrict__ rank,
-                          const int* __restrict__ cell_start, int* __restrict__ perm) {
+                          const int* __restrict__ cell_start, int* __restrict__ perm, int* __restrict__ big,
+                          int* __restrict__ nbig) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    perm[cell_start[cell_of[i]] + rank[i]] = i;
+    const int c = cell_of[i], r = rank[i], b = cell_start[c];
+    perm[b + r] = i;
+    if (r == 0 && cell_start[c + 1] - b > kSortSmall) big[atomicAdd(nbig, 1)] = c;
 }
 
 __device__ __forceinline__ void append(int* list, int* counter, bool pred, int value) {
@@ -145,6 +180,7 @@ __device__ __forceinline__ void append(int* list, int* counter, bool pred, int v
 template <bool SOIL>
 __global__ void k_reorder64(Consts c, const int* __restrict__ perm, Persist64 a, Persist64 b,
                             float4* __restrict__ pos32, float4* __restrict__ pos32l,
+                            const int* __restrict__ cell_of, const int* __restrict__ cell_start,
                             const long long* __restrict__ cell_src, long long* __restrict__ cell0,
                             unsigned char* __restrict__ cell_flow, int* __restrict__ list_flow,
                             int* __restrict__ list_bdy, int* __restrict__ list_count,
@@ -155,6 +191,14 @@ __global__ void k_reorder64(Consts c, const int* __restrict__ perm, Persist64 a,
     if (live) {
         const size_t n = c.n;
         const int s = perm[k];
+        // ascending old index inside the cell: this particle's rank among the cell's (a pass of
+        // its own, one thread per cell, took 15 us on a 2D grid and 158 us on the 3D benchmark's)
+        const int cell = cell_of[s], cb = cell_start[cell], ce = cell_start[cell + 1];
+        if (ce - cb <= kSortSmall) {
+            int r = 0;
+            for (int q = cb; q < ce; ++q) r += perm[q] < s;
+            k = cb + r;
+        }
         double xv[3];
         for (int d = 0; d < 3; ++d) {
             xv[d] = a.x[d * n + s];
@@ -195,6 +239,10 @@ inline int nblk(long long n) { return (int)((n + TPB - 1) / TPB); }
 }  // namespace
 
 void scan_exclusive(const int* in, int* out, int n, int* tile_sum, cudaStream_t s) {
+    if (n <= SCAN_ONE) {
+        TSG_LAUNCH(k_scan_one, 1, SCAN_ONE_TPB, s, in, n, out);
+        return;
+    }
     int ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     TSG_LAUNCH(k_tile_sums, ntiles, TPB, s, in, n, tile_sum);
     TSG_LAUNCH(k_scan_tiles, 1, TPB, s, tile_sum, ntiles);
@@ -204,15 +252,13 @@ void scan_exclusive(const int* in, int* out, int n, int* tile_sum, cudaStream_t 
 void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid& g, cudaStream_t s) {
     PhaseScope ph(s, PH_SORT);
     const long long nbins = c.G + 1;
-    cudaMemsetAsync(g.count, 0, sizeof(int) * nbins, s);
-    cudaMemsetAsync(g.list_count, 0, sizeof(int) * 2, s);
-    cudaMemsetAsync(g.cell_flow, 0, (size_t)c.G, s);
+    cudaMemsetAsync(g.count, 0, g.zero_bytes, s);
     TSG_LAUNCH(k_hash, nblk(c.n), TPB, s, c, cur.x, g.cell_of, g.rank, g.count, g.cell0_old, g.err);
     scan_exclusive(g.count, g.cell_start, (int)nbins, g.tile_sum, s);
-    TSG_LAUNCH(k_scatter, nblk(c.n), TPB, s, c.n, g.cell_of, g.rank, g.cell_start, g.perm);
-    sort_within_cells(nbins, g.cell_start, g.cell_of, c.n, g.perm, g.big, g.nbig, s);
+    TSG_LAUNCH(k_scatter, nblk(c.n), TPB, s, c.n, g.cell_of, g.rank, g.cell_start, g.perm, g.big, g.nbig);
+    TSG_LAUNCH(k_cell_sort_big, 152, kSortBlock, s, g.big, g.nbig, g.cell_start, g.cell_of, c.n, g.perm);
     if (c.solver == 1) {
-        TSG_LAUNCH(k_reorder64<false>, nblk(c.n), TPB, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell0_old,
+        TSG_LAUNCH(k_reorder64<false>, nblk(c.n), TPB, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, g.cell0_old,
                    t.cell0, g.cell_flow, g.list_flow, g.list_bdy, g.list_count, nullptr, nullptr);
     } else {
         // mu(I) keeps v_tmp across steps: stage it in aux3 (free until advect_pos) and gather
@@ -221,7 +267,7 @@ void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid
             cudaMemcpyAsync(t.aux3, t.v_tmp, sizeof(double) * 3 * (size_t)c.n, cudaMemcpyDeviceToDevice, s);
             src = t.aux3;
         }
-        TSG_LAUNCH(k_reorder64<true>, nblk(c.n), TPB, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell0_old,
+        TSG_LAUNCH(k_reorder64<true>, nblk(c.n), TPB, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, g.cell0_old,
                    t.cell0, g.cell_flow, g.list_flow, g.list_bdy, g.list_count, src, src ? t.v_tmp : nullptr);
     }
     Persist64 tmp = cur;
