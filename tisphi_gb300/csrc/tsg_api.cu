@@ -252,46 +252,10 @@ void own_rows(tsg_handle* h, bool geometry, cudaStream_t s) {
     if (geometry) fp64_geometry(h->c, h->cur, h->t, h->g, s);
 }
 
-// substep of the FP64 form on the current rows and geometry.
-int substep64(tsg_handle* h, cudaStream_t s) {
-    int stage = h->c.ti == 1 ? -1 : 0;
-    auto rates = [&] {
-        fp64_one_step(h->c, h->cur, h->t, h->g, stage, s);
-        if (stage >= 0) ++stage;
-    };
-    auto adv = [&](int which) { fp64_advect(h->c, h->cur, h->t, h->g, which, s); };
-    switch (h->c.ti) {
-    case 1: rates(); adv(TSG_ADVECT_FULL); break;
-    case 2: rates(); adv(TSG_ADVECT_LF_HALF); rates(); adv(TSG_ADVECT_FULL); break;
-    case 4: {
-        adv(TSG_RK_INIT);
-        const int m[4] = {1, 2, 2, 1};
-        for (int k = 0; k < 4; ++k) {
-            rates();
-            fp64_rk_update(h->c, h->cur, h->t, m[k], s);
-            if (k < 3) adv(TSG_RK_STAGE);
-        }
-        adv(TSG_RK_FINAL);
-        break;
-    }
-    default: return TSG_E_CONFIG;
-    }
-    return check_cuda();
-}
-
 // One step of the FP64 form after its sort.
-int step64(tsg_handle* h, bool collide, cudaStream_t s) {
-    const Consts& c = h->c;
-    fp64_build_rows(c, h->cur, h->t, h->g, true, s);
-    fp64_kernel_corr(c, h->cur, h->t, h->g, s);
-    fp64_init_tmp(c, h->cur, h->t, s);
-    if (int rc = substep64(h, s)) return rc;
-    fp64_advect(c, h->cur, h->t, h->g, TSG_ADVECT_POS, s);
+int step64(tsg_handle* h, bool collide, cudaStream_t s, const SideStream64* side = nullptr) {
+    fp64_step(h->c, h->cur, h->t, h->g, h->rigid, collide, s, side);
     h->pos32_dirty = true;
-    fp64_advect(c, h->cur, h->t, h->g, TSG_ADVECT_SOMETHING, s);
-    if (c.n_rigid_dyn) fp64_solve_rigid(c, h->cur, h->rigid, s);
-    // enforce_boundary also clamps dynamic rigid particles in every boundary mode
-    if (collide || c.n_rigid_dyn) fp64_advect(c, h->cur, h->t, h->g, TSG_ENFORCE_BOUNDARY, s);
     return check_cuda();
 }
 
@@ -313,15 +277,19 @@ tsg_handle::StepGraph* step_graph64(tsg_handle* h, int steps, bool collide) {
     if (g.exec && g.collide == collide) return &g;
     if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
     cudaStream_t cs = nullptr;
-    if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    SideStream64 side{};
+    bool ok = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming) == cudaSuccess &&
+              cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming) == cudaSuccess;
     const Persist64 cur = h->cur, nxt = h->nxt;
     const long long c0 = launch_total();
     cudaGraph_t graph = nullptr;
-    bool ok = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed) == cudaSuccess;
+    ok = ok && cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed) == cudaSuccess;
     if (ok) {
         for (int q = 0; q < steps && ok; ++q) {
             sort_fp64(h->c, h->cur, h->nxt, h->t, h->g, cs);
-            ok = step64(h, collide, cs) == 0;
+            ok = step64(h, collide, cs, &side) == 0;
         }
         ok = cudaStreamEndCapture(cs, &graph) == cudaSuccess && graph && ok;
     }
@@ -332,7 +300,10 @@ tsg_handle::StepGraph* step_graph64(tsg_handle* h, int steps, bool collide) {
     ok = ok && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
     if (!ok) g.exec = nullptr;
     if (graph) cudaGraphDestroy(graph);
-    cudaStreamDestroy(cs);
+    if (side.fork) cudaEventDestroy(side.fork);
+    if (side.join) cudaEventDestroy(side.join);
+    if (side.stream) cudaStreamDestroy(side.stream);
+    if (cs) cudaStreamDestroy(cs);
     cudaGetLastError();
     g.collide = collide;
     return ok ? &g : nullptr;
@@ -625,7 +596,7 @@ int tsg_init_tmp(tsg_handle* h, void* stream) {
     if (!h || !h->uploaded) return TSG_E_STATE;
     cudaStream_t s = S(stream);
     if (use_fp32(h)) fp32_init_tmp(*h->f32, s);
-    else fp64_init_tmp(h->c, h->cur, h->t, s);
+    else fp64_init_tmp(h->c, h->cur, h->t, h->g, s);
     return check_cuda();
 }
 
@@ -633,7 +604,7 @@ int tsg_one_step(tsg_handle* h, void* stream) {
     if (!h || !h->sorted) return TSG_E_STATE;
     cudaStream_t s = S(stream);
     if (use_fp32(h)) fp32_one_step(*h->f32, s);
-    else { own_rows(h, true, s); fp64_one_step(h->c, h->cur, h->t, h->g, -1, s); }
+    else { own_rows(h, true, s); fp64_one_step(h->c, h->cur, h->t, h->g, s); }
     return check_cuda();
 }
 
@@ -654,7 +625,7 @@ int tsg_advect(tsg_handle* h, int which, void* stream) {
 
 static void rk_update(tsg_handle* h, int m, cudaStream_t s) {
     if (use_fp32(h)) fp32_rk_update(*h->f32, m, s);
-    else fp64_rk_update(h->c, h->cur, h->t, m, s);
+    else fp64_rk_update(h->c, h->cur, h->t, h->g, m, s);
 }
 
 int tsg_rk_update(tsg_handle* h, int32_t m, void* stream) {
@@ -668,7 +639,8 @@ int tsg_substep(tsg_handle* h, void* stream) {
     if (!h || !h->sorted) return TSG_E_STATE;
     if (!use_fp32(h)) {
         own_rows(h, true, S(stream));
-        return substep64(h, S(stream));
+        fp64_substep(h->c, h->cur, h->t, h->g, S(stream));
+        return check_cuda();
     }
     int rc = 0;
     switch (h->c.ti) {

@@ -7,12 +7,12 @@
 // products: q1^4 = (q1*q1)*(q1*q1), q1^3 = (q1*q1)*q1, x**2 = x*x.
 //
 // Kernels (one thread per particle; boundary / flow particles through index lists):
-//   k_corr        Shepard factor for all particles, CSPM matrix for flow particles
-//                 (eng/solver_sph_base.py:386-423), one neighbour traversal.
-//   k_init_tmp    init_real2tmp (eng/solver_sph_base.py:67-74).
-//   k_pre         per-particle first phase of one_step: Tait EOS (WC,
-//                 eng/solver_sph_wc.py:86-88) or stress adaptation (DP,
-//                 eng/solver_sph_dp.py:215-217).
+//   k_corr_flow, k_corr_bdy  Shepard factor for all particles, CSPM matrix for flow particles
+//                 (eng/solver_sph_base.py:386-423), pair geometry of the rows.
+//   k_particle    the per-particle passes: init_real2tmp (eng/solver_sph_base.py:67-74), the
+//                 first phase of one_step (Tait EOS, eng/solver_sph_wc.py:86-88, or stress
+//                 adaptation, eng/solver_sph_dp.py:215-217), the integrators, advect_pos and
+//                 the solvers' post-steps (eng/solver_sph_base.py:79-247, solver overrides).
 //   k_bdy         dummy-boundary extrapolation of v_tmp, density_tmp, pressure / stress
 //                 (eng/solver_sph_wc.py:90-103, eng/solver_sph_muI.py:97-109,
 //                 eng/solver_sph_dp.py:219-234), all sums in one traversal.
@@ -21,7 +21,6 @@
 //   k_mui_mom     mu(I) stress divergence + damping (eng/solver_sph_muI.py:113-128).
 //   k_dp_rates    DP velocity gradient, continuity, Bui-2008 stress rate, stress
 //                 divergence, damping (eng/solver_sph_dp.py:236-270), one traversal.
-//   advection / post-step kernels (eng/solver_sph_base.py:79-247, solver overrides).
 #include <cfloat>
 
 #include "tsg_internal.h"
@@ -415,9 +414,7 @@ __global__ void k_density_sum(Consts c, Persist64 p, Trans64 t, const int* __res
     out[i] = ret;
 }
 
-__global__ void k_init_tmp(Consts c, Persist64 p, Trans64 t) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_init(const Consts& c, const Persist64& p, const Trans64& t, int i) {
     const int n = c.n;
     const int ti = p.mat_type[i];
     if (ti > 0) {
@@ -515,11 +512,8 @@ __device__ __forceinline__ void soil_record(const Consts& c, double* rec, int i,
     }
 }
 
-// First, per-particle phase of one_step.
-__global__ void k_pre(Consts c, Persist64 p, Trans64 t, const int* __restrict__ list, int count, Pairs64 pr) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int i = list[k];
+// First, per-particle phase of one_step (flow particles; mu(I) has none).
+__device__ __forceinline__ void do_pre(const Consts& c, const Persist64& p, const Trans64& t, int i, const Pairs64& pr) {
     const int n = c.n;
     const double rt = t.density_tmp[i], mV = p.m_V[i];
     double vt[3];
@@ -1090,9 +1084,7 @@ __global__ void __launch_bounds__(ROWS * G) k_dp_rates(Consts c, Persist64 p, Tr
 }
 
 // ---- integrators (eng/solver_sph_base.py:79-170) ----
-__global__ void k_advect_full(Consts c, Persist64 p, Trans64 t, int* err) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_full(const Consts& c, const Persist64& p, const Trans64& t, int i, int* err) {
     const int n = c.n;
     const int ti = p.mat_type[i];
     if (ti > 0) {
@@ -1106,9 +1098,7 @@ __global__ void k_advect_full(Consts c, Persist64 p, Trans64 t, int* err) {
         for (int q = 0; q < 9; ++q) p.stress[(size_t)q * n + i] += c.dt * t.d_stress[(size_t)q * n + i];
 }
 
-__global__ void k_advect_half(Consts c, Persist64 p, Trans64 t) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_half(const Consts& c, const Persist64& p, const Trans64& t, int i) {
     const int n = c.n;
     const int ti = p.mat_type[i];
     if (ti > 0) {
@@ -1121,9 +1111,7 @@ __global__ void k_advect_half(Consts c, Persist64 p, Trans64 t) {
         for (int q = 0; q < 9; ++q) t.stress_tmp[(size_t)q * n + i] += c.hdt * t.d_stress[(size_t)q * n + i];
 }
 
-__global__ void k_rk_init(Consts c, Persist64 p, Trans64 t) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_rk_init(const Consts& c, const Persist64& p, const Trans64& t, int i) {
     const int n = c.n;
     const int ti = p.mat_type[i];
     if (ti > 0) {
@@ -1134,9 +1122,7 @@ __global__ void k_rk_init(Consts c, Persist64 p, Trans64 t) {
         for (int q = 0; q < 9; ++q) t.d_stress_RK[(size_t)q * n + i] = 0.0;
 }
 
-__global__ void k_rk_update(Consts c, Persist64 p, Trans64 t, int m) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_rk_update(const Consts& c, const Persist64& p, const Trans64& t, int i, int m) {
     const int n = c.n;
     const int ti = p.mat_type[i];
     if (ti > 0) {
@@ -1147,9 +1133,7 @@ __global__ void k_rk_update(Consts c, Persist64 p, Trans64 t, int m) {
         for (int q = 0; q < 9; ++q) t.d_stress_RK[(size_t)q * n + i] += (double)m * t.d_stress[(size_t)q * n + i];
 }
 
-__global__ void k_rk_stage(Consts c, Persist64 p, Trans64 t) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_rk_stage(const Consts& c, const Persist64& p, const Trans64& t, int i) {
     const int n = c.n;
     const int ti = p.mat_type[i];
     if (ti > 0) {
@@ -1164,9 +1148,7 @@ __global__ void k_rk_stage(Consts c, Persist64 p, Trans64 t) {
             t.stress_tmp[(size_t)q * n + i] = c.hdt * t.d_stress[(size_t)q * n + i] + p.stress[(size_t)q * n + i];
 }
 
-__global__ void k_rk_final(Consts c, Persist64 p, Trans64 t, int* err) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_rk_final(const Consts& c, const Persist64& p, const Trans64& t, int i, int* err) {
     const int n = c.n;
     const int ti = p.mat_type[i];
     if (ti > 0) {
@@ -1245,9 +1227,7 @@ __global__ void k_xsph_rigid(Consts c, Persist64 p, Trans64 t, const int* __rest
     for (int d = 0; d < 3; ++d) t.aux3[(size_t)d * n + i] = s[d];
 }
 
-__global__ void k_advect_pos(Consts c, Persist64 p, Trans64 t, int* err) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_pos(const Consts& c, const Persist64& p, const Trans64& t, int i, int* err) {
     const int n = c.n;
     const int ti = p.mat_type[i];
     if (!(ti > 0)) return;
@@ -1264,18 +1244,14 @@ __global__ void k_advect_pos(Consts c, Persist64 p, Trans64 t, int* err) {
 }
 
 // ---- advect_something (solver post-steps) ----
-__global__ void k_post_wc(Consts c, Persist64 p) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_post_wc(const Consts& c, const Persist64& p, int i) {
     if (p.mat_type[i] != MAT_FLUID) return;
     double rho = fmax(c.rho0, p.density[i]);
     p.density[i] = rho;
     p.m_V[i] = p.mass[i] / rho;
 }
 
-__global__ void k_post_mui_a(Consts c, Persist64 p, Trans64 t) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_post_mui(const Consts& c, const Persist64& p, const Trans64& t, int i) {
     if (p.mat_type[i] != MAT_SOIL) return;
     const int n = c.n;
     double rho = fmax(c.rho0, p.density[i]);
@@ -1333,9 +1309,7 @@ __global__ void k_post_mui_c(Consts c, Persist64 p, Trans64 t) {
     for (int q = 0; q < 9; ++q) p.stress[(size_t)q * n + i] = t.aux9[(size_t)q * n + i];
 }
 
-__global__ void k_post_dp(Consts c, Persist64 p, Trans64 t) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void do_post_dp(const Consts& c, const Persist64& p, const Trans64& t, int i) {
     if (p.mat_type[i] != MAT_SOIL) return;
     const int n = c.n;
     double rho = fmax(c.rho0, p.density[i]);
@@ -1348,6 +1322,34 @@ __global__ void k_post_dp(Consts c, Persist64 p, Trans64 t) {
     for (int q = 0; q < 9; ++q) p.stress[(size_t)q * n + i] = st[q];
     p.strain_equ[i] += c.dt * t.d_strain_equ[i];
     p.strain_equ_p[i] += c.dt * t.d_strain_equ_p[i];
+}
+
+// ---- per-particle passes ----
+// The passes of a step between its pair loops, in the order of the bits; every value they
+// exchange belongs to one particle, so a launch runs all that lie between two loops (a leap-frog
+// step: 3 launches instead of 7 of about 3 us each on a small scene).
+enum : unsigned {
+    OP_INIT = 1, OP_RK_INIT = 2, OP_RK_UPDATE = 4, OP_HALF = 8, OP_RK_STAGE = 16, OP_FULL = 32, OP_RK_FINAL = 64,
+    OP_PRE = 128, OP_POS = 256, OP_POST = 512
+};
+__global__ void __launch_bounds__(TPB) k_particle(Consts c, Persist64 p, Trans64 t, Pairs64 pr, unsigned ops, int m,
+                                                  int* err) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n) return;
+    if (ops & OP_INIT) do_init(c, p, t, i);
+    if (ops & OP_RK_INIT) do_rk_init(c, p, t, i);
+    if (ops & OP_RK_UPDATE) do_rk_update(c, p, t, i, m);
+    if (ops & OP_HALF) do_half(c, p, t, i);
+    if (ops & OP_RK_STAGE) do_rk_stage(c, p, t, i);
+    if (ops & OP_FULL) do_full(c, p, t, i, err);
+    if (ops & OP_RK_FINAL) do_rk_final(c, p, t, i, err);
+    if ((ops & OP_PRE) && p.mat_type[i] == c.flow_type) do_pre(c, p, t, i, pr);
+    if (ops & OP_POS) do_pos(c, p, t, i, err);
+    if (ops & OP_POST) {
+        if (c.solver == 1) do_post_wc(c, p, i);
+        else if (c.solver == 2) do_post_mui(c, p, t, i);
+        else do_post_dp(c, p, t, i);
+    }
 }
 
 // ---- enforce_boundary (eng/solver_sph_base.py:525-601) ----
@@ -1735,15 +1737,33 @@ void fp64_geometry(const Consts& c, const Persist64& p, Trans64& t, const Grid& 
     if (c.n_bdy > 0) DISPATCH_ROWS(c, g, k_geom_bdy, c.n_bdy, c, p, g.list_bdy, c.n_bdy, g.pr);
 }
 
-void fp64_kernel_corr(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+static void particle_pass(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, unsigned ops, int m,
+                          cudaStream_t s) {
+    if (c.solver == 2) ops &= ~(unsigned)OP_PRE;
+    if (!ops) return;
+    PhaseScope ph(s, ops & (OP_HALF | OP_RK_STAGE | OP_RK_UPDATE | OP_FULL | OP_RK_FINAL | OP_RK_INIT) ? PH_INTEGRATE
+                     : ops & OP_INIT ? PH_INIT : ops & OP_PRE ? PH_PRE : ops & OP_POS ? PH_POS : PH_POST);
+    TSG_LAUNCH(k_particle, nblk(c.n), TPB, s, c, p, t, g.pr, ops, m, g.err);
+}
+
+static void corr_flow(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+    if (c.n_flow <= 0) return;
     PhaseScope ph(s, PH_CORR);
-    if (c.n_flow > 0) {
-        if (c.corr == 1)
-            DISPATCH_ROWS_B(c, g, k_corr_flow, true, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
-        else
-            DISPATCH_ROWS_B(c, g, k_corr_flow, false, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
-    }
-    if (c.n_bdy > 0) DISPATCH_ROWS(c, g, k_corr_bdy, c.n_bdy, c, p, t, g.cell_start, g.list_bdy, c.n_bdy, g.pr);
+    if (c.corr == 1)
+        DISPATCH_ROWS_B(c, g, k_corr_flow, true, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+    else
+        DISPATCH_ROWS_B(c, g, k_corr_flow, false, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+}
+
+static void corr_bdy(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+    if (c.n_bdy <= 0) return;
+    PhaseScope ph(s, PH_CORR);
+    DISPATCH_ROWS(c, g, k_corr_bdy, c.n_bdy, c, p, t, g.cell_start, g.list_bdy, c.n_bdy, g.pr);
+}
+
+void fp64_kernel_corr(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+    corr_flow(c, p, t, g, s);
+    corr_bdy(c, p, t, g, s);
 }
 
 void fp64_rest_cm(const Consts& c, const Persist64& p, const Rigid64& r, cudaStream_t s) {
@@ -1765,32 +1785,36 @@ void fp64_density_sum(const Consts& c, const Persist64& p, const Trans64& t, con
     DISPATCH_DIM(c, k_density_sum, nblk(c.n), c, p, t, g.cell_start, out);
 }
 
-void fp64_init_tmp(const Consts& c, const Persist64& p, Trans64& t, cudaStream_t s) {
-    PhaseScope ph(s, PH_INIT);
-    TSG_LAUNCH(k_init_tmp, nblk(c.n), TPB, s, c, p, t);
+void fp64_init_tmp(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+    particle_pass(c, p, t, g, OP_INIT, 0, s);
 }
 
-void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int stage, cudaStream_t s) {
-    // without the correction the gradient is grad W itself: nothing to keep
-    const int kc = c.corr != 1 || stage < 0 ? KC_MAKE : stage == 0 ? KC_KEEP : KC_READ;
-    if (c.n_flow > 0 && (c.solver == 1 || c.solver == 3)) {
-        PhaseScope ph(s, PH_PRE);
-        TSG_LAUNCH(k_pre, nblk(c.n_flow), TPB, s, c, p, t, g.list_flow, c.n_flow, g.pr);
-    }
-    if (c.solver == 2 && c.n_flow > 0) {
-        PhaseScope ph(s, PH_PRE);
-        const int kc1 = c.corr == 1 && kc == KC_MAKE ? KC_KEEP : kc;  // the momentum loop reads it
-        DISPATCH_KC3(c, g, k_mui_stress, LANES, kc1, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
-    }
-    if (c.n_bdy > 0) {
-        PhaseScope ph(s, PH_BDY);
-        if (c.solver == 1)
-            DISPATCH_ROWS_B(c, g, k_bdy, false, c.n_bdy, c, p, t, g.cell_start, g.list_bdy, c.n_bdy, g.pr);
-        else
-            DISPATCH_ROWS_B(c, g, k_bdy, true, c.n_bdy, c, p, t, g.cell_start, g.list_bdy, c.n_bdy, g.pr);
-    }
+// The loops of one_step after its per-particle first phase.  stage: how often this step's loops
+// have run before (the first stores the corrected gradients for the others); -1: the only time.
+// Without the correction the gradient is grad W itself: nothing to keep.
+static int gradient_mode(const Consts& c, int stage) {
+    return c.corr != 1 || stage < 0 ? KC_MAKE : stage == 0 ? KC_KEEP : KC_READ;
+}
+
+static void mui_stress(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int stage, cudaStream_t s) {
+    if (c.solver != 2 || c.n_flow <= 0) return;
+    PhaseScope ph(s, PH_PRE);
+    int kc = gradient_mode(c, stage);
+    if (c.corr == 1 && kc == KC_MAKE) kc = KC_KEEP;  // the momentum loop reads it
+    DISPATCH_KC3(c, g, k_mui_stress, LANES, kc, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+}
+
+static void bdy(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+    if (c.n_bdy <= 0) return;
+    PhaseScope ph(s, PH_BDY);
+    if (c.solver == 1) DISPATCH_ROWS_B(c, g, k_bdy, false, c.n_bdy, c, p, t, g.cell_start, g.list_bdy, c.n_bdy, g.pr);
+    else DISPATCH_ROWS_B(c, g, k_bdy, true, c.n_bdy, c, p, t, g.cell_start, g.list_bdy, c.n_bdy, g.pr);
+}
+
+static void rates(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int stage, cudaStream_t s) {
     if (c.n_flow > 0) {
         PhaseScope ph(s, PH_RATES);
+        const int kc = gradient_mode(c, stage);
         if (c.solver == 1)
             DISPATCH_KC3(c, g, k_wc_rates, LANES, kc, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
         else if (c.solver == 2 && c.corr == 1)
@@ -1806,45 +1830,122 @@ void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int
     }
 }
 
-void fp64_advect(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int which, cudaStream_t s) {
-    const int nb = nblk(c.n);
-    PhaseScope ph(s, which == TSG_ADVECT_POS ? PH_POS : which == TSG_ADVECT_SOMETHING ? PH_POST
-                     : which == TSG_ENFORCE_BOUNDARY ? PH_OTHER : PH_INTEGRATE);
-    switch (which) {
-    case TSG_ADVECT_FULL: TSG_LAUNCH(k_advect_full, nb, TPB, s, c, p, t, g.err); break;
-    case TSG_ADVECT_LF_HALF: TSG_LAUNCH(k_advect_half, nb, TPB, s, c, p, t); break;
-    case TSG_ADVECT_POS:
-        if (c.xsph) {
-            if (c.n_flow > 0)
-                DISPATCH_ROWS(c, g, k_xsph, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
-            if (c.n_rigid_dyn > 0)
-                DISPATCH_DIM(c, k_xsph_rigid, nblk(c.n_bdy), c, p, t, g.cell_start, g.list_bdy, c.n_bdy);
+void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+    particle_pass(c, p, t, g, OP_PRE, 0, s);
+    mui_stress(c, p, t, g, -1, s);
+    bdy(c, p, t, g, s);
+    rates(c, p, t, g, -1, s);
+}
+
+static void xsph(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+    if (!c.xsph) return;
+    PhaseScope ph(s, PH_POS);
+    if (c.n_flow > 0) DISPATCH_ROWS(c, g, k_xsph, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+    if (c.n_rigid_dyn > 0) DISPATCH_DIM(c, k_xsph_rigid, nblk(c.n_bdy), c, p, t, g.cell_start, g.list_bdy, c.n_bdy);
+}
+
+// mu(I): what follows the per-particle part of advect_something.
+static void mui_regularise(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+    if (c.solver != 2 || c.n_flow <= 0) return;
+    PhaseScope ph(s, PH_POST);
+    if (g.pr.cap_f) fp64_refresh_pos32(c, p, t, s);
+    build_rows(c, p, t, g, true, false, s);
+    DISPATCH_ROWS(c, g, k_post_mui_b, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+    TSG_LAUNCH(k_post_mui_c, nblk(c.n), TPB, s, c, p, t);
+}
+
+// substep by the integrator, from the per-particle first phase of its first loops (run by the
+// caller) to its last update, which `tail` follows in the same launch.  first_bdy: the first
+// boundary loop is still to run.
+static void substep_loops(const Consts& c, Persist64& p, Trans64& t, const Grid& g, unsigned tail, bool first_bdy,
+                          cudaStream_t s) {
+    auto loops = [&](int stage, bool with_bdy) {
+        mui_stress(c, p, t, g, stage, s);
+        if (with_bdy) bdy(c, p, t, g, s);
+        rates(c, p, t, g, stage, s);
+    };
+    if (c.ti == 1) {
+        loops(-1, first_bdy);
+        particle_pass(c, p, t, g, OP_FULL | tail, 0, s);
+    } else if (c.ti == 2) {
+        loops(0, first_bdy);
+        particle_pass(c, p, t, g, OP_HALF | OP_PRE, 0, s);
+        loops(1, true);
+        particle_pass(c, p, t, g, OP_FULL | tail, 0, s);
+    } else {
+        const int m[4] = {1, 2, 2, 1};
+        for (int k = 0; k < 4; ++k) {
+            loops(k, k > 0 || first_bdy);
+            particle_pass(c, p, t, g, OP_RK_UPDATE | (k < 3 ? OP_RK_STAGE | OP_PRE : OP_RK_FINAL | tail), m[k], s);
         }
-        TSG_LAUNCH(k_advect_pos, nb, TPB, s, c, p, t, g.err);
+    }
+}
+static unsigned substep_head(const Consts& c) { return (c.ti == 4 ? OP_RK_INIT : 0u) | OP_PRE; }
+
+void fp64_substep(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
+    particle_pass(c, p, t, g, substep_head(c), 0, s);
+    substep_loops(c, p, t, g, 0, true, s);
+}
+
+void fp64_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, const Rigid64& r, bool collide,
+               cudaStream_t s, const SideStream64* side) {
+    fp64_build_rows(c, p, t, g, true, s);
+    // The correction pass over the flow rows and what the first rates loop needs besides (the
+    // per-particle start, the boundary rows' Shepard factors and extrapolation) touch different
+    // arrays: two branches of the graph (a small scene fills neither the GPU nor a launch's
+    // latency with one of them).  mu(I) extrapolates after its stress loop.
+    const bool early_bdy = c.solver != 2;
+    cudaStream_t b = s;
+    if (side) {
+        b = side->stream;
+        cudaEventRecord(side->fork, s);
+        cudaStreamWaitEvent(b, side->fork, 0);
+    }
+    corr_flow(c, p, t, g, s);
+    particle_pass(c, p, t, g, OP_INIT | substep_head(c), 0, b);
+    corr_bdy(c, p, t, g, b);
+    if (early_bdy) bdy(c, p, t, g, b);
+    if (side) {
+        cudaEventRecord(side->join, b);
+        cudaStreamWaitEvent(s, side->join, 0);
+    }
+    substep_loops(c, p, t, g, c.xsph ? 0u : OP_POS | OP_POST, !early_bdy, s);
+    if (c.xsph) {
+        xsph(c, p, t, g, s);
+        particle_pass(c, p, t, g, OP_POS | OP_POST, 0, s);
+    }
+    mui_regularise(c, p, t, g, s);
+    if (c.n_rigid_dyn) fp64_solve_rigid(c, p, r, s);
+    // enforce_boundary also clamps dynamic rigid particles in every boundary mode
+    if (collide || c.n_rigid_dyn) fp64_advect(c, p, t, g, TSG_ENFORCE_BOUNDARY, s);
+}
+
+void fp64_advect(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int which, cudaStream_t s) {
+    switch (which) {
+    case TSG_ADVECT_FULL: particle_pass(c, p, t, g, OP_FULL, 0, s); break;
+    case TSG_ADVECT_LF_HALF: particle_pass(c, p, t, g, OP_HALF, 0, s); break;
+    case TSG_ADVECT_POS:
+        xsph(c, p, t, g, s);
+        particle_pass(c, p, t, g, OP_POS, 0, s);
         break;
     case TSG_ADVECT_SOMETHING:
-        if (c.solver == 1) TSG_LAUNCH(k_post_wc, nb, TPB, s, c, p);
-        else if (c.solver == 2) {
-            TSG_LAUNCH(k_post_mui_a, nb, TPB, s, c, p, t);
-            if (c.n_flow > 0) {
-                if (g.pr.cap_f) fp64_refresh_pos32(c, p, t, s);
-                build_rows(c, p, t, g, true, false, s);
-                DISPATCH_ROWS(c, g, k_post_mui_b, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
-            }
-            TSG_LAUNCH(k_post_mui_c, nb, TPB, s, c, p, t);
-        } else TSG_LAUNCH(k_post_dp, nb, TPB, s, c, p, t);
+        particle_pass(c, p, t, g, OP_POST, 0, s);
+        mui_regularise(c, p, t, g, s);
         break;
-    case TSG_ENFORCE_BOUNDARY: TSG_LAUNCH(k_enforce, nb, TPB, s, c, p); break;
-    case TSG_RK_INIT: TSG_LAUNCH(k_rk_init, nb, TPB, s, c, p, t); break;
-    case TSG_RK_STAGE: TSG_LAUNCH(k_rk_stage, nb, TPB, s, c, p, t); break;
-    case TSG_RK_FINAL: TSG_LAUNCH(k_rk_final, nb, TPB, s, c, p, t, g.err); break;
+    case TSG_ENFORCE_BOUNDARY: {
+        PhaseScope ph(s, PH_OTHER);
+        TSG_LAUNCH(k_enforce, nblk(c.n), TPB, s, c, p);
+        break;
+    }
+    case TSG_RK_INIT: particle_pass(c, p, t, g, OP_RK_INIT, 0, s); break;
+    case TSG_RK_STAGE: particle_pass(c, p, t, g, OP_RK_STAGE, 0, s); break;
+    case TSG_RK_FINAL: particle_pass(c, p, t, g, OP_RK_FINAL, 0, s); break;
     default: break;
     }
 }
 
-void fp64_rk_update(const Consts& c, Persist64& p, Trans64& t, int m, cudaStream_t s) {
-    PhaseScope ph(s, PH_INTEGRATE);
-    TSG_LAUNCH(k_rk_update, nblk(c.n), TPB, s, c, p, t, m);
+void fp64_rk_update(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int m, cudaStream_t s) {
+    particle_pass(c, p, t, g, OP_RK_UPDATE, m, s);
 }
 
 void fp64_neighbors(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g,

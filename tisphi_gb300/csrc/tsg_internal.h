@@ -193,12 +193,16 @@ void fp64_kernel_corr(const Consts& c, const Persist64& p, Trans64& t, const Gri
 void fp64_build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, bool sorted,
                      cudaStream_t s);
 void fp64_geometry(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
-void fp64_init_tmp(const Consts& c, const Persist64& p, Trans64& t, cudaStream_t s);
-// stage: how often this step's loops have run before (the first stores the corrected gradients
-// for the others); -1: a loop on its own.
-void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int stage, cudaStream_t s);
+void fp64_init_tmp(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
+void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
+// substep (its integrator's loops and updates) on current rows and geometry.
+void fp64_substep(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
+// A step after its sort.  side: a second stream and two events while capturing, else null.
+struct SideStream64 { cudaStream_t stream; cudaEvent_t fork, join; };
+void fp64_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, const Rigid64& r, bool collide,
+               cudaStream_t s, const SideStream64* side);
 void fp64_advect(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int which, cudaStream_t s);
-void fp64_rk_update(const Consts& c, Persist64& p, Trans64& t, int m, cudaStream_t s);
+void fp64_rk_update(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int m, cudaStream_t s);
 void fp64_neighbors(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g,
                     int* counts, int* offsets, int* list, cudaStream_t s);
 void fp64_diag(const Consts& c, const Persist64& p, double* out8, cudaStream_t s);
