@@ -414,17 +414,6 @@ __global__ void k_density_sum(Consts c, Persist64 p, Trans64 t, const int* __res
     out[i] = ret;
 }
 
-__device__ __forceinline__ void do_init(const Consts& c, const Persist64& p, const Trans64& t, int i) {
-    const int n = c.n;
-    const int ti = p.mat_type[i];
-    if (ti > 0) {
-        t.density_tmp[i] = p.density[i];
-        for (int d = 0; d < 3; ++d) t.v_tmp[(size_t)d * n + i] = p.v[(size_t)d * n + i];
-    }
-    if (ti == MAT_SOIL)
-        for (int q = 0; q < 9; ++q) t.stress_tmp[(size_t)q * n + i] = p.stress[(size_t)q * n + i];
-}
-
 // ---- Drucker-Prager invariants and return mapping (eng/solver_sph_dp.py:42-109) ----
 __device__ __forceinline__ double mtrace(const double* a) { return (a[0] + a[4]) + a[8]; }
 __device__ __forceinline__ double msum_sq(const double* a) {
@@ -512,27 +501,6 @@ __device__ __forceinline__ void soil_record(const Consts& c, double* rec, int i,
     }
 }
 
-// First, per-particle phase of one_step (flow particles; mu(I) has none).
-__device__ __forceinline__ void do_pre(const Consts& c, const Persist64& p, const Trans64& t, int i, const Pairs64& pr) {
-    const int n = c.n;
-    const double rt = t.density_tmp[i], mV = p.m_V[i];
-    double vt[3];
-    for (int d = 0; d < 3; ++d) vt[d] = t.v_tmp[(size_t)d * n + i];
-    if (c.solver == 1) {
-        double ratio = rt / c.rho0;
-        double pw = c.exponent_is_int ? powi(ratio, (long)c.gamma) : pow(ratio, c.gamma);
-        const double pres = fmax(c.B * (pw - 1.0), 0.0);
-        p.pressure[i] = pres;
-        wc_record(c, pr.rec, i, vt, pres, rt, mV, p.mat_type[i] == MAT_FLUID);
-    } else if (c.solver == 3) {
-        double st[9];
-        for (int q = 0; q < 9; ++q) st[q] = t.stress_tmp[(size_t)q * n + i];
-        dp_adapt(c, st);
-        for (int q = 0; q < 9; ++q) t.stress_tmp[(size_t)q * n + i] = st[q];
-        soil_record(c, pr.rec, i, vt, st, rt, mV);
-    }
-}
-
 // One flow neighbour's terms of the dummy extrapolation: v (DIM), then p (WCSPH) or density (1)
 // and stress (9).  w = W(r), r = x_i - x_j.
 template <int DIM, bool SOIL>
@@ -592,17 +560,17 @@ __global__ void __launch_bounds__(ROWS * G) k_bdy(Consts c, Persist64 p, Trans64
         });
     }
     const int ti = p.mat_type[i];
-    const double f = t.CSPM_f[i];
+    const double f = t.CSPM_f[i], mV = p.m_V[i];
+    const bool dyn = ti == MAT_RIGID && p.is_dynamic[i] != 0;
     double vt[3], rt;
-    for (int d = 0; d < 3; ++d) {
-        vt[d] = 2 * p.v[(size_t)d * n + i] - (d < DIM ? B[d < DIM ? d : 0] : 0.0) * f;
-        t.v_tmp[(size_t)d * n + i] = vt[d];
-    }
+    ld3(vt, p.v, n, i);
+    for (int d = 0; d < 3; ++d) vt[d] = 2 * vt[d] - (d < DIM ? B[d < DIM ? d : 0] : 0.0) * f;
+    st3(t.v_tmp, vt, n, i);
     if (!SOIL) {
         rt = c.rho0;
         const double pres = fmax(B[DIM] * f, 0.0);
         p.pressure[i] = pres;
-        wc_record(c, pr.rec, i, vt, pres, rt, p.m_V[i], false);
+        wc_record(c, pr.rec, i, vt, pres, rt, mV, false);
     } else {
         rt = c.solver == 2 ? fmax(B[DIM] * f, c.rho0) : c.rho0;
         double st[9];
@@ -610,7 +578,7 @@ __global__ void __launch_bounds__(ROWS * G) k_bdy(Consts c, Persist64 p, Trans64
             st[q] = B[(SOIL ? DIM + 1 : 0) + (SOIL ? q : 0)] * f;
             t.stress_tmp[(size_t)q * n + i] = st[q];
         }
-        soil_record(c, pr.rec, i, vt, st, rt, p.m_V[i]);
+        soil_record(c, pr.rec, i, vt, st, rt, mV);
     }
     t.density_tmp[i] = rt;
     // static rigid: rates stay zero; dynamic rigid: gravity, then the reaction.  Dummy and
@@ -618,7 +586,6 @@ __global__ void __launch_bounds__(ROWS * G) k_bdy(Consts c, Persist64 p, Trans64
     // never-written rates travel with it through the sort (the rate arrays here are not
     // reordered, so a slot may hold another particle's)
     t.d_density[i] = 0.0;
-    const bool dyn = ti == MAT_RIGID && p.is_dynamic[i] != 0;
     for (int d = 0; d < 3; ++d) t.d_vel[(size_t)d * n + i] = dyn ? c.g[d] : 0.0;
 }
 
@@ -1083,85 +1050,6 @@ __global__ void __launch_bounds__(ROWS * G) k_dp_rates(Consts c, Persist64 p, Tr
     for (int d = 0; d < 3; ++d) t.d_vel[(size_t)d * n + i] = (dv[d] + c.g[d]) + fd[d];
 }
 
-// ---- integrators (eng/solver_sph_base.py:79-170) ----
-__device__ __forceinline__ void do_full(const Consts& c, const Persist64& p, const Trans64& t, int i, int* err) {
-    const int n = c.n;
-    const int ti = p.mat_type[i];
-    if (ti > 0) {
-        double rho = p.density[i] + c.dt * t.d_density[i];
-        p.density[i] = rho;
-        p.m_V[i] = p.mass[i] / rho;
-        for (int d = 0; d < 3; ++d) p.v[(size_t)d * n + i] += c.dt * t.d_vel[(size_t)d * n + i];
-        if (!isfinite(rho)) atomicOr(err, TSG_ERR_NONFINITE);
-    }
-    if (ti == MAT_SOIL && c.solver == 3)
-        for (int q = 0; q < 9; ++q) p.stress[(size_t)q * n + i] += c.dt * t.d_stress[(size_t)q * n + i];
-}
-
-__device__ __forceinline__ void do_half(const Consts& c, const Persist64& p, const Trans64& t, int i) {
-    const int n = c.n;
-    const int ti = p.mat_type[i];
-    if (ti > 0) {
-        double rt = t.density_tmp[i] + c.hdt * t.d_density[i];
-        t.density_tmp[i] = rt;
-        p.m_V[i] = p.mass[i] / rt;
-        for (int d = 0; d < 3; ++d) t.v_tmp[(size_t)d * n + i] += c.hdt * t.d_vel[(size_t)d * n + i];
-    }
-    if (ti == MAT_SOIL && c.solver == 3)
-        for (int q = 0; q < 9; ++q) t.stress_tmp[(size_t)q * n + i] += c.hdt * t.d_stress[(size_t)q * n + i];
-}
-
-__device__ __forceinline__ void do_rk_init(const Consts& c, const Persist64& p, const Trans64& t, int i) {
-    const int n = c.n;
-    const int ti = p.mat_type[i];
-    if (ti > 0) {
-        t.d_density_RK[i] = 0.0;
-        for (int d = 0; d < 3; ++d) t.d_vel_RK[(size_t)d * n + i] = 0.0;
-    }
-    if (ti == MAT_SOIL && t.d_stress_RK)
-        for (int q = 0; q < 9; ++q) t.d_stress_RK[(size_t)q * n + i] = 0.0;
-}
-
-__device__ __forceinline__ void do_rk_update(const Consts& c, const Persist64& p, const Trans64& t, int i, int m) {
-    const int n = c.n;
-    const int ti = p.mat_type[i];
-    if (ti > 0) {
-        t.d_density_RK[i] += t.d_density[i] * m;
-        for (int d = 0; d < 3; ++d) t.d_vel_RK[(size_t)d * n + i] += t.d_vel[(size_t)d * n + i] * m;
-    }
-    if (ti == MAT_SOIL && t.d_stress_RK)
-        for (int q = 0; q < 9; ++q) t.d_stress_RK[(size_t)q * n + i] += (double)m * t.d_stress[(size_t)q * n + i];
-}
-
-__device__ __forceinline__ void do_rk_stage(const Consts& c, const Persist64& p, const Trans64& t, int i) {
-    const int n = c.n;
-    const int ti = p.mat_type[i];
-    if (ti > 0) {
-        double rt = c.hdt * t.d_density[i] + p.density[i];
-        t.density_tmp[i] = rt;
-        p.m_V[i] = p.mass[i] / rt;
-        for (int d = 0; d < 3; ++d)
-            t.v_tmp[(size_t)d * n + i] = c.hdt * t.d_vel[(size_t)d * n + i] + p.v[(size_t)d * n + i];
-    }
-    if (ti == MAT_SOIL && c.solver == 3)
-        for (int q = 0; q < 9; ++q)
-            t.stress_tmp[(size_t)q * n + i] = c.hdt * t.d_stress[(size_t)q * n + i] + p.stress[(size_t)q * n + i];
-}
-
-__device__ __forceinline__ void do_rk_final(const Consts& c, const Persist64& p, const Trans64& t, int i, int* err) {
-    const int n = c.n;
-    const int ti = p.mat_type[i];
-    if (ti > 0) {
-        double rho = p.density[i] + c.dt6 * t.d_density_RK[i];
-        p.density[i] = rho;
-        p.m_V[i] = p.mass[i] / rho;
-        for (int d = 0; d < 3; ++d) p.v[(size_t)d * n + i] += c.dt6 * t.d_vel_RK[(size_t)d * n + i];
-        if (!isfinite(rho)) atomicOr(err, TSG_ERR_NONFINITE);
-    }
-    if (ti == MAT_SOIL && c.solver == 3)
-        for (int q = 0; q < 9; ++q) p.stress[(size_t)q * n + i] += c.dt6 * t.d_stress_RK[(size_t)q * n + i];
-}
-
 // ---- advect_pos with XSPH (eng/solver_sph_base.py:224-238), two phases ----
 template <int DIM, int G>
 __global__ void __launch_bounds__(ROWS * G) k_xsph(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
@@ -1227,40 +1115,6 @@ __global__ void k_xsph_rigid(Consts c, Persist64 p, Trans64 t, const int* __rest
     for (int d = 0; d < 3; ++d) t.aux3[(size_t)d * n + i] = s[d];
 }
 
-__device__ __forceinline__ void do_pos(const Consts& c, const Persist64& p, const Trans64& t, int i, int* err) {
-    const int n = c.n;
-    const int ti = p.mat_type[i];
-    if (!(ti > 0)) return;
-    const bool xs = c.xsph && p.is_dynamic[i];
-    bool ok = true;
-    for (int d = 0; d < 3; ++d) {
-        double v = p.v[(size_t)d * n + i];
-        double nx = xs ? p.x[(size_t)d * n + i] + c.dt * (v + 0.5 * t.aux3[(size_t)d * n + i])
-                       : p.x[(size_t)d * n + i] + c.dt * v;
-        p.x[(size_t)d * n + i] = nx;
-        ok = ok && isfinite(nx);
-    }
-    if (!ok) atomicOr(err, TSG_ERR_NONFINITE);
-}
-
-// ---- advect_something (solver post-steps) ----
-__device__ __forceinline__ void do_post_wc(const Consts& c, const Persist64& p, int i) {
-    if (p.mat_type[i] != MAT_FLUID) return;
-    double rho = fmax(c.rho0, p.density[i]);
-    p.density[i] = rho;
-    p.m_V[i] = p.mass[i] / rho;
-}
-
-__device__ __forceinline__ void do_post_mui(const Consts& c, const Persist64& p, const Trans64& t, int i) {
-    if (p.mat_type[i] != MAT_SOIL) return;
-    const int n = c.n;
-    double rho = fmax(c.rho0, p.density[i]);
-    p.density[i] = rho;
-    p.m_V[i] = p.mass[i] / rho;
-    p.strain_equ[i] += c.dt * t.d_strain_equ[i];
-    for (int q = 0; q < 9; ++q) p.stress[(size_t)q * n + i] = t.stress_tmp[(size_t)q * n + i];
-}
-
 // Stress regularisation after advect_pos: centres use their moved positions, candidate
 // cells come from this step's sort (eng/solver_sph_muI.py:151-156).  The rows are rebuilt from
 // the moved positions first (flow neighbours only).
@@ -1309,21 +1163,6 @@ __global__ void k_post_mui_c(Consts c, Persist64 p, Trans64 t) {
     for (int q = 0; q < 9; ++q) p.stress[(size_t)q * n + i] = t.aux9[(size_t)q * n + i];
 }
 
-__device__ __forceinline__ void do_post_dp(const Consts& c, const Persist64& p, const Trans64& t, int i) {
-    if (p.mat_type[i] != MAT_SOIL) return;
-    const int n = c.n;
-    double rho = fmax(c.rho0, p.density[i]);
-    p.density[i] = rho;
-    p.m_V[i] = p.mass[i] / rho;
-    double st[9];
-    for (int q = 0; q < 9; ++q) st[q] = p.stress[(size_t)q * n + i];
-    p.flag_retmap[i] = dp_flag(c, st);
-    dp_adapt(c, st);
-    for (int q = 0; q < 9; ++q) p.stress[(size_t)q * n + i] = st[q];
-    p.strain_equ[i] += c.dt * t.d_strain_equ[i];
-    p.strain_equ_p[i] += c.dt * t.d_strain_equ_p[i];
-}
-
 // ---- per-particle passes ----
 // The passes of a step between its pair loops, in the order of the bits; every value they
 // exchange belongs to one particle, so a launch runs all that lie between two loops (a leap-frog
@@ -1332,23 +1171,154 @@ enum : unsigned {
     OP_INIT = 1, OP_RK_INIT = 2, OP_RK_UPDATE = 4, OP_HALF = 8, OP_RK_STAGE = 16, OP_FULL = 32, OP_RK_FINAL = 64,
     OP_PRE = 128, OP_POS = 256, OP_POST = 512
 };
+// All loads come first and all stores last: interleaved, each store held back the next plane's
+// load (the compiler cannot tell the planes apart) and the pass was a chain of round trips.
+template <bool SOIL>
 __global__ void __launch_bounds__(TPB) k_particle(Consts c, Persist64 p, Trans64 t, Pairs64 pr, unsigned ops, int m,
                                                   int* err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
-    if (ops & OP_INIT) do_init(c, p, t, i);
-    if (ops & OP_RK_INIT) do_rk_init(c, p, t, i);
-    if (ops & OP_RK_UPDATE) do_rk_update(c, p, t, i, m);
-    if (ops & OP_HALF) do_half(c, p, t, i);
-    if (ops & OP_RK_STAGE) do_rk_stage(c, p, t, i);
-    if (ops & OP_FULL) do_full(c, p, t, i, err);
-    if (ops & OP_RK_FINAL) do_rk_final(c, p, t, i, err);
-    if ((ops & OP_PRE) && p.mat_type[i] == c.flow_type) do_pre(c, p, t, i, pr);
-    if (ops & OP_POS) do_pos(c, p, t, i, err);
-    if (ops & OP_POST) {
-        if (c.solver == 1) do_post_wc(c, p, i);
-        else if (c.solver == 2) do_post_mui(c, p, t, i);
-        else do_post_dp(c, p, t, i);
+    const int ti = p.mat_type[i];
+    if (ti <= 0) return;
+    const size_t n = c.n;
+    const bool soil = SOIL && ti == MAT_SOIL, dp = soil && c.solver == 3;
+    const bool pre = (ops & OP_PRE) && ti == c.flow_type;
+    const bool post = (ops & OP_POST) && ti == (SOIL ? MAT_SOIL : MAT_FLUID);
+    const bool has = ops & (OP_INIT | OP_RK_STAGE);  // rho~, v~ set here
+    double rho = 0, mass = 0, mV = 0, rt = 0, dd = 0, ad = 0, v[3], x[3], vt[3], dv[3], av[3];
+    double st[9], stt[9], ds[9], as[9], eq = 0, eqp = 0, deq = 0, deqp = 0, xs[3] = {0, 0, 0};
+    const unsigned rates_in = OP_RK_UPDATE | OP_HALF | OP_RK_STAGE | OP_FULL;
+    const bool upd_rho = ops & (OP_FULL | OP_RK_FINAL);
+    if ((ops & (OP_INIT | OP_RK_STAGE)) || upd_rho || post) rho = p.density[i];
+    if (ops & (OP_INIT | OP_RK_STAGE | OP_FULL | OP_RK_FINAL | OP_POS)) ld3(v, p.v, n, i);
+    if (ops & (OP_HALF | OP_RK_STAGE | OP_FULL | OP_RK_FINAL) || post) mass = p.mass[i];
+    if (ops & rates_in) { dd = t.d_density[i]; ld3(dv, t.d_vel, n, i); }
+    if ((ops & (OP_RK_UPDATE | OP_RK_FINAL)) && !(ops & OP_RK_INIT)) { ad = t.d_density_RK[i]; ld3(av, t.d_vel_RK, n, i); }
+    if ((ops & OP_HALF) || (pre && !has)) { rt = t.density_tmp[i]; ld3(vt, t.v_tmp, n, i); }
+    if (pre && !(ops & (OP_HALF | OP_RK_STAGE))) mV = p.m_V[i];
+    const bool xsph = (ops & OP_POS) && c.xsph && p.is_dynamic[i];
+    if (ops & OP_POS) {
+        ld3(x, p.x, n, i);
+        if (xsph) ld3(xs, t.aux3, n, i);
+    }
+    if (SOIL && soil) {
+        if ((ops & OP_INIT) || (dp && ((ops & (OP_RK_STAGE | OP_FULL | OP_RK_FINAL)) || post))) ld9(st, p.stress, n, i);
+        if ((dp && ((ops & OP_HALF) || (pre && !has))) || (!dp && post)) ld9(stt, t.stress_tmp, n, i);
+        if (dp && (ops & rates_in)) ld9(ds, t.d_stress, n, i);
+        if (dp && (ops & (OP_RK_UPDATE | OP_RK_FINAL)) && !(ops & OP_RK_INIT)) ld9(as, t.d_stress_RK, n, i);
+        if (post) {
+            eq = p.strain_equ[i];
+            deq = t.d_strain_equ[i];
+            if (dp) { eqp = p.strain_equ_p[i]; deqp = t.d_strain_equ_p[i]; }
+        }
+    }
+
+    // init_real2tmp (eng/solver_sph_base.py:67-74)
+    if (ops & OP_INIT) {
+        rt = rho;
+        for (int d = 0; d < 3; ++d) vt[d] = v[d];
+        if (SOIL && soil)
+            for (int q = 0; q < 9; ++q) stt[q] = st[q];
+    }
+    // the integrators (eng/solver_sph_base.py:79-170)
+    if (ops & OP_RK_INIT) {
+        ad = 0.0;
+        for (int d = 0; d < 3; ++d) av[d] = 0.0;
+        if (SOIL && dp)
+            for (int q = 0; q < 9; ++q) as[q] = 0.0;
+    }
+    if (ops & OP_RK_UPDATE) {
+        ad += dd * m;
+        for (int d = 0; d < 3; ++d) av[d] += dv[d] * m;
+        if (SOIL && dp)
+            for (int q = 0; q < 9; ++q) as[q] += (double)m * ds[q];
+    }
+    if (ops & OP_HALF) {
+        rt = rt + c.hdt * dd;
+        mV = mass / rt;
+        for (int d = 0; d < 3; ++d) vt[d] += c.hdt * dv[d];
+        if (SOIL && dp)
+            for (int q = 0; q < 9; ++q) stt[q] += c.hdt * ds[q];
+    }
+    if (ops & OP_RK_STAGE) {
+        rt = c.hdt * dd + rho;
+        mV = mass / rt;
+        for (int d = 0; d < 3; ++d) vt[d] = c.hdt * dv[d] + v[d];
+        if (SOIL && dp)
+            for (int q = 0; q < 9; ++q) stt[q] = c.hdt * ds[q] + st[q];
+    }
+    bool bad = false;
+    if (ops & OP_FULL) {
+        rho = rho + c.dt * dd;
+        mV = mass / rho;
+        for (int d = 0; d < 3; ++d) v[d] += c.dt * dv[d];
+        bad = !isfinite(rho);
+        if (SOIL && dp)
+            for (int q = 0; q < 9; ++q) st[q] += c.dt * ds[q];
+    }
+    if (ops & OP_RK_FINAL) {
+        rho = rho + c.dt6 * ad;
+        mV = mass / rho;
+        for (int d = 0; d < 3; ++d) v[d] += c.dt6 * av[d];
+        bad = !isfinite(rho);
+        if (SOIL && dp)
+            for (int q = 0; q < 9; ++q) st[q] += c.dt6 * as[q];
+    }
+    // first phase of one_step: Tait EOS (eng/solver_sph_wc.py:86-88) or stress adaptation
+    // (eng/solver_sph_dp.py:215-217), and the record the loops read
+    double pres = 0.0;
+    if (pre) {
+        if (!SOIL) {
+            const double ratio = rt / c.rho0;
+            const double pw = c.exponent_is_int ? powi(ratio, (long)c.gamma) : pow(ratio, c.gamma);
+            pres = fmax(c.B * (pw - 1.0), 0.0);
+        } else if (dp) {
+            dp_adapt(c, stt);
+        }
+    }
+    // advect_pos (eng/solver_sph_base.py:224-238; the XSPH sums are in aux3)
+    if (ops & OP_POS) {
+        for (int d = 0; d < 3; ++d) {
+            x[d] = xsph ? x[d] + c.dt * (v[d] + 0.5 * xs[d]) : x[d] + c.dt * v[d];
+            bad = bad || !isfinite(x[d]);
+        }
+    }
+    // advect_something (the solvers' post-steps)
+    int flag = 0;
+    if (post) {
+        rho = fmax(c.rho0, rho);
+        mV = mass / rho;
+        if (SOIL) {
+            eq += c.dt * deq;
+            if (dp) {
+                flag = dp_flag(c, st);
+                dp_adapt(c, st);
+                eqp += c.dt * deqp;
+            }
+        }
+    }
+
+    if (bad) atomicOr(err, TSG_ERR_NONFINITE);
+    if (upd_rho || post) p.density[i] = rho;
+    if ((ops & (OP_HALF | OP_RK_STAGE)) || upd_rho || post) p.m_V[i] = mV;
+    if (upd_rho) st3(p.v, v, n, i);
+    if (ops & OP_POS) st3(p.x, x, n, i);
+    if (ops & (OP_INIT | OP_HALF | OP_RK_STAGE)) { t.density_tmp[i] = rt; st3(t.v_tmp, vt, n, i); }
+    if (ops & (OP_RK_INIT | OP_RK_UPDATE)) { t.d_density_RK[i] = ad; st3(t.d_vel_RK, av, n, i); }
+    if (pre && !SOIL) {
+        p.pressure[i] = pres;
+        wc_record(c, pr.rec, i, vt, pres, rt, mV, ti == MAT_FLUID);
+    }
+    if (SOIL && soil) {
+        if (pre && dp) soil_record(c, pr.rec, i, vt, stt, rt, mV);
+        if ((ops & OP_INIT) || (dp && ((ops & (OP_HALF | OP_RK_STAGE)) || pre))) st9(t.stress_tmp, stt, n, i);
+        if (dp && (ops & (OP_RK_INIT | OP_RK_UPDATE))) st9(t.d_stress_RK, as, n, i);
+        if (dp && (upd_rho || post)) st9(p.stress, st, n, i);
+        if (!dp && post) st9(p.stress, stt, n, i);
+        if (post) {
+            p.strain_equ[i] = eq;
+            if (dp) { p.strain_equ_p[i] = eqp; p.flag_retmap[i] = flag; }
+        }
     }
 }
 
@@ -1737,13 +1707,17 @@ void fp64_geometry(const Consts& c, const Persist64& p, Trans64& t, const Grid& 
     if (c.n_bdy > 0) DISPATCH_ROWS(c, g, k_geom_bdy, c.n_bdy, c, p, g.list_bdy, c.n_bdy, g.pr);
 }
 
+// Block size of the per-particle passes: small scenes in blocks of one warp, to reach every SM.
+static int tpb(int n) { return n < 152 * 4 * TPB ? 32 : TPB; }
+
 static void particle_pass(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, unsigned ops, int m,
                           cudaStream_t s) {
     if (c.solver == 2) ops &= ~(unsigned)OP_PRE;
     if (!ops) return;
     PhaseScope ph(s, ops & (OP_HALF | OP_RK_STAGE | OP_RK_UPDATE | OP_FULL | OP_RK_FINAL | OP_RK_INIT) ? PH_INTEGRATE
                      : ops & OP_INIT ? PH_INIT : ops & OP_PRE ? PH_PRE : ops & OP_POS ? PH_POS : PH_POST);
-    TSG_LAUNCH(k_particle, nblk(c.n), TPB, s, c, p, t, g.pr, ops, m, g.err);
+    if (c.solver == 1) TSG_LAUNCH(k_particle<false>, nblk(c.n, tpb(c.n)), tpb(c.n), s, c, p, t, g.pr, ops, m, g.err);
+    else TSG_LAUNCH(k_particle<true>, nblk(c.n, tpb(c.n)), tpb(c.n), s, c, p, t, g.pr, ops, m, g.err);
 }
 
 static void corr_flow(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {

@@ -209,6 +209,23 @@ __device__ __forceinline__ long long flat_cell(const Consts& c, const double* x)
     return idx[0] * c.gnum[1] * c.gnum[2] + idx[1] * c.gnum[2] + idx[2];
 }
 
+// Planar vectors and tensors.
+__device__ __forceinline__ void ld3(double* r, const double* a, size_t n, int i) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) r[d] = a[d * n + i];
+}
+__device__ __forceinline__ void st3(double* a, const double* r, size_t n, int i) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) a[d * n + i] = r[d];
+}
+__device__ __forceinline__ void ld9(double* r, const double* a, size_t n, int i) {
+#pragma unroll
+    for (int q = 0; q < 9; ++q) r[q] = a[q * n + i];
+}
+__device__ __forceinline__ void st9(double* a, const double* r, size_t n, int i) {
+#pragma unroll
+    for (int q = 0; q < 9; ++q) a[q * n + i] = r[q];
+}
 // f32 coordinates of a position: high part (w: flow flag) and what it rounds off.
 __device__ __forceinline__ void write_pos32(const Consts& c, const double* x, bool flow, float4* hi, float4* lo) {
     double d[3];

@@ -199,34 +199,46 @@ __global__ void k_reorder64(Consts c, const int* __restrict__ perm, Persist64 a,
             for (int q = cb; q < ce; ++q) r += perm[q] < s;
             k = cb + r;
         }
-        double xv[3];
-        for (int d = 0; d < 3; ++d) {
-            xv[d] = a.x[d * n + s];
-            b.x[d * n + k] = xv[d];
-            b.v[d * n + k] = a.v[d * n + s];
-            b.x0[d * n + k] = a.x0[d * n + s];
-        }
-        b.density[k] = a.density[s];
-        b.mass[k] = a.mass[s];
-        b.m_V[k] = a.m_V[s];
-        b.pressure[k] = a.pressure[s];
-        if (SOIL) {
-            for (int q = 0; q < 9; ++q) b.stress[q * n + k] = a.stress[q * n + s];
-            b.strain_equ[k] = a.strain_equ[s];
-            b.strain_equ_p[k] = a.strain_equ_p[s];
-            b.flag_retmap[k] = a.flag_retmap[s];
-        }
+        // every load before the first store: the compiler cannot tell the planes apart, and a
+        // store between them makes each load wait for the one before it
+        double xv[3], vv[3], x0[3], st[9], vt[3];
+        ld3(xv, a.x, n, s);
+        ld3(vv, a.v, n, s);
+        ld3(x0, a.x0, n, s);
+        const double rho = a.density[s], mass = a.mass[s], mV = a.m_V[s], pr = a.pressure[s];
         mt = a.mat_type[s];
+        const int mid = a.mat_id[s], oid = a.obj_id[s], dyn = a.is_dynamic[s], id = a.id0[s];
+        const long long f = cell_src[s];
+        double eq = 0.0, eqp = 0.0;
+        int flag = 0;
+        if (SOIL) {
+            ld9(st, a.stress, n, s);
+            eq = a.strain_equ[s];
+            eqp = a.strain_equ_p[s];
+            flag = a.flag_retmap[s];
+            if (vt_src) ld3(vt, vt_src, n, s);
+        }
+        st3(b.x, xv, n, k);
+        st3(b.v, vv, n, k);
+        st3(b.x0, x0, n, k);
+        b.density[k] = rho;
+        b.mass[k] = mass;
+        b.m_V[k] = mV;
+        b.pressure[k] = pr;
+        if (SOIL) {
+            st9(b.stress, st, n, k);
+            b.strain_equ[k] = eq;
+            b.strain_equ_p[k] = eqp;
+            b.flag_retmap[k] = flag;
+            if (vt_src) st3(vt_dst, vt, n, k);
+        }
         b.mat_type[k] = mt;
-        b.mat_id[k] = a.mat_id[s];
-        b.obj_id[k] = a.obj_id[s];
-        b.is_dynamic[k] = a.is_dynamic[s];
-        b.id0[k] = a.id0[s];
-        if (vt_src)
-            for (int d = 0; d < 3; ++d) vt_dst[d * n + k] = vt_src[d * n + s];
+        b.mat_id[k] = mid;
+        b.obj_id[k] = oid;
+        b.is_dynamic[k] = dyn;
+        b.id0[k] = id;
         const bool flow = mt == MAT_FLUID || mt == MAT_SOIL;
         write_pos32(c, xv, flow, pos32 + k, pos32l + k);
-        const long long f = cell_src[s];
         cell0[k] = f;
         if (flow && f >= 0 && f < c.G) cell_flow[f] = 1;
     }
@@ -257,8 +269,10 @@ void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid
     scan_exclusive(g.count, g.cell_start, (int)nbins, g.tile_sum, s);
     TSG_LAUNCH(k_scatter, nblk(c.n), TPB, s, c.n, g.cell_of, g.rank, g.cell_start, g.perm, g.big, g.nbig);
     TSG_LAUNCH(k_cell_sort_big, 152, kSortBlock, s, g.big, g.nbig, g.cell_start, g.cell_of, c.n, g.perm);
+    // small scenes in blocks of one warp, to reach every SM
+    const int tpb = c.n < 152 * 4 * TPB ? 32 : TPB, nb = (c.n + tpb - 1) / tpb;
     if (c.solver == 1) {
-        TSG_LAUNCH(k_reorder64<false>, nblk(c.n), TPB, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, g.cell0_old,
+        TSG_LAUNCH(k_reorder64<false>, nb, tpb, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, g.cell0_old,
                    t.cell0, g.cell_flow, g.list_flow, g.list_bdy, g.list_count, nullptr, nullptr);
     } else {
         // mu(I) keeps v_tmp across steps: stage it in aux3 (free until advect_pos) and gather
@@ -267,7 +281,7 @@ void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid
             cudaMemcpyAsync(t.aux3, t.v_tmp, sizeof(double) * 3 * (size_t)c.n, cudaMemcpyDeviceToDevice, s);
             src = t.aux3;
         }
-        TSG_LAUNCH(k_reorder64<true>, nblk(c.n), TPB, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, g.cell0_old,
+        TSG_LAUNCH(k_reorder64<true>, nb, tpb, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, g.cell0_old,
                    t.cell0, g.cell_flow, g.list_flow, g.list_bdy, g.list_count, src, src ? t.v_tmp : nullptr);
     }
     Persist64 tmp = cur;
