@@ -79,12 +79,42 @@ __device__ __forceinline__ bool pair(const K32& k, const Start& S, int a, int b,
     return true;
 }
 
-// Iterate the step's neighbour list of i (every list fits: the caller checks for overflow).
+// Iterate the step's neighbour list of i (a list above the capacity is cut off: the caller
+// reports it and drops the results).
 template <class F>
 __device__ __forceinline__ void for_list(const K32& k, const T32& t, int i, F&& body) {
-    const int m = t.cnt[i];
+    const int m = min(t.cnt[i], k.maxn);
     for (int s = 0; s < m; ++s) body(entry_index(k, t.nbr[(size_t)s * k.n + i]));
 }
+
+// The WCSPH sweep's lists by AL adjacent lanes a particle: lane g takes slots g, g + AL, ... and
+// the partial sums are added in a fixed tree.  A rollout's few thousand particles, one thread
+// each, leave most SMs idle and walk some thirty dependent gathers of heavy terms in a row
+// (3,274 particles: pair terms 52 us, boundary terms 26 and 14 us).
+template <int AL>
+struct ListLanes {
+    int i, g;
+    bool live;
+    __device__ __forceinline__ explicit ListLanes(int n) {
+        const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+        i = tid / AL;
+        g = tid % AL;
+        live = i < n;
+        if (!live) i = n - 1;
+    }
+    template <class F>
+    __device__ __forceinline__ void each(const K32& k, const T32& t, bool on, F&& body) const {
+        const int m = live && on ? min(t.cnt[i], k.maxn) : 0;
+        for (int s = g; s < m; s += AL) body(entry_index(k, t.nbr[(size_t)s * k.n + i]));
+    }
+    template <class T>
+    __device__ __forceinline__ void sum(T& v) const {
+#pragma unroll
+        for (int o = AL / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+    __device__ __forceinline__ void sum(float2& v) const { sum(v.x); sum(v.y); }
+    __device__ __forceinline__ bool writes() const { return live && g == 0; }
+};
 
 __device__ __forceinline__ void sym2(const T32& t, size_t n, int i, float& xx, float& yy, float& xy) {
     xx = t.sigt[i];
@@ -354,8 +384,11 @@ __global__ void k_adj_stress(K32 k, P32 p, T32 t, Start S, A32 A) {
 
 // Parameter adjoints summed in a fixed order (one block, strided partials, tree), so that
 // repeated reversals of the same step give the same bits.
-__global__ void k_adj_params(int n, const double2* __restrict__ gp, double* __restrict__ pbar) {
-    __shared__ double smu[256], sco[256];
+constexpr int kParamThreads = 1024;
+__global__ void __launch_bounds__(kParamThreads) k_adj_params(int n, const double2* __restrict__ gp,
+                                                             double* __restrict__ pbar, const int* __restrict__ novf) {
+    __shared__ double smu[kParamThreads], sco[kParamThreads];
+    if (*novf) return;
     double a = 0.0, b = 0.0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         a += gp[i].x;
@@ -525,9 +558,10 @@ __device__ __forceinline__ bool wpair(const K32& k, const Start& S, const T32& t
     return true;
 }
 
+template <int AL>
 __global__ void k_wadj_pairs(K32 k, P32 p, T32 t, Start S, A32 A) {
-    const int kk = blockIdx.x * blockDim.x + threadIdx.x;
-    if (kk >= k.n) return;
+    const ListLanes<AL> lanes(k.n);
+    const int kk = lanes.i;
     const bool kf = fluid(S.hi[kk].w);
     const float mvk = S.lo[kk].w;
     const float rho_k = k.rho0 + t.drt[kk];
@@ -536,7 +570,7 @@ __global__ void k_wadj_pairs(K32 k, P32 p, T32 t, Start S, A32 A) {
     double gnu = 0.0;
     const float2 ak = A.dv[kk];
     const float ck = A.dr[kk];
-    for_list(k, t, kk, [&](int j) {
+    lanes.each(k, t, true, [&](int j) {
         const bool jf = fluid(S.hi[j].w);
         if (kf) {  // kk the centre i, j the neighbour
             WPair P;
@@ -595,6 +629,8 @@ __global__ void k_wadj_pairs(K32 k, P32 p, T32 t, Start S, A32 A) {
             }
         }
     });
+    lanes.sum(ax); lanes.sum(av); lanes.sum(ar); lanes.sum(amv); lanes.sum(aP); lanes.sum(gnu);
+    if (!lanes.writes()) return;
     A.x[kk] = f2(A.x[kk].x + ax.x, A.x[kk].y + ax.y);
     A.v[kk] = f2(A.v[kk].x + av.x, A.v[kk].y + av.y);  // fluid: v; dummy: its v~
     A.rt[kk] += aP;                                      // P = p / rho^2
@@ -606,12 +642,14 @@ __global__ void k_wadj_pairs(K32 k, P32 p, T32 t, Start S, A32 A) {
 }
 
 // Boundary extrapolation reversed at each dummy: coefficients of its sums.
+template <int AL>
 __global__ void k_wadj_bdy(K32 k, P32 p, T32 t, Start S, A32 A) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= k.n || tf_type(S.hi[b].w) > 0 || t.cnt[b] == 0) return;
+    const ListLanes<AL> lanes(k.n);
+    const int b = lanes.i;
+    const bool on = tf_type(S.hi[b].w) <= 0 && t.cnt[b] != 0;
     float2 U = f2(0.f, 0.f);
     float Q = 0.f, Sb = 0.f;
-    for_list(k, t, b, [&](int j) {
+    lanes.each(k, t, on, [&](int j) {
         if (!fluid(S.hi[j].w)) return;
         float d[3];
         delta<2>(S.hi[b], S.lo[b], S.hi[j], S.lo[j], d);
@@ -624,6 +662,8 @@ __global__ void k_wadj_bdy(K32 k, P32 p, T32 t, Start S, A32 A) {
         Q += mw * (pr.x + pr.y * k.g[1] * d[1]);
         Sb += mw;
     });
+    lanes.sum(U); lanes.sum(Q); lanes.sum(Sb);
+    if (!on || !lanes.writes()) return;
     const float cf = t.cf[b];
     const float2 avt = A.v[b];                          // adjoint of v~_b
     const float pb = A.rt[b] / (k.rho0 * k.rho0);       // P_b = p_b / rho0^2
@@ -636,15 +676,17 @@ __global__ void k_wadj_bdy(K32 k, P32 p, T32 t, Start S, A32 A) {
 }
 
 // The boundary sums' terms gathered at each fluid particle.
+template <int AL>
 __global__ void k_wadj_bdy_fluid(K32 k, P32 p, T32 t, Start S, A32 A) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= k.n || !fluid(S.hi[j].w)) return;
+    const ListLanes<AL> lanes(k.n);
+    const int j = lanes.i;
+    const bool on = fluid(S.hi[j].w);
     const float mvj = S.lo[j].w;
     const float4 v = t.vt[j];
     const float2 pr = t.pr[j];
     float2 ax = f2(0.f, 0.f), av = f2(0.f, 0.f);
     float amv = 0.f, ap = 0.f, ar = 0.f;
-    for_list(k, t, j, [&](int b) {
+    lanes.each(k, t, on, [&](int b) {
         if (tf_type(S.hi[b].w) > 0) return;
         float d[3];
         delta<2>(S.hi[b], S.lo[b], S.hi[j], S.lo[j], d);  // d = x_b - x_j
@@ -664,6 +706,8 @@ __global__ void k_wadj_bdy_fluid(K32 k, P32 p, T32 t, Start S, A32 A) {
         ax.x += -wb * G * d[0];
         ax.y += -wb * G * d[1] - B2 * mvj * pr.y * k.g[1] * W;
     });
+    lanes.sum(ax); lanes.sum(av); lanes.sum(amv); lanes.sum(ap); lanes.sum(ar);
+    if (!on || !lanes.writes()) return;
     A.x[j] = f2(A.x[j].x + ax.x, A.x[j].y + ax.y);
     A.v[j] = f2(A.v[j].x + av.x, A.v[j].y + av.y);
     A.mv[j] += amv;
@@ -673,9 +717,9 @@ __global__ void k_wadj_bdy_fluid(K32 k, P32 p, T32 t, Start S, A32 A) {
 
 // EOS and m_V = m / rho reversed; adjoint out in canonical order.
 __global__ void k_wadj_out(K32 k, P32 p, T32 t, Start S, A32 A, double* __restrict__ ax, double* __restrict__ av,
-                           double* __restrict__ ar, double* __restrict__ avt) {
+                           double* __restrict__ ar, double* __restrict__ avt, const int* __restrict__ novf) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= k.n) return;
+    if (i >= k.n || *novf) return;
     const size_t c = (size_t)p.ids[i].x;
     avt[3 * c] = avt[3 * c + 1] = avt[3 * c + 2] = 0.0;
     if (!fluid(S.hi[i].w)) {
@@ -707,7 +751,28 @@ T* grab(Fp32State& st, size_t count) {
 struct AdjBuffers {
     Start S{};
     A32 A{};
+    int* novf_host = nullptr;  // pinned: the overflow count of the step's lists
+    cudaEvent_t novf_ready = nullptr;
 };
+
+// The step start back into the current buffers (WCSPH: all that the step's forward changes).
+__global__ void k_restore_start(int n, P32 p, RecView vt, Start S) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    p.hi[i] = S.hi[i];
+    p.lo[i] = S.lo[i];
+    p.vel[i] = S.vel[i];
+    p.drho[i] = S.drho[i];
+    vt[i] = S.vt[i];
+}
+
+template <int AL>
+void wadj_lists(Fp32State& st, const P32& p, AdjBuffers& B, cudaStream_t s) {
+    const int nb = nblk(AL * (long long)st.n);
+    TSG_LAUNCH(k_wadj_pairs<AL>, nb, TPB, s, st.k, p, st.T, B.S, B.A);
+    TSG_LAUNCH(k_wadj_bdy<AL>, nb, TPB, s, st.k, p, st.T, B.S, B.A);
+    TSG_LAUNCH(k_wadj_bdy_fluid<AL>, nb, TPB, s, st.k, p, st.T, B.S, B.A);
+}
 
 AdjBuffers* adj_buffers(Fp32State& st) {
     if (st.adj) return static_cast<AdjBuffers*>(st.adj);
@@ -725,7 +790,10 @@ AdjBuffers* adj_buffers(Fp32State& st) {
     A.b2 = grab<float>(st, n); A.bs = grab<float>(st, n); A.dds = grab<float>(st, n);
     A.s = grab<float4>(st, n); A.b3 = grab<float4>(st, n); A.vg = grab<float4>(st, n);
     if (!S.hi || !S.lo || !S.vel || !S.vt || !S.vlo || !A.gp || !S.drho || !A.x || !A.v || !A.dv || !A.vn || !A.b1 || !A.r || !A.mv ||
-        !A.rt || !A.dr || !A.b2 || !A.bs || !A.dds || !A.s || !A.b3 || !A.vg) {
+        !A.rt || !A.dr || !A.b2 || !A.bs || !A.dds || !A.s || !A.b3 || !A.vg ||
+        cudaMallocHost(reinterpret_cast<void**>(&b->novf_host), sizeof(int)) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->novf_ready, cudaEventDisableTiming) != cudaSuccess) {
+        if (b->novf_host) cudaFreeHost(b->novf_host);
         delete b;
         return nullptr;
     }
@@ -736,7 +804,11 @@ AdjBuffers* adj_buffers(Fp32State& st) {
 }  // namespace
 
 void fp32_free_adjoint(Fp32State& st) {
-    delete static_cast<AdjBuffers*>(st.adj);
+    if (AdjBuffers* b = static_cast<AdjBuffers*>(st.adj)) {
+        cudaEventDestroy(b->novf_ready);
+        cudaFreeHost(b->novf_host);
+        delete b;
+    }
     st.adj = nullptr;
 }
 
@@ -754,22 +826,33 @@ int fp32_adjoint_step(Fp32State& st, double* ax, double* av, double* ar, double*
     st.built = true;
     st.lists_valid = true;
     ++st.rebuilds;
-    int novf = 0;
-    cudaMemcpyAsync(&novf, st.novf, sizeof novf, cudaMemcpyDeviceToHost, s);
-    cudaStreamSynchronize(s);
-    if (novf) return TSG_E_CAPACITY;  // every list must hold all neighbours
     P32& p = st.P[st.cur];
     const int nb = nblk(st.n);
+    // every list must hold all neighbours
+    cudaMemcpyAsync(B->novf_host, st.novf, sizeof(int), cudaMemcpyDeviceToHost, s);
+    cudaEventRecord(B->novf_ready, s);
+    if (k.solver != 1) {
+        cudaEventSynchronize(B->novf_ready);
+        if (*B->novf_host) return TSG_E_CAPACITY;
+    }
     TSG_LAUNCH(k_copy_start, nb, TPB, s, st.n, p, st.T.vt, B->S);
     f32::step_body(st, s, false);
     // reverse sweep
     if (k.solver == 1) {
         TSG_LAUNCH(k_wadj_init, nb, TPB, s, k, p, st.T, B->S, B->A, ax, av, ar);
-        TSG_LAUNCH(k_wadj_pairs, nb, TPB, s, k, p, st.T, B->S, B->A);
-        TSG_LAUNCH(k_wadj_bdy, nb, TPB, s, k, p, st.T, B->S, B->A);
-        TSG_LAUNCH(k_wadj_bdy_fluid, nb, TPB, s, k, p, st.T, B->S, B->A);
-        TSG_LAUNCH(k_wadj_out, nb, TPB, s, k, p, st.T, B->S, B->A, ax, av, ar, avt);
-        TSG_LAUNCH(k_adj_params, 1, 256, s, st.n, B->A.gp, pbar);
+        // (larger scenes fill the GPU with a thread per particle, whose list reads coalesce)
+        if (st.n <= 65536) wadj_lists<8>(st, p, *B, s);
+        else wadj_lists<1>(st, p, *B, s);
+        TSG_LAUNCH(k_wadj_out, nb, TPB, s, k, p, st.T, B->S, B->A, ax, av, ar, avt, st.novf);
+        TSG_LAUNCH(k_adj_params, 1, kParamThreads, s, st.n, B->A.gp, pbar, st.novf);
+        // The count of overflowed lists has long arrived by now: the host waits for the rebuild
+        // only, and the sweep runs on while the next call is prepared.  The kernels above write
+        // none of the caller's arrays where it is not zero, and the step is put back.
+        cudaEventSynchronize(B->novf_ready);
+        if (*B->novf_host) {
+            TSG_LAUNCH(k_restore_start, nb, TPB, s, st.n, p, st.T.vt, B->S);
+            return TSG_E_CAPACITY;
+        }
         return cudaGetLastError() == cudaSuccess ? 0 : TSG_E_CUDA;
     }
     TSG_LAUNCH(k_adj_init, nb, TPB, s, k, p, st.T, B->S, B->A, ax, av, ar, avt);
@@ -777,7 +860,7 @@ int fp32_adjoint_step(Fp32State& st, double* ax, double* av, double* ar, double*
     TSG_LAUNCH(k_adj_bdy, nb, TPB, s, k, p, st.T, B->S, B->A);
     TSG_LAUNCH(k_adj_bdy_soil, nb, TPB, s, k, p, st.T, B->S, B->A);
     TSG_LAUNCH(k_adj_stress, nb, TPB, s, k, p, st.T, B->S, B->A);
-    TSG_LAUNCH(k_adj_params, 1, 256, s, st.n, B->A.gp, pbar);
+    TSG_LAUNCH(k_adj_params, 1, kParamThreads, s, st.n, B->A.gp, pbar, st.novf);
     TSG_LAUNCH(k_adj_vgrad, nb, TPB, s, k, p, st.T, B->S, B->A);
     TSG_LAUNCH(k_adj_out, nb, TPB, s, k, p, B->S, B->A, ax, av, ar, avt);
     return cudaGetLastError() == cudaSuccess ? 0 : TSG_E_CUDA;

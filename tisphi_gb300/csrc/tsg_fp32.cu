@@ -66,20 +66,34 @@ __global__ void k_hash32(K32 k, int count_n, int base, const float4* __restrict_
     rank[t] = atomicAdd(&count[f], 1);
 }
 
+// Arrival order inside the cells; cells above kSortSmall are listed for k_cell_sort_big, the
+// others' particles are ranked by k_reorder32.
 __global__ void k_scatter32(int count_n, const int* __restrict__ cell_of, const int* __restrict__ rank,
-                            const int* __restrict__ cell_start, int* __restrict__ perm) {
+                            const int* __restrict__ cell_start, int* __restrict__ perm, int* __restrict__ big,
+                            int* __restrict__ nbig) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count_n) return;
-    perm[cell_start[cell_of[t]] + rank[t]] = t;
+    const int c = cell_of[t], r = rank[t], b = cell_start[c];
+    perm[b + r] = t;
+    if (r == 0 && cell_start[c + 1] - b > kSortSmall) big[atomicAdd(nbig, 1)] = c;
 }
 
 // Gather block [base, base + count_n) from a into b (new order), renormalise hi/lo and
-// refresh the prefilter position.
-__global__ void k_reorder32(K32 k, int count_n, int base, const int* __restrict__ perm, P32 a, P32 b,
+// refresh the prefilter position.  Inside a cell, ascending old index: this particle's rank
+// among the cell's (one thread per cell sorting through global memory took 7 us of a 2D
+// scene's rebuild).
+__global__ void k_reorder32(K32 k, int count_n, int base, const int* __restrict__ perm,
+                            const int* __restrict__ cell_of, const int* __restrict__ cell_start, P32 a, P32 b,
                             float4* __restrict__ PF) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count_n) return;
-    const int dst = base + t, src = base + perm[t];
+    const int old = perm[t], cell = cell_of[old], cb = cell_start[cell], ce = cell_start[cell + 1];
+    if (ce - cb <= kSortSmall) {
+        int r = 0;
+        for (int q = cb; q < ce; ++q) r += perm[q] < old;
+        t = cb + r;
+    }
+    const int dst = base + t, src = base + old;
     float4 h = a.hi[src], l = a.lo[src];
     float hv[3] = {h.x, h.y, h.z}, lv[3] = {l.x, l.y, l.z};
     float pfv[3];
@@ -90,20 +104,34 @@ __global__ void k_reorder32(K32 k, int count_n, int base, const int* __restrict_
         lv[d] = (float)(x - hq);
         pfv[d] = (float)x;
     }
+    // every load before the first store (the compiler cannot tell the arrays apart)
+    const float4 vel = a.vel[src], vlo = a.vlo ? a.vlo[src] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float drho = a.drho[src], mass = a.mass[src];
+    const int4 ids = a.ids[src];
+    const size_t n = k.n;
+    float sig[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, eeq = 0.f, eeqp = 0.f;
+    int flag = 0;
+    if (a.sig) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) sig[q] = a.sig[q * n + src];
+        eeq = a.eeq[src];
+        eeqp = a.eeqp[src];
+        flag = a.flag[src];
+    }
     b.hi[dst] = make_float4(hv[0], hv[1], hv[2], h.w);
     b.lo[dst] = make_float4(lv[0], lv[1], lv[2], l.w);
-    b.vel[dst] = a.vel[src];
-    b.drho[dst] = a.drho[src];
-    b.mass[dst] = a.mass[src];
-    b.ids[dst] = a.ids[src];
+    b.vel[dst] = vel;
+    b.drho[dst] = drho;
+    b.mass[dst] = mass;
+    b.ids[dst] = ids;
     if (a.sig) {
-        const size_t n = k.n;
-        for (int q = 0; q < 6; ++q) b.sig[q * n + dst] = a.sig[q * n + src];
-        b.eeq[dst] = a.eeq[src];
-        b.eeqp[dst] = a.eeqp[src];
-        b.flag[dst] = a.flag[src];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) b.sig[q * n + dst] = sig[q];
+        b.eeq[dst] = eeq;
+        b.eeqp[dst] = eeqp;
+        b.flag[dst] = flag;
     }
-    if (a.vlo) b.vlo[dst] = a.vlo[src];
+    if (a.vlo) b.vlo[dst] = vlo;
     PF[dst] = make_float4(pfv[0], pfv[1], pfv[2], h.w);
 }
 
@@ -128,6 +156,75 @@ __global__ void k_lists(K32 k, const float4* __restrict__ HI, RecView LO,
     }, true);
     cnt[i] = m;
     if (m > k.maxn) note_overflow(ovf_list, novf, i);
+}
+
+// The same lists by a warp per particle, for scenes too small to fill the GPU with one thread
+// per particle: 32 candidates of a stencil row are tested at a time and the accepted ones take
+// their slots in order by ballot.  The tests are enum_neighbors' own, so the lists are equal.
+template <int DIM>
+__global__ void k_lists_warp(K32 k, const float4* __restrict__ HI, RecView LO, const float4* __restrict__ PF,
+                             const int* __restrict__ dstart, const int* __restrict__ sstart, int* __restrict__ cnt,
+                             int* __restrict__ nbr, int* __restrict__ ovf_list, int* __restrict__ novf) {
+    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (i >= k.n) return;
+    const float4 hi_i = HI[i], lo_i = LO[i], pf_i = PF[i];
+    const bool flow_i = is_flow(tf_type(pf_i.w));
+    constexpr int NR = DIM == 3 ? 9 : 3;
+    bool ok = true;
+    const long long cc0 = cell_coord(k, hi_i.x, lo_i.x, ok);
+    const long long cc1 = cell_coord(k, hi_i.y, lo_i.y, ok);
+    const long long cc2 = cell_coord(k, hi_i.z, lo_i.z, ok);
+    const bool pf = fabsf(pf_i.x) < k.pf_lim && fabsf(pf_i.y) < k.pf_lim && fabsf(pf_i.z) < k.pf_lim;
+    // lanes 0 .. 2 NR - 1 hold the candidate ranges: the dynamic block's stencil rows, then the
+    // static block's
+    int jb_l = 0, je_l = 0;
+    if (ok && lane < (flow_i ? 2 * NR : NR)) {
+        const int* cs = lane < NR ? dstart : sstart;
+        const int q = lane < NR ? lane : lane - NR;
+        const long long ny = k.gnum[1], nz = k.gnum[2], G = k.G;
+        const int ox = DIM == 3 ? q / 3 - 1 : q - 1, oy = DIM == 3 ? q % 3 - 1 : 0;
+        const long long f0 = (cc0 + ox) * ny * nz + (cc1 + oy) * nz + cc2;
+        const long long lo = f0 - 1 > 0 ? f0 - 1 : 0;
+        const long long hi = f0 + 1 < G - 1 ? f0 + 1 : G - 1;
+        if (lo <= hi) { jb_l = cs[lo]; je_l = cs[hi + 1]; }
+    }
+    int m = 0;
+    unsigned rows = __ballot_sync(0xffffffffu, jb_l < je_l);
+    while (rows) {
+        const int q = __ffs(rows) - 1;
+        rows &= rows - 1u;
+        const int jb = __shfl_sync(0xffffffffu, jb_l, q), je = __shfl_sync(0xffffffffu, je_l, q);
+        for (int b = jb; b < je; b += 32) {
+            const int j = b + lane;
+            bool in = false;
+            float4 hj = hi_i;
+            if (j < je && j != i) {
+                const float4 pj = PF[j];
+                bool near = flow_i || is_flow(tf_type(pj.w));
+                if (near && pf) {
+                    const float fx = pf_i.x - pj.x, fy = pf_i.y - pj.y, fz = pf_i.z - pj.z;
+                    float r2f = fx * fx + fy * fy;
+                    if (DIM == 3) r2f += fz * fz;
+                    near = !(r2f > k.R2Lhi);
+                }
+                if (near) {
+                    float d[3];
+                    hj = HI[j];
+                    delta<DIM>(hi_i, lo_i, hj, LO[j], d);
+                    in = dist2<DIM>(d) < k.R2L;
+                }
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, in);
+            const int slot = m + __popc(bal & ((1u << lane) - 1u));
+            if (in && slot < k.maxn) nbr[(size_t)slot * k.n + i] = entry_of(k, j, hi_i, hj);
+            m += __popc(bal);
+        }
+    }
+    if (lane == 0) {
+        cnt[i] = m;
+        if (m > k.maxn) note_overflow(ovf_list, novf, i);
+    }
 }
 
 // Warp-per-cell list build (3D): the lanes of a warp are the particles of one cell, so
@@ -1934,10 +2031,12 @@ void build_cells(Fp32State& st, int base, int count_n, int* count, int* start, c
     P32& a = st.P[st.cur];
     TSG_LAUNCH(k_hash32, nblk(count_n), TPB, s, k, count_n, base, a.hi, a.lo, st.cell_of, st.rank, count, st.err);
     scan_exclusive(count, start, (int)nbins, st.tiles, s);
-    TSG_LAUNCH(k_scatter32, nblk(count_n), TPB, s, count_n, st.cell_of, st.rank, start, st.perm);
-    sort_within_cells(nbins, start, st.cell_of, count_n, st.perm, st.sort_big, st.sort_nbig, s);
+    cudaMemsetAsync(st.sort_nbig, 0, sizeof(int), s);
+    TSG_LAUNCH(k_scatter32, nblk(count_n), TPB, s, count_n, st.cell_of, st.rank, start, st.perm, st.sort_big,
+               st.sort_nbig);
+    TSG_LAUNCH(k_cell_sort_big, 152, kSortBlock, s, st.sort_big, st.sort_nbig, start, st.cell_of, count_n, st.perm);
     P32& b = st.P[1 - st.cur];
-    TSG_LAUNCH(k_reorder32, nblk(count_n), TPB, s, k, count_n, base, st.perm, a, b, st.pf);
+    TSG_LAUNCH(k_reorder32, nblk(count_n), TPB, s, k, count_n, base, st.perm, st.cell_of, start, a, b, st.pf);
     (void)reorder_into_next;
 }
 
@@ -2212,10 +2311,18 @@ void lists_by_cell(Fp32State& st, const P32& p, cudaStream_t s) {
                st.dstart, st.sstart, st.T.cnt, st.T.nbr, st.ovf_list, st.novf);
 }
 
+// Up to this many particles a warp each builds the lists.
+constexpr int kWarpLists = 65536;
+
 template <int DIM>
 void build_lists(Fp32State& st, const P32& p, cudaStream_t s) {
     const K32& k = st.k;
     cudaMemsetAsync(st.novf, 0, sizeof(int), s);
+    if (st.cells_per_cta <= 0 && k.n <= kWarpLists) {
+        TSG_LAUNCH(k_lists_warp<DIM>, (k.n + 3) / 4, 128, s, k, p.hi, p.lo, st.pf, st.dstart, st.sstart, st.T.cnt,
+                   st.T.nbr, st.ovf_list, st.novf);
+        return;
+    }
     if (st.cells_per_cta <= 0) {  // one thread per particle
         TSG_LAUNCH(k_lists<DIM>, nblk(k.n), TPB, s, k, p.hi, p.lo, st.pf, st.dstart, st.sstart, st.T.cnt, st.T.nbr,
                    st.ovf_list, st.novf);
@@ -2714,6 +2821,11 @@ int capture_steps(Fp32State& st, int steps, bool collide, Fp32State::StepGraph& 
     cudaGraph_t graph = nullptr;
     if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed) != cudaSuccess) rc = TSG_E_CUDA;
     for (int q = 0; q < steps && !rc; ++q) {
+        if (k.disp2_limit <= 0.f) {  // no skin: every step rebuilds, without asking
+            rebuild(st, cs, true);
+            step_body(st, cs, collide, false);
+            continue;
+        }
         cudaStreamCaptureStatus status;
         cudaGraph_t cg = nullptr;
         if (cudaStreamGetCaptureInfo(cs, &status, nullptr, &cg) != cudaSuccess || !cg) { rc = TSG_E_CUDA; break; }
@@ -2791,7 +2903,8 @@ Fp32State::StepGraph* graph_for(Fp32State& st, int steps, bool collide, int* rc)
 
 int fp32_step_graph(Fp32State& st, int nsteps, bool collide, cudaStream_t s) {
     if (profiling_on()) return TSG_E_STATE;  // per-phase events need the eager path
-    if (!st.built) fp32_sort(st, s);
+    const bool always = st.k.disp2_limit <= 0.f;  // the graphs rebuild in every step
+    if (!st.built && !always) fp32_sort(st, s);
     const int K = st.steps_per_graph > 1 ? st.steps_per_graph : 1;
     int rc = 0;
     while (nsteps > 0) {
@@ -2800,6 +2913,7 @@ int fp32_step_graph(Fp32State& st, int nsteps, bool collide, cudaStream_t s) {
         if (!g) return rc;
         if (cudaGraphLaunch(g->exec, s) != cudaSuccess) return TSG_E_CUDA;
         add_launches(g->kernels);
+        if (always) { st.rebuilds += take; st.built = true; }
         nsteps -= take;
     }
     st.lists_valid = st.k.disp2_limit > 0.f;
@@ -2854,13 +2968,56 @@ size_t snap_bytes(Fp32State& st) {
     return total;
 }
 
-void snap_copy(Fp32State& st, void* buf, bool restore, cudaStream_t s) {
-    char* q = static_cast<char*>(buf);
-    for (auto& it : snap_items(st)) {
-        if (restore) cudaMemcpyAsync(it.first, q, it.second, cudaMemcpyDeviceToDevice, s);
-        else cudaMemcpyAsync(q, it.first, it.second, cudaMemcpyDeviceToDevice, s);
-        q += (it.second + 255) & ~size_t(255);
+// All fields in one launch (16-byte words; every field starts 256-byte aligned and its padding
+// stays inside the snapshot's 256-byte slots, the tail is copied by 4-byte words).  A rollout
+// saves or loads a state three times per step: six to eleven copies of a few microseconds each
+// cost more than the step's kernels on a small scene.
+struct SnapTable {
+    char* field[12];
+    long long bytes[12], off[12];  // off: in the snapshot
+    long long words[13];           // first 16-byte word of each field in the launch
+    int count;
+};
+__global__ void k_snap_copy(SnapTable t, char* buf, int restore) {
+    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < t.words[t.count];
+         w += (long long)gridDim.x * blockDim.x) {
+        int q = 0;
+        while (w >= t.words[q + 1]) ++q;
+        const long long o = (w - t.words[q]) * 16;
+        char* f = t.field[q] + o;
+        char* b = buf + t.off[q] + o;
+        const char* src = restore ? b : f;
+        char* dst = restore ? f : b;
+        if (o + 16 <= t.bytes[q]) *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(src);
+        else
+            for (long long e = 0; o + e < t.bytes[q]; e += 4)
+                *reinterpret_cast<int*>(dst + e) = *reinterpret_cast<const int*>(src + e);
     }
+}
+
+void snap_copy(Fp32State& st, void* buf, bool restore, cudaStream_t s) {
+    SnapTable t;
+    t.count = 0;
+    t.words[0] = 0;
+    long long off = 0;
+    for (auto& it : snap_items(st)) {
+        const int q = t.count++;
+        t.field[q] = static_cast<char*>(it.first);
+        t.bytes[q] = (long long)it.second;
+        t.off[q] = off;
+        t.words[q + 1] = t.words[q] + (t.bytes[q] + 15) / 16;
+        off += (t.bytes[q] + 255) & ~255ll;
+    }
+    if (t.words[t.count] == 0) return;
+    if ((reinterpret_cast<size_t>(buf) & 15) != 0) {  // a caller's unaligned buffer
+        for (int q = 0; q < t.count; ++q) {
+            char* b = static_cast<char*>(buf) + t.off[q];
+            cudaMemcpyAsync(restore ? t.field[q] : b, restore ? b : t.field[q], t.bytes[q], cudaMemcpyDeviceToDevice, s);
+        }
+        return;
+    }
+    const long long nb = (t.words[t.count] + 255) / 256;
+    TSG_LAUNCH(k_snap_copy, (int)(nb < 152 * 8 ? nb : 152 * 8), 256, s, t, static_cast<char*>(buf), restore ? 1 : 0);
 }
 
 int snapshot(Fp32State& st, cudaStream_t s, bool restore) {
