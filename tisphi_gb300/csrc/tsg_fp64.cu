@@ -189,14 +189,42 @@ __device__ __forceinline__ double det3(const double* a) {
 
 // The kernel functions behind a call (see slow_mul), their constants by value: grad W and W.
 struct KernelConsts { int kernel; unsigned div_span; double h1, kk; };
-struct KernelVals { double kd[3], W; };
+struct KernelVals { double kd[3], W, rr; };  // grad W, W, |r| |r|
 template <int DIM>
 __device__ __noinline__ KernelVals slow_kernel(KernelConsts c, double r0, double r1, double r2, double rn) {
     const double r[3] = {r0, r1, r2};
     KernelVals k;
     kernel_dW<DIM>(c, r, rn, k.kd);
     k.W = kernel_W(c, rn);
+    k.rr = rn * rn;
     return k;
+}
+
+// grad W (if asked for) and W of a separation r.  The Wendland kernel away from its ends runs on
+// the integer pipes but for its two sums; the others take the kernel functions.
+template <int DIM>
+__device__ __forceinline__ KernelVals pair_kernel(const Consts& c, const double* r, bool want_dW, bool want_W) {
+    const bool r_ok = usable_v<DIM>(r);
+    double r2;
+    on_pipe(r_ok, [&](auto mul) { r2 = dotv<DIM>(r, r, mul); });
+    KernelVals k;
+    k.W = 0.0;
+    if (c.wend_int && r_ok && above(r2, 0x1p-200)) {
+        const double rn = int_sqrt(r2);
+        const double q = int_mul(rn, c.h1), q1 = __fma_rn(-0.5, q, 1.0);
+        if (above(rn, EPS) && !above(q, 2.0) && above(q1, 0x1p-50)) {
+            const double q2 = int_mul(q1, q1);
+            if (want_dW) {
+                const unsigned long long X = recip63(rn);
+                const double s = int_mul(int_mul(int_mul(c.kk, int_mul(q2, q1)), int_mul(-5.0, q)), c.h1);
+                for (int d = 0; d < DIM; ++d) k.kd[d] = quot(int_mul(s, r[d]), rn, X);
+                k.rr = int_mul(rn, rn);
+            }
+            if (want_W) k.W = int_mul(int_mul(c.kk, int_mul(q2, q2)), __fma_rn(2.0, q, 1.0));
+            return k;
+        }
+    }
+    return slow_kernel<DIM>(KernelConsts{c.kernel, c.div_span, c.h1, c.kk}, r[0], r[1], r[2], slow_sqrt(r2));
 }
 
 // Pair geometry of row slot `slot` (entry j): r, grad W and, for a flow neighbour, W into
@@ -209,41 +237,24 @@ __device__ __forceinline__ double pair_geometry(const Consts& c, const double* _
     r[0] = xi[0] - X[j];
     r[1] = xi[1] - X[n + j];
     r[2] = DIM == 3 ? xi[2] - X[2 * n + j] : 0.0;
-    const bool r_ok = usable_v<DIM>(r);
-    double r2;
-    on_pipe(r_ok, [&](auto mul) { r2 = dotv<DIM>(r, r, mul); });
-    const double rn = sqrt(r2);
-    double W = 0.0, den;
-    const double q = rn * c.h1, q1 = __fma_rn(-0.5, q, 1.0);
-    if (c.wend_int && r_ok && above(rn, EPS) && !above(q, 2.0) && usable(q) && above(q1, 0x1p-50)) {
-        const double y = __drcp_rn(rn);
-        const double q2 = int_mul(q1, q1);
-        const double s = int_mul(int_mul(int_mul(c.kk, int_mul(q2, q1)), int_mul(-5.0, q)), c.h1);
-        for (int d = 0; d < DIM; ++d) kd[d] = div_by(int_mul(s, r[d]), rn, y, c.div_span);
-        if (want_W) W = int_mul(int_mul(c.kk, int_mul(q2, q2)), __fma_rn(2.0, q, 1.0));
-        den = int_mul(rn, rn);
-    } else {
-        const KernelVals k = slow_kernel<DIM>(KernelConsts{c.kernel, c.div_span, c.h1, c.kk}, r[0], r[1], r[2], rn);
-        for (int d = 0; d < DIM; ++d) kd[d] = k.kd[d];
-        W = k.W;
-        den = slow_mul(rn, rn);
+    const KernelVals k = pair_kernel<DIM>(c, r, true, want_W);
+    for (int d = 0; d < DIM; ++d) {
+        kd[d] = k.kd[d];
+        pr.gk[d * pr.slots_f + slot] = kd[d];
     }
-    for (int d = 0; d < DIM; ++d) pr.gk[d * pr.slots_f + slot] = kd[d];
     if (pr.gden) {
-        den = den + c.eps_h2;
-        pr.gden[slot] = make_double2(den, __drcp_rn(den));
+        const double den = k.rr + c.eps_h2;
+        pr.gden[slot] = make_double2(den, __longlong_as_double((long long)divisor(den)));
     }
-    return W;
+    return k.W;
 }
 
 // Kernel value of a boundary row's entry.
 template <int DIM>
 __device__ __forceinline__ double pair_W(const Consts& c, const double* __restrict__ X, const double* xi, int j) {
     const size_t n = c.n;
-    const double rx = xi[0] - X[j], ry = xi[1] - X[n + j];
-    double r2 = rx * rx + ry * ry;
-    if (DIM == 3) { const double rz = xi[2] - X[2 * n + j]; r2 = r2 + rz * rz; }
-    return kernel_W(c, sqrt(r2));
+    const double r[3] = {xi[0] - X[j], xi[1] - X[n + j], DIM == 3 ? xi[2] - X[2 * n + j] : 0.0};
+    return pair_kernel<DIM>(c, r, false, true).W;
 }
 
 // This thread's row in the row-sum phase: particle index and listed count (0 for a row past the
@@ -652,13 +663,11 @@ __device__ __forceinline__ void row_gradient(const Consts& c, const Pairs64& pr,
 
 // One neighbour's WCSPH terms: continuity, then the acceleration (DIM), from the neighbour's
 // record (v~, P = p / rho~^2, m_V, viscosity factor, -rho0 m_V) and the pair geometry
-// (den.y = 1 / den.x).
-struct Divisor {  // a divisor with its reciprocal; span 0 where div_by's window does not hold
-    double b, y;
-    unsigned span;
-    __device__ __forceinline__ Divisor(const Consts& c, double v) : b(v), y(1.0 / v) {
-        span = (unsigned)__double2hiint(v) - (923u << 20) < 200u << 20 ? c.div_span : 0u;
-    }
+// (den.y: den.x's divisor() bits).
+struct Divisor {  // a divisor with its divisor() bits
+    double b;
+    unsigned long long X;
+    __device__ __forceinline__ explicit Divisor(double v) : b(v), X(divisor(v)) {}
 };
 template <int DIM>
 __device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const double* v, double P, double mV, double cvj,
@@ -672,10 +681,13 @@ __device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const doub
         dr = dotv<DIM>(dvv, r, mul);
     });
     const double mn = min0(dr);
-    double cv = cvj;
-    if (!fluid) cv = div_by(cv, rti.b, rti.y, rti.span);
-    cv = div_by(cv * mn, den.x, den.y, c.div_span);
-    const double cp = cC * (pri + P);
+    double cv = cvj, cp = pri + P;
+    if (!fluid) cv = quot(cv, rti.b, rti.X);
+    on_pipe(usable(cv) && usable(mn) && usable(cC) && usable(cp), [&](auto mul) {
+        cv = mul(cv, mn);
+        cp = mul(cC, cp);
+    });
+    cv = quot(cv, den.x, (unsigned long long)__double_as_longlong(den.y));
     on_pipe(usable(cp) && usable(cv) && usable_v<DIM>(kd), [&](auto mul) {
         for (int d = 0; d < DIM; ++d) T[1 + d] = mul(cv, kd[d]) + mul(cp, kd[d]);
     });
@@ -693,7 +705,7 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
         double xi[3], vti[3], L[9];
         load_x<DIM>(p.x, q.i, n, xi);
         for (int d = 0; d < 3; ++d) vti[d] = t.v_tmp[(size_t)d * n + q.i];
-        const Divisor rti(c, t.density_tmp[q.i]);
+        const Divisor rti(t.density_tmp[q.i]);
         const double pri = pr.rec[(size_t)8 * q.i + 3];
         if (c.corr == 1 && KC != KC_READ)
             for (int e = 0; e < 9; ++e) L[e] = t.CSPM_L[(size_t)e * n + q.i];
@@ -716,7 +728,7 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
     const int row = blockIdx.x * ROWS + threadIdx.x;
     if (threadIdx.x >= ROWS || row >= count) return;
     const int i = list[row];
-    const Divisor rti(c, t.density_tmp[i]);
+    const Divisor rti(t.density_tmp[i]);
     double A[C];
     const bool listed = pr.cap_f && pr.cnt[row] <= pr.cap_f;
     const bool rep = c.boundary == 3 || c.boundary == 4;
@@ -738,7 +750,7 @@ __global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Tr
             corrected<DIM>(c, L, kd, kc);
             const double den = rn * rn + c.eps_h2;
             wc_terms<DIM>(c, p.mat_type[j] == MAT_FLUID, rj, rj[3], rj[4], rj[5], rj[6], vti, rti, pri, r,
-                          make_double2(den, __drcp_rn(den)), kd, kc, T);
+                          make_double2(den, __longlong_as_double((long long)divisor(den))), kd, kc, T);
             for (int q = 0; q < C; ++q) A[q] += T[q];
         });
     }
@@ -1067,7 +1079,11 @@ __global__ void __launch_bounds__(ROWS * G) k_xsph(Consts c, Persist64 p, Trans6
             if (!nb_flow(ent)) return;
             const double w = pair_W<DIM>(c, p.x, xi, ent);
             const double mVj = p.m_V[ent];
-            for (int d = 0; d < DIM; ++d) T[d] = mVj * (p.v[(size_t)d * n + ent] - vi[d]) * w;
+            double dv[3];
+            for (int d = 0; d < DIM; ++d) dv[d] = p.v[(size_t)d * n + ent] - vi[d];
+            on_pipe(usable(mVj) && usable(w) && usable_v<DIM>(dv), [&](auto mul) {
+                for (int d = 0; d < DIM; ++d) T[d] = mul(mul(mVj, dv[d]), w);
+            });
         });
     }
     const int row = blockIdx.x * ROWS + threadIdx.x;
@@ -1132,7 +1148,13 @@ __global__ void __launch_bounds__(ROWS * G) k_post_mui_b(Consts c, Persist64 p, 
             const int j = pr.nb_f[q.base + s];
             const double w = pair_W<DIM>(c, p.x, xi, j);
             const double mVj = p.m_V[j];
-            for (int e = 0; e < 9; ++e) T[e] = mVj * p.stress[(size_t)e * n + j] * w;
+            double st[9];
+            ld9(st, p.stress, n, j);
+            bool ok = usable(mVj) && usable(w);
+            for (int e = 0; e < 9; ++e) ok = ok && usable(st[e]);
+            on_pipe(ok, [&](auto mul) {
+                for (int e = 0; e < 9; ++e) T[e] = mul(mul(mVj, st[e]), w);
+            });
         });
     }
     const int row = blockIdx.x * ROWS + threadIdx.x;

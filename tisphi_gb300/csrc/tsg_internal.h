@@ -141,7 +141,7 @@ struct Pairs64 {
     int* nb_f;          // entries: particle index, sign bit set for a non-flow neighbour
     int* nb_b;
     double* gk;         // dim planes: kernel gradient of each flow entry
-    double2* gden;      // |r|^2 + 0.01 h^2 of each flow entry and its reciprocal (WCSPH)
+    double2* gden;      // |r|^2 + 0.01 h^2 of each flow entry and its divisor() bits (WCSPH)
     double* gc;         // dim planes: corrected gradient L_i grad W of each flow entry (CSPM);
                         // the soil solvers, which use no other gradient, keep it in gk
     double* gw;         // kernel value of each boundary entry

@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(256) k_list64(Consts c, const double* __restri
 // with every lane off holds the pipe like any other.
 __device__ __noinline__ double slow_mul(double a, double b) { return a * b; }
 __device__ __noinline__ double slow_div(double a, double b) { return a / b; }
+__device__ __noinline__ double slow_sqrt(double a) { return sqrt(a); }
 
 // a / b, correctly rounded, from y = RN(1 / b): one product and two fused multiply-adds instead
 // of the division's ten-odd FP64 instructions (Markstein 1990; Brisebarre, Muller and Raina,
@@ -184,6 +185,77 @@ __device__ __forceinline__ double int_mul(double a, double b) {
                             zero ? 0 : (int)(unsigned)r);
 }
 
+
+// Square roots and quotients on the integer pipes, correctly rounded.  All three start from the
+// f32 approximation of the special-function unit and refine it by Newton's iteration in fixed
+// point on exact residuals (the low 64 bits suffice, the residuals are small); the last bit is
+// then decided exactly: with M0 the truncated result and t = 2 M0 + 1 the midpoint above it,
+// the sign of v - t^2 (root) or a - t b (quotient) says whether to round up.  Neither a root
+// nor a quotient of 53-bit numbers is ever such a midpoint.  The tie test needs the refined
+// value to a fraction of the last place only, so approximations off by a few f32 ulp give the
+// same bits.
+__device__ __forceinline__ unsigned approx31(float y) {  // y in (0.5, 1 + 2^-22] as 31 fractional bits
+    return min(__float2uint_rz(y * 2147483648.f), 0x7fffffffu);
+}
+// 2^63 / B to within 2^-58 for a positive normal b = B 2^e, B in [1, 2).
+__device__ __forceinline__ unsigned long long recip63(double b) {
+    const unsigned bh = (unsigned)__double2hiint(b), bl = (unsigned)__double2loint(b);
+    const unsigned mh = (bh & 0xfffffu) | 0x100000u;
+    const unsigned long long mb = ((unsigned long long)mh << 32) | bl;
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(0x3f800000u | __funnelshift_l(bl, bh & 0xfffffu, 3))));
+    const unsigned X0 = approx31(y);
+    const long long R0 = (long long)(0ull - (unsigned long long)X0 * bl - ((unsigned long long)(X0 * mh) << 32));
+    const unsigned long long X1 = ((unsigned long long)X0 << 32)
+                                + (unsigned long long)(((long long)(int)X0 * (int)(R0 >> 32)) >> 19);
+    const unsigned long long Xp = X1 >> 15;
+    const long long R1 = (long long)(0ull - Xp * mb);
+    return (Xp << 15) + (unsigned long long)(((long long)(int)(Xp >> 17) * (int)(R1 >> 28)) >> 40);
+}
+// a / b with X = recip63(b); b positive, both normal, the quotient too.
+__device__ __forceinline__ double int_quot(double a, double b, unsigned long long X) {
+    const unsigned ah = (unsigned)__double2hiint(a), bh = (unsigned)__double2hiint(b);
+    const unsigned long long ma = ((unsigned long long)((ah & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(a);
+    const unsigned long long mb = ((unsigned long long)((bh & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(b);
+    const unsigned long long P = __umul64hi(ma << 11, X);
+    const unsigned sh = (unsigned)(P >> 62) ^ 1u;  // the quotient of the significands is below one
+    const unsigned long long M0 = (P << sh) >> 10;
+    const long long D = (long long)((ma << (53 + sh)) - (2 * M0 + 1) * mb);
+    const unsigned e = (1022u << 20) + (ah & 0x7ff00000u) - (bh & 0x7ff00000u) - (sh << 20);
+    const unsigned long long r = ((unsigned long long)e << 32) + M0 + (D > 0 ? 1u : 0u);
+    return __longlong_as_double((long long)(r | ((unsigned long long)(ah & 0x80000000u) << 32)));
+}
+// sqrt(v), v positive and normal.
+__device__ __forceinline__ double int_sqrt(double v) {
+    const unsigned vh = (unsigned)__double2hiint(v), vl = (unsigned)__double2loint(v);
+    const int u = (int)(vh >> 20) - 1023;
+    const unsigned odd = (unsigned)u & 1u;
+    const unsigned long long A = ((((unsigned long long)((vh & 0xfffffu) | 0x100000u)) << 32) | vl) << odd;
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y)
+        : "f"(__uint_as_float((0x3f800000u + (odd << 23)) | __funnelshift_l(vl, vh & 0xfffffu, 3))));
+    const unsigned Y0 = approx31(y);
+    const unsigned S0 = (unsigned)(((unsigned long long)(unsigned)(A >> 22) * Y0) >> 31);
+    const long long R0 = (long long)((A << 8) - (unsigned long long)S0 * S0);
+    const unsigned long long S1 = ((unsigned long long)S0 << 22)
+                                + (unsigned long long)(((long long)(int)(R0 >> 12) * (int)Y0) >> 28);
+    const unsigned long long Sp = S1 >> 8;
+    const long long R1 = (long long)((A << 36) - Sp * Sp);
+    const unsigned long long M0 = (Sp << 8) + (unsigned long long)(((long long)(int)(R1 >> 20) * (int)Y0) >> 48);
+    const unsigned long long t = 2 * M0 + 1;
+    const long long D = (long long)((A << 54) - t * t);
+    return __longlong_as_double((long long)(((unsigned long long)(unsigned)(1022 + (u >> 1)) << 52) + M0 + (D > 0 ? 1u : 0u)));
+}
+// A divisor prepared for int_quot (X 0: not usable, quotients take the call).
+__device__ __forceinline__ unsigned long long divisor(double b) {  // usable: 2^-200 <= b < 2^200
+    return (unsigned)__double2hiint(b) - (823u << 20) < 400u << 20 ? recip63(b) : 0ull;
+}
+__device__ __forceinline__ double quot(double a, double b, unsigned long long X) {
+    const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    if (X != 0ull && hi - (523u << 20) < 1000u << 20) return int_quot(a, b, X);
+    if (X != 0ull && (hi | (unsigned)__double2loint(a)) == 0u) return a;
+    return slow_div(a, b);
+}
 
 // a > b for b >= 0 and a that is not a NaN, on the bits (an FP64 comparison holds the pipe too).
 __device__ __forceinline__ bool above(double a, double b) {
