@@ -273,8 +273,11 @@ __device__ __forceinline__ RowRef row_ref(const int* __restrict__ list, int coun
 }
 
 // Flow rows: pair geometry, Shepard sum and CSPM matrix (eng/solver_sph_base.py:386-423).
+// Bounded to 80-odd registers: 24 warps an SM instead of 16 hide the integer chains (3D, 118 k
+// rows: 979 -> 893 us; 2D, 7.2 k rows: 11 us a step); the 3D rates passes likewise (642 -> 585
+// and 835 -> 798 us).  What holds them now is the FP64 pipe, about 80 % busy.
 template <int DIM, int G, bool CORR>
-__global__ void __launch_bounds__(ROWS * G) k_corr_flow(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+__global__ void __launch_bounds__(ROWS * G, G == 8 ? 3 : 6) k_corr_flow(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
                                                         const int* __restrict__ list, int count, Pairs64 pr) {
     constexpr int C = 1 + (CORR ? DIM * DIM : 0);
     __shared__ double S[C][ROWS];
@@ -289,12 +292,13 @@ __global__ void __launch_bounds__(ROWS * G) k_corr_flow(Consts c, Persist64 p, T
             const double W = pair_geometry<DIM>(c, p.x, xi, j, pr, q.base + s, nb_flow(ent), r, kd);
             if (nb_flow(ent)) {
                 const double mVj = p.m_V[j];
-                on_pipe(usable(mVj) && usable(W) && (!CORR || (usable_v<DIM>(r) && usable_v<DIM>(kd))), [&](auto mul) {
+                // (the matrix products stay on the FP64 pipe, which this pass no longer fills)
+                on_pipe(usable(mVj) && usable(W) && (!CORR || usable_v<DIM>(r)), [&](auto mul) {
                     T[0] = mul(mVj, W);
                     if (CORR)
                         for (int a = 0; a < DIM; ++a) {
                             const double av = mul(mVj, -r[a]);
-                            for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = mul(av, kd[b]);
+                            for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = av * kd[b];
                         }
                 });
             }
@@ -688,14 +692,14 @@ __device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const doub
         cp = mul(cC, cp);
     });
     cv = quot(cv, den.x, (unsigned long long)__double_as_longlong(den.y));
-    on_pipe(usable(cp) && usable(cv) && usable_v<DIM>(kd), [&](auto mul) {
-        for (int d = 0; d < DIM; ++d) T[1 + d] = mul(cv, kd[d]) + mul(cp, kd[d]);
+    on_pipe(usable(cp) && usable_v<DIM>(kd), [&](auto mul) {
+        for (int d = 0; d < DIM; ++d) T[1 + d] = cv * kd[d] + mul(cp, kd[d]);  // one product on each pipe
     });
 }
 
 // ---- WCSPH rates (eng/solver_sph_wc.py:108-126) ----
 template <int DIM, int G, int KC>
-__global__ void __launch_bounds__(ROWS * G) k_wc_rates(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+__global__ void __launch_bounds__(ROWS * G, G == 8 ? 2 : DIM == 3 && KC == KC_READ ? 6 : 5) k_wc_rates(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
                                                        const int* __restrict__ list, int count, Pairs64 pr) {
     constexpr int C = 1 + DIM;
     __shared__ double S[C][ROWS];
@@ -988,8 +992,10 @@ __global__ void __launch_bounds__(ROWS * G) k_mui_mom(Consts c, Persist64 p, Tra
 }
 
 // ---- DP rates (eng/solver_sph_dp.py:236-270, Bui 2008 :172-208) ----
+// The 2D bound holds five blocks of 128 threads on an SM: 20,000 rows then run in one wave
+// (8 lanes and no bound: two waves and a nearly empty third, 2,975 us per ten steps; 2,447 now).
 template <int DIM, int G, int KC>
-__global__ void __launch_bounds__(ROWS * G) k_dp_rates(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+__global__ void __launch_bounds__(ROWS * G, DIM == 2 ? 20 / G : 1) k_dp_rates(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
                                                        const int* __restrict__ list, int count, Pairs64 pr) {
     constexpr int C = DIM + DIM * DIM + 1;
     __shared__ double S[C][ROWS];
@@ -1668,37 +1674,37 @@ static void rigid_lists64(const Consts& c, const Persist64& p, const Rigid64& r,
         else TSG_LAUNCH(KERNEL<3>, GRID, TPB, s, __VA_ARGS__);                    \
     } while (0)
 
-// Lanes per row: about as many as a loop has sums (2 to 5 in most), so that the additions in
-// slot order cost what one thread's would; the Drucker-Prager loop has 7 (2D) or 13 sums and a
-// long epilogue, and wants the threads.  us per launch with 8 -> 4 lanes: 3D rates (118 k rows)
-// 1,915 -> 1,834, correction 2,141 -> 2,055; 2D mu(I) (20 k rows) correction 81 -> 66, stress
-// 56 -> 47, momentum 49 -> 40; 2D rates (7 k rows) 42 -> 36; Drucker-Prager 90 -> 101.
-constexpr int LANES = 4, LANES_DP = 8;
+// Lanes per row: four, about as many as a loop has sums (2 to 5 in most), so that the additions
+// in slot order cost what one thread's would (8 lanes: 3D, 118 k rows, 4,203 us a step against
+// 2,819; 2D mu(I), 20 k rows, 216 against 187); eight in 2D scenes whose rows leave the SMs
+// short of warps, where the loop is a chain of latencies (7.2 k rows: 905 us per ten steps
+// against 1,091; 600 rows: 75 us a step against 86; 16 lanes lose at both).
+// The line: 8 x 8,192 threads are a quarter of what the GPU holds.  3D rows have four times the
+// entries to share out and keep four.
+constexpr int LANES = 4, LANES_SMALL = 8, SMALL_ROWS = 8192;
+inline bool small_rows(const Consts& c) { return c.dim == 2 && c.n_flow <= SMALL_ROWS; }
 inline int nrows(int count) { return (count + ROWS - 1) / ROWS; }
 // Threads of a row kernel: without rows only the epilogue's threads have work.
 inline int row_threads(const Grid& g, int lanes) { return g.pr.cap_f ? ROWS * lanes : ROWS; }
 
-#define DISPATCH_LANES(c, g, KERNEL, LN, COUNT, ...)                                                          \
-    do {                                                                                                      \
-        if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LN>), nrows(COUNT), row_threads(g, LN), s, __VA_ARGS__);      \
-        else TSG_LAUNCH((KERNEL<3, LN>), nrows(COUNT), row_threads(g, LN), s, __VA_ARGS__);                   \
+#define ROWS_LAUNCH(g, LN, COUNT, KERNEL, ...) TSG_LAUNCH(KERNEL, nrows(COUNT), row_threads(g, LN), s, __VA_ARGS__)
+#define DISPATCH_ROWS(c, g, KERNEL, COUNT, ...)                                                            \
+    do {                                                                                                   \
+        if (small_rows(c)) ROWS_LAUNCH(g, LANES_SMALL, COUNT, (KERNEL<2, LANES_SMALL>), __VA_ARGS__);      \
+        else if ((c).dim == 2) ROWS_LAUNCH(g, LANES, COUNT, (KERNEL<2, LANES>), __VA_ARGS__);              \
+        else ROWS_LAUNCH(g, LANES, COUNT, (KERNEL<3, LANES>), __VA_ARGS__);                                \
     } while (0)
-#define DISPATCH_ROWS(c, g, KERNEL, COUNT, ...) DISPATCH_LANES(c, g, KERNEL, LANES, COUNT, __VA_ARGS__)
-#define DISPATCH_KC(c, g, KERNEL, LN, KC, COUNT, ...)                                                            \
-    do {                                                                                                         \
-        if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LN, KC>), nrows(COUNT), row_threads(g, LN), s, __VA_ARGS__);     \
-        else TSG_LAUNCH((KERNEL<3, LN, KC>), nrows(COUNT), row_threads(g, LN), s, __VA_ARGS__);                  \
+#define DISPATCH_ROWS_B(c, g, KERNEL, FLAG, COUNT, ...)                                                        \
+    do {                                                                                                       \
+        if (small_rows(c)) ROWS_LAUNCH(g, LANES_SMALL, COUNT, (KERNEL<2, LANES_SMALL, FLAG>), __VA_ARGS__);    \
+        else if ((c).dim == 2) ROWS_LAUNCH(g, LANES, COUNT, (KERNEL<2, LANES, FLAG>), __VA_ARGS__);            \
+        else ROWS_LAUNCH(g, LANES, COUNT, (KERNEL<3, LANES, FLAG>), __VA_ARGS__);                              \
     } while (0)
-#define DISPATCH_KC3(c, g, KERNEL, LN, MODE, COUNT, ...)                                                         \
-    do {                                                                                                         \
-        if ((MODE) == KC_READ) DISPATCH_KC(c, g, KERNEL, LN, KC_READ, COUNT, __VA_ARGS__);                       \
-        else if ((MODE) == KC_KEEP) DISPATCH_KC(c, g, KERNEL, LN, KC_KEEP, COUNT, __VA_ARGS__);                  \
-        else DISPATCH_KC(c, g, KERNEL, LN, KC_MAKE, COUNT, __VA_ARGS__);                                         \
-    } while (0)
-#define DISPATCH_ROWS_B(c, g, KERNEL, FLAG, COUNT, ...)                                                                 \
-    do {                                                                                                                \
-        if ((c).dim == 2) TSG_LAUNCH((KERNEL<2, LANES, FLAG>), nrows(COUNT), row_threads(g, LANES), s, __VA_ARGS__);    \
-        else TSG_LAUNCH((KERNEL<3, LANES, FLAG>), nrows(COUNT), row_threads(g, LANES), s, __VA_ARGS__);                 \
+#define DISPATCH_KC(c, g, KERNEL, MODE, COUNT, ...)                                                 \
+    do {                                                                                            \
+        if ((MODE) == KC_READ) DISPATCH_ROWS_B(c, g, KERNEL, KC_READ, COUNT, __VA_ARGS__);          \
+        else if ((MODE) == KC_KEEP) DISPATCH_ROWS_B(c, g, KERNEL, KC_KEEP, COUNT, __VA_ARGS__);     \
+        else DISPATCH_ROWS_B(c, g, KERNEL, KC_MAKE, COUNT, __VA_ARGS__);                            \
     } while (0)
 
 static void build_rows(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g, bool flow_only,
@@ -1797,7 +1803,7 @@ static void mui_stress(const Consts& c, Persist64& p, Trans64& t, const Grid& g,
     PhaseScope ph(s, PH_PRE);
     int kc = gradient_mode(c, stage);
     if (c.corr == 1 && kc == KC_MAKE) kc = KC_KEEP;  // the momentum loop reads it
-    DISPATCH_KC3(c, g, k_mui_stress, LANES, kc, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+    DISPATCH_KC(c, g, k_mui_stress, kc, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
 }
 
 static void bdy(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s) {
@@ -1812,13 +1818,13 @@ static void rates(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int 
         PhaseScope ph(s, PH_RATES);
         const int kc = gradient_mode(c, stage);
         if (c.solver == 1)
-            DISPATCH_KC3(c, g, k_wc_rates, LANES, kc, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+            DISPATCH_KC(c, g, k_wc_rates, kc, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
         else if (c.solver == 2 && c.corr == 1)
-            DISPATCH_KC(c, g, k_mui_mom, LANES, KC_READ, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+            DISPATCH_ROWS_B(c, g, k_mui_mom, KC_READ, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
         else if (c.solver == 2)
-            DISPATCH_KC(c, g, k_mui_mom, LANES, KC_MAKE, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+            DISPATCH_ROWS_B(c, g, k_mui_mom, KC_MAKE, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
         else
-            DISPATCH_KC3(c, g, k_dp_rates, LANES_DP, kc, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
+            DISPATCH_KC(c, g, k_dp_rates, kc, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
     }
     if (c.n_rigid_dyn > 0 && c.n_bdy > 0) {  // the flow's reaction on dynamic rigid particles
         PhaseScope ph(s, PH_RATES);
