@@ -66,16 +66,16 @@ __global__ void k_hash32(K32 k, int count_n, int base, const float4* __restrict_
     rank[t] = atomicAdd(&count[f], 1);
 }
 
-// Arrival order inside the cells; cells above kSortSmall are listed for k_cell_sort_big, the
+// Arrival order inside the cells; cells above `small` are listed for k_cell_sort_big, the
 // others' particles are ranked by k_reorder32.
 __global__ void k_scatter32(int count_n, const int* __restrict__ cell_of, const int* __restrict__ rank,
-                            const int* __restrict__ cell_start, int* __restrict__ perm, int* __restrict__ big,
-                            int* __restrict__ nbig) {
+                            const int* __restrict__ cell_start, int* __restrict__ perm, int small,
+                            int* __restrict__ big, int* __restrict__ nbig) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count_n) return;
     const int c = cell_of[t], r = rank[t], b = cell_start[c];
     perm[b + r] = t;
-    if (r == 0 && cell_start[c + 1] - b > kSortSmall) big[atomicAdd(nbig, 1)] = c;
+    if (r == 0 && cell_start[c + 1] - b > small) big[atomicAdd(nbig, 1)] = c;
 }
 
 // Gather block [base, base + count_n) from a into b (new order), renormalise hi/lo and
@@ -83,12 +83,12 @@ __global__ void k_scatter32(int count_n, const int* __restrict__ cell_of, const 
 // among the cell's (one thread per cell sorting through global memory took 7 us of a 2D
 // scene's rebuild).
 __global__ void k_reorder32(K32 k, int count_n, int base, const int* __restrict__ perm,
-                            const int* __restrict__ cell_of, const int* __restrict__ cell_start, P32 a, P32 b,
-                            float4* __restrict__ PF) {
+                            const int* __restrict__ cell_of, const int* __restrict__ cell_start, int small, P32 a,
+                            P32 b, float4* __restrict__ PF) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count_n) return;
     const int old = perm[t], cell = cell_of[old], cb = cell_start[cell], ce = cell_start[cell + 1];
-    if (ce - cb <= kSortSmall) {
+    if (ce - cb <= small) {
         int r = 0;
         for (int q = cb; q < ce; ++q) r += perm[q] < old;
         t = cb + r;
@@ -2024,19 +2024,20 @@ int ell_capacity(int dim, double R, double spacing) {
     return count + 8;
 }
 
+// (count and sort_nbig are zero on entry.)
 void build_cells(Fp32State& st, int base, int count_n, int* count, int* start, cudaStream_t s, bool reorder_into_next) {
     const K32& k = st.k;
     const long long nbins = k.G + 1;
-    cudaMemsetAsync(count, 0, sizeof(int) * nbins, s);
     P32& a = st.P[st.cur];
     TSG_LAUNCH(k_hash32, nblk(count_n), TPB, s, k, count_n, base, a.hi, a.lo, st.cell_of, st.rank, count, st.err);
     scan_exclusive(count, start, (int)nbins, st.tiles, s);
-    cudaMemsetAsync(st.sort_nbig, 0, sizeof(int), s);
-    TSG_LAUNCH(k_scatter32, nblk(count_n), TPB, s, count_n, st.cell_of, st.rank, start, st.perm, st.sort_big,
+    const int small = sort_small(count_n);
+    TSG_LAUNCH(k_scatter32, nblk(count_n), TPB, s, count_n, st.cell_of, st.rank, start, st.perm, small, st.sort_big,
                st.sort_nbig);
-    TSG_LAUNCH(k_cell_sort_big, 152, kSortBlock, s, st.sort_big, st.sort_nbig, start, st.cell_of, count_n, st.perm);
+    if (count_n > kSortAll)
+        TSG_LAUNCH(k_cell_sort_big, 152, kSortBlock, s, st.sort_big, st.sort_nbig, start, st.cell_of, count_n, st.perm);
     P32& b = st.P[1 - st.cur];
-    TSG_LAUNCH(k_reorder32, nblk(count_n), TPB, s, k, count_n, base, st.perm, st.cell_of, start, a, b, st.pf);
+    TSG_LAUNCH(k_reorder32, nblk(count_n), TPB, s, k, count_n, base, st.perm, st.cell_of, start, small, a, b, st.pf);
     (void)reorder_into_next;
 }
 
@@ -2155,21 +2156,23 @@ int fp32_create(const tsg_config& cfg, const Consts& c, const tsg_particles* pp,
     }
     st->pf = dal<float4>(*st, n);
     const size_t nb = (size_t)k.G + 1;
-    st->dcount = dal<int>(*st, nb); st->dstart = dal<int>(*st, nb + 1);
+    // dcount and the counters a rebuild starts from zero, one memory set
+    st->dcount = dal<int>(*st, nb + 4);
+    st->novf = st->dcount + nb; st->nsact = st->novf + 1; st->sort_nbig = st->novf + 2;
+    st->maxdisp = reinterpret_cast<unsigned*>(st->novf + 3);
+    st->dstart = dal<int>(*st, nb + 1);
     st->scount = dal<int>(*st, nb); st->sstart = dal<int>(*st, nb + 1);
     st->cell_of = dal<int>(*st, n); st->rank = dal<int>(*st, n); st->perm = dal<int>(*st, n);
     st->tiles = dal<int>(*st, nb / 2048 + 4); st->err = dal<int>(*st, 1);
     st->cells_d = dal<int>(*st, nb); st->cells_s = dal<int>(*st, nb); st->ncells = dal<int>(*st, 2);
-    st->ovf_list = dal<int>(*st, n); st->novf = dal<int>(*st, 1);
-    st->sact = dal<int>(*st, n - nd > 0 ? n - nd : 1); st->nsact = dal<int>(*st, 1);
-    st->maxdisp = dal<unsigned>(*st, 1);
+    st->ovf_list = dal<int>(*st, n);
+    st->sact = dal<int>(*st, n - nd > 0 ? n - nd : 1);
     st->sort_big = dal<int>(*st, cellsort_big_ints(n));
-    st->sort_nbig = dal<int>(*st, 1);
     st->d_rebuilds = dal<int>(*st, 1);
     st->cells_per_cta = c.dim == 3 ? 4 : 0;
     st->stage = dal<double>(*st, 9 * (size_t)n + 16);
     st->scratch = dal<double>(*st, 64);
-    if (!t.nbr || !st->stage || !st->sort_big || !st->sort_nbig || (soil && !t.srec)) { fp32_destroy(st); return TSG_E_CUDA; }
+    if (!t.nbr || !st->stage || !st->sort_big || !st->dcount || (soil && !t.srec)) { fp32_destroy(st); return TSG_E_CUDA; }
     // upload raw arrays through the staging buffer, then split on the device
     double* dx = st->stage;                 // 3n
     double* dv = dx + 3 * (size_t)n;        // 3n
@@ -2245,6 +2248,8 @@ int fp32_create(const tsg_config& cfg, const Consts& c, const tsg_particles* pp,
     cudaMemsetAsync(st->P[1].vel, 0, sizeof(float4) * n, s);
     // static block: sort once into P[1], copy the whole static block into both buffers
     if (n - nd > 0) {
+        cudaMemsetAsync(st->scount, 0, sizeof(int) * (k.G + 1), s);
+        cudaMemsetAsync(st->sort_nbig, 0, sizeof(int), s);
         build_cells(*st, nd, n - nd, st->scount, st->sstart, s, true);
         const long long m = k.G + 2;
         TSG_LAUNCH(k_offset, nblk(m, 256), 256, s, st->sstart, m, nd);
@@ -2317,7 +2322,6 @@ constexpr int kWarpLists = 65536;
 template <int DIM>
 void build_lists(Fp32State& st, const P32& p, cudaStream_t s) {
     const K32& k = st.k;
-    cudaMemsetAsync(st.novf, 0, sizeof(int), s);
     if (st.cells_per_cta <= 0 && k.n <= kWarpLists) {
         TSG_LAUNCH(k_lists_warp<DIM>, (k.n + 3) / 4, 128, s, k, p.hi, p.lo, st.pf, st.dstart, st.sstart, st.T.cnt,
                    st.T.nbr, st.ovf_list, st.novf);
@@ -2404,8 +2408,8 @@ __global__ void k_copy_back32(int nd, P32 b, P32 a, size_t n) {
 }  // namespace
 
 // List the static-block particles with a non-empty list and write the state of the others.
+// nsact is zero on entry.
 static void static_active(Fp32State& st, cudaStream_t s) {
-    cudaMemsetAsync(st.nsact, 0, sizeof(int), s);
     if (st.n > st.nd)
         TSG_LAUNCH(k_static_active, nblk(st.n - st.nd), TPB, s, st.k, st.P[st.cur], st.T, st.k.solver == 1 ? 1 : 0,
                    st.sact, st.nsact);
@@ -2414,6 +2418,7 @@ static void static_active(Fp32State& st, cudaStream_t s) {
 // Re-sort the dynamic block and rebuild every list.  in_place keeps the current buffer
 // (the sorted block is copied back), as a captured graph needs fixed pointers.
 void f32::rebuild(Fp32State& st, cudaStream_t s, bool in_place) {
+    cudaMemsetAsync(st.dcount, 0, sizeof(int) * (st.k.G + 5), s);
     {
         PhaseScope ph(s, PH_SORT);
         if (st.nd > 0) {
@@ -2430,7 +2435,6 @@ void f32::rebuild(Fp32State& st, cudaStream_t s, bool in_place) {
         else build_lists<2>(st, st.P[st.cur], s);
         static_active(st, s);
     }
-    cudaMemsetAsync(st.maxdisp, 0, sizeof(unsigned), s);
 }
 
 void fp32_sort(Fp32State& st, cudaStream_t s) {
@@ -3280,7 +3284,10 @@ int fp32_write(Fp32State& st, const char* name, const void* src, bool from_devic
     if (what == 0) st.lists_valid = false;
     // boundary particles without flow neighbours: their extrapolated state follows an
     // imported velocity / pressure at once (it is otherwise written at list builds only)
-    if (st.built && (what == 1 || what == 3)) static_active(st, s);
+    if (st.built && (what == 1 || what == 3)) {
+        cudaMemsetAsync(st.nsact, 0, sizeof(int), s);
+        static_active(st, s);
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : TSG_E_CUDA;
 }
 

@@ -70,6 +70,11 @@ struct Consts {
 // Largest cell segment the counting sort's last step gives to one thread (tsg_cellsort.cuh),
 // and the size of its list of larger cells (at most n / (kSortSmall + 1) of them).
 constexpr int kSortSmall = 256;
+// Up to this many particles the reorder pass ranks every cell itself, however large (all of them
+// in one cell: 16,384 loads a thread, a fraction of a millisecond), and the launch that orders
+// the larger cells is left out.
+constexpr int kSortAll = 16384;
+inline int sort_small(int n) { return n <= kSortAll ? 0x7fffffff : kSortSmall; }
 inline size_t cellsort_big_ints(long long n) { return (size_t)(n / kSortSmall + 2); }
 
 // Block size of the rigid-object list builder (tsg_rigid_list.cuh) and its scratch size.

@@ -150,16 +150,16 @@ __global__ void __launch_bounds__(SCAN_ONE_TPB) k_scan_one(const int* __restrict
     if (threadIdx.x == SCAN_ONE_TPB - 1) out[n] = e;  // grand total
 }
 
-// Places the particles in arrival order inside their cells and lists the cells above
-// kSortSmall, which k_cell_sort_big orders; k_reorder64 ranks the particles of the others.
+// Places the particles in arrival order inside their cells and lists the cells above `small`
+// particles, which k_cell_sort_big orders; k_reorder64 ranks the particles of the others.
 __global__ void k_scatter(int n, const int* __restrict__ cell_of, const int* __restrict__ rank,
-                          const int* __restrict__ cell_start, int* __restrict__ perm, int* __restrict__ big,
-                          int* __restrict__ nbig) {
+                          const int* __restrict__ cell_start, int* __restrict__ perm, int small,
+                          int* __restrict__ big, int* __restrict__ nbig) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int c = cell_of[i], r = rank[i], b = cell_start[c];
     perm[b + r] = i;
-    if (r == 0 && cell_start[c + 1] - b > kSortSmall) big[atomicAdd(nbig, 1)] = c;
+    if (r == 0 && cell_start[c + 1] - b > small) big[atomicAdd(nbig, 1)] = c;
 }
 
 __device__ __forceinline__ void append(int* list, int* counter, bool pred, int value) {
@@ -180,7 +180,7 @@ __device__ __forceinline__ void append(int* list, int* counter, bool pred, int v
 template <bool SOIL>
 __global__ void k_reorder64(Consts c, const int* __restrict__ perm, Persist64 a, Persist64 b,
                             float4* __restrict__ pos32, float4* __restrict__ pos32l,
-                            const int* __restrict__ cell_of, const int* __restrict__ cell_start,
+                            const int* __restrict__ cell_of, const int* __restrict__ cell_start, int small,
                             const long long* __restrict__ cell_src, long long* __restrict__ cell0,
                             unsigned char* __restrict__ cell_flow, int* __restrict__ list_flow,
                             int* __restrict__ list_bdy, int* __restrict__ list_count,
@@ -194,7 +194,7 @@ __global__ void k_reorder64(Consts c, const int* __restrict__ perm, Persist64 a,
         // ascending old index inside the cell: this particle's rank among the cell's (a pass of
         // its own, one thread per cell, took 15 us on a 2D grid and 158 us on the 3D benchmark's)
         const int cell = cell_of[s], cb = cell_start[cell], ce = cell_start[cell + 1];
-        if (ce - cb <= kSortSmall) {
+        if (ce - cb <= small) {
             int r = 0;
             for (int q = cb; q < ce; ++q) r += perm[q] < s;
             k = cb + r;
@@ -267,12 +267,13 @@ void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid
     cudaMemsetAsync(g.count, 0, g.zero_bytes, s);
     TSG_LAUNCH(k_hash, nblk(c.n), TPB, s, c, cur.x, g.cell_of, g.rank, g.count, g.cell0_old, g.err);
     scan_exclusive(g.count, g.cell_start, (int)nbins, g.tile_sum, s);
-    TSG_LAUNCH(k_scatter, nblk(c.n), TPB, s, c.n, g.cell_of, g.rank, g.cell_start, g.perm, g.big, g.nbig);
-    TSG_LAUNCH(k_cell_sort_big, 152, kSortBlock, s, g.big, g.nbig, g.cell_start, g.cell_of, c.n, g.perm);
+    const int small = sort_small(c.n);
+    TSG_LAUNCH(k_scatter, nblk(c.n), TPB, s, c.n, g.cell_of, g.rank, g.cell_start, g.perm, small, g.big, g.nbig);
+    if (c.n > kSortAll) TSG_LAUNCH(k_cell_sort_big, 152, kSortBlock, s, g.big, g.nbig, g.cell_start, g.cell_of, c.n, g.perm);
     // small scenes in blocks of one warp, to reach every SM
     const int tpb = c.n < 152 * 4 * TPB ? 32 : TPB, nb = (c.n + tpb - 1) / tpb;
     if (c.solver == 1) {
-        TSG_LAUNCH(k_reorder64<false>, nb, tpb, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, g.cell0_old,
+        TSG_LAUNCH(k_reorder64<false>, nb, tpb, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, small, g.cell0_old,
                    t.cell0, g.cell_flow, g.list_flow, g.list_bdy, g.list_count, nullptr, nullptr);
     } else {
         // mu(I) keeps v_tmp across steps: stage it in aux3 (free until advect_pos) and gather
@@ -281,7 +282,7 @@ void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid
             cudaMemcpyAsync(t.aux3, t.v_tmp, sizeof(double) * 3 * (size_t)c.n, cudaMemcpyDeviceToDevice, s);
             src = t.aux3;
         }
-        TSG_LAUNCH(k_reorder64<true>, nb, tpb, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, g.cell0_old,
+        TSG_LAUNCH(k_reorder64<true>, nb, tpb, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, small, g.cell0_old,
                    t.cell0, g.cell_flow, g.list_flow, g.list_bdy, g.list_count, src, src ? t.v_tmp : nullptr);
     }
     Persist64 tmp = cur;
