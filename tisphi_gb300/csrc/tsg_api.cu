@@ -171,7 +171,7 @@ int alloc_all(tsg_handle* h) {
     rc |= alloc_persist(h, h->nxt, soil);
     Trans64& t = h->t;
     rc |= dalloc(h, &t.v_tmp, 3 * n); rc |= dalloc(h, &t.density_tmp, n);
-    if (soil) { rc |= dalloc(h, &t.stress_tmp, 9 * n); rc |= dalloc(h, &t.v_grad, 9 * n); rc |= dalloc(h, &t.aux9, 9 * n); }
+    if (soil) { rc |= dalloc(h, &t.stress_tmp, 9 * n); rc |= dalloc(h, &t.v_grad, 9 * n); }
     if (c.solver == 3) rc |= dalloc(h, &t.d_stress, 9 * n);
     rc |= dalloc(h, &t.d_density, n); rc |= dalloc(h, &t.d_vel, 3 * n);
     rc |= dalloc(h, &t.CSPM_f, n);

@@ -1139,10 +1139,13 @@ __global__ void k_xsph_rigid(Consts c, Persist64 p, Trans64 t, const int* __rest
 
 // Stress regularisation after advect_pos: centres use their moved positions, candidate
 // cells come from this step's sort (eng/solver_sph_muI.py:151-156).  The rows are rebuilt from
-// the moved positions first (flow neighbours only).
+// the moved positions first (flow neighbours only).  The loop's stress is stress_tmp, which the
+// reference copies into stress just before (:148), so the sums read it there and go straight
+// into stress.  In 2D the four out-of-plane shears are zero unless a caller wrote some: their
+// products (+-0, which no sum starting at +0 notices) are formed only where one is not.
 template <int DIM, int G>
-__global__ void __launch_bounds__(ROWS * G) k_post_mui_b(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
-                                                         const int* __restrict__ list, int count, Pairs64 pr) {
+__global__ void __launch_bounds__(ROWS * G) k_post_mui(Consts c, Persist64 p, Trans64 t, const int* __restrict__ cs,
+                                                       const int* __restrict__ list, int count, Pairs64 pr) {
     constexpr int C = 9;
     __shared__ double S[C][ROWS];
     const int n = c.n;
@@ -1155,12 +1158,25 @@ __global__ void __launch_bounds__(ROWS * G) k_post_mui_b(Consts c, Persist64 p, 
             const double w = pair_W<DIM>(c, p.x, xi, j);
             const double mVj = p.m_V[j];
             double st[9];
-            ld9(st, p.stress, n, j);
-            bool ok = usable(mVj) && usable(w);
-            for (int e = 0; e < 9; ++e) ok = ok && usable(st[e]);
-            on_pipe(ok, [&](auto mul) {
-                for (int e = 0; e < 9; ++e) T[e] = mul(mul(mVj, st[e]), w);
+            ld9(st, t.stress_tmp, n, j);
+            const bool ok = usable(mVj) && usable(w);
+            const bool plane = usable(st[0]) && usable(st[1]) && usable(st[3]) && usable(st[4]) && usable(st[8]);
+            on_pipe(ok && plane, [&](auto mul) {
+                T[0] = mul(mul(mVj, st[0]), w);
+                T[1] = mul(mul(mVj, st[1]), w);
+                T[3] = mul(mul(mVj, st[3]), w);
+                T[4] = mul(mul(mVj, st[4]), w);
+                T[8] = mul(mul(mVj, st[8]), w);
             });
+            // (a factor that is not finite makes them NaN, not zero)
+            if (DIM == 3 || !ok || !(zero(st[2]) && zero(st[5]) && zero(st[6]) && zero(st[7]))) {
+                on_pipe(ok && usable(st[2]) && usable(st[5]) && usable(st[6]) && usable(st[7]), [&](auto mul) {
+                    T[2] = mul(mul(mVj, st[2]), w);
+                    T[5] = mul(mul(mVj, st[5]), w);
+                    T[6] = mul(mul(mVj, st[6]), w);
+                    T[7] = mul(mul(mVj, st[7]), w);
+                });
+            }
         });
     }
     const int row = blockIdx.x * ROWS + threadIdx.x;
@@ -1176,19 +1192,12 @@ __global__ void __launch_bounds__(ROWS * G) k_post_mui_b(Consts c, Persist64 p, 
             if (p.mat_type[j] != MAT_SOIL) return;
             const double w = kernel_W(c, rn);
             const double mVj = p.m_V[j];
-            for (int q = 0; q < 9; ++q) s[q] += mVj * p.stress[(size_t)q * n + j] * w;
+            for (int q = 0; q < 9; ++q) s[q] += mVj * t.stress_tmp[(size_t)q * n + j] * w;
         });
     }
     const double f = t.CSPM_f[i];
-    for (int q = 0; q < 9; ++q) t.aux9[(size_t)q * n + i] = s[q] * f;
-}
-
-__global__ void k_post_mui_c(Consts c, Persist64 p, Trans64 t) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    if (p.mat_type[i] != MAT_SOIL) return;
-    const int n = c.n;
-    for (int q = 0; q < 9; ++q) p.stress[(size_t)q * n + i] = t.aux9[(size_t)q * n + i];
+    for (int q = 0; q < 9; ++q) s[q] = s[q] * f;
+    st9(p.stress, s, n, i);
 }
 
 // ---- per-particle passes ----
@@ -1231,7 +1240,7 @@ __global__ void __launch_bounds__(TPB) k_particle(Consts c, Persist64 p, Trans64
     }
     if (SOIL && soil) {
         if ((ops & OP_INIT) || (dp && ((ops & (OP_RK_STAGE | OP_FULL | OP_RK_FINAL)) || post))) ld9(st, p.stress, n, i);
-        if ((dp && ((ops & OP_HALF) || (pre && !has))) || (!dp && post)) ld9(stt, t.stress_tmp, n, i);
+        if (dp && ((ops & OP_HALF) || (pre && !has))) ld9(stt, t.stress_tmp, n, i);
         if (dp && (ops & rates_in)) ld9(ds, t.d_stress, n, i);
         if (dp && (ops & (OP_RK_UPDATE | OP_RK_FINAL)) && !(ops & OP_RK_INIT)) ld9(as, t.d_stress_RK, n, i);
         if (post) {
@@ -1342,7 +1351,6 @@ __global__ void __launch_bounds__(TPB) k_particle(Consts c, Persist64 p, Trans64
         if ((ops & OP_INIT) || (dp && ((ops & (OP_HALF | OP_RK_STAGE)) || pre))) st9(t.stress_tmp, stt, n, i);
         if (dp && (ops & (OP_RK_INIT | OP_RK_UPDATE))) st9(t.d_stress_RK, as, n, i);
         if (dp && (upd_rho || post)) st9(p.stress, st, n, i);
-        if (!dp && post) st9(p.stress, stt, n, i);
         if (post) {
             p.strain_equ[i] = eq;
             if (dp) { p.strain_equ_p[i] = eqp; p.flag_retmap[i] = flag; }
@@ -1852,8 +1860,7 @@ static void mui_regularise(const Consts& c, Persist64& p, Trans64& t, const Grid
     PhaseScope ph(s, PH_POST);
     if (g.pr.cap_f) fp64_refresh_pos32(c, p, t, s);
     build_rows(c, p, t, g, true, false, s);
-    DISPATCH_ROWS(c, g, k_post_mui_b, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
-    TSG_LAUNCH(k_post_mui_c, nblk(c.n), TPB, s, c, p, t);
+    DISPATCH_ROWS(c, g, k_post_mui, c.n_flow, c, p, t, g.cell_start, g.list_flow, c.n_flow, g.pr);
 }
 
 // substep by the integrator, from the per-particle first phase of its first loops (run by the

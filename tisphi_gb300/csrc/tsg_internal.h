@@ -128,7 +128,6 @@ struct Trans64 {
     double* d_vel_RK;   // 3 planes
     double* d_stress_RK;// 9 planes or nullptr
     double* aux3;       // 3 planes: XSPH sums
-    double* aux9;       // 9 planes: regularised stress (mu(I))
     float4* pos32;      // (x - vdomain_start) as f32, candidate prefilter; w = 1 for flow particles
     float4* pos32l;     // what pos32 rounds off, as f32
     long long* cell0;   // flattened cell index of the position, kNoCell if it has none

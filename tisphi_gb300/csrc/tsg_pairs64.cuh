@@ -160,6 +160,9 @@ __device__ __forceinline__ bool usable(double a) {  // +-0 or 2^-255 <= |a| < 2^
     const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
     return hi - (768u << 20) < (512u << 20) || (hi | (unsigned)__double2loint(a)) == 0u;
 }
+__device__ __forceinline__ bool zero(double a) {
+    return (((unsigned)__double2hiint(a) & 0x7fffffffu) | (unsigned)__double2loint(a)) == 0u;
+}
 __device__ __forceinline__ double int_mul(double a, double b) {
     const unsigned ah = __double2hiint(a), al = __double2loint(a);
     const unsigned bh = __double2hiint(b), bl = __double2loint(b);
@@ -180,9 +183,9 @@ __device__ __forceinline__ double int_mul(double a, double b) {
     const unsigned ea = ah & 0x7ff00000u, eb = bh & 0x7ff00000u;
     const unsigned e = ea + eb - (1023u << 20) - (sh << 20) + h1;
     const unsigned long long r = (((unsigned long long)e << 32) | h0) + up;
-    const bool zero = min(ea, eb) == 0u;
-    return __hiloint2double((int)((zero ? 0u : (unsigned)(r >> 32)) | ((ah ^ bh) & 0x80000000u)),
-                            zero ? 0 : (int)(unsigned)r);
+    const bool none = min(ea, eb) == 0u;  // a zero factor
+    return __hiloint2double((int)((none ? 0u : (unsigned)(r >> 32)) | ((ah ^ bh) & 0x80000000u)),
+                            none ? 0 : (int)(unsigned)r);
 }
 
 
