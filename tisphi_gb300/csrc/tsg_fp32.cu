@@ -99,7 +99,7 @@ __global__ void k_reorder32(K32 k, int count_n, int base, const int* __restrict_
     float pfv[3];
     for (int d = 0; d < 3; ++d) {
         double x = (double)hv[d] + (double)lv[d];
-        double hq = (double)k.Q * rint(x / (double)k.Q);
+        double hq = (double)k.Q * rint(x * (double)k.inv_Q);  // Q is a power of two: exact, like the division
         hv[d] = (float)hq;
         lv[d] = (float)(x - hq);
         pfv[d] = (float)x;
@@ -158,19 +158,22 @@ __global__ void k_lists(K32 k, const float4* __restrict__ HI, RecView LO,
     if (m > k.maxn) note_overflow(ovf_list, novf, i);
 }
 
-// The same lists by a warp per particle, for scenes too small to fill the GPU with one thread
-// per particle: 32 candidates of a stencil row are tested at a time and the accepted ones take
+// The same lists by LP lanes per particle, for scenes too small to fill the GPU with one thread
+// per particle: LP candidates of a stencil row are tested at a time and the accepted ones take
 // their slots in order by ballot.  The tests are enum_neighbors' own, so the lists are equal.
-template <int DIM>
+template <int DIM, int LP>
 __global__ void k_lists_warp(K32 k, const float4* __restrict__ HI, RecView LO, const float4* __restrict__ PF,
                              const int* __restrict__ dstart, const int* __restrict__ sstart, int* __restrict__ cnt,
                              int* __restrict__ nbr, int* __restrict__ ovf_list, int* __restrict__ novf) {
-    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (i >= k.n) return;
+    const int lane = threadIdx.x & 31, g = lane % LP, gb = lane - g;
+    int i = (blockIdx.x * blockDim.x + threadIdx.x) / LP;
+    const bool live = i < k.n;
+    if (!live) i = k.n - 1;
+    const unsigned gmask = LP == 32 ? 0xffffffffu : ((1u << (LP & 31)) - 1u) << gb;  // this particle's lanes
     const float4 hi_i = HI[i], lo_i = LO[i], pf_i = PF[i];
     const bool flow_i = is_flow(tf_type(pf_i.w));
     constexpr int NR = DIM == 3 ? 9 : 3;
+    static_assert(2 * NR <= LP, "a lane per stencil row");
     bool ok = true;
     const long long cc0 = cell_coord(k, hi_i.x, lo_i.x, ok);
     const long long cc1 = cell_coord(k, hi_i.y, lo_i.y, ok);
@@ -179,9 +182,9 @@ __global__ void k_lists_warp(K32 k, const float4* __restrict__ HI, RecView LO, c
     // lanes 0 .. 2 NR - 1 hold the candidate ranges: the dynamic block's stencil rows, then the
     // static block's
     int jb_l = 0, je_l = 0;
-    if (ok && lane < (flow_i ? 2 * NR : NR)) {
-        const int* cs = lane < NR ? dstart : sstart;
-        const int q = lane < NR ? lane : lane - NR;
+    if (live && ok && g < (flow_i ? 2 * NR : NR)) {
+        const int* cs = g < NR ? dstart : sstart;
+        const int q = g < NR ? g : g - NR;
         const long long ny = k.gnum[1], nz = k.gnum[2], G = k.G;
         const int ox = DIM == 3 ? q / 3 - 1 : q - 1, oy = DIM == 3 ? q % 3 - 1 : 0;
         const long long f0 = (cc0 + ox) * ny * nz + (cc1 + oy) * nz + cc2;
@@ -191,12 +194,16 @@ __global__ void k_lists_warp(K32 k, const float4* __restrict__ HI, RecView LO, c
     }
     int m = 0;
     unsigned rows = __ballot_sync(0xffffffffu, jb_l < je_l);
+    if (LP < 32) {  // a row that any particle of the warp has
+        for (int o = LP; o < 32; o <<= 1) rows |= (rows >> o) | (rows << (32 - o));
+        rows &= (1u << (2 * NR)) - 1u;
+    }
     while (rows) {
         const int q = __ffs(rows) - 1;
         rows &= rows - 1u;
-        const int jb = __shfl_sync(0xffffffffu, jb_l, q), je = __shfl_sync(0xffffffffu, je_l, q);
-        for (int b = jb; b < je; b += 32) {
-            const int j = b + lane;
+        const int jb = __shfl_sync(0xffffffffu, jb_l, gb + q), je = __shfl_sync(0xffffffffu, je_l, gb + q);
+        for (int b = jb; __any_sync(0xffffffffu, b < je); b += LP) {
+            const int j = b + g;
             bool in = false;
             float4 hj = hi_i;
             if (j < je && j != i) {
@@ -215,13 +222,13 @@ __global__ void k_lists_warp(K32 k, const float4* __restrict__ HI, RecView LO, c
                     in = dist2<DIM>(d) < k.R2L;
                 }
             }
-            const unsigned bal = __ballot_sync(0xffffffffu, in);
+            const unsigned bal = __ballot_sync(0xffffffffu, in) & gmask;
             const int slot = m + __popc(bal & ((1u << lane) - 1u));
             if (in && slot < k.maxn) nbr[(size_t)slot * k.n + i] = entry_of(k, j, hi_i, hj);
             m += __popc(bal);
         }
     }
-    if (lane == 0) {
+    if (live && g == 0) {
         cnt[i] = m;
         if (m > k.maxn) note_overflow(ovf_list, novf, i);
     }
@@ -1048,11 +1055,12 @@ __global__ void k_mui_stress32(K32 k, P32 p, T32 t, const float4* __restrict__ P
             load_L(t.L, k.n, i, L);
         float vg[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         CSum dd;
-        for_nbrs<DIM, FB>(k, i, t.cnt, t.nbr, p.hi, p.lo, PF, dstart, sstart, true,
-                          [&](int j, const float* d, float r2, int sidx, int, float mVj) {
+        for_nbrs_g<DIM, FB, false, true>(
+            k, i, t.cnt, t.nbr, p.hi, p.lo, PF, dstart, sstart, true, [&](int j) { return t.vt[j]; },
+            [&](int j, const float* d, float r2, int sidx, int, float mVj, const float4& vtj) {
             float kc[3];
             grad_c<DIM, CORR>(L, w_grad(k, fast_sqrt(r2)), d, kc);
-            vgrad_add<DIM>(mVj, vti, vli, t.vt[j], t.vtlo[j], kc, vg, dd);
+            vgrad_add<DIM>(mVj, vti, vli, vtj, t.vtlo[j], kc, vg, dd);
             if (sidx % kFlushEvery == kFlushEvery - 1) dd.flush();
         });
         const size_t n = k.n;
@@ -1262,7 +1270,12 @@ __global__ void k_post_mui32(K32 k, P32 p, T32 t) {
 // order and the list offsets give the same displacement bits, so both visit the soil
 // neighbours within the support in the same order and give the same sums (for particles
 // that have not changed cell since the sort; otherwise the order, not the set, differs).
-template <int DIM>
+// PACKED (the step sequence, where no caller can have written stress_tmp since the momentum
+// pass): the neighbour's stress comes from that pass's record, one 128-bit read and zz in 2D, one
+// 256-bit read in 3D, instead of six 32-bit gathers; in 2D the out-of-plane shears it leaves out
+// are zero (0 times xx below: NaN after a blow-up, as their sums would be).  Four list entries
+// per trip, all their reads issued before the first is used.  320,000 particles in 2D: 62 -> 50 us.
+template <int DIM, bool PACKED>
 __global__ void k_reg_mui32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
                             const int* __restrict__ sstart, const unsigned* __restrict__ maxd, float list_d2) {
     const bool lists_ok = list_d2 > 0.f && __uint_as_float(*maxd) <= list_d2;
@@ -1273,17 +1286,50 @@ __global__ void k_reg_mui32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, 
         const int m = t.cnt[i];
         if (lists_ok && m <= k.maxn) {
             const float4 lo_i = p.lo[i];
-            for (int q = 0; q < m; ++q) {
-                const int e = t.nbr[(size_t)q * n + i];
-                if (class_type((e >> kEntryBits) & 7) != MAT_SOIL) continue;
-                const int j = e & kEntryMask;
-                const float4 l = p.lo[j];
-                float d[3];
-                const float r2 = list_delta<DIM>(k, e, lo_i, l, d);
-                if (!(r2 < k.R2)) continue;
-                const float mw = l.w * w_val(k, fast_sqrt(r2));
-                for (int c = 0; c < 6; ++c) s[c] += mw * t.sigt[c * n + j];
+            const int* lp = t.nbr + i;
+            constexpr int U = 4;
+            int e[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) e[u] = u < m ? __ldcs(lp + u * n) : 0;
+            for (int q = 0; q < m; q += U) {
+                int nx[U];
+                float4 l[U];
+                float st[U][6];
+#pragma unroll
+                for (int u = 0; u < U; ++u) nx[u] = q + U + u < m ? __ldcs(lp + (q + U + u) * n) : 0;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (q + u >= m) continue;
+                    const int j = e[u] & kEntryMask;
+                    l[u] = p.lo[j];
+                    if (!PACKED) {
+#pragma unroll
+                        for (int c = 0; c < 6; ++c) st[u][c] = t.sigt[c * n + j];
+                    } else if (DIM == 2) {
+                        const float4 sa = t.srec[j];
+                        st[u][0] = sa.x; st[u][1] = sa.y; st[u][3] = sa.z;
+                        st[u][2] = t.sigt[2 * n + j];
+                    } else {
+                        float4 sa, sb;
+                        ldg_rec(t.srec, j, sa, sb);
+                        st[u][0] = sa.x; st[u][1] = sa.y; st[u][2] = sa.z;
+                        st[u][3] = sb.x; st[u][4] = sb.y; st[u][5] = sb.z;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (q + u >= m || class_type((e[u] >> kEntryBits) & 7) != MAT_SOIL) continue;
+                    float d[3];
+                    const float r2 = list_delta<DIM>(k, e[u], lo_i, l[u], d);
+                    if (!(r2 < k.R2)) continue;
+                    const float mw = l[u].w * w_val(k, fast_sqrt(r2));
+#pragma unroll
+                    for (int c = 0; c < (PACKED && DIM == 2 ? 4 : 6); ++c) s[c] += mw * st[u][c];
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) e[u] = nx[u];
             }
+            if (PACKED && DIM == 2) s[4] = s[5] = s[0] * 0.f;
         } else {
             enum_neighbors<DIM>(k, i, p.hi, p.lo, PF, dstart, sstart, false, [&](int j, const float*, float r2) {
                 if (tf_type(p.hi[j].w) != MAT_SOIL) return;
@@ -2316,14 +2362,19 @@ void lists_by_cell(Fp32State& st, const P32& p, cudaStream_t s) {
                st.dstart, st.sstart, st.T.cnt, st.T.nbr, st.ovf_list, st.novf);
 }
 
-// Up to this many particles a warp each builds the lists.
+// Up to this many particles a half warp (2D; a row of three cells holds some 30) or a warp each
+// builds the lists: 3,274 particles 42 us with a thread each, 13 us with a warp; 2D dambreak of
+// 9,144, ten steps, 818 us with a warp, 790 us with a half.  A batch of 536,000 particles fills
+// the GPU either way and loses by the uncoalesced list writes (1,992 -> 2,581 us).
 constexpr int kWarpLists = 65536;
+template <int DIM>
+constexpr int kListLanes = DIM == 3 ? 32 : 16;
 
 template <int DIM>
 void build_lists(Fp32State& st, const P32& p, cudaStream_t s) {
     const K32& k = st.k;
     if (st.cells_per_cta <= 0 && k.n <= kWarpLists) {
-        TSG_LAUNCH(k_lists_warp<DIM>, (k.n + 3) / 4, 128, s, k, p.hi, p.lo, st.pf, st.dstart, st.sstart, st.T.cnt,
+        TSG_LAUNCH((k_lists_warp<DIM, kListLanes<DIM>>), nblk(kListLanes<DIM> * (long long)k.n, 128), 128, s, k, p.hi, p.lo, st.pf, st.dstart, st.sstart, st.T.cnt,
                    st.T.nbr, st.ovf_list, st.novf);
         return;
     }
@@ -2666,6 +2717,30 @@ static void advect_pos(Fp32State& st, cudaStream_t s, bool post) {
     if (k.disp2_limit <= 0.f) st.lists_valid = false;
 }
 
+// packed: the momentum pass's stress records still hold stress_tmp (see k_reg_mui32).
+static void advect_something(Fp32State& st, cudaStream_t s, bool packed) {
+    const K32& k = st.k;
+    P32& p = st.P[st.cur];
+    PhaseScope ph(s, PH_POST);
+    if (k.solver == 1) TSG_LAUNCH(k_post_wc32, nblk(k.nd), TPB, s, k, p);
+    else if (k.solver == 2) {
+        TSG_LAUNCH(k_post_mui32, nblk(k.nd), TPB, s, k, p, st.T);
+        // the regularisation reads the lists while no particle has moved more than 0.49
+        // skin since their build ((0.49 / 0.45)^2 = 1.1857 times the rebuild threshold),
+        // measured here from the moved positions (the next step's check finds the same)
+        float list_d2 = -1.f;
+        if (st.lists_valid && k.disp2_limit > 0.f) {
+            TSG_LAUNCH(k_disp32, nblk(k.nd), TPB, s, k, p.hi, p.lo, st.pf, st.maxdisp);
+            list_d2 = k.disp2_limit * 1.185f;
+        }
+#define REG_MUI(D, PK) \
+    TSG_LAUNCH((k_reg_mui32<D, PK>), nblk(k.nd), TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, st.maxdisp, list_d2)
+        if (k.dim == 2) { if (packed) REG_MUI(2, true); else REG_MUI(2, false); }
+        else { if (packed) REG_MUI(3, true); else REG_MUI(3, false); }
+#undef REG_MUI
+    } else TSG_LAUNCH(k_post_dp32, nblk(k.nd), TPB, s, k, p, st.T);
+}
+
 void fp32_advect(Fp32State& st, int which, cudaStream_t s) {
     const K32& k = st.k;
     P32& p = st.P[st.cur];
@@ -2673,28 +2748,7 @@ void fp32_advect(Fp32State& st, int which, cudaStream_t s) {
     case TSG_ADVECT_FULL: { PhaseScope ph(s, PH_INTEGRATE); TSG_LAUNCH(k_advect_full32, nblk(k.nd), TPB, s, k, p, st.T, st.err); break; }
     case TSG_ADVECT_LF_HALF: { PhaseScope ph(s, PH_INTEGRATE); TSG_LAUNCH(k_advect_half32<false>, nblk(k.nd), TPB, s, k, p, st.T); break; }
     case TSG_ADVECT_POS: advect_pos(st, s, false); break;
-    case TSG_ADVECT_SOMETHING: {
-        PhaseScope ph(s, PH_POST);
-        if (k.solver == 1) TSG_LAUNCH(k_post_wc32, nblk(k.nd), TPB, s, k, p);
-        else if (k.solver == 2) {
-            TSG_LAUNCH(k_post_mui32, nblk(k.nd), TPB, s, k, p, st.T);
-            // the regularisation reads the lists while no particle has moved more than 0.49
-            // skin since their build ((0.49 / 0.45)^2 = 1.1857 times the rebuild threshold),
-            // measured here from the moved positions (the next step's check finds the same)
-            float list_d2 = -1.f;
-            if (st.lists_valid && k.disp2_limit > 0.f) {
-                TSG_LAUNCH(k_disp32, nblk(k.nd), TPB, s, k, p.hi, p.lo, st.pf, st.maxdisp);
-                list_d2 = k.disp2_limit * 1.185f;
-            }
-            if (k.dim == 2)
-                TSG_LAUNCH(k_reg_mui32<2>, nblk(k.nd), TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, st.maxdisp,
-                           list_d2);
-            else
-                TSG_LAUNCH(k_reg_mui32<3>, nblk(k.nd), TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, st.maxdisp,
-                           list_d2);
-        } else TSG_LAUNCH(k_post_dp32, nblk(k.nd), TPB, s, k, p, st.T);
-        break;
-    }
+    case TSG_ADVECT_SOMETHING: advect_something(st, s, false); break;
     case TSG_ENFORCE_BOUNDARY: { PhaseScope ph(s, PH_OTHER); TSG_LAUNCH(k_enforce32, nblk(k.nd), TPB, s, k, p); break; }
     case TSG_RK_INIT: { PhaseScope ph(s, PH_INTEGRATE); TSG_LAUNCH(k_rk_init32, nblk(k.nd), TPB, s, k, p, st.T); break; }
     case TSG_RK_STAGE: { PhaseScope ph(s, PH_INTEGRATE); TSG_LAUNCH(k_rk_stage32, nblk(k.nd), TPB, s, k, p, st.T); break; }
@@ -2768,7 +2822,7 @@ void f32::step_body(Fp32State& st, cudaStream_t s, bool collide, bool fold_disp)
         advect_pos(st, s, true);  // advect_something of WCSPH is the density clamp, fused
     } else {
         advect_pos(st, s, false);
-        fp32_advect(st, TSG_ADVECT_SOMETHING, s);
+        advect_something(st, s, true);
     }
     fp32_solve_rigid(st, s);
     if (collide || st.rnobj) fp32_advect(st, TSG_ENFORCE_BOUNDARY, s);
