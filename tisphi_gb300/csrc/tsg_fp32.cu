@@ -924,8 +924,8 @@ __global__ void __launch_bounds__(kRigidBlock) k_rigid_rest32(const int* __restr
 // with the inverse CSPM matrix (built by the same loop in the first pass, read back in the
 // second): (L (v_i - v_j)) . dx = sum_ab L_ab dv_b dx_a and L is symmetric, so a neighbour
 // costs six multiply-adds into the tensor instead of L applied to its velocity difference.
-template <int DIM, bool FB, bool CORR, int KT, int REP, bool FL = false>
-__global__ void __launch_bounds__(256, 4) k_rates32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+template <int DIM, bool FB, bool CORR, int KT, int REP, bool FL = false, int U = 2>
+__global__ void __launch_bounds__(256, U == 2 ? 4 : 2) k_rates32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
                           const int* __restrict__ sstart, Ovf ovf) {
     constexpr bool FLC = FL && CORR;  // the CSPM matrix is built in this pass
     // with CORR both passes sum the continuity tensor and contract it with L after the loop
@@ -951,7 +951,7 @@ __global__ void __launch_bounds__(256, 4) k_rates32(K32 k, P32 p, T32 t, const f
         // viscosity factor for fluid and for boundary neighbours; -rho0 p_i / rho_i^2
         const float vf_f = visc_fac, vf_b = visc_fac * visc_b;
         const float pi_n = -k.rho0 * vti.w;
-        for_nbrs_g<DIM, FB, true, true>(k, i, t.cnt, t.nbr, p.hi, p.lo, PF, dstart, sstart, true,
+        for_nbrs_g<DIM, FB, true, true, U>(k, i, t.cnt, t.nbr, p.hi, p.lo, PF, dstart, sstart, true,
                                         [&](int j) { return t.vt[j]; },
                                   [&](int, const float* d, float r2, int sidx, int cj, float mVj, const float4& vtj) {
             const WG wg = w_pair<FL, true, KT>(k, r2);
@@ -2555,18 +2555,23 @@ void corr_launch(Fp32State& st, cudaStream_t s, const Ovf& ovf, bool skip_fluid,
                sf, ovf);
 }
 
+// Up to this many particles a thread each leaves every SM short of warps, and the rates pass
+// reads four records per trip (2D dambreak of 9,144, ten steps: 804 -> 783 us; a larger scene
+// loses by the registers).
+constexpr int kFewParticles = 152 * 128;
+
 // WCSPH boundary extrapolation over [base, base + count_n); the static block (base = nd)
 // visits its listed particles only.
 template <int DIM, bool SH>
 void bdy_launch(Fp32State& st, const P32& p, int base, int count_n, cudaStream_t s, const Ovf& ovf) {
     const K32& k = st.k;
-    const int nb = nblk(count_n, st.tpb);
+    const int tpb = st.tpb, nb = nblk(count_n, tpb);
     const int* act = base == k.nd ? st.sact : nullptr;
     if (k.kernel == 1)
-        TSG_LAUNCH((k_bdy32<DIM, false, 1, SH>), nb, st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n,
+        TSG_LAUNCH((k_bdy32<DIM, false, 1, SH>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n,
                    act, st.nsact, ovf);
     else
-        TSG_LAUNCH((k_bdy32<DIM, false, 0, SH>), nb, st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n,
+        TSG_LAUNCH((k_bdy32<DIM, false, 0, SH>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n,
                    act, st.nsact, ovf);
     TSG_LAUNCH((k_bdy32<DIM, true, -1, SH>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n, act,
                st.nsact, ovf);
@@ -2575,11 +2580,13 @@ void bdy_launch(Fp32State& st, const P32& p, int base, int count_n, cudaStream_t
 template <int DIM, bool CORR, int KT, bool FL>
 void rates_main(Fp32State& st, const P32& p, cudaStream_t s, const Ovf& ovf) {
     const K32& k = st.k;
-    const int nb = nblk(k.nd, st.tpb);
+    const int tpb = st.tpb, nb = nblk(k.nd, tpb);
     if (k.boundary == 3 || k.boundary == 4)
-        TSG_LAUNCH((k_rates32<DIM, false, CORR, KT, 1, FL>), nb, st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
+        TSG_LAUNCH((k_rates32<DIM, false, CORR, KT, 1, FL>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
+    else if (k.nd <= kFewParticles)
+        TSG_LAUNCH((k_rates32<DIM, false, CORR, KT, 0, FL, 4>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
     else
-        TSG_LAUNCH((k_rates32<DIM, false, CORR, KT, 0, FL>), nb, st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
+        TSG_LAUNCH((k_rates32<DIM, false, CORR, KT, 0, FL>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
 }
 
 template <int DIM, bool CORR, bool FL = false>
@@ -2611,13 +2618,13 @@ void soil_one_step(Fp32State& st, cudaStream_t s) {
     const K32& k = st.k;
     P32& p = st.P[st.cur];
     const Ovf ovf{st.ovf_list, st.novf};
-    const int nb = nblk(k.nd, st.tpb);
+    const int tpb = st.tpb, nb = nblk(k.nd, tpb);
     {
         PhaseScope ph(s, PH_PRE);
         if (k.solver == 2) {
-            if (k.corr) { TSG_LAUNCH((k_mui_stress32<DIM, false, true>), nb, st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
+            if (k.corr) { TSG_LAUNCH((k_mui_stress32<DIM, false, true>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
                           TSG_LAUNCH((k_mui_stress32<DIM, true, true>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf); }
-            else { TSG_LAUNCH((k_mui_stress32<DIM, false, false>), nb, st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
+            else { TSG_LAUNCH((k_mui_stress32<DIM, false, false>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
                    TSG_LAUNCH((k_mui_stress32<DIM, true, false>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf); }
         } else {
             TSG_LAUNCH(k_pre_dp32, nblk(k.nd), TPB, s, k, p, st.T);
@@ -2627,7 +2634,7 @@ void soil_one_step(Fp32State& st, cudaStream_t s) {
         PhaseScope ph(s, PH_BDY);
         auto bdy = [&](int base, int count_n) {
             if (count_n <= 0) return;
-            TSG_LAUNCH((k_bdy_soil32<DIM, false>), nblk(count_n, st.tpb), st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n, ovf);
+            TSG_LAUNCH((k_bdy_soil32<DIM, false>), nblk(count_n, tpb), tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n, ovf);
             TSG_LAUNCH((k_bdy_soil32<DIM, true>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n, ovf);
         };
         bdy(k.nd, k.n - k.nd);
@@ -2638,7 +2645,7 @@ void soil_one_step(Fp32State& st, cudaStream_t s) {
         TSG_LAUNCH(k_pack_stress32<DIM>, nblk(k.n), TPB, s, k, st.T);
 #define SOIL_MOM(CORR, DP)                                                                                       \
         do {                                                                                                     \
-            TSG_LAUNCH((k_soil_mom32<DIM, false, CORR, DP>), nb, st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf); \
+            TSG_LAUNCH((k_soil_mom32<DIM, false, CORR, DP>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf); \
             TSG_LAUNCH((k_soil_mom32<DIM, true, CORR, DP>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);  \
         } while (0)
         if (k.solver == 2) { if (k.corr) SOIL_MOM(true, false); else SOIL_MOM(false, false); }

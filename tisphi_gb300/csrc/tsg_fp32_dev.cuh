@@ -302,7 +302,9 @@ __device__ __forceinline__ float list_delta(const K32& k, int e, const float4& l
 // REC: the payload is the neighbour's v_tmp record, loaded together with its lo record in
 // one 256-bit read (ldg_rec) instead of through gather(j) (the overflow traversal still
 // calls gather).
-template <int DIM, bool FB, bool CODE = false, bool REC = false, class G, class F>
+// U = 4 (with REC): four entries per trip, for scenes that leave the SMs short of warps and
+// wait on the entry -> record chain; the visits keep their order, so sums keep their bits.
+template <int DIM, bool FB, bool CODE = false, bool REC = false, int U = 2, class G, class F>
 __device__ __forceinline__ void for_nbrs_g(const K32& k, int i, const int* __restrict__ cnt, const int* __restrict__ nbr,
                                            const float4* __restrict__ HI, RecView LO,
                                            const float4* __restrict__ PF, const int* __restrict__ dstart,
@@ -319,6 +321,26 @@ __device__ __forceinline__ void for_nbrs_g(const K32& k, int i, const int* __res
             const int c = (e >> kEntryBits) & 7;
             if (r2 < k.R2) body(e & kEntryMask, d, r2, s, CODE ? c : class_type(c), l.w, g);
         };
+        if constexpr (U > 2) {
+            int e[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) e[u] = u < m ? __ldcs(lp + u * stride) : 0;
+            for (int q = 0; q < m; q += U) {
+                int nx[U];
+                float4 l[U], g[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) nx[u] = q + U + u < m ? __ldcs(lp + (q + U + u) * stride) : 0;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (q + u < m) ldg_rec(LO.p, e[u] & kEntryMask, l[u], g[u]);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (q + u < m) visit(e[u], l[u], g[u], q + u);
+#pragma unroll
+                for (int u = 0; u < U; ++u) e[u] = nx[u];
+            }
+            return;
+        }
         int s = 0;
         int e0 = 0, e1 = 0;
         if (m > 1) { e0 = __ldcs(lp); e1 = __ldcs(lp + stride); lp += 2 * stride; }
