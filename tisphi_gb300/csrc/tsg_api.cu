@@ -438,7 +438,8 @@ int tsg_create(const tsg_config* cfg, tsg_handle** out) {
     c.div_span = c.R < 0x1p100 && c.eps_h2 > 0x1p-200 ? 1000u << 20 : 0u;
     c.rgrid = 1.0 / c.grid;
     c.grid_span = c.grid > 0x1p-100 && c.grid < 0x1p100 ? 1000u << 20 : 0u;
-    c.wend_int = f.kernel == 1 && c.kk > 0x1p-100 && c.kk < 0x1p100 && c.h1 > 0x1p-100 && c.h1 < 0x1p100;
+    c.kk6 = c.kk / 6.0;
+    c.kern_int = c.kk > 0x1p-100 && c.kk < 0x1p100 && c.h1 > 0x1p-100 && c.h1 < 0x1p100;
     c.pf_lo2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 262144.0)), 0.f);
     c.pf_hi2 = std::nextafter((float)(c.R * c.R * (1.0 + 1.0 / 262144.0)), 1e30f);
     c.R2T = c.R * c.R;

@@ -200,8 +200,8 @@ __device__ __noinline__ KernelVals slow_kernel(KernelConsts c, double r0, double
     return k;
 }
 
-// grad W (if asked for) and W of a separation r.  The Wendland kernel away from its ends runs on
-// the integer pipes but for its two sums; the others take the kernel functions.
+// grad W (if asked for) and W of a separation r.  Both kernels away from their ends run on the
+// integer pipes but for their sums; separations at the ends take the kernel functions.
 template <int DIM>
 __device__ __forceinline__ KernelVals pair_kernel(const Consts& c, const double* r, bool want_dW, bool want_W) {
     const bool r_ok = usable_v<DIM>(r);
@@ -209,18 +209,35 @@ __device__ __forceinline__ KernelVals pair_kernel(const Consts& c, const double*
     on_pipe(r_ok, [&](auto mul) { r2 = dotv<DIM>(r, r, mul); });
     KernelVals k;
     k.W = 0.0;
-    if (c.wend_int && r_ok && above(r2, 0x1p-200)) {
+    if (c.kern_int && r_ok && above(r2, 0x1p-200)) {
         const double rn = int_sqrt(r2);
-        const double q = int_mul(rn, c.h1), q1 = __fma_rn(-0.5, q, 1.0);
+        const double q = int_mul(rn, c.h1);
+        // 1 - q / 2 (Wendland) or 2 - q (cubic) must not vanish
+        const double q1 = c.kernel == 1 ? __fma_rn(-0.5, q, 1.0) : 2.0 - q;
         if (above(rn, EPS) && !above(q, 2.0) && above(q1, 0x1p-50)) {
-            const double q2 = int_mul(q1, q1);
-            if (want_dW) {
-                const unsigned long long X = recip63(rn);
-                const double s = int_mul(int_mul(int_mul(c.kk, int_mul(q2, q1)), int_mul(-5.0, q)), c.h1);
-                for (int d = 0; d < DIM; ++d) k.kd[d] = quot(int_mul(s, r[d]), rn, X);
-                k.rr = int_mul(rn, rn);
+            const unsigned long long X = want_dW ? recip63(rn) : 0ull;
+            if (want_dW) k.rr = int_mul(rn, rn);
+            if (c.kernel == 1) {
+                const double q2 = int_mul(q1, q1);
+                if (want_dW) {
+                    const double s = int_mul(int_mul(int_mul(c.kk, int_mul(q2, q1)), int_mul(-5.0, q)), c.h1);
+                    for (int d = 0; d < DIM; ++d) k.kd[d] = quot(int_mul(s, r[d]), rn, X);
+                }
+                if (want_W) k.W = int_mul(int_mul(c.kk, int_mul(q2, q2)), __fma_rn(2.0, q, 1.0));
+                return k;
             }
-            if (want_W) k.W = int_mul(int_mul(c.kk, int_mul(q2, q2)), __fma_rn(2.0, q, 1.0));
+            double s, w;
+            if (!above(q, 1.0)) {
+                const double q2 = int_mul(q, q);
+                w = int_mul(c.kk, __fma_rn(0.5, int_mul(q2, q), -q2) + 2.0 / 3.0);
+                s = int_mul(int_mul(c.kk, q), int_mul(1.5, q) - 2.0);
+            } else {
+                w = int_mul(c.kk6, int_mul(int_mul(q1, q1), q1));
+                s = int_mul(c.kk, int_mul(int_mul(-0.5, q1), q1));
+            }
+            if (want_dW)
+                for (int d = 0; d < DIM; ++d) k.kd[d] = int_mul(s, int_mul(quot(r[d], rn, X), c.h1));
+            if (want_W) k.W = w;
             return k;
         }
     }
