@@ -69,6 +69,11 @@ struct tsg_handle {
     const double* x_first = nullptr;  // cur.x at upload: tells the buffer parity
     int eager_steps = 0;
     bool no_graphs = false;         // a capture failed: launch eagerly
+    // While the FP64 arrays are laid out: offset into (and, once it is known, base of) the one
+    // allocation that holds them (see alloc_all)
+    char* slab = nullptr;
+    size_t slab_off = 0;
+    int slab_pass = 0;              // 0: separate allocations, 1: measuring, 2: placing
 };
 
 namespace {
@@ -80,6 +85,11 @@ template <class T>
 int dalloc(tsg_handle* h, T** p, size_t count) {
     *p = nullptr;
     if (count == 0) return 0;
+    if (h->slab_pass) {
+        if (h->slab_pass == 2) *p = reinterpret_cast<T*>(h->slab + h->slab_off);
+        h->slab_off += (count * sizeof(T) + 255) & ~size_t(255);
+        return 0;
+    }
     void* q = nullptr;
     if (cudaMalloc(&q, count * sizeof(T)) != cudaSuccess) return TSG_E_CUDA;
     cudaMemset(q, 0, count * sizeof(T));
@@ -144,25 +154,30 @@ int alloc_rows(tsg_handle* h) {
     if (cf <= 0 || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     const size_t bytes = sf * (4 + 8 * (size_t)planes) + sb * 12 + 4 * (size_t)h->n;
     if (bytes > free_b / 2) return 0;
-    auto take = [&](auto** p, size_t count) {
-        void* q = nullptr;
-        if (count && cudaMalloc(&q, count * sizeof(**p)) != cudaSuccess) { cudaGetLastError(); return false; }
-        if (q) h->allocs.push_back(q);
-        *reinterpret_cast<void**>(p) = q;
-        return true;
-    };
+    auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
+    const size_t parts[] = {up(4 * ((size_t)c.n_flow + c.n_bdy)), up(4 * sf), up(4 * sb), up(8 * sf * c.dim), up(8 * sb),
+                            c.solver == 1 ? up(16 * sf) : 0, own_gc ? up(8 * sf * c.dim) : 0};
+    size_t all = 0;
+    for (size_t b : parts) all += b;
+    void* q = nullptr;
+    if (cudaMalloc(&q, all ? all : 256) != cudaSuccess) { cudaGetLastError(); return 0; }
+    h->allocs.push_back(q);
+    char* at = static_cast<char*>(q);
+    auto place = [&](int part) { char* p = at; at += parts[part]; return p; };
     r.slots_f = sf;
-    if (take(&r.cnt, (size_t)c.n_flow + c.n_bdy) && take(&r.nb_f, sf) && take(&r.nb_b, sb) &&
-        take(&r.gk, sf * c.dim) && take(&r.gw, sb) && (c.solver != 1 || take(&r.gden, sf)) &&
-        (!own_gc || take(&r.gc, sf * c.dim))) {
-        if (!own_gc) r.gc = r.gk;
-        r.cap_f = cap_f;
-        r.cap_b = cap_b;
-    }
+    r.cnt = reinterpret_cast<int*>(place(0));
+    r.nb_f = reinterpret_cast<int*>(place(1));
+    r.nb_b = reinterpret_cast<int*>(place(2));
+    r.gk = reinterpret_cast<double*>(place(3));
+    r.gw = reinterpret_cast<double*>(place(4));
+    r.gden = c.solver == 1 ? reinterpret_cast<double2*>(place(5)) : nullptr;
+    r.gc = own_gc ? reinterpret_cast<double*>(place(6)) : r.gk;
+    r.cap_f = cap_f;
+    r.cap_b = cap_b;
     return 0;
 }
 
-int alloc_all(tsg_handle* h) {
+int alloc_arrays(tsg_handle* h) {
     const size_t n = h->n;
     const Consts& c = h->c;
     const bool soil = c.solver != 1;
@@ -199,8 +214,30 @@ int alloc_all(tsg_handle* h) {
     rc |= dalloc(h, &g.err, 1);
     rc |= dalloc(h, &h->d_stage, 9 * n + 16);
     rc |= dalloc(h, &h->d_scratch, 64);
-    if (!rc) rc = alloc_rows(h);
     return rc ? TSG_E_CUDA : 0;
+}
+
+// The FP64 form's arrays in one zeroed allocation (some sixty small ones cost a 2D scene more
+// than its upload); separate ones where no single block is left.
+int alloc_all(tsg_handle* h) {
+    h->slab_pass = 1;
+    h->slab_off = 0;
+    int rc = alloc_arrays(h);
+    const size_t bytes = h->slab_off;
+    void* q = nullptr;
+    if (!rc && cudaMalloc(&q, bytes) == cudaSuccess) {
+        cudaMemset(q, 0, bytes);
+        h->allocs.push_back(q);
+        h->slab = static_cast<char*>(q);
+        h->slab_off = 0;
+        h->slab_pass = 2;
+    } else {
+        cudaGetLastError();
+        h->slab_pass = 0;
+    }
+    if (!rc) rc = alloc_arrays(h);
+    h->slab_pass = 0;
+    return rc ? rc : alloc_rows(h);
 }
 
 __global__ void k_deinterleave(const double* __restrict__ src, double* __restrict__ dst, int n, int k) {
