@@ -158,13 +158,55 @@ __global__ void k_lists(K32 k, const float4* __restrict__ HI, RecView LO,
     if (m > k.maxn) note_overflow(ovf_list, novf, i);
 }
 
+// A static-block particle (fixed boundary) with an empty neighbour list has no flow particle
+// within support + skin: no flow particle reads its extrapolated state, and the values of the
+// list kernels for it (Shepard factor 1, identity CSPM matrix, WCSPH extrapolation 2 v with zero
+// pressure) depend on nothing but its own constant velocity.  They are written here, once per
+// list build, and the per-step kernels visit the particles with lists only.
+__device__ __forceinline__ void static_values(const K32& k, const P32& p, const T32& t, int wc, int i, bool listed) {
+    if (t.L) {  // no static particle is a flow particle: its CSPM matrix is the identity
+        const size_t n = k.n;
+        for (int q = 0; q < 6; ++q) t.L[q * n + i] = q < 3 ? 1.f : 0.f;
+    }
+    if (listed) return;
+    t.cf[i] = 1.f;
+    if (!wc) return;
+    const int ti = tf_type(p.hi[i].w);
+    if (ti == MAT_DUMMY || ti == MAT_REP || ti == MAT_RIGID) {
+        const float4 v = p.vel[i];
+        t.vt[i] = make_float4(2.f * v.x, 2.f * v.y, 2.f * v.z, 0.f);
+        t.pr[i] = make_float2(0.f, k.rho0);
+        t.drt[i] = 0.f;
+        p.vel[i].w = 0.f;
+        if (ti == MAT_RIGID) { t.dd[i] = 0.f; t.dv[i] = make_float4(0.f, 0.f, 0.f, 0.f); }
+    }
+}
+
+// The static-block particles with a non-empty list, in warp-sized runs of the block's order (a
+// run's place in the list depends on scheduling; every consumer treats its particles
+// independently, so results do not), and the values of the others.
+__global__ void k_static_active(K32 k, P32 p, T32 t, int wc, int* __restrict__ act, int* __restrict__ nact) {
+    const int i = k.nd + blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = i < k.n;
+    const bool on = in && t.cnt[i] != 0;
+    const unsigned ball = __ballot_sync(0xffffffffu, on);
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (lane == 0 && ball) base = atomicAdd(nact, __popc(ball));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (on) act[base + __popc(ball & ((1u << lane) - 1u))] = i;
+    if (in) static_values(k, p, t, wc, i, on);
+}
+
 // The same lists by LP lanes per particle, for scenes too small to fill the GPU with one thread
 // per particle: LP candidates of a stencil row are tested at a time and the accepted ones take
 // their slots in order by ballot.  The tests are enum_neighbors' own, so the lists are equal.
+// The static particles' part of the build (k_static_active) is done in the same launch.
 template <int DIM, int LP>
 __global__ void k_lists_warp(K32 k, const float4* __restrict__ HI, RecView LO, const float4* __restrict__ PF,
                              const int* __restrict__ dstart, const int* __restrict__ sstart, int* __restrict__ cnt,
-                             int* __restrict__ nbr, int* __restrict__ ovf_list, int* __restrict__ novf) {
+                             int* __restrict__ nbr, int* __restrict__ ovf_list, int* __restrict__ novf, P32 p, T32 t,
+                             int wc, int* __restrict__ act, int* __restrict__ nact) {
     const int lane = threadIdx.x & 31, g = lane % LP, gb = lane - g;
     int i = (blockIdx.x * blockDim.x + threadIdx.x) / LP;
     const bool live = i < k.n;
@@ -231,6 +273,10 @@ __global__ void k_lists_warp(K32 k, const float4* __restrict__ HI, RecView LO, c
     if (live && g == 0) {
         cnt[i] = m;
         if (m > k.maxn) note_overflow(ovf_list, novf, i);
+        if (i >= k.nd) {
+            if (m != 0) act[atomicAdd(nact, 1)] = i;
+            static_values(k, p, t, wc, i, m != 0);
+        }
     }
 }
 
@@ -2394,18 +2440,19 @@ constexpr int kWarpLists = 65536;
 template <int DIM>
 constexpr int kListLanes = DIM == 3 ? 32 : 16;
 
+// True if the static particles' part (k_static_active) is done too.
 template <int DIM>
-void build_lists(Fp32State& st, const P32& p, cudaStream_t s) {
+bool build_lists(Fp32State& st, const P32& p, cudaStream_t s) {
     const K32& k = st.k;
     if (st.cells_per_cta <= 0 && k.n <= kWarpLists) {
         TSG_LAUNCH((k_lists_warp<DIM, kListLanes<DIM>>), nblk(kListLanes<DIM> * (long long)k.n, 128), 128, s, k, p.hi, p.lo, st.pf, st.dstart, st.sstart, st.T.cnt,
-                   st.T.nbr, st.ovf_list, st.novf);
-        return;
+                   st.T.nbr, st.ovf_list, st.novf, p, st.T, k.solver == 1 ? 1 : 0, st.sact, st.nsact);
+        return true;
     }
     if (st.cells_per_cta <= 0) {  // one thread per particle
         TSG_LAUNCH(k_lists<DIM>, nblk(k.n), TPB, s, k, p.hi, p.lo, st.pf, st.dstart, st.sstart, st.T.cnt, st.T.nbr,
                    st.ovf_list, st.novf);
-        return;
+        return false;
     }
     cudaMemsetAsync(st.ncells, 0, sizeof(int), s);
     TSG_LAUNCH(k_nonempty_cells, nblk(k.G, 256), 256, s, (long long)k.G, st.dstart, st.cells_d, st.ncells);
@@ -2422,43 +2469,7 @@ void build_lists(Fp32State& st, const P32& p, cudaStream_t s) {
                st.T.nbr, st.ovf_list, st.novf);
     TSG_LAUNCH(k_lists_fixup<DIM>, 2 * 152, TPB, s, k, p.hi, p.lo, st.pf, st.dstart, st.sstart, st.T.cnt, st.T.nbr,
                st.ovf_list, st.novf);
-}
-
-// Static-block particles (fixed boundary) with a non-empty neighbour list, in warp-sized
-// runs of the block's order (a run's place in the list depends on scheduling; every consumer
-// treats its particles independently, so results do not).  A boundary particle with an
-// empty list has no flow particle within support + skin: no flow particle reads its
-// extrapolated state, and the values of the list kernels for it (Shepard factor 1, identity
-// CSPM matrix, WCSPH extrapolation 2 v with zero pressure) depend on nothing but its own
-// constant velocity; they are written here, once per list build, and the per-step kernels
-// visit the listed particles only.
-__global__ void k_static_active(K32 k, P32 p, T32 t, int wc, int* __restrict__ act, int* __restrict__ nact) {
-    const int i = k.nd + blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = i < k.n;
-    const bool on = in && t.cnt[i] != 0;
-    const unsigned ball = __ballot_sync(0xffffffffu, on);
-    const int lane = threadIdx.x & 31;
-    int base = 0;
-    if (lane == 0 && ball) base = atomicAdd(nact, __popc(ball));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (on) act[base + __popc(ball & ((1u << lane) - 1u))] = i;
-    if (!in) return;
-    if (t.L) {  // no static particle is a flow particle: its CSPM matrix is the identity
-        const size_t n = k.n;
-        for (int q = 0; q < 6; ++q) t.L[q * n + i] = q < 3 ? 1.f : 0.f;
-    }
-    if (on) return;
-    t.cf[i] = 1.f;
-    if (!wc) return;
-    const int ti = tf_type(p.hi[i].w);
-    if (ti == MAT_DUMMY || ti == MAT_REP || ti == MAT_RIGID) {
-        const float4 v = p.vel[i];
-        t.vt[i] = make_float4(2.f * v.x, 2.f * v.y, 2.f * v.z, 0.f);
-        t.pr[i] = make_float2(0.f, k.rho0);
-        t.drt[i] = 0.f;
-        p.vel[i].w = 0.f;
-        if (ti == MAT_RIGID) { t.dd[i] = 0.f; t.dv[i] = make_float4(0.f, 0.f, 0.f, 0.f); }
-    }
+    return false;
 }
 
 // Copy the dynamic block of b back into a (graph mode keeps one current buffer).
@@ -2506,9 +2517,8 @@ void f32::rebuild(Fp32State& st, cudaStream_t s, bool in_place) {
     }
     {
         PhaseScope ph2(s, PH_LISTS);
-        if (st.k.dim == 3) build_lists<3>(st, st.P[st.cur], s);
-        else build_lists<2>(st, st.P[st.cur], s);
-        static_active(st, s);
+        const bool done = st.k.dim == 3 ? build_lists<3>(st, st.P[st.cur], s) : build_lists<2>(st, st.P[st.cur], s);
+        if (!done) static_active(st, s);
     }
 }
 
