@@ -102,10 +102,45 @@ __device__ __forceinline__ void on_pipe(bool usable_operands, F&& f) {
     if (usable_operands) f(IntMul());
     else f(SlowMul());
 }
+struct IntQuot {
+    __device__ __forceinline__ double operator()(double a, double b, unsigned long long X) const {
+        const double q = int_quot(a, b, X);
+        return zero(a) ? a : q;
+    }
+};
+struct SlowQuot {
+    __device__ __forceinline__ double operator()(double a, double b, unsigned long long) const { return slow_div(a, b); }
+};
+struct Check {
+    bool& ok;
+    __device__ __forceinline__ void operator()(double x) const { ok = ok & usable(x); }
+    __device__ __forceinline__ void operator()(bool cond) const { ok = ok & cond; }
+    template <int N>
+    __device__ __forceinline__ void all(const double* x) const {
+#pragma unroll
+        for (int q = 0; q < N; ++q) ok = ok & usable(x[q]);
+    }
+};
+struct NoCheck {
+    __device__ __forceinline__ void operator()(double) const {}
+    __device__ __forceinline__ void operator()(bool) const {}
+    template <int N>
+    __device__ __forceinline__ void all(const double*) const {}
+};
+// eval(mul, quot, check) evaluates a pair's terms and names every operand that the integer
+// routines must be able to use; they return garbage (no fault, no loop) for others, so the terms
+// are formed first, without a branch, and once more by the FP64 unit where a check failed.  A
+// branch before each run of products kept the compiler from overlapping their chains.
+template <class E>
+__device__ __forceinline__ void on_pipes(E&& eval) {
+    bool ok = true;
+    eval(IntMul(), IntQuot(), Check{ok});
+    if (!ok) eval(SlowMul(), SlowQuot(), NoCheck());
+}
 // Every entry usable by int_mul.
 template <int DIM>
 __device__ __forceinline__ bool usable_v(const double* a) {
-    return usable(a[0]) && usable(a[1]) && (DIM == 2 || usable(a[2]));
+    return usable(a[0]) & usable(a[1]) & (DIM == 2 || usable(a[2]));
 }
 template <int DIM>
 __device__ __forceinline__ bool usable_m(const double* L) {
@@ -200,61 +235,60 @@ __device__ __noinline__ KernelVals slow_kernel(KernelConsts c, double r0, double
     return k;
 }
 
-// grad W (if asked for) and W of a separation r.  Both kernels away from their ends run on the
+// grad W (DW) and W (WV) of a separation r.  Both kernels away from their ends run on the
 // integer pipes but for their sums; separations at the ends take the kernel functions.
-template <int DIM>
-__device__ __forceinline__ KernelVals pair_kernel(const Consts& c, const double* r, bool want_dW, bool want_W) {
-    const bool r_ok = usable_v<DIM>(r);
-    double r2;
-    on_pipe(r_ok, [&](auto mul) { r2 = dotv<DIM>(r, r, mul); });
+template <int DIM, bool DW, bool WV>
+__device__ __forceinline__ KernelVals pair_kernel(const Consts& c, const double* r) {
     KernelVals k;
     k.W = 0.0;
-    if (c.kern_int && r_ok && above(r2, 0x1p-200)) {
-        const double rn = int_sqrt(r2);
-        const double q = int_mul(rn, c.h1);
-        // 1 - q / 2 (Wendland) or 2 - q (cubic) must not vanish
-        const double q1 = c.kernel == 1 ? __fma_rn(-0.5, q, 1.0) : 2.0 - q;
-        if (above(rn, EPS) && !above(q, 2.0) && above(q1, 0x1p-50)) {
-            const unsigned long long X = want_dW ? recip63(rn) : 0ull;
-            if (want_dW) k.rr = int_mul(rn, rn);
-            if (c.kernel == 1) {
-                const double q2 = int_mul(q1, q1);
-                if (want_dW) {
-                    const double s = int_mul(int_mul(int_mul(c.kk, int_mul(q2, q1)), int_mul(-5.0, q)), c.h1);
-                    for (int d = 0; d < DIM; ++d) k.kd[d] = quot(int_mul(s, r[d]), rn, X);
-                }
-                if (want_W) k.W = int_mul(int_mul(c.kk, int_mul(q2, q2)), __fma_rn(2.0, q, 1.0));
-                return k;
-            }
-            double s, w;
-            if (!above(q, 1.0)) {
-                const double q2 = int_mul(q, q);
-                w = int_mul(c.kk, __fma_rn(0.5, int_mul(q2, q), -q2) + 2.0 / 3.0);
-                s = int_mul(int_mul(c.kk, q), int_mul(1.5, q) - 2.0);
-            } else {
-                w = int_mul(c.kk6, int_mul(int_mul(q1, q1), q1));
-                s = int_mul(c.kk, int_mul(int_mul(-0.5, q1), q1));
-            }
-            if (want_dW)
-                for (int d = 0; d < DIM; ++d) k.kd[d] = int_mul(s, int_mul(quot(r[d], rn, X), c.h1));
-            if (want_W) k.W = w;
-            return k;
+    const double r2 = dotv<DIM>(r, r, IntMul());
+    const double rn = int_sqrt(r2);
+    const double q = int_mul(rn, c.h1);
+    // 1 - q / 2 (Wendland) or 2 - q (cubic) must not vanish
+    const double q1 = c.kernel == 1 ? __fma_rn(-0.5, q, 1.0) : 2.0 - q;
+    const bool ok = (c.kern_int != 0) & usable_v<DIM>(r) & above(r2, 0x1p-200) & above(rn, EPS) & !above(q, 2.0) &
+                    above(q1, 0x1p-50);
+    const unsigned long long X = DW ? recip63(rn) : 0ull;
+    if (DW) k.rr = int_mul(rn, rn);
+    if (c.kernel == 1) {
+        const double q2 = int_mul(q1, q1);
+        if (DW) {
+            const double s = int_mul(int_mul(int_mul(c.kk, int_mul(q2, q1)), int_mul(-5.0, q)), c.h1);
+            for (int d = 0; d < DIM; ++d) k.kd[d] = IntQuot()(int_mul(s, r[d]), rn, X);
         }
+        if (WV) k.W = int_mul(int_mul(c.kk, int_mul(q2, q2)), __fma_rn(2.0, q, 1.0));
+    } else {
+        double s, w;
+        if (!above(q, 1.0)) {
+            const double q2 = int_mul(q, q);
+            w = int_mul(c.kk, __fma_rn(0.5, int_mul(q2, q), -q2) + 2.0 / 3.0);
+            s = int_mul(int_mul(c.kk, q), int_mul(1.5, q) - 2.0);
+        } else {
+            w = int_mul(c.kk6, int_mul(int_mul(q1, q1), q1));
+            s = int_mul(c.kk, int_mul(int_mul(-0.5, q1), q1));
+        }
+        if (DW)
+            for (int d = 0; d < DIM; ++d) k.kd[d] = int_mul(s, int_mul(IntQuot()(r[d], rn, X), c.h1));
+        if (WV) k.W = w;
     }
-    return slow_kernel<DIM>(KernelConsts{c.kernel, c.div_span, c.h1, c.kk}, r[0], r[1], r[2], slow_sqrt(r2));
+    if (!ok) {
+        const double d2 = dotv<DIM>(r, r, SlowMul());
+        k = slow_kernel<DIM>(KernelConsts{c.kernel, c.div_span, c.h1, c.kk}, r[0], r[1], r[2], slow_sqrt(d2));
+    }
+    return k;
 }
 
 // Pair geometry of row slot `slot` (entry j): r, grad W and, for a flow neighbour, W into
 // registers, grad W and the viscosity denominator into the row's planes.  The Wendland kernel
 // away from its ends runs its products on the integer pipes; the others take the kernel functions.
-template <int DIM>
+template <int DIM, bool WV>
 __device__ __forceinline__ double pair_geometry(const Consts& c, const double* __restrict__ X, const double* xi, int j,
-                                                const Pairs64& pr, size_t slot, bool want_W, double* r, double* kd) {
+                                                const Pairs64& pr, size_t slot, double* r, double* kd) {
     const size_t n = c.n;
     r[0] = xi[0] - X[j];
     r[1] = xi[1] - X[n + j];
     r[2] = DIM == 3 ? xi[2] - X[2 * n + j] : 0.0;
-    const KernelVals k = pair_kernel<DIM>(c, r, true, want_W);
+    const KernelVals k = pair_kernel<DIM, true, WV>(c, r);
     for (int d = 0; d < DIM; ++d) {
         kd[d] = k.kd[d];
         pr.gk[d * pr.slots_f + slot] = kd[d];
@@ -271,7 +305,7 @@ template <int DIM>
 __device__ __forceinline__ double pair_W(const Consts& c, const double* __restrict__ X, const double* xi, int j) {
     const size_t n = c.n;
     const double r[3] = {xi[0] - X[j], xi[1] - X[n + j], DIM == 3 ? xi[2] - X[2 * n + j] : 0.0};
-    return pair_kernel<DIM>(c, r, false, true).W;
+    return pair_kernel<DIM, false, true>(c, r).W;
 }
 
 // This thread's row in the row-sum phase: particle index and listed count (0 for a row past the
@@ -306,19 +340,23 @@ __global__ void __launch_bounds__(ROWS * G, G == 8 ? 3 : 6) k_corr_flow(Consts c
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const int ent = pr.nb_f[q.base + s], j = nb_index(ent);
             double r[3], kd[3];
-            const double W = pair_geometry<DIM>(c, p.x, xi, j, pr, q.base + s, nb_flow(ent), r, kd);
-            if (nb_flow(ent)) {
-                const double mVj = p.m_V[j];
-                // (the matrix products stay on the FP64 pipe, which this pass no longer fills)
-                on_pipe(usable(mVj) && usable(W) && (!CORR || usable_v<DIM>(r)), [&](auto mul) {
-                    T[0] = mul(mVj, W);
-                    if (CORR)
-                        for (int a = 0; a < DIM; ++a) {
-                            const double av = mul(mVj, -r[a]);
-                            for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = av * kd[b];
-                        }
-                });
-            }
+            // a boundary neighbour adds nothing: zero mass gives +-0 terms
+            const double mVj = nb_flow(ent) ? p.m_V[j] : 0.0;
+            const double W = pair_geometry<DIM, true>(c, p.x, xi, j, pr, q.base + s, r, kd);
+            double av[3];
+            on_pipes([&](auto mul, auto, auto check) {
+                check(mVj);
+                check(W);
+                T[0] = mul(mVj, W);
+                if (CORR) {
+                    check.template all<DIM>(r);
+                    for (int a = 0; a < DIM; ++a) av[a] = mul(mVj, -r[a]);
+                }
+            });
+            // (the matrix products stay on the FP64 pipe, which this pass no longer fills)
+            if (CORR)
+                for (int a = 0; a < DIM; ++a)
+                    for (int b = 0; b < DIM; ++b) T[1 + a * DIM + b] = av[a] * kd[b];
         });
     }
     const int row = blockIdx.x * ROWS + threadIdx.x;
@@ -417,7 +455,7 @@ __global__ void __launch_bounds__(ROWS * G) k_geom_flow(Consts c, Persist64 p, c
     double xi[3], r[3], kd[3];
     load_x<DIM>(p.x, q.i, c.n, xi);
     for (int s = threadIdx.x % G; s < q.cnt; s += G)
-        pair_geometry<DIM>(c, p.x, xi, nb_index(pr.nb_f[q.base + s]), pr, q.base + s, false, r, kd);
+        pair_geometry<DIM, false>(c, p.x, xi, nb_index(pr.nb_f[q.base + s]), pr, q.base + s, r, kd);
 }
 
 template <int DIM, int G>
@@ -665,19 +703,28 @@ __device__ __forceinline__ void corrected(const Consts& c, const double* L, cons
     if (c.corr == 1) matvec_corr<DIM>(L, kd, kc, PlainMul());
     else { kc[0] = kd[0]; kc[1] = kd[1]; kc[2] = kd[2]; }
 }
-template <int DIM, int KC>
+// kd: grad W (KC_READ: not used); inside on_pipes.
+template <int DIM, int KC, class M, class K>
 __device__ __forceinline__ void row_gradient(const Consts& c, const Pairs64& pr, size_t slot, const double* L,
-                                             bool L_ok, double* kc) {
+                                             bool L_ok, const double* kd, double* kc, M mul, K check) {
     if (KC == KC_READ) {
         for (int d = 0; d < DIM; ++d) kc[d] = pr.gc[d * pr.slots_f + slot];
-        return;
+    } else if (c.corr == 1) {
+        check(L_ok);
+        check.template all<DIM>(kd);
+        matvec_corr<DIM>(L, kd, kc, mul);
+    } else {
+        for (int d = 0; d < DIM; ++d) kc[d] = kd[d];
     }
-    double kd[3] = {0.0, 0.0, 0.0};
-    for (int d = 0; d < DIM; ++d) kd[d] = pr.gk[d * pr.slots_f + slot];
-    if (c.corr == 1)
-        on_pipe(L_ok && usable_v<DIM>(kd), [&](auto mul) { matvec_corr<DIM>(L, kd, kc, mul); });
-    else
-        for (int d = 0; d < 3; ++d) kc[d] = kd[d];
+    check.template all<DIM>(kc);
+}
+template <int DIM, int KC>
+__device__ __forceinline__ void load_gradient(const Pairs64& pr, size_t slot, double* kd) {
+    if (KC != KC_READ)
+        for (int d = 0; d < DIM; ++d) kd[d] = pr.gk[d * pr.slots_f + slot];
+}
+template <int DIM, int KC>
+__device__ __forceinline__ void keep_gradient(const Pairs64& pr, size_t slot, const double* kc) {
     if (KC == KC_KEEP)
         for (int d = 0; d < DIM; ++d) pr.gc[d * pr.slots_f + slot] = kc[d];
 }
@@ -690,28 +737,34 @@ struct Divisor {  // a divisor with its divisor() bits
     unsigned long long X;
     __device__ __forceinline__ explicit Divisor(double v) : b(v), X(divisor(v)) {}
 };
-template <int DIM>
-__device__ __forceinline__ void wc_terms(const Consts& c, bool fluid, const double* v, double P, double mV, double cvj,
-                                         double cC, const double* vti, const Divisor& rti, double pri, const double* r,
-                                         double2 den, const double* kd, const double* kc, double* T) {
-    double dvv[3], a[3], dr;
+template <int DIM, class M, class Q, class K>
+__device__ __forceinline__ void wc_terms(bool fluid, const double* v, double P, double mV, double cvj, double cC,
+                                         const double* vti, const Divisor& rti, double pri, const double* r,
+                                         double2 den, const double* kd, const double* kc, double* T, M mul, Q quot,
+                                         K check) {
+    double dvv[3], a[3];
     for (int d = 0; d < DIM; ++d) dvv[d] = vti[d] - v[d];
-    on_pipe(usable(mV) && usable_v<DIM>(dvv) && usable_v<DIM>(r) && usable_v<DIM>(kc), [&](auto mul) {
-        for (int d = 0; d < DIM; ++d) a[d] = mul(mV, dvv[d]);
-        T[0] = dotv<DIM>(a, kc, mul);
-        dr = dotv<DIM>(dvv, r, mul);
-    });
-    const double mn = min0(dr);
+    check(mV);
+    check.template all<DIM>(dvv);
+    check.template all<DIM>(r);
+    for (int d = 0; d < DIM; ++d) a[d] = mul(mV, dvv[d]);
+    T[0] = dotv<DIM>(a, kc, mul);
+    const double mn = min0(dotv<DIM>(dvv, r, mul));
     double cv = cvj, cp = pri + P;
-    if (!fluid) cv = quot(cv, rti.b, rti.X);
-    on_pipe(usable(cv) && usable(mn) && usable(cC) && usable(cp), [&](auto mul) {
-        cv = mul(cv, mn);
-        cp = mul(cC, cp);
-    });
-    cv = quot(cv, den.x, (unsigned long long)__double_as_longlong(den.y));
-    on_pipe(usable(cp) && usable_v<DIM>(kd), [&](auto mul) {
-        for (int d = 0; d < DIM; ++d) T[1 + d] = cv * kd[d] + mul(cp, kd[d]);  // one product on each pipe
-    });
+    check(cv);
+    check(cp);
+    check(cC);
+    check(mn);
+    if (!fluid) {
+        check(rti.X != 0ull);
+        cv = quot(cv, rti.b, rti.X);
+    }
+    const unsigned long long X = (unsigned long long)__double_as_longlong(den.y);
+    check(X != 0ull);
+    cv = quot(mul(cv, mn), den.x, X);
+    cp = mul(cC, cp);
+    check.template all<DIM>(kd);
+    for (int d = 0; d < DIM; ++d) T[1 + d] = cv * kd[d] + mul(cp, kd[d]);  // one product on each pipe
 }
 
 // ---- WCSPH rates (eng/solver_sph_wc.py:108-126) ----
@@ -736,14 +789,18 @@ __global__ void __launch_bounds__(ROWS * G, G == 8 ? 2 : DIM == 3 && KC == KC_RE
             const int ent = pr.nb_f[slot], j = nb_index(ent);
             const double2* rj = reinterpret_cast<const double2*>(pr.rec + (size_t)8 * j);
             const double2 r0 = rj[0], r1 = rj[1], r2 = rj[2], r3 = rj[3];
+            const double2 den = pr.gden[slot];
             double r[3] = {0.0, 0.0, 0.0}, kd[3] = {0.0, 0.0, 0.0}, kc[3];
             for (int d = 0; d < DIM; ++d) {
                 r[d] = xi[d] - p.x[(size_t)d * n + j];
                 kd[d] = pr.gk[d * pr.slots_f + slot];
             }
-            row_gradient<DIM, KC>(c, pr, slot, L, L_ok, kc);
             const double v[3] = {r0.x, r0.y, r1.x};
-            wc_terms<DIM>(c, nb_flow(ent), v, r1.y, r2.x, r2.y, r3.x, vti, rti, pri, r, pr.gden[slot], kd, kc, T);
+            on_pipes([&](auto mul, auto quot, auto check) {
+                row_gradient<DIM, KC>(c, pr, slot, L, L_ok, kd, kc, mul, check);
+                wc_terms<DIM>(nb_flow(ent), v, r1.y, r2.x, r2.y, r3.x, vti, rti, pri, r, den, kd, kc, T, mul, quot, check);
+            });
+            keep_gradient<DIM, KC>(pr, slot, kc);
         });
     }
     const int row = blockIdx.x * ROWS + threadIdx.x;
@@ -770,8 +827,8 @@ __global__ void __launch_bounds__(ROWS * G, G == 8 ? 2 : DIM == 3 && KC == KC_RE
             kernel_dW<DIM>(c, r, rn, kd);
             corrected<DIM>(c, L, kd, kc);
             const double den = rn * rn + c.eps_h2;
-            wc_terms<DIM>(c, p.mat_type[j] == MAT_FLUID, rj, rj[3], rj[4], rj[5], rj[6], vti, rti, pri, r,
-                          make_double2(den, __longlong_as_double((long long)divisor(den))), kd, kc, T);
+            wc_terms<DIM>(p.mat_type[j] == MAT_FLUID, rj, rj[3], rj[4], rj[5], rj[6], vti, rti, pri, r,
+                          make_double2(den, 0.0), kd, kc, T, SlowMul(), SlowQuot(), NoCheck());
             for (int q = 0; q < C; ++q) A[q] += T[q];
         });
     }
@@ -794,16 +851,17 @@ __device__ __forceinline__ void damping_acc(const Consts& c, double rti, const d
 // One neighbour's velocity-gradient terms (DIM x DIM) and continuity term (last): the
 // continuity product m_V (v_i - v_j) is the exact negation of the gradient's, so its dot
 // product is the negated trace.
-template <int DIM>
-__device__ __forceinline__ void vgrad_terms(const double* v, double mV, const double* vti, const double* kc, double* T) {
+template <int DIM, class M, class K>
+__device__ __forceinline__ void vgrad_terms(const double* v, double mV, const double* vti, const double* kc, double* T,
+                                            M mul, K check) {
     double dv[3];
     for (int a = 0; a < DIM; ++a) dv[a] = v[a] - vti[a];
-    on_pipe(usable(mV) && usable_v<DIM>(dv) && usable_v<DIM>(kc), [&](auto mul) {
-        for (int a = 0; a < DIM; ++a) {
-            const double av = mul(mV, dv[a]);
-            for (int b = 0; b < DIM; ++b) T[a * DIM + b] = mul(av, kc[b]);
-        }
-    });
+    check(mV);
+    check.template all<DIM>(dv);
+    for (int a = 0; a < DIM; ++a) {
+        const double av = mul(mV, dv[a]);
+        for (int b = 0; b < DIM; ++b) T[a * DIM + b] = mul(av, kc[b]);
+    }
     double s = T[0] + T[DIM + 1];
     if (DIM == 3) s = s + T[8];
     T[DIM * DIM] = -s;
@@ -827,10 +885,15 @@ __global__ void __launch_bounds__(ROWS * G) k_mui_stress(Consts c, Persist64 p, 
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
             const int j = nb_index(pr.nb_f[slot]);
-            double kc[3], v[3];
+            double kd[3], kc[3], v[3];
             for (int d = 0; d < DIM; ++d) v[d] = t.v_tmp[(size_t)d * n + j];
-            row_gradient<DIM, KC>(c, pr, slot, L, L_ok, kc);
-            vgrad_terms<DIM>(v, p.m_V[j], vti, kc, T);
+            load_gradient<DIM, KC>(pr, slot, kd);
+            const double mVj = p.m_V[j];
+            on_pipes([&](auto mul, auto, auto check) {
+                row_gradient<DIM, KC>(c, pr, slot, L, L_ok, kd, kc, mul, check);
+                vgrad_terms<DIM>(v, mVj, vti, kc, T, mul, check);
+            });
+            keep_gradient<DIM, KC>(pr, slot, kc);
         });
     }
     const int row = blockIdx.x * ROWS + threadIdx.x;
@@ -851,7 +914,7 @@ __global__ void __launch_bounds__(ROWS * G) k_mui_stress(Consts c, Persist64 p, 
             kernel_dW<DIM>(c, r, rn, kd);
             corrected<DIM>(c, L, kd, kc);
             for (int d = 0; d < DIM; ++d) v[d] = t.v_tmp[(size_t)d * n + j];
-            vgrad_terms<DIM>(v, p.m_V[j], vti, kc, T);
+            vgrad_terms<DIM>(v, p.m_V[j], vti, kc, T, SlowMul(), NoCheck());
             for (int q = 0; q < C; ++q) A[q] += T[q];
         });
     }
@@ -897,18 +960,14 @@ __device__ __forceinline__ void stress_div_val(const double* sti, double ri2, co
 }
 // The same sum from the neighbour's record: S_j = stress_j / rho~_j^2 (DIM x DIM), sc = m_V rho~_j,
 // and S_i likewise.
-template <int DIM>
+template <int DIM, class M, class K>
 __device__ __forceinline__ void stress_div_rec(const double* Si, const double* Sj, double sc, const double* kc,
-                                               double* out) {
+                                               double* out, M mul, K check) {
     double m[DIM * DIM];
-    bool ok = usable(sc) && usable_v<DIM>(kc);
-    for (int q = 0; q < DIM * DIM; ++q) {
-        m[q] = Sj[q] + Si[q];
-        ok = ok && usable(m[q]);
-    }
-    on_pipe(ok, [&](auto mul) {
-        for (int q = 0; q < DIM * DIM; ++q) m[q] = mul(mul(sc, m[q]), kc[q % DIM]);
-    });
+    for (int q = 0; q < DIM * DIM; ++q) m[q] = Sj[q] + Si[q];
+    check(sc);
+    check.template all<DIM * DIM>(m);
+    for (int q = 0; q < DIM * DIM; ++q) m[q] = mul(mul(sc, m[q]), kc[q % DIM]);
     for (int a = 0; a < DIM; ++a) {
         out[a] = m[a * DIM] + m[a * DIM + 1];
         if (DIM == 3) out[a] = out[a] + m[a * DIM + 2];
@@ -954,11 +1013,15 @@ __device__ __forceinline__ void soil_sums(const Consts& c, const Persist64& p, c
         block_row_sums<C, G>(q.cnt, S, [&](int s, double* T) {
             const size_t slot = q.base + s;
             const int j = nb_index(pr.nb_f[slot]);
-            double kc[3];
-            row_gradient<DIM, KC>(c, pr, slot, L, L_ok, kc);
+            double kd[3], kc[3];
+            load_gradient<DIM, KC>(pr, slot, kd);
             const SoilRec<DIM> rj(pr.rec, j);
-            stress_div_rec<DIM>(ri.S(), rj.S(), rj.sc(), kc, T);
-            if (DP) vgrad_terms<DIM>(rj.v(), rj.mV(), ri.v(), kc, T + DIM);
+            on_pipes([&](auto mul, auto, auto check) {
+                row_gradient<DIM, KC>(c, pr, slot, L, L_ok, kd, kc, mul, check);
+                stress_div_rec<DIM>(ri.S(), rj.S(), rj.sc(), kc, T, mul, check);
+                if (DP) vgrad_terms<DIM>(rj.v(), rj.mV(), ri.v(), kc, T + DIM, mul, check);
+            });
+            keep_gradient<DIM, KC>(pr, slot, kc);
         });
     }
     const int row = blockIdx.x * ROWS + threadIdx.x;
@@ -980,8 +1043,8 @@ __device__ __forceinline__ void soil_sums(const Consts& c, const Persist64& p, c
             kernel_dW<DIM>(c, r, rn, kd);
             corrected<DIM>(c, L, kd, kc);
             const SoilRec<DIM> rj(pr.rec, j);
-            stress_div_rec<DIM>(ri.S(), rj.S(), rj.sc(), kc, T);
-            if (DP) vgrad_terms<DIM>(rj.v(), rj.mV(), ri.v(), kc, T + DIM);
+            stress_div_rec<DIM>(ri.S(), rj.S(), rj.sc(), kc, T, SlowMul(), NoCheck());
+            if (DP) vgrad_terms<DIM>(rj.v(), rj.mV(), ri.v(), kc, T + DIM, SlowMul(), NoCheck());
             for (int q = 0; q < C; ++q) A[q] += T[q];
         });
     }

@@ -158,7 +158,7 @@ __device__ __forceinline__ double div_by(double a, double b, double y, unsigned 
 // up to three of them).
 __device__ __forceinline__ bool usable(double a) {  // +-0 or 2^-255 <= |a| < 2^257
     const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
-    return hi - (768u << 20) < (512u << 20) || (hi | (unsigned)__double2loint(a)) == 0u;
+    return (hi - (768u << 20) < (512u << 20)) | ((hi | (unsigned)__double2loint(a)) == 0u);
 }
 __device__ __forceinline__ bool zero(double a) {
     return (((unsigned)__double2hiint(a) & 0x7fffffffu) | (unsigned)__double2loint(a)) == 0u;
