@@ -143,8 +143,7 @@ int alloc_rows(tsg_handle* h) {
     const Consts& c = h->c;
     Pairs64& r = h->g.pr;
     r = Pairs64{};
-    r.rec_stride = c.solver != 1 && c.dim == 3 ? 16 : 8;
-    if (int rc = dalloc(h, &r.rec, (size_t)r.rec_stride * h->n)) return rc;
+    if (int rc = dalloc(h, &r.rec, (size_t)(c.solver != 1 && c.dim == 3 ? 16 : 8) * h->n)) return rc;
     const int cf = row_capacity(c);
     const int cap_f = (cf + 7) / 8 * 8, cap_b = ((cf * 6) / 10 + 7) / 8 * 8;
     const size_t sf = (size_t)c.n_flow * cap_f, sb = (size_t)c.n_bdy * cap_b;

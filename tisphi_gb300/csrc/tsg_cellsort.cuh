@@ -1,15 +1,15 @@
-// The last step of the counting sort, shared by the FP64 and FP32-mixed forms: inside every
-// cell, ascending old index (the stable order of the reference's serial sort; the scatter
-// before it places a cell's particles in atomic arrival order).
+// Large cells of the counting sort, shared by the FP64 and FP32-mixed forms: inside every cell,
+// ascending old index (the stable order of the reference's serial sort; the scatter before it
+// places a cell's particles in atomic arrival order).
 //
-// Ordinary cells hold a few dozen particles and are insertion-sorted by one thread each
-// (k_cell_sort_small).  A segment above kSortSmall - the out-of-grid bin after particles
-// left the grid, or a very coarse grid - would make that quadratic in one thread (a
-// blown-up run with every particle out of the grid would keep the GPU busy for hours), so
-// such cells are listed instead and sorted by k_cell_sort_big, one block per cell: up to
-// kSortMid particles by a bitonic sort in shared memory, above that rebuilt in ascending
-// order from a block-wide scan over every particle of the flag "cell_of[i] == c" (n / 256
-// trips; at most n / kSortMid cells are that large).  Both paths give the same order.
+// Ordinary cells hold a few dozen particles, and the reorder passes rank each particle among its
+// cell's themselves.  For a segment above kSortSmall - the out-of-grid bin after particles left
+// the grid, or a very coarse grid - that would be quadratic (a blown-up run with every particle
+// out of the grid would keep the GPU busy for hours), so the scatter lists such cells and
+// k_cell_sort_big sorts them first, one block per cell: up to kSortMid particles by a bitonic
+// sort in shared memory, above that rebuilt in ascending order from a block-wide scan over every
+// particle of the flag "cell_of[i] == c" (n / 256 trips; at most n / kSortMid cells are that
+// large).  Both paths give the same order.
 // Scratch: big (cellsort_big_ints, tsg_internal.h) and its counter nbig, zeroed before each
 // sort.
 #pragma once
@@ -23,23 +23,6 @@ namespace {
 
 constexpr int kSortMid = 4096;
 constexpr int kSortBlock = 256;
-
-__global__ void k_cell_sort_small(long long ncell, const int* __restrict__ cell_start, int* __restrict__ perm,
-                                  int* __restrict__ big, int* __restrict__ nbig) {
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
-    const int b = cell_start[c], e = cell_start[c + 1];
-    if (e - b > kSortSmall) {
-        big[atomicAdd(nbig, 1)] = (int)c;
-        return;
-    }
-    for (int q = b + 1; q < e; ++q) {
-        const int v = perm[q];
-        int m = q - 1;
-        while (m >= b && perm[m] > v) { perm[m + 1] = perm[m]; --m; }
-        perm[m + 1] = v;
-    }
-}
 
 __global__ void __launch_bounds__(kSortBlock) k_cell_sort_big(const int* __restrict__ big, const int* __restrict__ nbig,
                                                               const int* __restrict__ cell_start,
@@ -92,16 +75,6 @@ __global__ void __launch_bounds__(kSortBlock) k_cell_sort_big(const int* __restr
             }
         }
     }
-}
-
-// Ascending old index inside every cell: ncell cells (bins) starting at cell_start, the
-// particles' cells in cell_of (n entries, the same index base as perm's values).
-inline void sort_within_cells(long long ncell, const int* cell_start, const int* cell_of, int n, int* perm, int* big,
-                              int* nbig, cudaStream_t s) {
-    cudaMemsetAsync(nbig, 0, sizeof(int), s);
-    TSG_LAUNCH(k_cell_sort_small, (int)((ncell + kSortBlock - 1) / kSortBlock), kSortBlock, s, ncell, cell_start,
-               perm, big, nbig);
-    TSG_LAUNCH(k_cell_sort_big, 152, kSortBlock, s, big, nbig, cell_start, cell_of, n, perm);
 }
 
 }  // namespace

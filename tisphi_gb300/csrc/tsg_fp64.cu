@@ -695,8 +695,9 @@ __device__ __forceinline__ void wc_force_pair(const Consts& c, int tj, double mV
 }
 
 // The corrected gradient L_i grad W of a pair is the same in every loop of a step.  KC_MAKE
-// forms it, KC_KEEP also stores it in the row, KC_READ reads it back (3D WCSPH: 15 of a pair's
-// 57 FP64 operations for 24 bytes of stream).
+// forms it, KC_KEEP also stores it in the row, KC_READ reads it back (3D WCSPH: nine products and
+// six additions of a pair for 24 bytes of stream; 118 k rows: 778 us with KC_KEEP, 578 with
+// KC_READ).
 enum { KC_MAKE = 0, KC_KEEP = 1, KC_READ = 2 };
 template <int DIM>
 __device__ __forceinline__ void corrected(const Consts& c, const double* L, const double* kd, double* kc) {

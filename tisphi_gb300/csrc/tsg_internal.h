@@ -68,8 +68,8 @@ struct Consts {
 // (from the uploaded positions, in upload order) and, per object, the slice of `list`
 // that the list builder (tsg_rigid_list.cuh) fills with the object's particles in
 // ascending order before every shape matching.
-// Largest cell segment the counting sort's last step gives to one thread (tsg_cellsort.cuh),
-// and the size of its list of larger cells (at most n / (kSortSmall + 1) of them).
+// Largest cell segment whose particles the reorder passes rank among themselves
+// (tsg_cellsort.cuh), and the size of the list of larger cells (at most n / (kSortSmall + 1) of them).
 constexpr int kSortSmall = 256;
 // Up to this many particles the reorder pass ranks every cell itself, however large (all of them
 // in one cell: 16,384 loads a thread, a fraction of a millisecond), and the launch that orders
@@ -150,8 +150,7 @@ struct Pairs64 {
     double* gc;         // dim planes: corrected gradient L_i grad W of each flow entry (CSPM);
                         // the soil solvers, which use no other gradient, keep it in gk
     double* gw;         // kernel value of each boundary entry
-    double* rec;        // rec_stride doubles per particle: what the rates loop reads of a neighbour
-    int rec_stride;
+    double* rec;        // 8 doubles per particle (16 for 3D soil): what a rates loop reads of a neighbour
 };
 
 // Sort scratch and cell table.

@@ -10,7 +10,8 @@
 // What bounds these loops is the FP64 pipe: sm_103a issues one FP64 warp instruction per SM
 // in 16 cycles, against four of any other kind per cycle, so everything that is not FP64
 // arithmetic (list and record traffic, shared-memory exchange) hides behind it and every FP64
-// operation saved counts.  A traversal of the cells ran the FP64 body for a third of a warp's
+// operation saved counts.  What can leave that pipe runs on the integer pipes beside it (int_mul,
+// int_sqrt, int_quot); the additions stay.  A traversal of the cells ran the FP64 body for a third of a warp's
 // lanes (the candidates of different particles pass the distance test at different trips);
 // rows keep the lanes full.
 //
@@ -151,7 +152,8 @@ __device__ __forceinline__ double div_by(double a, double b, double y, unsigned 
 // in 16 cycles; this takes about as long on the other pipes and runs beside it (measured: 18.5
 // cycles at the nominal clock for the FP64 product, 15.8 for this one, 9.3 for each of two in
 // parallel), so the pair loops give it most of their products.  3D, 118 k rows, us per launch:
-// rates 1,835 -> 855 (first loop) and 1,476 -> 655 (second), correction 2,057 -> 1,376.  The 53 x 53 bit product of the
+// rates 1,835 -> 855 (first loop) and 1,476 -> 655 (second), correction 2,057 -> 1,376; with the
+// roots and quotients below and the registers bounded 778, 578 and 897.  The 53 x 53 bit product of the
 // significands is formed in 128 bits, normalised, and rounded to nearest even with the bits
 // below jammed into one word; the sign and the exponent are put together beside it.  Operands
 // are +-0 or normal numbers with normal products (usable(a), usable(b): then so are products of
@@ -249,15 +251,9 @@ __device__ __forceinline__ double int_sqrt(double v) {
     const long long D = (long long)((A << 54) - t * t);
     return __longlong_as_double((long long)(((unsigned long long)(unsigned)(1022 + (u >> 1)) << 52) + M0 + (D > 0 ? 1u : 0u)));
 }
-// A divisor prepared for int_quot (X 0: not usable, quotients take the call).
+// A divisor prepared for int_quot (0: not usable, quotients take the call).
 __device__ __forceinline__ unsigned long long divisor(double b) {  // usable: 2^-200 <= b < 2^200
     return (unsigned)__double2hiint(b) - (823u << 20) < 400u << 20 ? recip63(b) : 0ull;
-}
-__device__ __forceinline__ double quot(double a, double b, unsigned long long X) {
-    const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
-    if (X != 0ull && hi - (523u << 20) < 1000u << 20) return int_quot(a, b, X);
-    if (X != 0ull && (hi | (unsigned)__double2loint(a)) == 0u) return a;
-    return slow_div(a, b);
 }
 
 // a > b for b >= 0 and a that is not a NaN, on the bits (an FP64 comparison holds the pipe too).
