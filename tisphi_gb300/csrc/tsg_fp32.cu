@@ -37,7 +37,6 @@
 #include "tsg_fp32_dev.cuh"
 #include "tsg_polar.cuh"
 #include "tsg_rigid_list.cuh"
-#include "tsg_cellsort.cuh"
 
 namespace tsg {
 
@@ -64,18 +63,6 @@ __global__ void k_hash32(K32 k, int count_n, int base, const float4* __restrict_
     }
     cell_of[t] = (int)f;
     rank[t] = atomicAdd(&count[f], 1);
-}
-
-// Arrival order inside the cells; cells above `small` are listed for k_cell_sort_big, the
-// others' particles are ranked by k_reorder32.
-__global__ void k_scatter32(int count_n, const int* __restrict__ cell_of, const int* __restrict__ rank,
-                            const int* __restrict__ cell_start, int* __restrict__ perm, int small,
-                            int* __restrict__ big, int* __restrict__ nbig) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count_n) return;
-    const int c = cell_of[t], r = rank[t], b = cell_start[c];
-    perm[b + r] = t;
-    if (r == 0 && cell_start[c + 1] - b > small) big[atomicAdd(nbig, 1)] = c;
 }
 
 // Gather block [base, base + count_n) from a into b (new order), renormalise hi/lo and
@@ -2146,12 +2133,8 @@ void build_cells(Fp32State& st, int base, int count_n, int* count, int* start, c
     const long long nbins = k.G + 1;
     P32& a = st.P[st.cur];
     TSG_LAUNCH(k_hash32, nblk(count_n), TPB, s, k, count_n, base, a.hi, a.lo, st.cell_of, st.rank, count, st.err);
-    scan_exclusive(count, start, (int)nbins, st.tiles, s);
+    sort_cells(count_n, (int)nbins, count, start, st.tiles, st.cell_of, st.rank, st.perm, st.sort_big, st.sort_nbig, s);
     const int small = sort_small(count_n);
-    TSG_LAUNCH(k_scatter32, nblk(count_n), TPB, s, count_n, st.cell_of, st.rank, start, st.perm, small, st.sort_big,
-               st.sort_nbig);
-    if (count_n > kSortAll)
-        TSG_LAUNCH(k_cell_sort_big, 152, kSortBlock, s, st.sort_big, st.sort_nbig, start, st.cell_of, count_n, st.perm);
     P32& b = st.P[1 - st.cur];
     TSG_LAUNCH(k_reorder32, nblk(count_n), TPB, s, k, count_n, base, st.perm, st.cell_of, start, small, a, b, st.pf);
     (void)reorder_into_next;

@@ -188,6 +188,10 @@ int visual_launch(const VisFields& f, const tsg_visual_cfg& vc, double* scratch,
 // ---- launchers (tsg_sort.cu) ----
 void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid& g, cudaStream_t s);
 void scan_exclusive(const int* in, int* out, int n, int* tile_sum, cudaStream_t s);
+// Counting sort between the hash and the reorder: cell_start from the counts, perm in arrival
+// order inside the cells, the cells that the reorder pass does not rank ordered.
+void sort_cells(int n, int nbins, const int* count, int* cell_start, int* tile_sum, const int* cell_of, const int* rank,
+                int* perm, int* big, int* nbig, cudaStream_t s);
 
 // ---- launchers (tsg_fp64.cu) ----
 void fp64_kernel_corr(const Consts& c, const Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
