@@ -97,3 +97,12 @@ ODD = {
 def test_operands_outside_the_integer_pipes(oracle_lib, native, scene):
     d, names, steps = ODD[scene]()
     _check(d, oracle_lib, names, steps)
+
+
+@pytest.mark.parametrize("spacing,size,domain", [
+    (0.0085, (0.5, 0.3, 0.2), (0.9, 0.5, 0.25)),  # 113 k rows: three a warp
+    (0.02, (0.3, 0.2, 0.02), (0.6, 0.4, 0.02)),   # three cells in z: none is left out
+    (0.02, (0.3, 0.2, 0.08), (0.6, 0.4, 0.08)),   # few cells in z, some left out
+])
+def test_row_builder_in_3d(oracle_lib, native, spacing, size, domain):
+    _check(small_dambreak_3d(spacing=spacing, size=size, domain=domain), oracle_lib, WC, 2)

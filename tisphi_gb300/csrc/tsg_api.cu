@@ -478,6 +478,12 @@ int tsg_create(const tsg_config* cfg, tsg_handle** out) {
     c.kern_int = c.kk > 0x1p-100 && c.kk < 0x1p100 && c.h1 > 0x1p-100 && c.h1 < 0x1p100;
     c.pf_lo2 = std::nextafter((float)(c.R * c.R * (1.0 - 1.0 / 262144.0)), 0.f);
     c.pf_hi2 = std::nextafter((float)(c.R * c.R * (1.0 + 1.0 / 262144.0)), 1e30f);
+    // k_list64's cell test: in f32 a centre's place in its cell is off by less than 2^-12 R, the
+    // squared distance to a cell by less than 2^-10 R^2.  Four cells or more in y and z: a
+    // flattened offset then stands for one cell only.
+    c.cell_inv = (float)(1.0 / c.grid);
+    c.cell_lim = c.dim == 3 && c.grid >= c.R && c.gnum[1] >= 4 && c.gnum[2] >= 4
+                     ? (float)((c.R / c.grid) * (c.R / c.grid) * (1.0 + 1.0 / 256.0)) : HUGE_VALF;
     c.R2T = c.R * c.R;
     while (std::sqrt(c.R2T) >= c.R) c.R2T = std::nextafter(c.R2T, 0.0);
     while (std::sqrt(c.R2T) < c.R) c.R2T = std::nextafter(c.R2T, 1e300);

@@ -55,6 +55,7 @@ struct Consts {
     float pf_r2, pf_lim;
     float pf_in2;       // below this f32 distance^2 a pair is certainly a neighbour
     float pf_lo2, pf_hi2;  // the same two bounds for the distance^2 with the low parts added
+    float cell_inv, cell_lim;  // 1 / cell size; support radius^2 in cells, widened (inf: cells are not tested)
     int kern_int;       // kernel constants inside 2^+-100 (int_mul chains stay normal)
     double kk6;         // kk / 6
     double rgrid;       // 1 / grid, and div_by's window for it

@@ -33,19 +33,31 @@ constexpr int NB_BDY = 1 << 31;    // entry flag: not a flow particle (sign bit)
 __device__ __forceinline__ int nb_index(int ent) { return ent & 0x7fffffff; }
 __device__ __forceinline__ bool nb_flow(int ent) { return ent >= 0; }
 
-// One warp per row.  The candidates of one stencil row of cells are contiguous; 32 of them are
-// tested at a time and the accepted ones compacted in order by ballot.  An FP64 instruction
-// costs a warp the same 16 cycles for one lane as for 32, so no FP64 runs here but for pairs
-// within 2^-18 of R^2: the f32 distance decides all but those within 2^-10 (the rounding of f32
-// coordinates below 500 R stays under a fifth of that), the same distance with the low parts of
-// the coordinates added all but those within 2^-18 (its error is below 2^-20), and the rest
-// take the reference's test: r2 < R2T is sqrt(r2) < support_radius, exactly, sqrt being
-// monotone.  The cell index comes from the sort (or the position refresh), one division per
-// particle there instead of one per warp here.  Boundary rows skip stencil rows without flow
-// particles (three quarters of a tank's dummies see none).
-// 118 k fluid + 357 k dummy particles in 3D: 301 us (911,754 + 1,413,114: 6.34 ms with FP64 cell
-// indices and shell tests in the warp, about 2 ms without).
-template <int DIM>
+// Distance, in cells, from coordinate t to the next cell in direction o (0: its own), or 0 where
+// f32 leaves open which cell t lies in.  Coordinates below 0 truncate towards it, which only
+// widens the gap.
+__device__ __forceinline__ float edge(float t, int o) {
+    const float f = t - floorf(t), d = o < 0 ? f : 1.f - f;
+    return o != 0 && fabsf(f - 0.5f) < 0.5f - 0x1p-9f ? d : 0.f;
+}
+
+// One warp per row, or RPW rows.  The candidates of one stencil row of cells are contiguous; 32
+// of them are tested at a time and the accepted ones compacted in order by ballot.  An FP64
+// instruction costs a warp the same 16 cycles for one lane as for 32, so no FP64 runs here but
+// for pairs within 2^-18 of R^2: the f32 distance decides all but those within 2^-10 (the
+// rounding of f32 coordinates below 500 R stays under a fifth of that), the same distance with
+// the low parts of the coordinates added all but those within 2^-18 (its error is below 2^-20),
+// and the rest take the reference's test: r2 < R2T is sqrt(r2) < support_radius, exactly, sqrt
+// being monotone.  The cell index comes from the sort (or the position refresh), one division
+// per particle there instead of one per warp here.
+// The pass is bound by issue, so what can be left out is: in 3D cells that lie wholly outside
+// the support (a quarter of the 27; only while the cells are those of the current positions),
+// and for boundary rows stencil rows without flow particles (three quarters of a tank's dummies
+// see none).
+// 118 k fluid + 357 k dummy particles in 3D: 210 us (294 us with all 27 cells tested, one row a
+// warp and the tests of a candidate in branches; 282 with the cells left out, 226 with three
+// rows a warp).  911,754 + 1,413,114: 6.34 ms with FP64 cell indices and shell tests in the warp.
+template <int DIM, int RPW>
 __global__ void __launch_bounds__(256) k_list64(Consts c, const double* __restrict__ X,
                                                 const float4* __restrict__ P32, const float4* __restrict__ P32L,
                                                 const long long* __restrict__ cell0, const int* __restrict__ cs,
@@ -53,76 +65,95 @@ __global__ void __launch_bounds__(256) k_list64(Consts c, const double* __restri
                                                 const int* __restrict__ list_flow, int n_flow,
                                                 const int* __restrict__ list_bdy, int n_bdy, bool flow_only,
                                                 Pairs64 pr) {
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= n_flow + n_bdy) return;
-    const bool bdy = row >= n_flow;
-    const int i = bdy ? list_bdy[row - n_flow] : list_flow[row];
-    const bool want_flow = bdy || flow_only;
-    const int cap = bdy ? pr.cap_b : pr.cap_f;
-    int* out = bdy ? pr.nb_b + (size_t)(row - n_flow) * cap : pr.nb_f + (size_t)row * cap;
-    const size_t n = c.n;
     constexpr int NR = DIM == 3 ? 9 : 3;
-    const long long fc = cell0[i];
-    int jb_l = 0, je_l = 0;
-    if (fc != kNoCell && lane < NR) {
-        const long long nz = c.gnum[2], sx = c.gnum[1] * nz, G = c.G;
-        const int ox = DIM == 3 ? lane / 3 - 1 : lane - 1, oy = DIM == 3 ? lane % 3 - 1 : 0;
-        const long long f0 = fc + ox * sx + oy * nz;
-        const long long lo = f0 - 1 > 0 ? f0 - 1 : 0;
-        const long long hi = f0 + 1 < G - 1 ? f0 + 1 : G - 1;
-        bool any = lo <= hi;
-        if (any && want_flow && cell_flow) {
-            any = false;
-            for (long long f = lo; f <= hi; ++f) any = any || cell_flow[f];
+    const int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * RPW, rows = n_flow + n_bdy;
+    const int lane = threadIdx.x & 31;
+    if (row0 >= rows) return;
+    const size_t n = c.n;
+    const auto near_origin = [&](const float4& p) {
+        return c.pf_on && fabsf(p.x) < c.pf_lim && fabsf(p.y) < c.pf_lim && fabsf(p.z) < c.pf_lim;
+    };
+    // lane NR r + q: the candidates of row row0 + r in its stencil row q
+    int i_l = 0, jb_l = 0, je_l = 0;
+    const int row_l = row0 + lane / NR;
+    if (lane < NR * RPW && row_l < rows) {
+        const int q = lane % NR;
+        i_l = row_l < n_flow ? list_flow[row_l] : list_bdy[row_l - n_flow];
+        const long long fc = cell0[i_l];
+        bool any = fc != kNoCell, below = true, above = true;
+        const int ox = DIM == 3 ? q / 3 - 1 : q - 1, oy = DIM == 3 ? q % 3 - 1 : 0;
+        if (DIM == 3 && cell_flow) {
+            const float4 p = P32[i_l];
+            if (near_origin(p)) {
+                const float ex = edge(p.x * c.cell_inv, ox), ey = edge(p.y * c.cell_inv, oy);
+                const float el = edge(p.z * c.cell_inv, -1), eh = edge(p.z * c.cell_inv, 1);
+                const float d2 = ex * ex + ey * ey;
+                any = any && !(d2 > c.cell_lim);
+                below = !(d2 + el * el > c.cell_lim);
+                above = !(d2 + eh * eh > c.cell_lim);
+            }
         }
-        if (any) { jb_l = cs[lo]; je_l = cs[hi + 1]; }
+        if (any) {
+            const long long nz = c.gnum[2], f0 = fc + ox * (c.gnum[1] * nz) + oy * nz;
+            const long long f_lo = below ? f0 - 1 : f0, f_hi = above ? f0 + 1 : f0;
+            const long long lo = f_lo > 0 ? f_lo : 0;
+            const long long hi = f_hi < c.G - 1 ? f_hi : c.G - 1;
+            any = lo <= hi;
+            if (any && (row_l >= n_flow || flow_only) && cell_flow) {
+                any = false;
+                for (long long f = lo; f <= hi; ++f) any = any || cell_flow[f];
+            }
+            if (any) { jb_l = cs[lo]; je_l = cs[hi + 1]; }
+        }
     }
-    int m = 0;
-    if (__any_sync(0xffffffffu, jb_l < je_l)) {
-        const float4 pi = P32[i];
-        const bool pf = c.pf_on && fabsf(pi.x) < c.pf_lim && fabsf(pi.y) < c.pf_lim && fabsf(pi.z) < c.pf_lim;
-        for (int q = 0; q < NR; ++q) {
-            const int jb = __shfl_sync(0xffffffffu, jb_l, q), je = __shfl_sync(0xffffffffu, je_l, q);
-            for (int b = jb; b < je; b += 32) {
-                const int j = b + lane;
-                bool in = false, flow = false;
-                if (j < je && j != i) {
-                    const float4 pj = P32[j];
-                    flow = pj.w != 0.f;
-                    if (flow || !want_flow) {
-                        bool exact = !pf;
-                        if (pf) {
-                            float fx = pi.x - pj.x, fy = pi.y - pj.y, fz = pi.z - pj.z;
-                            float r2f = fx * fx + fy * fy;
-                            if (DIM == 3) r2f += fz * fz;
-                            in = r2f < c.pf_in2;
-                            if (!in && !(r2f > c.pf_r2)) {
-                                const float4 li = P32L[i], lj = P32L[j];
-                                fx += li.x - lj.x;
-                                fy += li.y - lj.y;
-                                r2f = fx * fx + fy * fy;
-                                if (DIM == 3) { fz += li.z - lj.z; r2f += fz * fz; }
-                                in = r2f < c.pf_lo2;
-                                exact = !in && !(r2f > c.pf_hi2);
-                            }
-                        }
-                        if (exact) {
+    const unsigned some = __ballot_sync(0xffffffffu, jb_l < je_l);
+    for (int r = 0; r < RPW && row0 + r < rows; ++r) {
+        const int row = row0 + r;
+        unsigned left = RPW == 1 ? some : (some >> (NR * r)) & ((1u << NR) - 1u);
+        int m = 0;
+        if (left) {
+            const bool bdy = row >= n_flow, want_flow = bdy || flow_only;
+            const int i = __shfl_sync(0xffffffffu, i_l, NR * r);
+            const int cap = bdy ? pr.cap_b : pr.cap_f;
+            int* out = bdy ? pr.nb_b + (size_t)(row - n_flow) * cap : pr.nb_f + (size_t)row * cap;
+            const float4 pi = P32[i];
+            const bool pf = near_origin(pi);
+            const float in2 = pf ? c.pf_in2 : -1.f, out2 = pf ? c.pf_r2 : __int_as_float(0x7f800000);
+            do {
+                const int q = NR * r + __ffs(left) - 1;
+                left &= left - 1u;
+                const int jb = __shfl_sync(0xffffffffu, jb_l, q), je = __shfl_sync(0xffffffffu, je_l, q);
+                for (int b = jb; b < je; b += 32) {
+                    const int j = b + lane;
+                    const float4 pj = P32[min(j, je - 1)];
+                    const bool flow = pj.w != 0.f;
+                    float fx = pi.x - pj.x, fy = pi.y - pj.y, fz = pi.z - pj.z;
+                    float r2f = fx * fx + fy * fy;
+                    if (DIM == 3) r2f += fz * fz;
+                    bool in = j < je && j != i && (flow || !want_flow) && !(r2f > out2);
+                    if (in && !(r2f < in2)) {
+                        const float4 li = P32L[i], lj = P32L[j];
+                        fx += li.x - lj.x;
+                        fy += li.y - lj.y;
+                        r2f = fx * fx + fy * fy;
+                        if (DIM == 3) { fz += li.z - lj.z; r2f += fz * fz; }
+                        in = pf && r2f < c.pf_lo2;
+                        if (!in && !(pf && r2f > c.pf_hi2)) {
                             const double rx = X[i] - X[j], ry = X[n + i] - X[n + j];
                             double r2 = rx * rx + ry * ry;
                             if (DIM == 3) { const double rz = X[2 * n + i] - X[2 * n + j]; r2 = r2 + rz * rz; }
                             in = r2 < c.R2T;
                         }
                     }
+                    const unsigned bal = __ballot_sync(0xffffffffu, in);
+                    const int pos = m + __popc(bal & ((1u << lane) - 1u));
+                    if (in && pos < cap) out[pos] = flow ? j : j | NB_BDY;
+                    m += __popc(bal);
                 }
-                const unsigned bal = __ballot_sync(0xffffffffu, in);
-                const int pos = m + __popc(bal & ((1u << lane) - 1u));
-                if (in && pos < cap) out[pos] = flow ? j : j | NB_BDY;
-                m += __popc(bal);
-            }
+            } while (left);
         }
+        if (lane == 0) pr.cnt[row] = m;
     }
-    if (lane == 0) pr.cnt[row] = m;
 }
 
 // FP64 products and quotients of the rare operands that the paths below leave out.  Calls, so
