@@ -239,3 +239,36 @@ def test_soil_steps_close(oracle_lib, native, method, ti, skin, corr):
     else:
         assert e_s < 1e-4, report
     sim.ps.check_errors()
+
+
+@pytest.mark.parametrize("method,corr,steps", [(2, 0, 1), (2, 1, 1), (3, 0, 0), (3, 1, 0)])
+def test_soil_overflowed_lists(oracle_lib, native, method, corr, steps):
+    """A second, moving block over a quarter of the column: lists that overflow beside lists that
+    do not, both served by one launch.  A sum of some 60 terms of like size in f32 is good to
+    60 x 6e-8 = 4e-6 of its largest partial sum; the bound is the columns' 1e-4 normwise.
+    (Drucker-Prager from rest only: zero stress there takes the same branch in both forms.)"""
+    import copy
+    d = small_column(method, corr=corr)
+    h = d["Configuration"]["particleRadius"]
+    b = copy.deepcopy(d["Blocks"][0])
+    b["size"] = [b["size"][0] / 2, b["size"][1] / 2] + b["size"][2:]
+    b["translation"] = [b["translation"][0] + h, b["translation"][1] + h, b["translation"][2]]
+    b["velocity"] = [0.1, -0.05, 0.0]
+    d["Blocks"].append(b)
+    sim, orc = _pair(d, oracle_lib)
+    if steps:
+        _advance(sim, orc, oracle_lib, steps)
+    sim.ps.initialize_particle_system()
+    orc.sort()
+    over = sim.ps.list_stats()["overflowed"]
+    f = orc.get("mat_type") == 2
+    assert 100 < over < f.sum()
+    sim.solver.calc_kernel_corr()
+    orc.call(oracle_lib.ORC_KERNEL_CORR)
+    sim.solver.init_real2tmp()
+    orc.call(oracle_lib.ORC_INIT_TMP)
+    sim.solver.one_step()
+    orc.call(oracle_lib.ORC_ONE_STEP)
+    names = ["d_density", "d_vel"] + (["stress_tmp"] if method == 2 else ["d_stress"])
+    errs = {nm: _normwise(_by_id(sim, orc, nm)[f], orc.get(nm)[f]) for nm in names}
+    assert all(e < 1e-4 for e in errs.values()), f"normwise errors {errs}"

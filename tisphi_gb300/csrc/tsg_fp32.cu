@@ -498,9 +498,10 @@ template <int DIM, bool FB, int KT>
 // build.  The overflow pass takes the overflowed particles below nmax.  skip_fluid: the
 // fluid's factors are computed by the first rates pass of the step, so fluid particles are
 // passed over.
-__global__ void __launch_bounds__(256, 6) k_corr32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
-                         const int* __restrict__ sstart, const int* __restrict__ act, const int* __restrict__ nact,
-                         int lim, int nmax, int skip_fluid, Ovf ovf) {
+__device__ __forceinline__ void corr_pass(const K32& k, const P32& p, const T32& t, const float4* __restrict__ PF,
+                                          const int* __restrict__ dstart, const int* __restrict__ sstart,
+                                          const int* __restrict__ act, const int* __restrict__ nact, int lim,
+                                          int nmax, int skip_fluid, const Ovf& ovf) {
     FOR_PARTICLES_ACT(FB, 0, lim, act, nact, nmax, ovf, t.cnt, k.maxn, {
         const int ti = tf_type(p.hi[i].w);
         if (!(skip_fluid && ti == MAT_FLUID)) {
@@ -523,6 +524,16 @@ __global__ void __launch_bounds__(256, 6) k_corr32(K32 k, P32 p, T32 t, const fl
             if (k.corr == 1) inv_store<DIM>(k, t.L, i, L, want_L);
         }
     });
+}
+template <int DIM, int KT>
+__global__ void __launch_bounds__(256, 6)
+k_corr32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+         const int* __restrict__ sstart, const int* __restrict__ act, const int* __restrict__ nact, int lim, int nmax,
+         int skip_fluid, Ovf ovf) {
+    if ((int)blockIdx.x < ovf.first)
+        corr_pass<DIM, false, KT>(k, p, t, PF, dstart, sstart, act, nact, lim, nmax, skip_fluid, ovf);
+    else
+        corr_pass<DIM, true, -1>(k, p, t, PF, dstart, sstart, act, nact, lim, nmax, skip_fluid, ovf);
 }
 
 // Density summation (eng/solver_sph_wc.py:30-31): sum_j mass_j W_ij over every neighbour
@@ -609,9 +620,10 @@ __global__ void k_pre32(K32 k, P32 p, T32 t) {
 // stored, instead of read (the first one_step of a WCSPH step, whose correction kernel
 // then skips the static block).
 template <int DIM, bool FB, int KT, bool SH = false>
-__global__ void k_bdy32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
-                        const int* __restrict__ sstart, int base, int count_n, const int* __restrict__ act,
-                        const int* __restrict__ nact, Ovf ovf) {
+__device__ __forceinline__ void bdy_pass(const K32& k, const P32& p, const T32& t, const float4* __restrict__ PF,
+                                         const int* __restrict__ dstart, const int* __restrict__ sstart, int base,
+                                         int count_n, const int* __restrict__ act, const int* __restrict__ nact,
+                                         const Ovf& ovf) {
     const int lim = base + count_n;
     // with act: the listed particles of [base, lim) (the main pass's direct range is empty)
     FOR_PARTICLES_ACT(FB, base, act ? base : lim, act, nact, lim, ovf, t.cnt, k.maxn, {
@@ -665,6 +677,15 @@ __global__ void k_bdy32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, cons
             }
         }
     });
+}
+template <int DIM, int KT, bool SH>
+__global__ void k_bdy32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+                        const int* __restrict__ sstart, int base, int count_n, const int* __restrict__ act,
+                        const int* __restrict__ nact, Ovf ovf) {
+    if ((int)blockIdx.x < ovf.first)
+        bdy_pass<DIM, false, KT, SH>(k, p, t, PF, dstart, sstart, base, count_n, act, nact, ovf);
+    else
+        bdy_pass<DIM, true, -1, SH>(k, p, t, PF, dstart, sstart, base, count_n, act, nact, ovf);
 }
 
 // The reaction of the fluid on dynamic rigid particles (eng/solver_sph_wc.py:70-71, where
@@ -958,8 +979,9 @@ __global__ void __launch_bounds__(kRigidBlock) k_rigid_rest32(const int* __restr
 // second): (L (v_i - v_j)) . dx = sum_ab L_ab dv_b dx_a and L is symmetric, so a neighbour
 // costs six multiply-adds into the tensor instead of L applied to its velocity difference.
 template <int DIM, bool FB, bool CORR, int KT, int REP, bool FL = false, int U = 2>
-__global__ void __launch_bounds__(256, U == 2 ? 4 : 2) k_rates32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
-                          const int* __restrict__ sstart, Ovf ovf) {
+__device__ __forceinline__ void rates_pass(const K32& k, const P32& p, const T32& t, const float4* __restrict__ PF,
+                                           const int* __restrict__ dstart, const int* __restrict__ sstart,
+                                           const Ovf& ovf) {
     constexpr bool FLC = FL && CORR;  // the CSPM matrix is built in this pass
     // with CORR both passes sum the continuity tensor and contract it with L after the loop
     constexpr bool TEN = CORR;
@@ -1063,6 +1085,13 @@ __global__ void __launch_bounds__(256, U == 2 ? 4 : 2) k_rates32(K32 k, P32 p, T
       }
     });
 }
+template <int DIM, bool CORR, int KT, int REP, bool FL = false, int U = 2>
+__global__ void __launch_bounds__(256, U == 2 ? 4 : 2)
+k_rates32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+          const int* __restrict__ sstart, Ovf ovf) {
+    if ((int)blockIdx.x < ovf.first) rates_pass<DIM, false, CORR, KT, REP, FL, U>(k, p, t, PF, dstart, sstart, ovf);
+    else rates_pass<DIM, true, CORR, -1, -1, FL>(k, p, t, PF, dstart, sstart, ovf);
+}
 
 // Drucker-Prager first phase of one_step: adapt stress_tmp (eng/solver_sph_dp.py:215-217).
 __global__ void k_pre_dp32(K32 k, P32 p, T32 t) {
@@ -1078,8 +1107,9 @@ __global__ void k_pre_dp32(K32 k, P32 p, T32 t) {
 // mu(I) loop 1 (eng/solver_sph_muI.py:67-92): velocity gradient, continuity, pressure from
 // density (not density_tmp), mu(I) stress, equivalent strain rate.
 template <int DIM, bool FB, bool CORR>
-__global__ void k_mui_stress32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
-                               const int* __restrict__ sstart, Ovf ovf) {
+__device__ __forceinline__ void mui_stress_pass(const K32& k, const P32& p, const T32& t,
+                                                const float4* __restrict__ PF, const int* __restrict__ dstart,
+                                                const int* __restrict__ sstart, const Ovf& ovf) {
     FOR_PARTICLES(FB, 0, k.nd, ovf, t.cnt, k.maxn, {
       if (tf_type(p.hi[i].w) == MAT_SOIL) {
         const float4 vti = t.vt[i], vli = t.vtlo[i];
@@ -1109,13 +1139,20 @@ __global__ void k_mui_stress32(K32 k, P32 p, T32 t, const float4* __restrict__ P
       }
     });
 }
+template <int DIM, bool CORR>
+__global__ void k_mui_stress32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+                               const int* __restrict__ sstart, Ovf ovf) {
+    if ((int)blockIdx.x < ovf.first) mui_stress_pass<DIM, false, CORR>(k, p, t, PF, dstart, sstart, ovf);
+    else mui_stress_pass<DIM, true, CORR>(k, p, t, PF, dstart, sstart, ovf);
+}
 
 // Boundary extrapolation for the granular solvers (eng/solver_sph_muI.py:97-109,
 // eng/solver_sph_dp.py:219-234): velocity, density (mu(I)) and stress with the
 // hydrostatic correction rho_j g_a (x_i - x_j)_a on the diagonal.
 template <int DIM, bool FB>
-__global__ void k_bdy_soil32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
-                             const int* __restrict__ sstart, int base, int count_n, Ovf ovf) {
+__device__ __forceinline__ void bdy_soil_pass(const K32& k, const P32& p, const T32& t, const float4* __restrict__ PF,
+                                              const int* __restrict__ dstart, const int* __restrict__ sstart,
+                                              int base, int count_n, const Ovf& ovf) {
     const int lim = base + count_n;
     FOR_PARTICLES(FB, base, lim, ovf, t.cnt, k.maxn, {
         const int ti = tf_type(p.hi[i].w);
@@ -1151,6 +1188,13 @@ __global__ void k_bdy_soil32(K32 k, P32 p, T32 t, const float4* __restrict__ PF,
         }
     });
 }
+template <int DIM>
+__global__ void __maxnreg__(DIM == 3 ? 64 : 56)
+k_bdy_soil32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+             const int* __restrict__ sstart, int base, int count_n, Ovf ovf) {
+    if ((int)blockIdx.x < ovf.first) bdy_soil_pass<DIM, false>(k, p, t, PF, dstart, sstart, base, count_n, ovf);
+    else bdy_soil_pass<DIM, true>(k, p, t, PF, dstart, sstart, base, count_n, ovf);
+}
 
 // The stress and rho_tmp - rho0 of every particle packed for the stress-divergence pass's
 // neighbour reads: one 128-bit read per neighbour in 2D, (s_xx, s_yy, s_xy, rho~ - rho0), and
@@ -1174,8 +1218,9 @@ __global__ void k_pack_stress32(K32 k, T32 t) {
 // velocity gradient, continuity and Bui-2008 stress rate (eng/solver_sph_dp.py:172-208,
 // :236-270), all in one traversal.
 template <int DIM, bool FB, bool CORR, bool DP>
-__global__ void k_soil_mom32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
-                             const int* __restrict__ sstart, Ovf ovf) {
+__device__ __forceinline__ void soil_mom_pass(const K32& k, const P32& p, const T32& t, const float4* __restrict__ PF,
+                                              const int* __restrict__ dstart, const int* __restrict__ sstart,
+                                              const Ovf& ovf) {
     FOR_PARTICLES(FB, 0, k.nd, ovf, t.cnt, k.maxn, {
       if (tf_type(p.hi[i].w) == MAT_SOIL) {
         const size_t n = k.n;
@@ -1277,6 +1322,13 @@ __global__ void k_soil_mom32(K32 k, P32 p, T32 t, const float4* __restrict__ PF,
         }
       }
     });
+}
+template <int DIM, bool CORR, bool DP>
+__global__ void __maxnreg__(DP ? (DIM == 3 ? 96 : 72) : DIM == 3 ? 64 : 56)
+k_soil_mom32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+             const int* __restrict__ sstart, Ovf ovf) {
+    if ((int)blockIdx.x < ovf.first) soil_mom_pass<DIM, false, CORR, DP>(k, p, t, PF, dstart, sstart, ovf);
+    else soil_mom_pass<DIM, true, CORR, DP>(k, p, t, PF, dstart, sstart, ovf);
 }
 
 // mu(I) post-step, part 1 (eng/solver_sph_muI.py:134-149): density clamp, volume, equivalent
@@ -1651,8 +1703,9 @@ __global__ void k_advect_final_mui32(K32 k, P32 p, T32 t, int* err, const float4
 }
 
 template <int DIM, bool FB>
-__global__ void k_xsph32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
-                         const int* __restrict__ sstart, Ovf ovf) {
+__device__ __forceinline__ void xsph_pass(const K32& k, const P32& p, const T32& t, const float4* __restrict__ PF,
+                                          const int* __restrict__ dstart, const int* __restrict__ sstart,
+                                          const Ovf& ovf) {
     FOR_PARTICLES(FB, 0, k.nd, ovf, t.cnt, k.maxn, {
         const int ti = tf_type(p.hi[i].w);
         if (ti > 0 && tf_dyn(p.hi[i].w)) {
@@ -1671,6 +1724,13 @@ __global__ void k_xsph32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, con
             t.xs[i] = make_float4(s[0].get(), s[1].get(), DIM == 3 ? s[2].get() : 0.f, 0.f);
         }
     });
+}
+template <int DIM>
+__global__ void __maxnreg__(DIM == 3 ? 48 : 40)
+k_xsph32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+         const int* __restrict__ sstart, Ovf ovf) {
+    if ((int)blockIdx.x < ovf.first) xsph_pass<DIM, false>(k, p, t, PF, dstart, sstart, ovf);
+    else xsph_pass<DIM, true>(k, p, t, PF, dstart, sstart, ovf);
 }
 
 // POST: also the WCSPH density clamp of advect_something (k_post_wc32, which touches density
@@ -2545,14 +2605,26 @@ bool fp32_rebuild_due(Fp32State& st, cudaStream_t s) {
 }
 
 // The list kernels' main pass is compiled per kernel function (and, for the rates, per
-// repulsive-boundary mode); their overflow pass (a few particles) decides both at run time.
+// repulsive-boundary mode); their overflow pass (a few particles, the last blocks of the same
+// launch) decides both at run time.
 // Grids of the main passes cover the largest possible count of listed static particles;
 // the threads past the device count return at once.
 // skip_fluid: the first rates pass computes the fluid's factors; when the dynamic block holds
 // fluid only, the main pass then visits the listed static particles alone.  skip_static:
 // the first boundary pass computes the static block's Shepard factors.
+// (Where the overflow pass takes more registers than the main pass, the kernel is held to the
+// main pass's.)
+struct Passes {
+    Ovf ovf;
+    int grid, tpb;
+};
+// main_blocks of the main pass over n particles, then 16,384 threads at most for the overflow pass.
+Passes passes(const Fp32State& st, int main_blocks, int n) {
+    return {{st.ovf_list, st.novf, main_blocks}, main_blocks + nblk(std::min(std::max(n, 1), 64 * TPB), st.tpb), st.tpb};
+}
+
 template <int DIM>
-void corr_launch(Fp32State& st, cudaStream_t s, const Ovf& ovf, bool skip_fluid, bool skip_static) {
+void corr_launch(Fp32State& st, cudaStream_t s, bool skip_fluid, bool skip_static) {
     const K32& k = st.k;
     const P32& p = st.P[st.cur];
     const int lim = skip_fluid && st.c.n_bdy <= k.n - k.nd ? 0 : k.nd;
@@ -2560,16 +2632,13 @@ void corr_launch(Fp32State& st, cudaStream_t s, const Ovf& ovf, bool skip_fluid,
     const int nmax = skip_static ? k.nd : k.n;
     const int nb = nblk(lim + (skip_static ? 0 : k.n - k.nd), st.tpb);
     const int sf = skip_fluid ? 1 : 0;
-    if (nb > 0) {
-        if (k.kernel == 1)
-            TSG_LAUNCH((k_corr32<DIM, false, 1>), nb, st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, act, st.nsact,
-                       lim, nmax, sf, ovf);
-        else
-            TSG_LAUNCH((k_corr32<DIM, false, 0>), nb, st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, act, st.nsact,
-                       lim, nmax, sf, ovf);
-    }
-    TSG_LAUNCH((k_corr32<DIM, true, -1>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, act, st.nsact, lim, nmax,
-               sf, ovf);
+    const Passes q = passes(st, nb, nmax);
+    if (k.kernel == 1)
+        TSG_LAUNCH((k_corr32<DIM, 1>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, act, st.nsact, lim, nmax,
+                   sf, q.ovf);
+    else
+        TSG_LAUNCH((k_corr32<DIM, 0>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, act, st.nsact, lim, nmax,
+                   sf, q.ovf);
 }
 
 // Up to this many particles a thread each leaves every SM short of warps, and the rates pass
@@ -2580,46 +2649,40 @@ constexpr int kFewParticles = 152 * 128;
 // WCSPH boundary extrapolation over [base, base + count_n); the static block (base = nd)
 // visits its listed particles only.
 template <int DIM, bool SH>
-void bdy_launch(Fp32State& st, const P32& p, int base, int count_n, cudaStream_t s, const Ovf& ovf) {
+void bdy_launch(Fp32State& st, const P32& p, int base, int count_n, cudaStream_t s) {
     const K32& k = st.k;
-    const int tpb = st.tpb, nb = nblk(count_n, tpb);
+    const Passes q = passes(st, nblk(count_n, st.tpb), count_n);
     const int* act = base == k.nd ? st.sact : nullptr;
     if (k.kernel == 1)
-        TSG_LAUNCH((k_bdy32<DIM, false, 1, SH>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n,
-                   act, st.nsact, ovf);
+        TSG_LAUNCH((k_bdy32<DIM, 1, SH>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n, act,
+                   st.nsact, q.ovf);
     else
-        TSG_LAUNCH((k_bdy32<DIM, false, 0, SH>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n,
-                   act, st.nsact, ovf);
-    TSG_LAUNCH((k_bdy32<DIM, true, -1, SH>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n, act,
-               st.nsact, ovf);
+        TSG_LAUNCH((k_bdy32<DIM, 0, SH>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n, act,
+                   st.nsact, q.ovf);
 }
 
 template <int DIM, bool CORR, int KT, bool FL>
-void rates_main(Fp32State& st, const P32& p, cudaStream_t s, const Ovf& ovf) {
+void rates_kernel(Fp32State& st, const P32& p, cudaStream_t s) {
     const K32& k = st.k;
-    const int tpb = st.tpb, nb = nblk(k.nd, tpb);
+    const Passes q = passes(st, nblk(k.nd, st.tpb), k.nd);
     if (k.boundary == 3 || k.boundary == 4)
-        TSG_LAUNCH((k_rates32<DIM, false, CORR, KT, 1, FL>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
+        TSG_LAUNCH((k_rates32<DIM, CORR, KT, 1, FL>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf);
     else if (k.nd <= kFewParticles)
-        TSG_LAUNCH((k_rates32<DIM, false, CORR, KT, 0, FL, 4>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
+        TSG_LAUNCH((k_rates32<DIM, CORR, KT, 0, FL, 4>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf);
     else
-        TSG_LAUNCH((k_rates32<DIM, false, CORR, KT, 0, FL>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
+        TSG_LAUNCH((k_rates32<DIM, CORR, KT, 0, FL>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf);
 }
 
 template <int DIM, bool CORR, bool FL = false>
-void rates_launch(Fp32State& st, const P32& p, cudaStream_t s, const Ovf& ovf) {
-    const K32& k = st.k;
-    if (k.kernel == 1) rates_main<DIM, CORR, 1, FL>(st, p, s, ovf);
-    else rates_main<DIM, CORR, 0, FL>(st, p, s, ovf);
-    TSG_LAUNCH((k_rates32<DIM, true, CORR, -1, -1, FL>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
+void rates_launch(Fp32State& st, const P32& p, cudaStream_t s) {
+    if (st.k.kernel == 1) rates_kernel<DIM, CORR, 1, FL>(st, p, s);
+    else rates_kernel<DIM, CORR, 0, FL>(st, p, s);
 }
 
 static void kernel_corr(Fp32State& st, cudaStream_t s, bool skip_fluid, bool skip_static) {
     PhaseScope ph(s, PH_CORR);
-    const K32& k = st.k;
-    const Ovf ovf{st.ovf_list, st.novf};
-    if (k.dim == 2) corr_launch<2>(st, s, ovf, skip_fluid, skip_static);
-    else corr_launch<3>(st, s, ovf, skip_fluid, skip_static);
+    if (st.k.dim == 2) corr_launch<2>(st, s, skip_fluid, skip_static);
+    else corr_launch<3>(st, s, skip_fluid, skip_static);
 }
 
 void fp32_kernel_corr(Fp32State& st, cudaStream_t s) { kernel_corr(st, s, false, false); }
@@ -2634,15 +2697,14 @@ template <int DIM>
 void soil_one_step(Fp32State& st, cudaStream_t s) {
     const K32& k = st.k;
     P32& p = st.P[st.cur];
-    const Ovf ovf{st.ovf_list, st.novf};
-    const int tpb = st.tpb, nb = nblk(k.nd, tpb);
+    const Passes q = passes(st, nblk(k.nd, st.tpb), k.nd);
     {
         PhaseScope ph(s, PH_PRE);
         if (k.solver == 2) {
-            if (k.corr) { TSG_LAUNCH((k_mui_stress32<DIM, false, true>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
-                          TSG_LAUNCH((k_mui_stress32<DIM, true, true>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf); }
-            else { TSG_LAUNCH((k_mui_stress32<DIM, false, false>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
-                   TSG_LAUNCH((k_mui_stress32<DIM, true, false>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf); }
+            if (k.corr)
+                TSG_LAUNCH((k_mui_stress32<DIM, true>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf);
+            else
+                TSG_LAUNCH((k_mui_stress32<DIM, false>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf);
         } else {
             TSG_LAUNCH(k_pre_dp32, nblk(k.nd), TPB, s, k, p, st.T);
         }
@@ -2651,8 +2713,8 @@ void soil_one_step(Fp32State& st, cudaStream_t s) {
         PhaseScope ph(s, PH_BDY);
         auto bdy = [&](int base, int count_n) {
             if (count_n <= 0) return;
-            TSG_LAUNCH((k_bdy_soil32<DIM, false>), nblk(count_n, tpb), tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n, ovf);
-            TSG_LAUNCH((k_bdy_soil32<DIM, true>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n, ovf);
+            const Passes b = passes(st, nblk(count_n, st.tpb), count_n);
+            TSG_LAUNCH(k_bdy_soil32<DIM>, b.grid, b.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, base, count_n, b.ovf);
         };
         bdy(k.nd, k.n - k.nd);
         if (st.c.n_bdy > k.n - k.nd) bdy(0, k.nd);
@@ -2660,11 +2722,8 @@ void soil_one_step(Fp32State& st, cudaStream_t s) {
     {
         PhaseScope ph(s, PH_RATES);
         TSG_LAUNCH(k_pack_stress32<DIM>, nblk(k.n), TPB, s, k, st.T);
-#define SOIL_MOM(CORR, DP)                                                                                       \
-        do {                                                                                                     \
-            TSG_LAUNCH((k_soil_mom32<DIM, false, CORR, DP>), nb, tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf); \
-            TSG_LAUNCH((k_soil_mom32<DIM, true, CORR, DP>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);  \
-        } while (0)
+#define SOIL_MOM(CORR, DP) \
+        TSG_LAUNCH((k_soil_mom32<DIM, CORR, DP>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf)
         if (k.solver == 2) { if (k.corr) SOIL_MOM(true, false); else SOIL_MOM(false, false); }
         else { if (k.corr) SOIL_MOM(true, true); else SOIL_MOM(false, true); }
 #undef SOIL_MOM
@@ -2689,15 +2748,14 @@ static void one_step(Fp32State& st, cudaStream_t s, bool eos, bool fl = false, b
     }
     {
         PhaseScope ph(s, PH_BDY);
-        const Ovf ovf{st.ovf_list, st.novf};
         auto bdy = [&](int base, int count_n, bool shep) {
             if (count_n <= 0) return;
             if (shep) {
-                if (k.dim == 2) bdy_launch<2, true>(st, p, base, count_n, s, ovf);
-                else bdy_launch<3, true>(st, p, base, count_n, s, ovf);
+                if (k.dim == 2) bdy_launch<2, true>(st, p, base, count_n, s);
+                else bdy_launch<3, true>(st, p, base, count_n, s);
             } else {
-                if (k.dim == 2) bdy_launch<2, false>(st, p, base, count_n, s, ovf);
-                else bdy_launch<3, false>(st, p, base, count_n, s, ovf);
+                if (k.dim == 2) bdy_launch<2, false>(st, p, base, count_n, s);
+                else bdy_launch<3, false>(st, p, base, count_n, s);
             }
         };
         bdy(k.nd, k.n - k.nd, sh);
@@ -2705,12 +2763,11 @@ static void one_step(Fp32State& st, cudaStream_t s, bool eos, bool fl = false, b
     }
     {
         PhaseScope ph(s, PH_RATES);
-        const Ovf ovf{st.ovf_list, st.novf};
         if (fl) {
-            if (k.dim == 2) { if (k.corr) rates_launch<2, true, true>(st, p, s, ovf); else rates_launch<2, false, true>(st, p, s, ovf); }
-            else { if (k.corr) rates_launch<3, true, true>(st, p, s, ovf); else rates_launch<3, false, true>(st, p, s, ovf); }
-        } else if (k.dim == 2) { if (k.corr) rates_launch<2, true>(st, p, s, ovf); else rates_launch<2, false>(st, p, s, ovf); }
-        else { if (k.corr) rates_launch<3, true>(st, p, s, ovf); else rates_launch<3, false>(st, p, s, ovf); }
+            if (k.dim == 2) { if (k.corr) rates_launch<2, true, true>(st, p, s); else rates_launch<2, false, true>(st, p, s); }
+            else { if (k.corr) rates_launch<3, true, true>(st, p, s); else rates_launch<3, false, true>(st, p, s); }
+        } else if (k.dim == 2) { if (k.corr) rates_launch<2, true>(st, p, s); else rates_launch<2, false>(st, p, s); }
+        else { if (k.corr) rates_launch<3, true>(st, p, s); else rates_launch<3, false>(st, p, s); }
         if (st.rnobj) {  // the fluid's reaction on dynamic rigid particles, after the rates pass
             if (k.dim == 2) TSG_LAUNCH(k_rigid_reaction32<2>, nblk(k.nd), TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart);
             else TSG_LAUNCH(k_rigid_reaction32<3>, nblk(k.nd), TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart);
@@ -2727,14 +2784,11 @@ static void advect_pos(Fp32State& st, cudaStream_t s, bool post) {
     P32& p = st.P[st.cur];
     PhaseScope ph(s, PH_POS);
     if (k.xsph) {
-        const Ovf ovf{st.ovf_list, st.novf};
-        if (k.dim == 2) {
-            TSG_LAUNCH((k_xsph32<2, false>), nblk(k.nd, st.tpb), st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
-            TSG_LAUNCH((k_xsph32<2, true>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
-        } else {
-            TSG_LAUNCH((k_xsph32<3, false>), nblk(k.nd, st.tpb), st.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
-            TSG_LAUNCH((k_xsph32<3, true>), 64, TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, ovf);
-        }
+        const Passes q = passes(st, nblk(k.nd, st.tpb), k.nd);
+        if (k.dim == 2)
+            TSG_LAUNCH(k_xsph32<2>, q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf);
+        else
+            TSG_LAUNCH(k_xsph32<3>, q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf);
     }
     if (post) TSG_LAUNCH(k_advect_pos32<true>, nblk(k.nd), TPB, s, k, p, st.T, st.err);
     else TSG_LAUNCH(k_advect_pos32<false>, nblk(k.nd), TPB, s, k, p, st.T, st.err);
