@@ -700,9 +700,9 @@ struct Fp32State {
 namespace f32 {
 // Host helpers shared with the adjoint unit (defined in tsg_fp32.cu).
 // Re-sort the dynamic block and rebuild every list (in_place keeps the current buffer).
-void rebuild(Fp32State& st, cudaStream_t s, bool in_place);
+void rebuild(Fp32State& st, cudaStream_t s, bool in_place, bool init = false);
 // One step after the re-sort: correction, init_real2tmp, integrator, advect_pos, post-step.
-void step_body(Fp32State& st, cudaStream_t s, bool collide, bool fold_disp = false);
+void step_body(Fp32State& st, cudaStream_t s, bool collide, bool fold_disp = false, bool inited = false);
 }  // namespace f32
 
 }  // namespace tsg
