@@ -3,7 +3,7 @@
 // places a cell's particles in atomic arrival order).
 //
 // Ordinary cells hold a few dozen particles, and the reorder passes rank each particle among its
-// cell's themselves.  For a segment above kSortSmall - the out-of-grid bin after particles left
+// cell's themselves (tsg_cellrank.cuh).  For a segment above kSortSmall - the out-of-grid bin after particles left
 // the grid, or a very coarse grid - that would be quadratic (a blown-up run with every particle
 // out of the grid would keep the GPU busy for hours), so the scatter lists such cells and
 // k_cell_sort_big sorts them first, one block per cell: up to kSortMid particles by a bitonic

@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "tsg_fp32_dev.cuh"
+#include "tsg_cellrank.cuh"
 #include "tsg_polar.cuh"
 #include "tsg_rigid_list.cuh"
 
@@ -72,14 +73,20 @@ __global__ void k_hash32(K32 k, int count_n, int base, const float4* __restrict_
 __global__ void k_reorder32(K32 k, int count_n, int base, const int* __restrict__ perm,
                             const int* __restrict__ cell_of, const int* __restrict__ cell_start, int small, P32 a,
                             P32 b, float4* __restrict__ PF) {
+    __shared__ int sh_rank[TPB / 32][64];
     int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count_n) return;
-    const int old = perm[t], cell = cell_of[old], cb = cell_start[cell], ce = cell_start[cell + 1];
-    if (ce - cb <= small) {
-        int r = 0;
-        for (int q = cb; q < ce; ++q) r += perm[q] < old;
-        t = cb + r;
+    const bool live = t < count_n;
+    int old = 0, cb = 0, ce = 0;
+    if (live) {
+        old = perm[t];
+        const int cell = cell_of[old];
+        cb = cell_start[cell];
+        ce = cell_start[cell + 1];
     }
+    const bool ranks = live && ce - cb <= small;
+    const int r = rank_in_cell(perm, cb, ce, old, ranks, sh_rank[threadIdx.x >> 5]);
+    if (!live) return;
+    if (ranks) t = cb + r;
     const int dst = base + t, src = base + old;
     float4 h = a.hi[src], l = a.lo[src];
     float hv[3] = {h.x, h.y, h.z}, lv[3] = {l.x, l.y, l.z};

@@ -72,9 +72,8 @@ struct Consts {
 // Largest cell segment whose particles the reorder passes rank among themselves
 // (tsg_cellsort.cuh), and the size of the list of larger cells (at most n / (kSortSmall + 1) of them).
 constexpr int kSortSmall = 256;
-// Up to this many particles the reorder pass ranks every cell itself, however large (all of them
-// in one cell: 16,384 loads a thread, a fraction of a millisecond), and the launch that orders
-// the larger cells is left out.
+// Up to this many particles the reorder pass ranks every cell itself, however large
+// (rank_in_cell), and the launch that orders the larger cells is left out.
 constexpr int kSortAll = 16384;
 inline int sort_small(int n) { return n <= kSortAll ? 0x7fffffff : kSortSmall; }
 inline size_t cellsort_big_ints(long long n) { return (size_t)(n / kSortSmall + 2); }

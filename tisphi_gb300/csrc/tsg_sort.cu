@@ -16,6 +16,7 @@
 // Compiled with -fmad=false: the f64 cell arithmetic must round exactly like the oracle's.
 #include <cstdio>
 
+#include "tsg_cellrank.cuh"
 #include "tsg_cellsort.cuh"
 #include "tsg_internal.h"
 #include "tsg_pairs64.cuh"
@@ -202,20 +203,24 @@ __global__ void k_reorder64(Consts c, const int* __restrict__ perm, Persist64 a,
                             unsigned char* __restrict__ cell_flow, int* __restrict__ list_flow,
                             int* __restrict__ list_bdy, int* __restrict__ list_count,
                             const double* __restrict__ vt_src, double* __restrict__ vt_dst) {
+    __shared__ int sh_rank[TPB / 32][64];
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = k < c.n;
     int mt = 0;
+    // ascending old index inside the cell: this particle's rank among the cell's (a pass of
+    // its own, one thread per cell, took 15 us on a 2D grid and 158 us on the 3D benchmark's)
+    int s = 0, cb = 0, ce = 0;
+    if (live) {
+        s = perm[k];
+        const int cell = cell_of[s];
+        cb = cell_start[cell];
+        ce = cell_start[cell + 1];
+    }
+    const bool ranks = live && ce - cb <= small;
+    const int r = rank_in_cell(perm, cb, ce, s, ranks, sh_rank[threadIdx.x >> 5]);
+    if (ranks) k = cb + r;
     if (live) {
         const size_t n = c.n;
-        const int s = perm[k];
-        // ascending old index inside the cell: this particle's rank among the cell's (a pass of
-        // its own, one thread per cell, took 15 us on a 2D grid and 158 us on the 3D benchmark's)
-        const int cell = cell_of[s], cb = cell_start[cell], ce = cell_start[cell + 1];
-        if (ce - cb <= small) {
-            int r = 0;
-            for (int q = cb; q < ce; ++q) r += perm[q] < s;
-            k = cb + r;
-        }
         // every load before the first store: the compiler cannot tell the planes apart, and a
         // store between them makes each load wait for the one before it
         double xv[3], vv[3], x0[3], st[9], vt[3];
