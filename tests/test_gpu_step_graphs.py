@@ -1,0 +1,42 @@
+"""Step graphs of the FP32-mixed form: what tsg_get_launch says of them."""
+import ctypes
+
+import pytest
+
+from helpers import cfg_of, small_dambreak_2d
+
+pytestmark = pytest.mark.gpu
+
+
+def _steps_per_graph(lib, ps):
+    from tisphi_gb300 import _native as nat
+    c = nat.tsg_launch_cfg()
+    nat.check(lib.tsg_get_launch(ps._h, ctypes.byref(c)), "tsg_get_launch")
+    return c.steps_per_graph
+
+
+def _launches_of(lib, sim, steps):
+    before = lib.tsg_launch_count()
+    sim.solver.step(steps)
+    return lib.tsg_launch_count() - before
+
+
+def test_get_launch_reports_the_graphs_replayed(native):
+    """Single-step graphs for ten steps, five-step graphs after that; a caller's choice as given."""
+    from tisphi_gb300 import _native as nat
+    from tisphi_gb300.simulation import Simulation
+    lib = native
+    sim = Simulation(cfg_of(small_dambreak_2d()), precision="fp32_mixed")
+    assert _steps_per_graph(lib, sim.ps) == 1
+    sim.solver.step(4)
+    assert _steps_per_graph(lib, sim.ps) == 1
+    sim.solver.step(6)
+    assert _steps_per_graph(lib, sim.ps) == 5
+    # (a five-step graph checks the lists' expiry once: fewer launches than five single steps)
+    five = _launches_of(lib, sim, 5)
+    assert five < sum(_launches_of(lib, sim, 1) for _ in range(5))
+    cfg = nat.tsg_launch_cfg(128, 0, 3)
+    nat.check(lib.tsg_set_launch(sim.ps._h, ctypes.byref(cfg)), "tsg_set_launch")
+    assert _steps_per_graph(lib, sim.ps) == 3
+    sim.solver.step(20)
+    assert _steps_per_graph(lib, sim.ps) == 3

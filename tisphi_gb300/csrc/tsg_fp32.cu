@@ -3079,15 +3079,20 @@ Fp32State::StepGraph* graph_for(Fp32State& st, int steps, bool collide, int* rc)
 
 constexpr int kWarmSteps = 10;
 
+// Steps of the graph that the next tsg_step replays where it has that many to run.  Without a
+// caller's choice: single-step graphs at first, then graphs of five, which check the list expiry
+// once (10 steps: batch of 64 scenes 1,356 -> 1,272 us, 3D benchmark 9,413 -> 9,183) and cost a
+// few hundred microseconds to capture.
+static int graph_length(const Fp32State& st) {
+    if (!st.graph_chosen && st.graph_steps >= kWarmSteps) return 5;
+    return st.steps_per_graph > 1 ? st.steps_per_graph : 1;
+}
+
 int fp32_step_graph(Fp32State& st, int nsteps, bool collide, cudaStream_t s) {
     if (profiling_on()) return TSG_E_STATE;  // per-phase events need the eager path
     const bool always = st.k.disp2_limit <= 0.f;  // the graphs rebuild in every step
     if (!st.built && !always) fp32_sort(st, s);
-    // Without a caller's choice: single-step graphs at first, then graphs of five, which check the
-    // list expiry once (10 steps: batch of 64 scenes 1,356 -> 1,272 us, 3D benchmark 9,413 -> 9,183)
-    // and cost a few hundred microseconds to capture.
-    int K = st.steps_per_graph > 1 ? st.steps_per_graph : 1;
-    if (!st.graph_chosen && st.graph_steps >= kWarmSteps) K = 5;
+    const int K = graph_length(st);
     st.graph_steps = st.graph_steps < kWarmSteps ? st.graph_steps + nsteps : st.graph_steps;
     int rc = 0;
     while (nsteps > 0) {
@@ -3108,7 +3113,7 @@ void fp32_flush_counters(Fp32State& st, cudaStream_t s) { fold_rebuilds(st, s); 
 void fp32_get_launch(const Fp32State& st, int* tpb, int* cpc, int* spg) {
     *tpb = st.tpb;
     *cpc = st.cells_per_cta;
-    *spg = st.steps_per_graph;
+    *spg = graph_length(st);
 }
 
 int fp32_set_launch(Fp32State& st, int tpb, int cpc, int spg) {
