@@ -290,8 +290,9 @@ int tsg_sort_noalloc(const tsg_config* cfg, const double* x, int64_t n, int32_t*
  * its own launch shapes): threads_per_block of the neighbour-traversal kernels (64, 128,
  * 256); cells_per_cta of the neighbour-list build, one warp per cell (2, 4, 8; 0 = one
  * thread per particle); steps_per_graph, how many steps one captured CUDA graph replays
- * (1..64; until tsg_set_launch or tsg_autotune chooses it, 1 for a handle's first ten steps
- * and 5 from then on, which tsg_get_launch reports as it stands).  tsg_step runs FP32-mixed
+ * (1..64; until tsg_set_launch or tsg_autotune chooses it, 1 for the first ten steps after
+ * the upload or a tsg_set_fluid / tsg_set_soil and 5 from then on, which tsg_get_launch
+ * reports as it stands).  tsg_step runs FP32-mixed
  * steps as graph replays (each step re-sorts inside the graph only when the device-side
  * displacement check asks for it); while tsg_profile is on it runs them eagerly. */
 typedef struct tsg_launch_cfg {

@@ -3,7 +3,7 @@ import ctypes
 
 import pytest
 
-from helpers import cfg_of, small_dambreak_2d
+from helpers import cfg_of, small_column, small_dambreak_2d
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +40,20 @@ def test_get_launch_reports_the_graphs_replayed(native):
     assert _steps_per_graph(lib, sim.ps) == 3
     sim.solver.step(20)
     assert _steps_per_graph(lib, sim.ps) == 3
+
+
+@pytest.mark.parametrize("method", [1, 2])
+def test_parameter_changes_start_with_single_step_graphs(native, method):
+    """A five-step graph takes as long to capture as several steps take to run: a caller that
+    sets a parameter every few steps gets single-step graphs, as a new handle does."""
+    from tisphi_gb300.simulation import Simulation
+    sim = Simulation(cfg_of(small_dambreak_2d() if method == 1 else small_column(2)), precision="fp32_mixed")
+    sim.solver.step(12)
+    assert _steps_per_graph(native, sim.ps) == 5
+    if method == 1:
+        sim.solver.viscosity = 0.006
+    else:
+        sim.solver.coh = 1.0
+    assert _steps_per_graph(native, sim.ps) == 1
+    sim.solver.step(10)
+    assert _steps_per_graph(native, sim.ps) == 5

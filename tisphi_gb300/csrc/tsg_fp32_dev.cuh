@@ -678,7 +678,8 @@ struct Fp32State {
     // particle), steps per captured graph
     int tpb = 128, cells_per_cta = 4, steps_per_graph = 1;
     bool graph_chosen = false;  // steps_per_graph set by the caller or by tuning
-    int graph_steps = 0;        // steps run by graphs (counted up to the switch to longer ones)
+    int graph_steps = 0;        // steps run by graphs since the constants last changed (counted up to
+                                // the switch to longer ones)
     // captured step graphs: [0] one step, [1] steps_per_graph steps
     struct StepGraph {
         cudaGraphExec_t exec = nullptr;
