@@ -57,3 +57,16 @@ def test_parameter_changes_start_with_single_step_graphs(native, method):
     assert _steps_per_graph(native, sim.ps) == 1
     sim.solver.step(10)
     assert _steps_per_graph(native, sim.ps) == 5
+
+
+def test_a_write_of_x_leaves_no_trace_in_later_graphs(native):
+    """mu(I): graphs captured after a write of x hold the same kernels as others (the five-step
+    graph one displacement check, the regularisation the lists)."""
+    from tisphi_gb300.simulation import Simulation
+    a, b = (Simulation(cfg_of(small_column(2)), precision="fp32_mixed") for _ in range(2))
+    for s in (a, b):
+        s.solver.step(10)
+    b.ps.write_field("x", b.ps.field("x").contiguous())
+    for s in (a, b):
+        s.solver.step(5)
+    assert _launches_of(native, a, 5) == _launches_of(native, b, 5)

@@ -2621,7 +2621,9 @@ bool fp32_rebuild_due(Fp32State& st, cudaStream_t s) {
     cudaStreamSynchronize(s);
     float d2;
     std::memcpy(&d2, &bits, sizeof d2);
-    return !(d2 <= k.disp2_limit);
+    if (!(d2 <= k.disp2_limit)) return true;
+    st.lists_valid = true;  // (also after a write of x, which leaves the flag unset)
+    return false;
 }
 
 // The list kernels' main pass is compiled per kernel function (and, for the rates, per
@@ -2990,6 +2992,7 @@ int capture_steps(Fp32State& st, int steps, bool collide, Fp32State::StepGraph& 
     if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) return TSG_E_CUDA;
     if (cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking) != cudaSuccess) { cudaStreamDestroy(cs); return TSG_E_CUDA; }
     const K32& k = st.k;
+    const bool valid0 = st.lists_valid;
     const long long c0 = launch_total();
     long long body = 0;
     int rc = 0;
@@ -3040,6 +3043,9 @@ int capture_steps(Fp32State& st, int steps, bool collide, Fp32State::StepGraph& 
         cudaGraph_t done = nullptr;
         if (cudaStreamEndCapture(bs, &done) != cudaSuccess) { rc = TSG_E_CUDA; break; }
         body = launch_total() - b0;
+        // The check above, with its rebuild, leaves valid lists in every replay, whatever a write of
+        // x has left behind on the host: step_body decides by the flag what the graph holds.
+        st.lists_valid = true;
         step_body(st, cs, collide, q + 1 < steps && folds_disp(st, collide));
     }
     cudaError_t e = cudaStreamEndCapture(cs, &graph);
@@ -3054,7 +3060,10 @@ int capture_steps(Fp32State& st, int steps, bool collide, Fp32State::StepGraph& 
     cudaStreamDestroy(bs);
     cudaStreamDestroy(cs);
     cudaGetLastError();
-    if (rc) return rc;
+    if (rc) {
+        st.lists_valid = valid0;
+        return rc;
+    }
     g.steps = steps;
     g.cur = st.cur;
     g.tpb = st.tpb;
