@@ -1,7 +1,9 @@
-"""Step graphs of the FP32-mixed form: what tsg_get_launch says of them."""
+"""Captured steps: what tsg_get_launch says of them, what they hold, and how they are counted."""
 import ctypes
+import threading
 
 import pytest
+import torch
 
 from helpers import cfg_of, small_column, small_dambreak_2d
 
@@ -70,3 +72,73 @@ def test_a_write_of_x_leaves_no_trace_in_later_graphs(native):
     for s in (a, b):
         s.solver.step(5)
     assert _launches_of(native, a, 5) == _launches_of(native, b, 5)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_mixed"])
+def test_launches_counted_while_other_threads_launch(native, precision):
+    """Two threads, a handle each: every parameter change has the next step captured again, and
+    neither thread's launches enter what the other counts for its graphs."""
+    from tisphi_gb300.simulation import Simulation
+
+    def work(sim):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for q in range(60):
+                sim.solver.viscosity = 0.005 + 1e-6 * (q % 3)
+                sim.solver.step(1 + 3 * (q % 2))
+            torch.cuda.synchronize()
+
+    def total(together):
+        sims = [Simulation(cfg_of(small_dambreak_2d()), precision=precision) for _ in range(2)]
+        for s in sims:
+            s.solver.step(2)
+        torch.cuda.synchronize()
+        before = native.tsg_launch_count()
+        if together:
+            threads = [threading.Thread(target=work, args=(s,)) for s in sims]
+            for t in threads:
+                t.start()
+            for t in threads:
+                t.join()
+        else:
+            for s in sims:
+                work(s)
+        return native.tsg_launch_count() - before
+
+    alone = total(False)
+    assert alone > 0 and [total(True) for _ in range(3)] == [alone] * 3
+
+
+@pytest.mark.parametrize("precision,method", [("fp64", 1), ("fp64", 2), ("fp32_mixed", 1), ("fp32_mixed", 2)])
+def test_graphs_made_while_another_thread_synchronises(native, precision, method):
+    """A thread that waits for the device all the time, while parameter changes have every step's
+    graph made anew: neither side fails, and the state is that of an undisturbed run, bit for bit."""
+    from tisphi_gb300.simulation import Simulation
+
+    def run():
+        sim = Simulation(cfg_of(small_dambreak_2d() if method == 1 else small_column(2)), precision=precision)
+        for q in range(40):
+            if method == 1:
+                sim.solver.viscosity = 0.005 + 1e-6 * (q % 3)
+            else:
+                sim.solver.coh = 0.1 * (q % 3)
+            sim.solver.step(1 + q % 3)
+        return [sim.ps.field(nm).cpu() for nm in ("x", "v", "density", "id0")]
+
+    want = run()
+    stop, failed, waits = threading.Event(), [], [0]
+
+    def wait():
+        try:
+            while not stop.is_set():
+                torch.cuda.synchronize()
+                waits[0] += 1
+        except RuntimeError as e:
+            failed.append(e)
+
+    t = threading.Thread(target=wait)
+    t.start()
+    got = run()
+    stop.set()
+    t.join()
+    assert not failed and waits[0] > 10
+    assert all(torch.equal(a, b) for a, b in zip(want, got))

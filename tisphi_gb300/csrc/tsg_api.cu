@@ -21,6 +21,52 @@ void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 void add_launches(long long delta) { g_launches.fetch_add(delta, std::memory_order_relaxed); }
 long long launch_total() { return g_launches.load(std::memory_order_relaxed); }
 
+Tape*& tape() {
+    static thread_local Tape* t = nullptr;
+    return t;
+}
+void Tape::added(cudaError_t e, cudaGraphNode_t n) {
+    ok = ok && e == cudaSuccess;
+    if (e == cudaSuccess) deps.assign(1, n);
+}
+void Tape::node(void* f, dim3 grid, dim3 block, void** args) {
+    cudaKernelNodeParams kp{};
+    kp.func = f;
+    kp.gridDim = grid;
+    kp.blockDim = block;
+    kp.kernelParams = args;
+    cudaGraphNode_t n = nullptr;
+    added(cudaGraphAddKernelNode(&n, graph, deps.data(), deps.size(), &kp), n);
+    ++kernels;
+}
+void Tape::zero(void* p, size_t bytes) {
+    cudaMemsetParams mp{};
+    mp.dst = p;
+    mp.elementSize = bytes % 4 == 0 ? 4 : 1;
+    mp.width = bytes / mp.elementSize;
+    mp.height = 1;
+    cudaGraphNode_t n = nullptr;
+    added(cudaGraphAddMemsetNode(&n, graph, deps.data(), deps.size(), &mp), n);
+}
+void Tape::copy(void* dst, const void* src, size_t bytes) {
+    cudaGraphNode_t n = nullptr;
+    added(cudaGraphAddMemcpyNode1D(&n, graph, deps.data(), deps.size(), dst, src, bytes, cudaMemcpyDeviceToDevice), n);
+}
+void Fork::join() {
+    if (!tape()) return;
+    auto& d = tape()->deps;
+    for (cudaGraphNode_t n : first)
+        if (std::find(d.begin(), d.end(), n) == d.end()) d.push_back(n);
+}
+void zero_async(void* p, size_t bytes, cudaStream_t s) {
+    if (tape()) tape()->zero(p, bytes);
+    else cudaMemsetAsync(p, 0, bytes, s);
+}
+void copy_async(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    if (tape()) tape()->copy(dst, src, bytes);
+    else cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s);
+}
+
 struct ProfRec { int phase; cudaEvent_t a, b; };
 struct Profiler {
     bool on = false;
@@ -63,12 +109,12 @@ struct tsg_handle {
     int nscenes = 0;                // batched ensemble (tsg_batch_create): scenes and x pitch
     double batch_pitch = 0.0;
     Rigid64 rigid{};                // dynamic rigid bodies (FP64 form)
-    // Captured steps of the FP64 form, [buffer parity][1 or 2 steps] (see step_graph64)
+    // Step graphs of the FP64 form, [buffer parity][1 or 2 steps] (see step_graph64)
     struct StepGraph { cudaGraphExec_t exec = nullptr; long long kernels = 0; bool collide = false; };
     StepGraph graphs[2][2];
     const double* x_first = nullptr;  // cur.x at upload: tells the buffer parity
     int eager_steps = 0;
-    bool no_graphs = false;         // a capture failed: launch eagerly
+    bool no_graphs = false;         // a graph could not be made: launch eagerly
     // While the FP64 arrays are laid out: offset into (and, once it is known, base of) the one
     // allocation that holds them (see alloc_all)
     char* slab = nullptr;
@@ -289,8 +335,8 @@ void own_rows(tsg_handle* h, bool geometry, cudaStream_t s) {
 }
 
 // One step of the FP64 form after its sort.
-int step64(tsg_handle* h, bool collide, cudaStream_t s, const SideStream64* side = nullptr) {
-    fp64_step(h->c, h->cur, h->t, h->g, h->rigid, collide, s, side);
+int step64(tsg_handle* h, bool collide, cudaStream_t s) {
+    fp64_step(h->c, h->cur, h->t, h->g, h->rigid, collide, s);
     h->pos32_dirty = true;
     return check_cuda();
 }
@@ -303,7 +349,7 @@ void drop_graphs64(tsg_handle* h) {
         }
 }
 
-// The captured graph of one or two FP64 steps from the current buffers.  A small scene's step is
+// The graph of one or two FP64 steps from the current buffers.  A small scene's step is
 // some twenty-five launches of a few microseconds, each waiting for the host's next one when
 // launched one by one; the graph issues them back to back.  Nothing in a step depends on the
 // host, the constants are the launches' own copies (dropped when a material is set), and the
@@ -312,35 +358,25 @@ tsg_handle::StepGraph* step_graph64(tsg_handle* h, int steps, bool collide) {
     tsg_handle::StepGraph& g = h->graphs[h->cur.x == h->x_first ? 0 : 1][steps - 1];
     if (g.exec && g.collide == collide) return &g;
     if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
-    cudaStream_t cs = nullptr;
-    SideStream64 side{};
-    bool ok = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming) == cudaSuccess &&
-              cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming) == cudaSuccess;
     const Persist64 cur = h->cur, nxt = h->nxt;
-    const long long c0 = launch_total();
     cudaGraph_t graph = nullptr;
-    ok = ok && cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed) == cudaSuccess;
-    if (ok) {
+    if (cudaGraphCreate(&graph, 0) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    Tape tape(graph);
+    bool ok = true;
+    {
+        Recording rec(tape);
         for (int q = 0; q < steps && ok; ++q) {
-            sort_fp64(h->c, h->cur, h->nxt, h->t, h->g, cs);
-            ok = step64(h, collide, cs, &side) == 0;
+            sort_fp64(h->c, h->cur, h->nxt, h->t, h->g, nullptr);
+            ok = step64(h, collide, nullptr) == 0;
         }
-        ok = cudaStreamEndCapture(cs, &graph) == cudaSuccess && graph && ok;
     }
-    g.kernels = launch_total() - c0;
-    add_launches(-g.kernels);  // nodes, not launches
     h->cur = cur;
     h->nxt = nxt;
-    ok = ok && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
+    ok = ok && tape.ok && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
     if (!ok) g.exec = nullptr;
-    if (graph) cudaGraphDestroy(graph);
-    if (side.fork) cudaEventDestroy(side.fork);
-    if (side.join) cudaEventDestroy(side.join);
-    if (side.stream) cudaStreamDestroy(side.stream);
-    if (cs) cudaStreamDestroy(cs);
+    cudaGraphDestroy(graph);
     cudaGetLastError();
+    g.kernels = tape.kernels;
     g.collide = collide;
     return ok ? &g : nullptr;
 }
@@ -352,7 +388,7 @@ bool capturing(cudaStream_t s) {
 }
 
 // FP64 steps.  The first two of a handle run eagerly (a script that steps once or twice does
-// not pay for a capture), as do profiled steps and steps inside a caller's own capture.
+// not pay for a graph), as do profiled steps and steps inside a caller's own capture.
 int steps64(tsg_handle* h, int nsteps, bool collide, cudaStream_t s) {
     bool graphs = !h->no_graphs && !profiling_on() && !capturing(s);
     while (nsteps > 0) {

@@ -2508,7 +2508,7 @@ bool build_lists(Fp32State& st, const P32& p, cudaStream_t s) {
                    st.ovf_list, st.novf);
         return false;
     }
-    cudaMemsetAsync(st.ncells, 0, sizeof(int), s);
+    zero_async(st.ncells, sizeof(int), s);
     TSG_LAUNCH(k_nonempty_cells, nblk(k.G, 256), 256, s, (long long)k.G, st.dstart, st.cells_d, st.ncells);
     switch (st.cells_per_cta) {
     case 2: lists_by_cell<DIM, 2>(st, p, s); break;
@@ -2565,7 +2565,7 @@ static void static_active(Fp32State& st, cudaStream_t s) {
 // (the sorted block is copied back), as a captured graph needs fixed pointers.
 // init: the fused init_real2tmp of the step that follows (step_body's inited) goes with the copy.
 void f32::rebuild(Fp32State& st, cudaStream_t s, bool in_place, bool init) {
-    cudaMemsetAsync(st.dcount, 0, sizeof(int) * (st.k.G + 5), s);
+    zero_async(st.dcount, sizeof(int) * (st.k.G + 5), s);
     {
         PhaseScope ph(s, PH_SORT);
         if (st.nd > 0) {
@@ -2575,7 +2575,7 @@ void f32::rebuild(Fp32State& st, cudaStream_t s, bool in_place, bool init) {
             else if (init) TSG_LAUNCH(k_copy_back32<true>, nblk(st.nd), TPB, s, st.k, from, to, st.T);
             else TSG_LAUNCH(k_copy_back32<false>, nblk(st.nd), TPB, s, st.k, from, to, st.T);
         } else {
-            cudaMemsetAsync(st.dstart, 0, sizeof(int) * (st.k.G + 2), s);
+            zero_async(st.dstart, sizeof(int) * (st.k.G + 2), s);
         }
     }
     {
@@ -2975,7 +2975,6 @@ void fold_rebuilds(Fp32State& st, cudaStream_t s) {
     }
 }
 
-// Capture `steps` steps into one executable graph.  Each step: displacement check, then an
 // Whether step_body ends with the fused final update (which folds the new positions into
 // the displacement maximum) and moves no particle after it.
 bool folds_disp(const Fp32State& st, bool collide) {
@@ -2986,90 +2985,78 @@ bool folds_disp(const Fp32State& st, bool collide) {
     return st.k.solver == 1 && st.c.ti != 4 && !st.k.xsph;
 }
 
-// IF node whose body re-sorts in place and rebuilds the lists, then the step body.
-int capture_steps(Fp32State& st, int steps, bool collide, Fp32State::StepGraph& g) {
-    cudaStream_t cs = nullptr, bs = nullptr;
-    if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) return TSG_E_CUDA;
-    if (cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking) != cudaSuccess) { cudaStreamDestroy(cs); return TSG_E_CUDA; }
+// An IF node after what `t` holds; its body graph, or null.
+cudaGraph_t add_if(Tape& t, cudaGraphConditionalHandle hnd) {
+    // (the union inside has no default constructor: zeroed storage, then fields)
+    alignas(cudaGraphNodeParams) unsigned char cp_buf[sizeof(cudaGraphNodeParams)];
+    std::memset(cp_buf, 0, sizeof cp_buf);
+    cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(cp_buf);
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = hnd;
+    cp.conditional.type = cudaGraphCondTypeIf;
+    cp.conditional.size = 1;
+    cudaGraphNode_t node = nullptr;
+    t.added(cudaGraphAddNode(&node, t.graph, t.deps.data(), nullptr, t.deps.size(), &cp), node);
+    return t.ok ? cp.conditional.phGraph_out[0] : nullptr;
+}
+
+// `steps` steps as one executable graph.  Each step: displacement check, then an IF node whose
+// body re-sorts in place and rebuilds the lists, then the step body.
+int make_graph(Fp32State& st, int steps, bool collide, Fp32State::StepGraph& g) {
     const K32& k = st.k;
     const bool valid0 = st.lists_valid;
-    const long long c0 = launch_total();
-    long long body = 0;
-    int rc = 0;
     cudaGraph_t graph = nullptr;
-    if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed) != cudaSuccess) rc = TSG_E_CUDA;
-    for (int q = 0; q < steps && !rc; ++q) {
+    if (cudaGraphCreate(&graph, 0) != cudaSuccess) { cudaGetLastError(); return TSG_E_CUDA; }
+    Tape t(graph);
+    long long body = 0;
+    for (int q = 0; q < steps && t.ok; ++q) {
+        Recording rec(t);
         if (k.disp2_limit <= 0.f) {  // no skin: every step rebuilds, without asking
             const bool init = fuses_eos(st) && st.nd > 0;
-            rebuild(st, cs, true, init);
-            step_body(st, cs, collide, false, init);
+            rebuild(st, nullptr, true, init);
+            step_body(st, nullptr, collide, false, init);
             continue;
         }
-        cudaStreamCaptureStatus status;
-        cudaGraph_t cg = nullptr;
-        if (cudaStreamGetCaptureInfo(cs, &status, nullptr, &cg) != cudaSuccess || !cg) { rc = TSG_E_CUDA; break; }
         cudaGraphConditionalHandle hnd;
-        if (cudaGraphConditionalHandleCreate(&hnd, cg, 0, cudaGraphCondAssignDefault) != cudaSuccess) { rc = TSG_E_CUDA; break; }
+        t.ok = t.ok && cudaGraphConditionalHandleCreate(&hnd, graph, 0, cudaGraphCondAssignDefault) == cudaSuccess;
+        if (!t.ok) break;
         P32& p = st.P[st.cur];
         // after the first step of the graph, the previous step's fused final update has folded
         // its new positions into the displacement maximum already
         if (q == 0 || !folds_disp(st, collide))
-            TSG_LAUNCH(k_disp32, nblk(k.nd), TPB, cs, k, p.hi, p.lo, st.pf, st.maxdisp);
-        TSG_LAUNCH(k_set_rebuild32, 1, 1, cs, hnd, st.maxdisp, k.disp2_limit, st.d_rebuilds);
-        const cudaGraphNode_t* deps = nullptr;
-        size_t ndeps = 0;
-        if (cudaStreamGetCaptureInfo(cs, &status, nullptr, &cg, &deps, nullptr, &ndeps) != cudaSuccess) { rc = TSG_E_CUDA; break; }
-        // (the union inside has no default constructor: zeroed storage, then fields)
-        alignas(cudaGraphNodeParams) unsigned char cp_buf[sizeof(cudaGraphNodeParams)];
-        std::memset(cp_buf, 0, sizeof cp_buf);
-        cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(cp_buf);
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = hnd;
-        cp.conditional.type = cudaGraphCondTypeIf;
-        cp.conditional.size = 1;
-        cudaGraphNode_t node;
-        if (cudaGraphAddNode(&node, cg, deps, nullptr, ndeps, &cp) != cudaSuccess) { rc = TSG_E_CUDA; break; }
-        cudaGraph_t bodyg = cp.conditional.phGraph_out[0];
-        if (cudaStreamUpdateCaptureDependencies(cs, &node, nullptr, 1, cudaStreamSetCaptureDependencies) != cudaSuccess) {
-            rc = TSG_E_CUDA;
-            break;
+            TSG_LAUNCH(k_disp32, nblk(k.nd), TPB, nullptr, k, p.hi, p.lo, st.pf, st.maxdisp);
+        TSG_LAUNCH(k_set_rebuild32, 1, 1, nullptr, hnd, st.maxdisp, k.disp2_limit, st.d_rebuilds);
+        cudaGraph_t bodyg = add_if(t, hnd);
+        if (!bodyg) break;
+        {
+            Tape b(bodyg);
+            Recording in_body(b);
+            rebuild(st, nullptr, true);
+            body = b.kernels;
+            t.ok = t.ok && b.ok;
         }
-        const long long b0 = launch_total();
-        if (cudaStreamBeginCaptureToGraph(bs, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
-            rc = TSG_E_CUDA;
-            break;
-        }
-        rebuild(st, bs, true);
-        cudaGraph_t done = nullptr;
-        if (cudaStreamEndCapture(bs, &done) != cudaSuccess) { rc = TSG_E_CUDA; break; }
-        body = launch_total() - b0;
         // The check above, with its rebuild, leaves valid lists in every replay, whatever a write of
         // x has left behind on the host: step_body decides by the flag what the graph holds.
         st.lists_valid = true;
-        step_body(st, cs, collide, q + 1 < steps && folds_disp(st, collide));
+        step_body(st, nullptr, collide, q + 1 < steps && folds_disp(st, collide));
     }
-    cudaError_t e = cudaStreamEndCapture(cs, &graph);
-    if (!rc && (e != cudaSuccess || !graph)) rc = TSG_E_CUDA;
-    const long long captured = launch_total() - c0;
-    add_launches(-captured);  // nodes, not launches
-    if (!rc) {
+    bool ok = t.ok;
+    if (ok) {
         if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
-        if (cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess) { rc = TSG_E_CUDA; g.exec = nullptr; }
+        if (cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess) { ok = false; g.exec = nullptr; }
     }
-    if (graph) cudaGraphDestroy(graph);
-    cudaStreamDestroy(bs);
-    cudaStreamDestroy(cs);
+    cudaGraphDestroy(graph);
     cudaGetLastError();
-    if (rc) {
+    if (!ok) {
         st.lists_valid = valid0;
-        return rc;
+        return TSG_E_CUDA;
     }
     g.steps = steps;
     g.cur = st.cur;
     g.tpb = st.tpb;
     g.cpc = st.cells_per_cta;
     g.collide = collide;
-    g.kernels = captured - body * steps;
+    g.kernels = t.kernels;
     st.body_kernels = body;
     return 0;
 }
@@ -3080,7 +3067,7 @@ Fp32State::StepGraph* graph_for(Fp32State& st, int steps, bool collide, int* rc)
     if (g.exec && g.steps == steps && g.cur == st.cur && g.tpb == st.tpb && g.cpc == st.cells_per_cta &&
         g.collide == collide)
         return &g;
-    *rc = capture_steps(st, steps, collide, g);
+    *rc = make_graph(st, steps, collide, g);
     return *rc ? nullptr : &g;
 }
 

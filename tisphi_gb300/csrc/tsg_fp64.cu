@@ -1982,27 +1982,20 @@ void fp64_substep(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cuda
 }
 
 void fp64_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, const Rigid64& r, bool collide,
-               cudaStream_t s, const SideStream64* side) {
+               cudaStream_t s) {
     fp64_build_rows(c, p, t, g, true, s);
     // The correction pass over the flow rows and what the first rates loop needs besides (the
     // per-particle start, the boundary rows' Shepard factors and extrapolation) touch different
     // arrays: two branches of the graph (a small scene fills neither the GPU nor a launch's
     // latency with one of them).  mu(I) extrapolates after its stress loop.
     const bool early_bdy = c.solver != 2;
-    cudaStream_t b = s;
-    if (side) {
-        b = side->stream;
-        cudaEventRecord(side->fork, s);
-        cudaStreamWaitEvent(b, side->fork, 0);
-    }
+    Fork branches;
     corr_flow(c, p, t, g, s);
-    particle_pass(c, p, t, g, OP_INIT | substep_head(c), 0, b);
-    corr_bdy(c, p, t, g, b);
-    if (early_bdy) bdy(c, p, t, g, b);
-    if (side) {
-        cudaEventRecord(side->join, b);
-        cudaStreamWaitEvent(s, side->join, 0);
-    }
+    branches.second();
+    particle_pass(c, p, t, g, OP_INIT | substep_head(c), 0, s);
+    corr_bdy(c, p, t, g, s);
+    if (early_bdy) bdy(c, p, t, g, s);
+    branches.join();
     substep_loops(c, p, t, g, c.xsph ? 0u : OP_POS | OP_POST, !early_bdy, s);
     if (c.xsph) {
         xsph(c, p, t, g, s);

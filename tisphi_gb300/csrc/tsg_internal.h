@@ -2,23 +2,71 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <tuple>
+#include <utility>
+#include <vector>
 
 #include "../../include/tisphi_gb300.h"
 
 namespace tsg {
 
 // Host-side count of kernel launches issued by this library (all handles).  Graph replays
-// add their kernel-node counts through add_launches; launches recorded while a stream is
-// being captured are taken back out (they are nodes, not launches).
+// add their kernel-node counts through add_launches.
 void note_launch();
 void add_launches(long long delta);
 long long launch_total();
 // True while tsg_profile is on (steps then run eagerly, with per-phase events).
 bool profiling_on();
-#define TSG_LAUNCH(kernel, grid, block, stream, ...)                   \
-    do {                                                                \
-        ::tsg::note_launch();                                           \
-        kernel<<<(grid), (block), 0, (stream)>>>(__VA_ARGS__);          \
+
+// A graph under construction on the calling thread: while one is set (Recording), launches and
+// copies are added to it as nodes, each after the one before, instead of going to their stream.
+// Not a stream capture: while one is open anywhere in the process, a device-wide
+// synchronisation on any other thread fails and breaks the capture, and what the capturing
+// thread launches after that runs at once.
+struct Tape {
+    cudaGraph_t graph;
+    std::vector<cudaGraphNode_t> deps;  // what the next node waits for
+    long long kernels = 0;
+    bool ok = true;
+    explicit Tape(cudaGraph_t g) : graph(g) {}
+    template <class... P, class... A>
+    void launch(void (*f)(P...), dim3 grid, dim3 block, A&&... a) {
+        std::tuple<P...> v(std::forward<A>(a)...);
+        std::apply([&](auto&... x) {
+            void* args[] = {&x...};
+            node(reinterpret_cast<void*>(f), grid, block, args);
+        }, v);
+    }
+    void node(void* f, dim3 grid, dim3 block, void** args);
+    void zero(void* p, size_t bytes);
+    void copy(void* dst, const void* src, size_t bytes);
+    void added(cudaError_t e, cudaGraphNode_t n);
+};
+Tape*& tape();
+struct Recording {
+    Tape* outer;
+    explicit Recording(Tape& t) : outer(tape()) { tape() = &t; }
+    ~Recording() { tape() = outer; }
+};
+// Two branches of a graph from here on; launched eagerly, one after the other.
+struct Fork {
+    std::vector<cudaGraphNode_t> from, first;
+    Fork() { if (tape()) from = tape()->deps; }
+    void second() { if (tape()) { first = tape()->deps; tape()->deps = from; } }
+    void join();
+};
+// Device memory set to zero, or copied on the device, in stream order.
+void zero_async(void* p, size_t bytes, cudaStream_t s);
+void copy_async(void* dst, const void* src, size_t bytes, cudaStream_t s);
+
+#define TSG_LAUNCH(kernel, grid, block, stream, ...)                       \
+    do {                                                                    \
+        if (::tsg::Tape* tape_ = ::tsg::tape()) {                           \
+            tape_->launch(kernel, dim3(grid), dim3(block), __VA_ARGS__);    \
+        } else {                                                            \
+            ::tsg::note_launch();                                           \
+            kernel<<<(grid), (block), 0, (stream)>>>(__VA_ARGS__);          \
+        }                                                                   \
     } while (0)
 
 // Phase profiling: when enabled, every launcher brackets its kernels with CUDA events
@@ -205,10 +253,9 @@ void fp64_init_tmp(const Consts& c, const Persist64& p, Trans64& t, const Grid& 
 void fp64_one_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
 // substep (its integrator's loops and updates) on current rows and geometry.
 void fp64_substep(const Consts& c, Persist64& p, Trans64& t, const Grid& g, cudaStream_t s);
-// A step after its sort.  side: a second stream and two events while capturing, else null.
-struct SideStream64 { cudaStream_t stream; cudaEvent_t fork, join; };
+// A step after its sort.
 void fp64_step(const Consts& c, Persist64& p, Trans64& t, const Grid& g, const Rigid64& r, bool collide,
-               cudaStream_t s, const SideStream64* side);
+               cudaStream_t s);
 void fp64_advect(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int which, cudaStream_t s);
 void fp64_rk_update(const Consts& c, Persist64& p, Trans64& t, const Grid& g, int m, cudaStream_t s);
 void fp64_neighbors(const Consts& c, const Persist64& p, const Trans64& t, const Grid& g,

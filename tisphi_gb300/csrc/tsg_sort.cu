@@ -297,7 +297,7 @@ void sort_cells(int n, int nbins, const int* count, int* cell_start, int* tile_s
 void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid& g, cudaStream_t s) {
     PhaseScope ph(s, PH_SORT);
     const long long nbins = c.G + 1;
-    cudaMemsetAsync(g.count, 0, g.zero_bytes, s);
+    zero_async(g.count, g.zero_bytes, s);
     TSG_LAUNCH(k_hash, nblk(c.n), TPB, s, c, cur.x, g.cell_of, g.rank, g.count, g.cell0_old, g.err);
     sort_cells(c.n, (int)nbins, g.count, g.cell_start, g.tile_sum, g.cell_of, g.rank, g.perm, g.big, g.nbig, s);
     const int small = sort_small(c.n);
@@ -310,7 +310,7 @@ void sort_fp64(const Consts& c, Persist64& cur, Persist64& nxt, Trans64& t, Grid
         // mu(I) keeps v_tmp across steps: stage it in aux3 (free until advect_pos) and gather
         const double* src = nullptr;
         if (c.solver == 2) {
-            cudaMemcpyAsync(t.aux3, t.v_tmp, sizeof(double) * 3 * (size_t)c.n, cudaMemcpyDeviceToDevice, s);
+            copy_async(t.aux3, t.v_tmp, sizeof(double) * 3 * (size_t)c.n, s);
             src = t.aux3;
         }
         TSG_LAUNCH(k_reorder64<true>, nb, tpb, s, c, g.perm, cur, nxt, t.pos32, t.pos32l, g.cell_of, g.cell_start, small, g.cell0_old,
