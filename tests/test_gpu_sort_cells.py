@@ -1,9 +1,11 @@
 """Order and cost of the sort where one cell holds most of the particles.
 
 Up to 16,384 particles the reorder pass ranks every cell itself, whatever its size; the
-out-of-grid bin of a run that has blown up then holds thousands.  The order is the stable
-counting sort's (eng/particle_system.py:228-257) for any start and length of the cell, and the
-sort of such a scene stays within a few times that of a healthy one.
+out-of-grid bin of a run that has blown up then holds thousands.  Above that, cells of more than
+256 particles are listed and ordered by a block each: in shared memory up to 4,096 particles, by a
+scan over all particles above.  The order is the stable counting sort's
+(eng/particle_system.py:228-257) for any start and length of the cell, and the sort of a blown-up
+scene stays within a few times that of a healthy one.
 """
 import contextlib
 import ctypes
@@ -49,6 +51,21 @@ def test_order_in_one_large_cell(native, precision, count):
     ids = ps.field("id0").cpu().numpy()
     end = ids.size if precision == "fp64" else fl.size  # FP32-mixed: the bin ends the fluid's block
     np.testing.assert_array_equal(ids[end - count:end], before[moved])
+
+
+# (256 / 257: ranked / listed; 4,096 / 4,097: shared memory / scan)
+@pytest.mark.parametrize("precision", ["fp64", "fp32_mixed"])
+@pytest.mark.parametrize("count", [256, 257, 1000, 4096, 4097, 20000])
+def test_order_in_listed_cells(native, precision, count):
+    sim, fl, moved = _moved(precision, 0.003, count)
+    ps = sim.ps
+    assert fl.size > 16384  # the FP32-mixed form sorts the fluid by itself
+    before = ps.field("id0").cpu().numpy().copy()
+    _sort(ps)
+    ids = ps.field("id0").cpu().numpy()
+    end = ids.size if precision == "fp64" else fl.size
+    np.testing.assert_array_equal(ids[end - count:end], before[moved])
+    assert np.array_equal(np.sort(ids), np.arange(ids.size))
 
 
 def _sort_ms(lib, ps, reps=20):
