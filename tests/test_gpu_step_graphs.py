@@ -1,4 +1,4 @@
-"""Captured steps: what tsg_get_launch says of them, what they hold, and how they are counted."""
+"""Step graphs: what tsg_get_launch says of them, what they hold, and how they are counted."""
 import ctypes
 import threading
 
@@ -142,3 +142,47 @@ def test_graphs_made_while_another_thread_synchronises(native, precision, method
     t.join()
     assert not failed and waits[0] > 10
     assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+FIELDS = ["x", "v", "density", "pressure", "id0"]
+
+
+@pytest.mark.parametrize("precision,method", [(p, m) for p in ("fp64", "fp32_mixed") for m in (1, 2, 3)])
+@pytest.mark.parametrize("warm", [12, 13])
+def test_parameter_changes_reach_the_graphs(native, precision, method, warm):
+    """Graphs hold the constants by value.  After enough steps for every length of graph, from
+    either buffer of the FP64 sort, a changed parameter gives what steps launched one by one with
+    it give, bit for bit, and not what the old one gives."""
+    from tisphi_gb300.simulation import Simulation
+    lib = native
+
+    def sim():
+        return Simulation(cfg_of(small_dambreak_2d() if method == 1 else small_column(method)), precision=precision)
+
+    def change(s):
+        if method == 1:
+            s.solver.stiffness = 6.0e4
+        elif method == 2:
+            s.solver.mu = 0.5
+        else:
+            s.solver.coh = 500.0
+            s.solver.fric = 0.3
+
+    names = FIELDS + (["stress"] if method != 1 else [])
+    graphs, eager, old = sim(), sim(), sim()
+    for s in (graphs, eager, old):
+        s.solver.step(warm)
+        s.solver.step(1)  # (both lengths of graph)
+    for s in (graphs, eager):
+        change(s)
+    for n in (1, 2, 6):
+        graphs.solver.step(n)
+        old.solver.step(n)
+        lib.tsg_profile(1)
+        try:
+            eager.solver.step(n)
+        finally:
+            lib.tsg_profile(0)
+        for nm in names:
+            assert torch.equal(graphs.ps.field(nm), eager.ps.field(nm)), nm
+    assert not torch.equal(graphs.ps.field("v"), old.ps.field("v"))
