@@ -186,3 +186,55 @@ def test_parameter_changes_reach_the_graphs(native, precision, method, warm):
         for nm in names:
             assert torch.equal(graphs.ps.field(nm), eager.ps.field(nm)), nm
     assert not torch.equal(graphs.ps.field("v"), old.ps.field("v"))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_mixed"])
+def test_steps_while_another_thread_captures(native, precision):
+    """A thread that captures a graph of its own in the default mode, which forbids every other
+    thread what may touch the capture, while steps make, replay and drop theirs: neither notices."""
+    from tisphi_gb300.simulation import Simulation
+
+    def run(sim):
+        for n in (1, 1, 2, 1, 5, 6, 12, 5):
+            sim.solver.step(n)
+        sim.solver.viscosity = 0.006
+        sim.solver.step(4)
+
+    a, b = (Simulation(cfg_of(small_dambreak_2d()), precision=precision) for _ in range(2))
+    run(a)
+    x = torch.ones(1000, device="cuda")
+    y = torch.empty_like(x)
+    torch.cuda.synchronize()
+    inside, stepped, got = threading.Event(), threading.Event(), []
+
+    def capture():
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                g = torch.cuda.CUDAGraph()
+                g.capture_begin()
+                torch.mul(x, 2, out=y)
+                inside.set()
+                stepped.wait(60)
+                torch.add(y, 1, out=y)
+                g.capture_end()
+                g.replay()
+                torch.cuda.current_stream().synchronize()
+                got.append(float(y[0]))
+        except RuntimeError as e:
+            got.append(e)
+        finally:
+            inside.set()
+
+    t = threading.Thread(target=capture)
+    t.start()
+    inside.wait(60)
+    try:
+        with torch.cuda.stream(torch.cuda.Stream()):
+            run(b)
+    finally:
+        stepped.set()
+        t.join()
+    torch.cuda.synchronize()
+    assert got == [3.0]
+    for nm in ("x", "v", "density", "id0"):
+        assert torch.equal(a.ps.field(nm), b.ps.field(nm)), nm

@@ -344,6 +344,7 @@ int step64(tsg_handle* h, bool collide, cudaStream_t s) {
 }
 
 void drop_graphs64(tsg_handle* h) {
+    RelaxedCapture relaxed;
     for (auto& side : h->graphs)
         for (auto& g : side) {
             if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -393,6 +394,7 @@ bool capturing(cudaStream_t s) {
 // not pay for a graph), as do profiled steps and steps inside a caller's own capture.
 int steps64(tsg_handle* h, int nsteps, bool collide, cudaStream_t s) {
     bool graphs = !h->no_graphs && !profiling_on() && !capturing(s);
+    RelaxedCapture relaxed;
     while (nsteps > 0) {
         if (graphs && h->eager_steps >= 2) {
             const int take = nsteps >= 2 ? 2 : 1;

@@ -3086,6 +3086,7 @@ static int graph_length(const Fp32State& st) {
 
 int fp32_step_graph(Fp32State& st, int nsteps, bool collide, cudaStream_t s) {
     if (profiling_on()) return TSG_E_STATE;  // per-phase events need the eager path
+    RelaxedCapture relaxed;
     const bool always = st.k.disp2_limit <= 0.f;  // the graphs rebuild in every step
     if (!st.built && !always) fp32_sort(st, s);
     const int K = graph_length(st);
@@ -3271,6 +3272,7 @@ int fp32_snapshot_copy(Fp32State& st, void* buf, bool load, cudaStream_t s) {
 // graphs: a caller that changes a parameter every few steps would otherwise capture a five-step
 // graph each time (set_fluid + 5 steps, 1,038 particles: 505 us against 420).
 static void drop_graphs(Fp32State& st) {
+    RelaxedCapture relaxed;
     for (auto& g : st.graphs)
         if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
     st.graph_steps = 0;

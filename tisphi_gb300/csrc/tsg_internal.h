@@ -55,6 +55,15 @@ struct Fork {
     void second() { if (tape()) { first = tape()->deps; tape()->deps = from; } }
     void join();
 };
+// While it lives, this thread may make, launch and destroy graphs although another thread
+// captures a stream in the default (global) mode; without it the first such call fails and breaks
+// that capture.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+};
 // Device memory set to zero, or copied on the device, in stream order.
 void zero_async(void* p, size_t bytes, cudaStream_t s);
 void copy_async(void* dst, const void* src, size_t bytes, cudaStream_t s);
