@@ -1151,8 +1151,9 @@ __device__ __forceinline__ void mui_stress_pass(const K32& k, const P32& p, cons
     });
 }
 template <int DIM, bool CORR>
-__global__ void k_mui_stress32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
-                               const int* __restrict__ sstart, Ovf ovf) {
+__global__ void __maxnreg__(DIM == 3 ? 64 : 56)
+k_mui_stress32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+               const int* __restrict__ sstart, Ovf ovf) {
     if ((int)blockIdx.x < ovf.first) mui_stress_pass<DIM, false, CORR>(k, p, t, PF, dstart, sstart, ovf);
     else mui_stress_pass<DIM, true, CORR>(k, p, t, PF, dstart, sstart, ovf);
 }
