@@ -1150,12 +1150,21 @@ __device__ __forceinline__ void mui_stress_pass(const K32& k, const P32& p, cons
       }
     });
 }
-template <int DIM, bool CORR>
-__global__ void __maxnreg__(DIM == 3 ? 64 : 56)
-k_mui_stress32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
-               const int* __restrict__ sstart, Ovf ovf) {
-    if ((int)blockIdx.x < ovf.first) mui_stress_pass<DIM, false, CORR>(k, p, t, PF, dstart, sstart, ovf);
-    else mui_stress_pass<DIM, true, CORR>(k, p, t, PF, dstart, sstart, ovf);
+// (3D: with the overflow pass in the launch the compiler takes 72 registers with CSPM, one block
+// less an SM; 119,000 soil particles 132 us, held to the main pass's 64 92 us.  2D: it takes 56 by
+// itself and is faster left to it than held to them.)
+template <bool CORR>
+__global__ void k_mui_stress32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+                               const int* __restrict__ sstart, Ovf ovf) {
+    if ((int)blockIdx.x < ovf.first) mui_stress_pass<2, false, CORR>(k, p, t, PF, dstart, sstart, ovf);
+    else mui_stress_pass<2, true, CORR>(k, p, t, PF, dstart, sstart, ovf);
+}
+template <bool CORR>
+__global__ void __maxnreg__(64)
+k_mui_stress32_3d(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
+                  const int* __restrict__ sstart, Ovf ovf) {
+    if ((int)blockIdx.x < ovf.first) mui_stress_pass<3, false, CORR>(k, p, t, PF, dstart, sstart, ovf);
+    else mui_stress_pass<3, true, CORR>(k, p, t, PF, dstart, sstart, ovf);
 }
 
 // Boundary extrapolation for the granular solvers (eng/solver_sph_muI.py:97-109,
@@ -2724,10 +2733,11 @@ void soil_one_step(Fp32State& st, cudaStream_t s) {
     {
         PhaseScope ph(s, PH_PRE);
         if (k.solver == 2) {
-            if (k.corr)
-                TSG_LAUNCH((k_mui_stress32<DIM, true>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf);
-            else
-                TSG_LAUNCH((k_mui_stress32<DIM, false>), q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf);
+            const auto launch = [&](auto* f) {
+                TSG_LAUNCH(f, q.grid, q.tpb, s, k, p, st.T, st.pf, st.dstart, st.sstart, q.ovf);
+            };
+            if (DIM == 3) launch(k.corr ? k_mui_stress32_3d<true> : k_mui_stress32_3d<false>);
+            else launch(k.corr ? k_mui_stress32<true> : k_mui_stress32<false>);
         } else {
             TSG_LAUNCH(k_pre_dp32, nblk(k.nd), TPB, s, k, p, st.T);
         }
