@@ -360,6 +360,7 @@ void drop_graphs64(tsg_handle* h) {
 tsg_handle::StepGraph* step_graph64(tsg_handle* h, int steps, bool collide) {
     tsg_handle::StepGraph& g = h->graphs[h->cur.x == h->x_first ? 0 : 1][steps - 1];
     if (g.exec && g.collide == collide) return &g;
+    RelaxedCapture relaxed;
     if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
     const Persist64 cur = h->cur, nxt = h->nxt;
     cudaGraph_t graph = nullptr;
@@ -394,7 +395,6 @@ bool capturing(cudaStream_t s) {
 // not pay for a graph), as do profiled steps and steps inside a caller's own capture.
 int steps64(tsg_handle* h, int nsteps, bool collide, cudaStream_t s) {
     bool graphs = !h->no_graphs && !profiling_on() && !capturing(s);
-    RelaxedCapture relaxed;
     while (nsteps > 0) {
         if (graphs && h->eager_steps >= 2) {
             const int take = nsteps >= 2 ? 2 : 1;

@@ -3016,6 +3016,7 @@ cudaGraph_t add_if(Tape& t, cudaGraphConditionalHandle hnd) {
 int make_graph(Fp32State& st, int steps, bool collide, Fp32State::StepGraph& g) {
     const K32& k = st.k;
     const bool valid0 = st.lists_valid;
+    RelaxedCapture relaxed;
     cudaGraph_t graph = nullptr;
     if (cudaGraphCreate(&graph, 0) != cudaSuccess) { cudaGetLastError(); return TSG_E_CUDA; }
     Tape t(graph);
@@ -3097,7 +3098,6 @@ static int graph_length(const Fp32State& st) {
 
 int fp32_step_graph(Fp32State& st, int nsteps, bool collide, cudaStream_t s) {
     if (profiling_on()) return TSG_E_STATE;  // per-phase events need the eager path
-    RelaxedCapture relaxed;
     const bool always = st.k.disp2_limit <= 0.f;  // the graphs rebuild in every step
     if (!st.built && !always) fp32_sort(st, s);
     const int K = graph_length(st);

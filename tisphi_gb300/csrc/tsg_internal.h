@@ -55,7 +55,7 @@ struct Fork {
     void second() { if (tape()) { first = tape()->deps; tape()->deps = from; } }
     void join();
 };
-// While it lives, this thread may make, launch and destroy graphs although another thread
+// While it lives, this thread may make and destroy graphs although another thread
 // captures a stream in the default (global) mode; without it the first such call fails and breaks
 // that capture.
 struct RelaxedCapture {
