@@ -2644,15 +2644,23 @@ bool fp32_rebuild_due(Fp32State& st, cudaStream_t s) {
 // skip_fluid: the first rates pass computes the fluid's factors; when the dynamic block holds
 // fluid only, the main pass then visits the listed static particles alone.  skip_static:
 // the first boundary pass computes the static block's Shepard factors.
-// (Where the overflow pass takes more registers than the main pass, the kernel is held to the
-// main pass's.)
+// Where the overflow pass takes more registers than the main pass, the kernel is held to the main
+// pass's; the overflow pass then spills a little (-Xptxas -v: 16 to 84 bytes in 3D).
 struct Passes {
     Ovf ovf;
     int grid, tpb;
 };
-// main_blocks of the main pass over n particles, then 16,384 threads at most for the overflow pass.
+// main_blocks of the main pass over n particles, then kOvfBlocks x TPB threads at most for the
+// overflow pass.  As the last blocks of a launch its blocks do not spread over the SMs as evenly as
+// a launch of their own did, and in some passes the traversal spills at the main pass's registers:
+// 64 blocks took up to 12 % longer than that launch, 96 take less (us a step with launches of their
+// own / 64 / 96 blocks: mu(I) in 3D with CSPM, 75,454 overflowed lists, 21,600 / 22,700 / 16,900;
+// Drucker-Prager likewise with XSPH 30,000 / 32,000 / 23,500; 2D dambreak with CSPM and XSPH,
+// 22,600 lists, 970 / 1,070 / 773); 152 cost a step without any 0.3 %, 96 nothing measurable.
+constexpr int kOvfBlocks = 96;
 Passes passes(const Fp32State& st, int main_blocks, int n) {
-    return {{st.ovf_list, st.novf, main_blocks}, main_blocks + nblk(std::min(std::max(n, 1), 64 * TPB), st.tpb), st.tpb};
+    return {{st.ovf_list, st.novf, main_blocks},
+            main_blocks + nblk(std::min(std::max(n, 1), kOvfBlocks * TPB), st.tpb), st.tpb};
 }
 
 template <int DIM>
