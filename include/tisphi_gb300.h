@@ -293,7 +293,7 @@ int tsg_sort_noalloc(const tsg_config* cfg, const double* x, int64_t n, int32_t*
 /* Launch configuration of the FP32-mixed form.  No reference counterpart (Taichi picks
  * its own launch shapes): threads_per_block of the neighbour-traversal kernels (64, 128,
  * 256); cells_per_cta of the neighbour-list build, one warp per cell (2, 4, 8; 0 = one
- * thread per particle); steps_per_graph, how many steps one captured CUDA graph replays
+ * thread per particle); steps_per_graph, how many steps one CUDA graph replays
  * (1..64; until tsg_set_launch or tsg_autotune chooses it, 1 for the first ten steps after
  * the upload or a tsg_set_fluid / tsg_set_soil and 5 from then on, which tsg_get_launch
  * reports as it stands).  tsg_step runs FP32-mixed

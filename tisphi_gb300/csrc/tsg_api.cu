@@ -761,7 +761,7 @@ int tsg_step(tsg_handle* h, int nsteps, void* stream) {
     if (!h || !h->uploaded) return TSG_E_STATE;
     if (nsteps < 0) return TSG_E_ARG;
     const bool collide = h->c.boundary == 1;
-    // FP32-mixed: replay captured step graphs (no host round trip per step) unless per-phase
+    // FP32-mixed: replay step graphs (no host round trip per step) unless per-phase
     // profiling wants its events, which the eager path below records
     if (use_fp32(h) && !profiling_on() && nsteps > 0) {
         int rc = fp32_step_graph(*h->f32, nsteps, collide, S(stream));
@@ -770,7 +770,7 @@ int tsg_step(tsg_handle* h, int nsteps, void* stream) {
         return check_cuda();
     }
     if (!use_fp32(h)) return steps64(h, nsteps, collide, S(stream));
-    for (int k = 0; k < nsteps; ++k) {  // FP32-mixed, profiled: what the captured graphs replay, eagerly
+    for (int k = 0; k < nsteps; ++k) {  // FP32-mixed, profiled: what the step graphs replay, eagerly
         int rc;
         // with a neighbour skin the particles are re-sorted only when the lists expire
         if (fp32_rebuild_due(*h->f32, S(stream)))

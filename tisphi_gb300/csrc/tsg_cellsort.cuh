@@ -3,10 +3,10 @@
 // places a cell's particles in atomic arrival order).
 //
 // Ordinary cells hold a few dozen particles, and the reorder passes rank each particle among its
-// cell's themselves (tsg_cellrank.cuh).  For a segment above kSortSmall - the out-of-grid bin after particles left
-// the grid, or a very coarse grid - that would be quadratic (a blown-up run with every particle
-// out of the grid would keep the GPU busy for hours), so the scatter lists such cells and
-// k_cell_sort_big sorts them first, one block per cell: up to kSortMid particles by a bitonic
+// cell's themselves (tsg_cellrank.cuh).  In scenes above kSortAll particles a segment above
+// kSortSmall - the out-of-grid bin after particles left the grid, or a very coarse grid - is listed
+// by the scatter (every warp of the reorder reading all of it would be quadratic) and sorted by
+// k_cell_sort_big first, one block per cell: up to kSortMid particles by a bitonic
 // sort in shared memory, above that rebuilt in ascending order from a block-wide scan over every
 // particle of the flag "cell_of[i] == c" (n / 256 trips; at most n / kSortMid cells are that
 // large).  Both paths give the same order.

@@ -1683,7 +1683,7 @@ __device__ __forceinline__ float4 advect_final_one(const K32& k, P32& p, T32& t,
 // multiply-adds here and there, so the compiler's contraction choices cannot make the two
 // paths round differently.  maxd (may be null): the largest squared displacement since the
 // list build is folded in from the new positions, as the next step's list-expiry check
-// would compute it (a captured multi-step graph drops that check after its first step
+// would compute it (a multi-step graph drops that check after its first step
 // and has the steps before the last fold their positions in).
 __global__ void k_advect_final_wc32(K32 k, P32 p, T32 t, int* err, const float4* __restrict__ PF,
                                     unsigned* __restrict__ maxd) {
@@ -2572,7 +2572,7 @@ static void static_active(Fp32State& st, cudaStream_t s) {
 }
 
 // Re-sort the dynamic block and rebuild every list.  in_place keeps the current buffer
-// (the sorted block is copied back), as a captured graph needs fixed pointers.
+// (the sorted block is copied back), as a graph needs fixed pointers.
 // init: the fused init_real2tmp of the step that follows (step_body's inited) goes with the copy.
 void f32::rebuild(Fp32State& st, cudaStream_t s, bool in_place, bool init) {
     zero_async(st.dcount, sizeof(int) * (st.k.G + 5), s);
@@ -2882,7 +2882,7 @@ void fp32_rk_update(Fp32State& st, int m, cudaStream_t s) {
     TSG_LAUNCH(k_rk_update32, nblk(st.k.nd), TPB, s, st.k, st.P[st.cur], st.T, (float)m);
 }
 
-// ---------------------------------------------------------------- captured steps
+// ---------------------------------------------------------------- step graphs
 // WCSPH with symplectic Euler or leap-frog: the fluid EOS (first phase of each one_step)
 // runs inside init_real2tmp and the half step, which produce its input density_tmp.
 static bool fuses_eos(const Fp32State& st) { return st.k.solver == 1 && st.c.ti != 4; }
@@ -2891,7 +2891,7 @@ static bool fuses_eos(const Fp32State& st) { return st.k.solver == 1 && st.c.ti 
 // the integrator's one_step / advect sequence, advect_pos, advect_something and, in
 // collision mode, enforce_boundary (eng/solver_sph_base.py:41-61, :79-120).
 // fold_disp: the fused final update folds the new positions into the displacement maximum
-// (the next step, captured in the same graph, skips its list-expiry check).
+// (the next step of the same graph skips its list-expiry check).
 // inited: the rebuild before has run the fused init_real2tmp (fuses_eos).
 void f32::step_body(Fp32State& st, cudaStream_t s, bool collide, bool fold_disp, bool inited) {
     const bool fuse = fuses_eos(st);
@@ -3098,7 +3098,7 @@ constexpr int kWarmSteps = 10;
 // Steps of the graph that the next tsg_step replays where it has that many to run.  Without a
 // caller's choice: single-step graphs at first, then graphs of five, which check the list expiry
 // once (10 steps: batch of 64 scenes 1,356 -> 1,272 us, 3D benchmark 9,413 -> 9,183) and cost a
-// few hundred microseconds to capture.
+// few hundred microseconds to make.
 static int graph_length(const Fp32State& st) {
     if (!st.graph_chosen && st.graph_steps >= kWarmSteps) return 5;
     return st.steps_per_graph > 1 ? st.steps_per_graph : 1;
@@ -3238,7 +3238,7 @@ int snapshot(Fp32State& st, cudaStream_t s, bool restore) {
 float time_steps(Fp32State& st, int steps, bool collide, cudaStream_t s, int* rc) {
     snapshot(st, s, true);
     rebuild(st, s, true);
-    *rc = fp32_step_graph(st, 1, collide, s);  // captures the graphs outside the timed region
+    *rc = fp32_step_graph(st, 1, collide, s);  // makes the graphs outside the timed region
     if (st.steps_per_graph > 1 && !*rc) *rc = fp32_step_graph(st, st.steps_per_graph, collide, s);
     if (*rc) return 1e30f;
     cudaEvent_t a, b;
@@ -3287,8 +3287,8 @@ int fp32_snapshot_copy(Fp32State& st, void* buf, bool load, cudaStream_t s) {
     return cudaGetLastError() == cudaSuccess ? 0 : TSG_E_CUDA;
 }
 
-// The captured launches hold the constants by value.  The handle starts over with single-step
-// graphs: a caller that changes a parameter every few steps would otherwise capture a five-step
+// The graphs hold the constants by value.  The handle starts over with single-step
+// graphs: a caller that changes a parameter every few steps would otherwise make a five-step
 // graph each time (set_fluid + 5 steps, 1,038 particles: 505 us against 420).
 static void drop_graphs(Fp32State& st) {
     RelaxedCapture relaxed;

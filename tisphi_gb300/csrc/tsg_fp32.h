@@ -29,7 +29,7 @@ void fp32_destroy(Fp32State* st);
 void fp32_sort(Fp32State& st, cudaStream_t s);
 // True when the neighbour lists must be rebuilt before the next step (always without a skin).
 bool fp32_rebuild_due(Fp32State& st, cudaStream_t s);
-// One step of the FP32-mixed sequence the captured graphs replay (kernel correction through
+// One step of the FP32-mixed sequence the step graphs replay (kernel correction through
 // advect_something), launched eagerly; the caller re-sorts first when lists expire.
 void fp32_step_body(Fp32State& st, bool collide, cudaStream_t s);
 void fp32_kernel_corr(Fp32State& st, cudaStream_t s);
@@ -47,7 +47,7 @@ int* fp32_err_ptr(Fp32State& st);
 // particles, out[3] list builds since creation.
 int fp32_list_stats(Fp32State& st, int64_t* out5, cudaStream_t s);
 
-// Graph mode: nsteps full steps replayed from captured graphs (the re-sort runs inside the
+// Graph mode: nsteps full steps replayed from graphs (the re-sort runs inside the
 // graph when the device-side displacement check asks for it).  TSG_E_STATE while
 // per-phase profiling is on.
 int fp32_step_graph(Fp32State& st, int nsteps, bool collide, cudaStream_t s);
@@ -63,7 +63,7 @@ int fp32_autotune(Fp32State& st, int trial_steps, bool collide, cudaStream_t s, 
 size_t fp32_snapshot_bytes(Fp32State& st);
 int fp32_snapshot_copy(Fp32State& st, void* buf, bool load, cudaStream_t s);
 // Replace the granular material constants (mu(I): tan(friction), cohesion; Drucker-Prager:
-// the yield-surface constants) of a created state; captured graphs are dropped.
+// the yield-surface constants) of a created state; step graphs are dropped.
 void fp32_set_soil(Fp32State& st, const Consts& c);
 void fp32_set_fluid(Fp32State& st, const Consts& c);
 // Adjoint of one mu(I) symplectic-Euler step from the loaded state (tsg_adjoint.cu).

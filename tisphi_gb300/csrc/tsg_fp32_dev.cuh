@@ -675,12 +675,12 @@ struct Fp32State {
     int nscenes = 0;               // > 0 for a batched ensemble
     // launch configuration (tsg_set_launch / tsg_autotune): threads per block of the
     // neighbour kernels, cells per CTA of the warp-per-cell list build (0: one thread per
-    // particle), steps per captured graph
+    // particle), steps per graph
     int tpb = 128, cells_per_cta = 4, steps_per_graph = 1;
     bool graph_chosen = false;  // steps_per_graph set by the caller or by tuning
     int graph_steps = 0;        // steps run by graphs since the constants last changed (counted up to
                                 // the switch to longer ones)
-    // captured step graphs: [0] one step, [1] steps_per_graph steps
+    // step graphs: [0] one step, [1] steps_per_graph steps
     struct StepGraph {
         cudaGraphExec_t exec = nullptr;
         int steps = 0, cur = -1, tpb = 0, cpc = 0;

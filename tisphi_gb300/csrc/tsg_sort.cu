@@ -10,8 +10,10 @@
 //   scan        exclusive prefix sum of the G + 1 counts (the extra bin collects
 //               particles whose flattened index falls outside [0, G));
 //   k_scatter   perm[cell_start + rank] = old index (unstable inside a cell);
-//   k_cell_sort_big (tsg_cellsort.cuh) orders cells above kSortSmall by old index;
-//   k_reorder64 ranks the others' particles by old index (stable result), gathers every persistent field into the other buffer set, writes the f32
+//   k_cell_sort_big (tsg_cellsort.cuh) orders cells above kSortSmall by old index in scenes
+//               above kSortAll particles;
+//   k_reorder64 ranks the others' particles by old index (tsg_cellrank.cuh; stable result),
+//               gathers every persistent field into the other buffer set, writes the f32
 //               prefilter positions and the flow / boundary index lists.
 // Compiled with -fmad=false: the f64 cell arithmetic must round exactly like the oracle's.
 #include <cstdio>
