@@ -122,12 +122,8 @@ struct Consts {
     int n_rigid_dyn;    // dynamic rigid particles (shape-matched bodies)
 };
 
-// Dynamic rigid bodies (eng/solver_sph_base.py:467-518): object ids, rest centres of mass
-// (from the uploaded positions, in upload order) and, per object, the slice of `list`
-// that the list builder (tsg_rigid_list.cuh) fills with the object's particles in
-// ascending order before every shape matching.
-// Largest cell segment whose particles the reorder passes rank among themselves
-// (tsg_cellsort.cuh), and the size of the list of larger cells (at most n / (kSortSmall + 1) of them).
+// Largest cell segment whose particles the reorder passes rank among themselves in scenes above
+// kSortAll particles (larger ones: tsg_cellsort.cuh), and the size of the list of larger cells (at most n / (kSortSmall + 1) of them).
 constexpr int kSortSmall = 256;
 // Up to this many particles the reorder pass ranks every cell itself, however large
 // (rank_in_cell), and the launch that orders the larger cells is left out.
@@ -140,6 +136,10 @@ constexpr int kRListBlock = 256;
 inline int rlist_blocks(int n) { return (n + kRListBlock - 1) / kRListBlock; }
 inline size_t rlist_scratch_ints(int n, int nobj) { return (size_t)nobj * (size_t)rlist_blocks(n); }
 
+// Dynamic rigid bodies (eng/solver_sph_base.py:467-518): object ids, rest centres of mass
+// (from the uploaded positions, in upload order) and, per object, the slice of `list`
+// that the list builder (tsg_rigid_list.cuh) fills with the object's particles in
+// ascending order before every shape matching.
 struct Rigid64 {
     int nobj = 0;
     int* obj_id = nullptr;      // nobj (device)
