@@ -40,3 +40,36 @@ def test_out_of_plane_shears_are_positive_zeros(native):
     assert np.any(st[:, 0, 0] < 0)  # compressed, where 0 times xx is -0
     for a, b in ((0, 2), (1, 2), (2, 0), (2, 1)):
         assert not st[:, a, b].any() and not np.signbit(st[:, a, b]).any()
+
+
+def _column_3d():
+    d = small_column(2, spacing=0.008, width=0.1, height=0.05, domain=(0.2, 0.08))
+    d["Configuration"]["is2D"] = False
+    d["Configuration"]["domainEnd"] = [0.2, 0.08, 0.048]
+    d["Blocks"][0]["size"] = [0.1, 0.05, 0.048]
+    return d
+
+
+@pytest.mark.parametrize("skin", [0.05, 1e-6, 0.0])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_steps_by_lists_and_by_enumeration(oracle_lib, native, dim, skin):
+    """The neighbours from the lists; from the cells because every particle has moved too far for a
+    tiny skin; and from the cells because there is no skin: the oracle's stress at the bound of the
+    granular columns, 1e-4 of the largest entry."""
+    from tisphi_gb300.simulation import Simulation
+    d = _column_3d() if dim == 3 else small_column(2)
+    d["Configuration"]["neighbourSkin"] = skin
+    cfg = cfg_of(d)
+    sim = Simulation(cfg, precision="fp32_mixed")
+    orc = oracle_lib.OracleSim(cfg)
+    sim.solver.step(12)
+    orc.step(12)
+    gid = sim.ps.field("id0").cpu().numpy()
+    take = np.empty_like(gid)
+    take[gid] = np.arange(gid.size)
+    take = take[orc.get("id0").astype(np.int64)]
+    f = orc.get("mat_type") == 2
+    a = sim.ps.field("stress").cpu().numpy().astype(np.float64)[take][f].reshape(-1, 9)
+    b = orc.get("stress")[f].reshape(-1, 9)
+    assert np.max(np.abs(b)) > 0
+    assert np.max(np.abs(a - b)) / np.max(np.abs(b)) < 1e-4

@@ -1379,12 +1379,17 @@ __global__ void k_post_mui32(K32 k, P32 p, T32 t) {
 // PACKED (the step sequence, where no caller can have written stress_tmp since the momentum
 // pass): the neighbour's stress comes from that pass's record, one 128-bit read and zz in 2D, one
 // 256-bit read in 3D, instead of six 32-bit gathers; in 2D the out-of-plane shears it leaves out
-// are zero (0 times |xx| below: +0, or NaN after a blow-up, as their sums would be).  Four list entries
-// per trip, all their reads issued before the first is used.  320,000 particles in 2D: 62 -> 50 us.
-template <int DIM, bool PACKED>
+// are zero (0 times |xx| below: +0, or NaN after a blow-up, as their sums would be).  Two list entries
+// per trip, their reads issued before the first is used.  LISTS = false (no skin, so no lists at
+// the moved positions): the enumeration alone, at its own registers.  us a launch, one entry per
+// trip and no records / four entries / two: 2D, 320,000 soil particles 76 / 51 / 43, and 119 / 145
+// by enumeration (107 with LISTS = false); 3D, 119,000 particles 141 / 133 / 102 and 340 / 516 (339);
+// 20,000 particles in 2D 33 / 16 / 16.
+template <int DIM, bool PACKED, bool LISTS>
 __global__ void k_reg_mui32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, const int* __restrict__ dstart,
                             const int* __restrict__ sstart, const unsigned* __restrict__ maxd, float list_d2) {
-    const bool lists_ok = list_d2 > 0.f && __uint_as_float(*maxd) <= list_d2;
+    constexpr int U = 2;
+    const bool lists_ok = LISTS && __uint_as_float(*maxd) <= list_d2;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k.nd; i += gridDim.x * blockDim.x) {
         if (tf_type(p.hi[i].w) != MAT_SOIL) continue;
         const size_t n = k.n;
@@ -1393,7 +1398,6 @@ __global__ void k_reg_mui32(K32 k, P32 p, T32 t, const float4* __restrict__ PF, 
         if (lists_ok && m <= k.maxn) {
             const float4 lo_i = p.lo[i];
             const int* lp = t.nbr + i;
-            constexpr int U = 4;
             int e[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) e[u] = u < m ? __ldcs(lp + u * n) : 0;
@@ -2853,10 +2857,11 @@ static void advect_something(Fp32State& st, cudaStream_t s, bool packed, bool fi
             if (!final_done) TSG_LAUNCH(k_disp32, nblk(k.nd), TPB, s, k, p.hi, p.lo, st.pf, st.maxdisp);
             list_d2 = k.disp2_limit * 1.185f;
         }
-#define REG_MUI(D, PK) \
-    TSG_LAUNCH((k_reg_mui32<D, PK>), nblk(k.nd), TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, st.maxdisp, list_d2)
-        if (k.dim == 2) { if (packed) REG_MUI(2, true); else REG_MUI(2, false); }
-        else { if (packed) REG_MUI(3, true); else REG_MUI(3, false); }
+#define REG_MUI(D, PK, LISTS) \
+    TSG_LAUNCH((k_reg_mui32<D, PK, LISTS>), nblk(k.nd), TPB, s, k, p, st.T, st.pf, st.dstart, st.sstart, st.maxdisp, list_d2)
+        if (list_d2 <= 0.f) { if (k.dim == 2) REG_MUI(2, false, false); else REG_MUI(3, false, false); }
+        else if (k.dim == 2) { if (packed) REG_MUI(2, true, true); else REG_MUI(2, false, true); }
+        else { if (packed) REG_MUI(3, true, true); else REG_MUI(3, false, true); }
 #undef REG_MUI
     } else TSG_LAUNCH(k_post_dp32, nblk(k.nd), TPB, s, k, p, st.T);
 }
