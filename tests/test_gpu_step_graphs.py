@@ -238,3 +238,26 @@ def test_steps_while_another_thread_captures(native, precision):
     assert got == [3.0]
     for nm in ("x", "v", "density", "id0"):
         assert torch.equal(a.ps.field(nm), b.ps.field(nm)), nm
+
+
+@pytest.mark.parametrize("warm", [0, 7])
+@pytest.mark.parametrize("method", [1, 2])
+def test_fp64_steps_inside_a_callers_capture(native, method, warm):
+    """Two FP64 steps captured by the caller are the launches themselves, before and after the
+    handle has graphs of its own: three replays are six steps, bit for bit."""
+    from tisphi_gb300.simulation import Simulation
+    a, b = (Simulation(cfg_of(small_dambreak_2d() if method == 1 else small_column(2)), precision="fp64")
+            for _ in range(2))
+    for s in (a, b):
+        if warm:
+            s.solver.step(warm)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        a.solver.step(2)
+    for _ in range(3):
+        g.replay()
+    b.solver.step(6)
+    torch.cuda.synchronize()
+    for nm in FIELDS:
+        assert torch.equal(a.ps.field(nm), b.ps.field(nm)), nm
