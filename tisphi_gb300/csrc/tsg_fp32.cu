@@ -2654,17 +2654,17 @@ struct Passes {
     Ovf ovf;
     int grid, tpb;
 };
-// main_blocks of the main pass over n particles, then kOvfBlocks x TPB threads at most for the
-// overflow pass.  As the last blocks of a launch its blocks do not spread over the SMs as evenly as
-// a launch of their own did, and in some passes the traversal spills at the main pass's registers:
-// 64 blocks took up to 12 % longer than that launch, 96 take less (us a step with launches of their
-// own / 64 / 96 blocks: mu(I) in 3D with CSPM, 75,454 overflowed lists, 21,600 / 22,700 / 16,900;
-// Drucker-Prager likewise with XSPH 30,000 / 32,000 / 23,500; 2D dambreak with CSPM and XSPH,
-// 22,600 lists, 970 / 1,070 / 773); 152 cost a step without any 0.3 %, 96 nothing measurable.
-constexpr int kOvfBlocks = 96;
+// main_blocks of the main pass over n particles, then 64 x TPB threads at most for the overflow pass.
+// In scenes twice as dense as a lattice some passes of these blocks take up to 12 % longer than in
+// a launch of their own (they do not spread over the SMs as evenly and spill at the main pass's
+// registers: mu(I) in 3D with CSPM, 75,454 overflowed lists, 21,600 -> 22,700 us a step; 2D dambreak
+// with CSPM and XSPH, 22,600 lists, 970 -> 1,070; WCSPH in 3D 4,620 -> 4,400).  More blocks would mend
+// that (96: 16,900 and 773) but cost scenes without overflow more than the joined launch gives them:
+// 2D dambreaks of 108,000 and 204,000 fluid particles 85 -> 88 and 115 -> 117 us a step with 96.
+// The blocks first in the grid, or the overflow pass behind the main pass in its threads: the 3D
+// benchmark 3 % slower.
 Passes passes(const Fp32State& st, int main_blocks, int n) {
-    return {{st.ovf_list, st.novf, main_blocks},
-            main_blocks + nblk(std::min(std::max(n, 1), kOvfBlocks * TPB), st.tpb), st.tpb};
+    return {{st.ovf_list, st.novf, main_blocks}, main_blocks + nblk(std::min(std::max(n, 1), 64 * TPB), st.tpb), st.tpb};
 }
 
 template <int DIM>
